@@ -214,9 +214,9 @@ int lamino_plan_autotune(lamino_plan_t p, const lamino_geom_t *geoms, int ngeom,
     auto gs = geoms_of(geoms, ngeom);
     double ms = p->p->autotune_bins(gs, objective, S(stream));
     if (bins) {
-        bins[0] = p->p->bins.b1;
-        bins[1] = p->p->bins.b2;
-        bins[2] = p->p->bins.b3;
+        bins[0] = p->p->b1;
+        bins[1] = p->p->b2;
+        bins[2] = p->p->b3;
     }
     if (best_ms) *best_ms = ms;
     API_END

@@ -43,6 +43,7 @@ struct Geom {
     uint64_t uid = next_geom_uid();
     int64_t nproj = 0, nrows = 0, ncols = 0;
     float gamma = 0.f, sg = 0.f, cg = 0.f;
+    double offX = 0.0, offY = 0.0;  // mean of the column / row frequencies (float rounding)
     std::vector<float> theta;
     std::vector<float> h_coeff;  // [3][nproj]
     DevBuf<float> qX, qY, st, ct, coeff;
@@ -65,6 +66,8 @@ struct Geom {
             beam_dir_vector_f(g, theta[i], c);
             for (int q = 0; q < 3; ++q) h_coeff[q * np + i] = c[q];
         }
+        for (int64_t k = 0; k < nc; ++k) offX += (double)hx[k] / (double)nc;
+        for (int64_t j = 0; j < nr; ++j) offY += (double)hy[j] / (double)nr;
         sg = std::sin(g);
         cg = std::cos(g);
         qX.alloc(nc); qY.alloc(nr); st.alloc(np); ct.alloc(np); coeff.alloc(3 * np);

@@ -5,16 +5,48 @@
 // upsampfac 2, tol 1.2e-6 in float), src/projection.cpp:42-126 (forward /
 // adjoint) and src/gradient.cpp:34-89 (sysmat).
 //
-// Design: point coordinates are never stored; each kernel regenerates a point
-// from the per-column / per-row / per-projection factors (geometry.cuh).  Point
-// ids are bin-sorted once per geometry and plan (a counting sort keyed by the
-// fine-grid bin of the first cell of the point's kernel footprint, cached), and
-// spreading / interpolation run one CTA per bin with the bin's tile of the fine
-// grid in shared memory.  The fine grid is (nf1, nf2, nf3) complex64 with nf the
-// smallest even 2,3,5-smooth size >= 2n; the uniform FFTs on it use cuFFT.
-// Deconvolution, the pad into the fine grid and the crop out of it are fused
-// into the kernels on either side of cuFFT, and so are the fftshift2 /
-// ifftshift2 index maps and the per-projection beam-vector weighting.
+// Design.  The points of one geometry are a lattice, and the transform is
+// factorised over it.  With the detector axis a = (cos g, 0, -sin g) and
+// b(theta) = (cos th sin g, -sin th, cos th cos g) in (x, y, z), point
+// (p, j, k) is q = X_k a + Y_j b(theta_p); a is the same for every angle, and
+// b's part outside y lies along the fixed axis t = (sin g, 0, cos g).  So
+//     q = X_k a + T t + y e_y,   T = Y_j cos(th_p),   y = -Y_j sin(th_p):
+// one regular axis X shared by all detector rows of all angles, and a 2-D
+// scattered set of (T, y) positions, one per detector row.  Interpolation from
+// the fine grid (type 2) then takes two 2-D steps instead of one 3-D step of
+// w^3 taps per point:
+//   1. (z, x) -> (T, X): the values at the nodes of a regular (T, X) grid, for
+//      every fine-grid y (k_nodes_gather: w^2 taps per node, lanes along y);
+//   2. (T, y) -> detector rows: w^2 taps per row, the same taps for all columns
+//      (k_rows_gather: lanes along X).
+// The T axis is oversampled by 2 with respect to the volume's extent along t,
+// n3 |sin g| + n1 |cos g|, and deconvolved per mode (its frequency along t is
+// k3 sin g + k1 cos g, not an integer).  Type 1 is the transpose.  At the
+// padded README size (721 x 71 x 721, 361 x 1233^2 points) that is 49 taps for
+// 3.0e8 node values and 49 for 5.5e8 points, all of it contiguous along y or X,
+// in place of 343 taps per point from scattered tiles.
+// Measured on B200 against antipodal point pairs spread through 3-D tiles (the
+// form before): adjoint at that size 333.6 -> 38.2 ms, forward of 181 x 362^2
+// points from 362 x 44 x 362 19.5 -> 3.4 ms, sysmat of 2 x 91 x 309^2 points on
+// 180 x 16 x 180 20.3 -> 2.05 ms, and no sort of the points on the first call
+// (adjoint of a new geometry 346 -> 42 ms).
+//
+// The three components need one complex transform, not three.  The beam vector
+// (sin g sin th, cos th, cos g sin th) spans two dimensions:
+//   S = sin g m0 + cos g m2 and C = m1 are projected with weights sin th, cos th.
+// S and C are real, so W = S + i C has V_S(q) = (F(q) + conj F(-q)) / 2 and
+// V_C(q) = (F(q) - conj F(-q)) / 2i, F the transform of W.  With
+// a_p = (sin th - i cos th) / 2 the projection spectrum is
+//   P(q) = a_p F(q) + conj(a_p F(-q)),
+// and -q is the lattice point (p, nrows-1-j, ncols-1-k).  The second term is
+// folded into the 2-D transform over the detector as a real factor and a phase
+// (twist below), so only F(q) is evaluated.  The adjoint runs the same steps
+// transposed.  This needs a lattice that is symmetric under q -> -q to more than
+// float rounding.  The reference's float frequencies are not (their grid is off
+// centre by up to 3e-7, which alone would move a 721-wide result by 2e-5), so
+// these operators take the antisymmetric part of the float frequencies, with
+// products and sums in double; the raw transforms, whose data have no such
+// symmetry, keep the float positions.
 #include <array>
 #include <cmath>
 #include <map>
@@ -37,13 +69,15 @@ int64_t next_smooth_even(int64_t n) {
     }
 }
 
-// p(k) = (w/2) int_{-1}^{1} phi(t) cos(k pi w t / nf) dt by Gauss-Legendre
-// quadrature in double (nodes by Newton iteration on P_n).
-static std::vector<double> es_fourier(int64_t nf, int64_t N, int w, double beta) {
-    const int nq = 200;
-    std::vector<double> xs(nq), ws(nq);
-    for (int i = 0; i < nq; ++i) {
-        double x = std::cos(M_PI * (i + 0.75) / (nq + 0.5));
+// Gauss-Legendre nodes on (0, 1) of an even rule on [-1, 1] (Newton iteration on
+// P_n), with the weights times the ES kernel: the transform of the kernel at
+// frequency k of a grid of nf cells is p(k) = w sum_q wphi_q cos(k pi w x_q / nf).
+static constexpr int kQuad = 100;
+static std::vector<double2> es_quadrature(double beta) {
+    const int nq = 2 * kQuad;
+    std::vector<double2> out(kQuad);
+    for (int i = 0; i < kQuad; ++i) {
+        double x = std::cos(M_PI * (i + 0.75) / (nq + 0.5)), wt = 0.0;
         for (int it = 0; it < 100; ++it) {
             double p0 = 1.0, p1 = x;
             for (int k = 2; k <= nq; ++k) {
@@ -54,25 +88,12 @@ static std::vector<double> es_fourier(int64_t nf, int64_t N, int w, double beta)
             double dp = nq * (x * p1 - p0) / (x * x - 1.0);
             double dx = p1 / dp;
             x -= dx;
-            if (std::fabs(dx) < 1e-16) {
-                ws[i] = 2.0 / ((1.0 - x * x) * dp * dp);
-                break;
-            }
-            ws[i] = 2.0 / ((1.0 - x * x) * dp * dp);
+            wt = 2.0 / ((1.0 - x * x) * dp * dp);
+            if (std::fabs(dx) < 1e-16) break;
         }
-        xs[i] = x;
+        out[i] = make_double2(x, wt * std::exp(beta * (std::sqrt(1.0 - x * x) - 1.0)));
     }
-    std::vector<double> p(N);
-    for (int64_t i = 0; i < N; ++i) {
-        double k = (double)(i - N / 2);
-        double s = 0.0;
-        for (int q = 0; q < nq; ++q) {
-            double phi = std::exp(beta * (std::sqrt(1.0 - xs[q] * xs[q]) - 1.0));
-            s += ws[q] * phi * std::cos(k * M_PI * w * xs[q] / (double)nf);
-        }
-        p[i] = 0.5 * w * s;
-    }
-    return p;
+    return out;
 }
 
 NufftPlan::NufftPlan(Dims3 d, double eps_) : vol(d), eps(eps_) {
@@ -84,26 +105,33 @@ NufftPlan::NufftPlan(Dims3 d, double eps_) : vol(d), eps(eps_) {
     nf2 = next_smooth_even(std::max<int64_t>(2 * d.n2, 2 * w));
     nf3 = next_smooth_even(std::max<int64_t>(2 * d.n3, 2 * w));
     if (nf() > (int64_t)INT32_MAX) throw Error(ERR_ARG, "fine grid too large");
+    const std::vector<double2> q = es_quadrature(beta);
+    quad.alloc(kQuad);
+    upload(quad.p, q.data(), (size_t)kQuad);
     auto up = [&](DevBuf<float> &buf, int64_t nf_, int64_t N) {
-        auto p = es_fourier(nf_, N, w, beta);
         std::vector<float> ip(N);
-        for (int64_t i = 0; i < N; ++i) ip[i] = (float)(1.0 / p[i]);
+        for (int64_t i = 0; i < N; ++i) {
+            const double k = (double)(i - N / 2);
+            double p = 0.0;
+            for (int t = 0; t < kQuad; ++t) p += q[t].y * std::cos(k * M_PI * w * q[t].x / (double)nf_);
+            ip[i] = (float)(1.0 / (w * p));
+        }
         buf.alloc(N);
         upload(buf.p, ip.data(), (size_t)N);
     };
     up(ip1, nf1, d.n1);
     up(ip2, nf2, d.n2);
     up(ip3, nf3, d.n3);
-    gin.alloc(3 * nf());
-    gwork.alloc(3 * nf());
-    zero_bytes(gin.p, gin.bytes());
-    int n[3] = {(int)nf1, (int)nf2, (int)nf3};
+    grid.alloc(nf());
+    // node grids are 0.9 to 1.2 fine grids for the detectors and volumes that the
+    // MBIR drivers pad together
+    work.alloc(nf() + nf() / 4);
+    int n[3] = {(int)nf1, (int)nf3, (int)nf2};
     fft3.make(3, n, CUFFT_C2C, 1);
-    set_bins(4, 8, 16);
 }
 
 // ---------------------------------------------------------------------------
-// kernels
+// the ES kernel on the fine grid
 // ---------------------------------------------------------------------------
 
 struct Fine {
@@ -112,299 +140,770 @@ struct Fine {
     float beta;
 };
 
-// first tap of a coordinate on the fine grid (wrapped) and its offset d0 in
-// [-W/2, -W/2 + 1) from the coordinate, in grid units; lu: the first tap unwrapped
+// first tap of a coordinate xc on a grid of s cells per unit (not wrapped), and
+// its offset d0 in [-W/2, -W/2 + 1) from the coordinate, in grid units
 template <int W>
-__device__ __forceinline__ int es_start(float xc, int nf, double s, float &d0, double &lu) {
-    double u = (double)xc * s;
-    double l0 = ceil(u - 0.5 * W);
+__device__ __forceinline__ int es_first(double xc, double s, float &d0) {
+    const double u = xc * s;
+    const double l0 = ceil(u - 0.5 * W);
     d0 = (float)(l0 - u);
-    lu = l0;
-    int64_t l = (int64_t)l0;
+    return (int)l0;
+}
+__device__ __forceinline__ int wrap(int l, int nf) {
     l %= nf;
-    if (l < 0) l += nf;
-    return (int)l;
+    return l < 0 ? l + nf : l;
+}
+// kernel value at tap t of a footprint with offset d0; 0 outside the footprint
+template <int W>
+__device__ __forceinline__ float es_weight(float d0, int t, float beta) {
+    const float a = (d0 + (float)t) * (2.0f / W);
+    const float q = 1.0f - a * a;
+    return q > 0.f ? expf(beta * (sqrtf(q) - 1.0f)) : 0.f;
 }
 template <int W>
-__device__ __forceinline__ int es_start(float xc, int nf, double s, float &d0) {
-    double lu;
-    return es_start<W>(xc, nf, s, d0, lu);
-}
-// offset d0 of a coordinate from another point's first tap lu (unwrapped);
-// true if the coordinate's own first tap is within one cell of lu, so that its
-// w taps on lu's footprint miss at most one edge tap (kernel value ~exp(-beta))
-template <int W>
-__device__ __forceinline__ bool es_offset_from(float xc, double s, double lu, float &d0) {
-    double u = (double)xc * s;
-    d0 = (float)(lu - u);
-    return fabs(ceil(u - 0.5 * W) - lu) <= 1.0;
-}
-
-template <int W>
-__device__ __forceinline__ void es_weights(float d0, float beta, float *wt) {
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-        float a = (d0 + (float)t) * (2.0f / W);
-        float q = 1.0f - a * a;
-        wt[t] = q > 0.f ? expf(beta * (sqrtf(q) - 1.0f)) : 0.f;
-    }
-}
-
-template <int W>
-__device__ __forceinline__ int es_taps(float xc, int nf, double s, float beta, float *wt) {
-    float d0;
-    const int l = es_start<W>(xc, nf, s, d0);
-    es_weights<W>(d0, beta, wt);
-    return l;
-}
-
-// deconvolve + place modes into the (zero) fine grid; real volume input
-__global__ void k_pad_real(const float *__restrict__ x, int n1, int n2, int n3,
-                           float2 *__restrict__ g, Fine F, const float *__restrict__ ip1,
-                           const float *__restrict__ ip2, const float *__restrict__ ip3) {
-    const int comp = blockIdx.y;
-    const int64_t V = (int64_t)n1 * n2 * n3;
-    const int64_t NF = (int64_t)F.nf1 * F.nf2 * F.nf3;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < V;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i3 = (int)(idx % n3);
-        int64_t r = idx / n3;
-        int i2 = (int)(r % n2);
-        int i1 = (int)(r / n2);
-        int l1 = i1 - n1 / 2; if (l1 < 0) l1 += F.nf1;
-        int l2 = i2 - n2 / 2; if (l2 < 0) l2 += F.nf2;
-        int l3 = i3 - n3 / 2; if (l3 < 0) l3 += F.nf3;
-        float v = x[comp * V + idx] * (__ldg(ip1 + i1) * __ldg(ip2 + i2) * __ldg(ip3 + i3));
-        g[comp * NF + ((int64_t)l1 * F.nf2 + l2) * F.nf3 + l3] = make_float2(v, 0.f);
-    }
-}
-
-__global__ void k_pad_complex(const float2 *__restrict__ f, int n1, int n2, int n3,
-                              float2 *__restrict__ g, Fine F, const float *__restrict__ ip1,
-                              const float *__restrict__ ip2, const float *__restrict__ ip3) {
-    const int64_t V = (int64_t)n1 * n2 * n3;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < V;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i3 = (int)(idx % n3);
-        int64_t r = idx / n3;
-        int i2 = (int)(r % n2);
-        int i1 = (int)(r / n2);
-        int l1 = i1 - n1 / 2; if (l1 < 0) l1 += F.nf1;
-        int l2 = i2 - n2 / 2; if (l2 < 0) l2 += F.nf2;
-        int l3 = i3 - n3 / 2; if (l3 < 0) l3 += F.nf3;
-        float c = __ldg(ip1 + i1) * __ldg(ip2 + i2) * __ldg(ip3 + i3);
-        float2 v = f[idx];
-        g[((int64_t)l1 * F.nf2 + l2) * F.nf3 + l3] = make_float2(v.x * c, v.y * c);
-    }
-}
-
-// fine grid -> modes: y = (acc ? y : 0) + Re(G[k mod nf]) / p(k) * scale
-__global__ void k_extract_real(const float2 *__restrict__ g, int n1, int n2, int n3,
-                               float *__restrict__ y, Fine F, const float *__restrict__ ip1,
-                               const float *__restrict__ ip2, const float *__restrict__ ip3,
-                               float scale, int accumulate) {
-    const int comp = blockIdx.y;
-    const int64_t V = (int64_t)n1 * n2 * n3;
-    const int64_t NF = (int64_t)F.nf1 * F.nf2 * F.nf3;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < V;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i3 = (int)(idx % n3);
-        int64_t r = idx / n3;
-        int i2 = (int)(r % n2);
-        int i1 = (int)(r / n2);
-        int l1 = i1 - n1 / 2; if (l1 < 0) l1 += F.nf1;
-        int l2 = i2 - n2 / 2; if (l2 < 0) l2 += F.nf2;
-        int l3 = i3 - n3 / 2; if (l3 < 0) l3 += F.nf3;
-        float c = __ldg(ip1 + i1) * __ldg(ip2 + i2) * __ldg(ip3 + i3) * scale;
-        float v = g[comp * NF + ((int64_t)l1 * F.nf2 + l2) * F.nf3 + l3].x * c;
-        if (accumulate) v += y[comp * V + idx];
-        y[comp * V + idx] = v;
-    }
-}
-
-__global__ void k_extract_complex(const float2 *__restrict__ g, int n1, int n2, int n3,
-                                  float2 *__restrict__ f, Fine F, const float *__restrict__ ip1,
-                                  const float *__restrict__ ip2, const float *__restrict__ ip3) {
-    const int64_t V = (int64_t)n1 * n2 * n3;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < V;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i3 = (int)(idx % n3);
-        int64_t r = idx / n3;
-        int i2 = (int)(r % n2);
-        int i1 = (int)(r / n2);
-        int l1 = i1 - n1 / 2; if (l1 < 0) l1 += F.nf1;
-        int l2 = i2 - n2 / 2; if (l2 < 0) l2 += F.nf2;
-        int l3 = i3 - n3 / 2; if (l3 < 0) l3 += F.nf3;
-        float c = __ldg(ip1 + i1) * __ldg(ip2 + i2) * __ldg(ip3 + i3);
-        float2 v = g[((int64_t)l1 * F.nf2 + l2) * F.nf3 + l3];
-        f[idx] = make_float2(v.x * c, v.y * c);
-    }
-}
-
-// interpolate NC fine grids at one point
-template <int W, int NC>
-__device__ __forceinline__ void interp_point(const float2 *__restrict__ G, int64_t NF, const Fine &F,
-                                             float x, float y, float z, float2 *out) {
-    float w1[W], w2[W], w3[W];
-    int b3 = es_taps<W>(x, F.nf3, F.s3, F.beta, w3);
-    int b2 = es_taps<W>(y, F.nf2, F.s2, F.beta, w2);
-    int b1 = es_taps<W>(z, F.nf1, F.s1, F.beta, w1);
-    int i3s[W];
-#pragma unroll
-    for (int t = 0; t < W; ++t) { int v = b3 + t; i3s[t] = v >= F.nf3 ? v - F.nf3 : v; }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) out[c] = make_float2(0.f, 0.f);
-#pragma unroll 1
-    for (int t1 = 0; t1 < W; ++t1) {
-        int i1 = b1 + t1; if (i1 >= F.nf1) i1 -= F.nf1;
-#pragma unroll
-        for (int t2 = 0; t2 < W; ++t2) {
-            int i2 = b2 + t2; if (i2 >= F.nf2) i2 -= F.nf2;
-            const int64_t rowo = ((int64_t)i1 * F.nf2 + i2) * F.nf3;
-            float k12 = w1[t1] * w2[t2];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const float2 *row = G + c * NF + rowo;
-                float rr = 0.f, ri = 0.f;
-#pragma unroll
-                for (int t3 = 0; t3 < W; ++t3) {
-                    float2 v = __ldg(row + i3s[t3]);
-                    rr = fmaf(w3[t3], v.x, rr);
-                    ri = fmaf(w3[t3], v.y, ri);
-                }
-                out[c].x = fmaf(k12, rr, out[c].x);
-                out[c].y = fmaf(k12, ri, out[c].y);
-            }
-        }
-    }
-}
-
-// spread NC strengths at one point into NC fine grids (float2 vector atomics)
-template <int W, int NC>
-__device__ __forceinline__ void spread_point(float2 *__restrict__ H, int64_t NF, const Fine &F,
-                                             float x, float y, float z, const float2 *str) {
-    float w1[W], w2[W], w3[W];
-    int b3 = es_taps<W>(x, F.nf3, F.s3, F.beta, w3);
-    int b2 = es_taps<W>(y, F.nf2, F.s2, F.beta, w2);
-    int b1 = es_taps<W>(z, F.nf1, F.s1, F.beta, w1);
-    int i3s[W];
-#pragma unroll
-    for (int t = 0; t < W; ++t) { int v = b3 + t; i3s[t] = v >= F.nf3 ? v - F.nf3 : v; }
-#pragma unroll 1
-    for (int t1 = 0; t1 < W; ++t1) {
-        int i1 = b1 + t1; if (i1 >= F.nf1) i1 -= F.nf1;
-#pragma unroll
-        for (int t2 = 0; t2 < W; ++t2) {
-            int i2 = b2 + t2; if (i2 >= F.nf2) i2 -= F.nf2;
-            const int64_t rowo = ((int64_t)i1 * F.nf2 + i2) * F.nf3;
-            float k12 = w1[t1] * w2[t2];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                float2 *row = H + c * NF + rowo;
-                float sr = k12 * str[c].x, si = k12 * str[c].y;
-#pragma unroll
-                for (int t3 = 0; t3 < W; ++t3)
-                    atomicAdd(row + i3s[t3], make_float2(w3[t3] * sr, w3[t3] * si));
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void decode_pid(uint32_t pid, const GeomView &g, int &p, int &j, int &k) {
-    uint32_t plane = (uint32_t)g.nrows * (uint32_t)g.ncols;
-    p = (int)(pid / plane);
-    uint32_t r = pid - (uint32_t)p * plane;
-    j = (int)(r / (uint32_t)g.ncols);
-    k = (int)(r - (uint32_t)j * (uint32_t)g.ncols);
-}
-
-// Antipodal pairs (the adjoint).  The detector frequencies are symmetric about
-// zero (qX[k] = -qX[nc-1-k] and qY[j] = -qY[nr-1-j] up to float rounding), so
-// the points at in-plane flat index i and N-1-i of a projection (N = nrows
-// ncols) are antipodal: x_{N-1-i} = -x_i + d, |d| at the rounding level.  The
-// adjoint keeps only the real part of the type-1 sum, and on the periodic fine
-// grid (m -> -m, phi even) the term of a point i' with strength f equals, in
-// real part, the term of strength conj(f) at -x_{i'}.  That position lies next
-// to x_i, so one staged record carries both points and spreads them through
-// x_i's footprint: half the tile read-modify-writes per point.  Pair q of a
-// projection is (q, N-1-q), q in [0, (N+1)/2); for odd N the middle point is
-// its own partner and the pair's second strength is zero.
-__device__ __forceinline__ uint32_t pairs_per_proj(const GeomView &g) {
-    return ((uint32_t)g.nrows * (uint32_t)g.ncols + 1u) / 2u;
-}
-__device__ __forceinline__ void decode_pair(uint32_t pid, const GeomView &g, int &p, int &j, int &k, int &j2,
-                                            int &k2) {
-    const uint32_t H = pairs_per_proj(g);
-    p = (int)(pid / H);
-    const uint32_t q = pid - (uint32_t)p * H;
-    j = (int)(q / (uint32_t)g.ncols);
-    k = (int)(q - (uint32_t)j * (uint32_t)g.ncols);
-    j2 = g.nrows - 1 - j;
-    k2 = g.ncols - 1 - k;
+__device__ __forceinline__ float es_tap(float d0, int t, float beta) {
+    return (unsigned)t < (unsigned)W ? es_weight<W>(d0, t, beta) : 0.f;
 }
 
 // ---------------------------------------------------------------------------
-// bin sort: point (or pair) ids grouped by the fine-grid bin of their
-// footprint's first cell (a pair's: its first point's)
+// volume <-> fine grid
+// ---------------------------------------------------------------------------
 
-// first cell of the kernel footprint along one dimension, in [0, nf) (as es_taps)
+// CTA -> (i1, first i2, first i3) of its 32 x 32 tile
+__device__ __forceinline__ void volume_tile(int n2, int n3, int &i1, int &b2, int &b3) {
+    const unsigned t3 = (n3 + 31) / 32, t2 = (n2 + 31) / 32, r = blockIdx.x / t3;
+    b3 = (int)(blockIdx.x - r * t3) * 32;
+    i1 = (int)(r / t2);
+    b2 = (int)(r - i1 * t2) * 32;
+}
+// Volumes have n3 fastest, the fine grid n2: both sides transpose 32 x 32 tiles
+// of (i3, i2) through shared memory so that reads and writes are contiguous.
+// W = S + i C (real volume, gamma's sines) or the complex modes, deconvolved.
+template <bool CPLX>
+__global__ void __launch_bounds__(256) k_pad(const float *__restrict__ x, const float2 *__restrict__ modes, int n1,
+                                             int n2, int n3, float sg, float cg, float2 *__restrict__ g, Fine F,
+                                             const float *__restrict__ ip1, const float *__restrict__ ip2,
+                                             const float *__restrict__ ip3, const float *__restrict__ ipT) {
+    __shared__ float2 tile[32][33];
+    int i1, b2, b3;
+    volume_tile(n2, n3, i1, b2, b3);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t V = (int64_t)n1 * n2 * n3;
+    int l1 = i1 - n1 / 2; if (l1 < 0) l1 += F.nf1;
+    const float c1 = __ldg(ip1 + i1);
+    const int i3 = b3 + tx;
+    if (i3 < n3) {
+        float c = c1 * __ldg(ip3 + i3);
+        if (ipT) c *= __ldg(ipT + (int64_t)i1 * n3 + i3);
+        for (int r = ty; r < 32 && b2 + r < n2; r += 8) {
+            const int64_t idx = ((int64_t)i1 * n2 + b2 + r) * n3 + i3;
+            const float d = c * __ldg(ip2 + b2 + r);
+            if (CPLX) {
+                const float2 v = modes[idx];
+                tile[r][tx] = make_float2(v.x * d, v.y * d);
+            } else {
+                tile[r][tx] = make_float2((sg * x[idx] + cg * x[2 * V + idx]) * d, x[V + idx] * d);
+            }
+        }
+    }
+    __syncthreads();
+    const int i2 = b2 + tx;
+    if (i2 >= n2) return;
+    int l2 = i2 - n2 / 2; if (l2 < 0) l2 += F.nf2;
+    for (int r = ty; r < 32 && b3 + r < n3; r += 8) {
+        int l3 = b3 + r - n3 / 2; if (l3 < 0) l3 += F.nf3;
+        g[((int64_t)l1 * F.nf3 + l3) * F.nf2 + l2] = tile[tx][r];
+    }
+}
+
+// fine grid -> modes: y_i (+)= the beam components of U = S + i C, or the complex modes
+template <bool CPLX>
+__global__ void __launch_bounds__(256) k_extract(const float2 *__restrict__ g, int n1, int n2, int n3, float sg,
+                                                 float cg, float *__restrict__ y, float2 *__restrict__ modes, Fine F,
+                                                 const float *__restrict__ ip1, const float *__restrict__ ip2,
+                                                 const float *__restrict__ ip3, const float *__restrict__ ipT,
+                                                 float scale, int accumulate) {
+    __shared__ float2 tile[32][33];
+    int i1, b2, b3;
+    volume_tile(n2, n3, i1, b2, b3);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t V = (int64_t)n1 * n2 * n3;
+    int l1 = i1 - n1 / 2; if (l1 < 0) l1 += F.nf1;
+    const int i2 = b2 + tx;
+    if (i2 < n2) {
+        int l2 = i2 - n2 / 2; if (l2 < 0) l2 += F.nf2;
+        for (int r = ty; r < 32 && b3 + r < n3; r += 8) {
+            int l3 = b3 + r - n3 / 2; if (l3 < 0) l3 += F.nf3;
+            tile[tx][r] = g[((int64_t)l1 * F.nf3 + l3) * F.nf2 + l2];
+        }
+    }
+    __syncthreads();
+    const int i3 = b3 + tx;
+    if (i3 >= n3) return;
+    float c = __ldg(ip1 + i1) * __ldg(ip3 + i3) * scale;
+    if (ipT) c *= __ldg(ipT + (int64_t)i1 * n3 + i3);
+    for (int r = ty; r < 32 && b2 + r < n2; r += 8) {
+        const int64_t idx = ((int64_t)i1 * n2 + b2 + r) * n3 + i3;
+        const float d = c * __ldg(ip2 + b2 + r);
+        const float2 v = tile[r][tx];
+        const float re = v.x * d, im = v.y * d;
+        if (CPLX) {
+            modes[idx] = make_float2(re, im);
+        } else if (accumulate) {
+            y[idx] += sg * re;
+            y[V + idx] += im;
+            y[2 * V + idx] += cg * re;
+        } else {
+            y[idx] = sg * re;
+            y[V + idx] = im;
+            y[2 * V + idx] = cg * re;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// building a lattice
+// ---------------------------------------------------------------------------
+
+// column frequencies, beam factors and the twist factors: for detector-space
+// index m of a dimension of n, d = n / 2,
+//   (cos, sin)(pi m (2 d + 1) / n + off u) and (cos, sin)(pi m / n),
+// u the centred index of m and off the mean of the dimension's float
+// frequencies: a spectrum sampled off centre is an image times e^{-i off u}, of
+// which the operators take the real part
+__device__ __forceinline__ double odd_part(const float *q, int i, int n) {
+    return 0.5 * ((double)__ldg(q + i) - (double)__ldg(q + n - 1 - i));
+}
+__global__ void k_lat_tables(GeomView g, bool raw, double offX, double offY, double *__restrict__ X, float2 *__restrict__ a,
+                             float4 *__restrict__ trow, float4 *__restrict__ tcol) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < g.ncols) X[i] = raw ? (double)g.qX[i] : odd_part(g.qX, i, g.ncols);
+    if (i < g.nproj) a[i] = make_float2(0.5f * g.st[i], -0.5f * g.ct[i]);
+    for (int d = 0; d < 2; ++d) {
+        const int n = d ? g.ncols : g.nrows;
+        if (i >= n) continue;
+        double s0, c0, s1, c1;
+        const long long r = ((long long)i * (2 * (n / 2) + 1)) % (2LL * n);
+        const int u = i < (n + 1) / 2 ? i : i - n;
+        sincos(r * (M_PI / n) + u * (d ? offX : offY), &s0, &c0);
+        sincospi((double)i / n, &s1, &c1);
+        (d ? tcol : trow)[i] = make_float4((float)c0, (float)s0, (float)c1, (float)s1);
+    }
+}
+
+// 1 / p_T at every mode's frequency along t, from the plan's quadrature
+__global__ void k_lat_deconv(const double2 *__restrict__ quad, int n1, int n3, double sg, double cg, int w, int nTf,
+                             float *__restrict__ ipT) {
+    __shared__ double2 q[kQuad];
+    for (int i = threadIdx.x; i < kQuad; i += blockDim.x) q[i] = quad[i];
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n1 * n3) return;
+    const int i1 = i / n3, i3 = i - i1 * n3;
+    const double k = (i3 - n3 / 2) * sg + (i1 - n1 / 2) * cg;
+    double p = 0.0;
+    for (int t = 0; t < kQuad; ++t) p += q[t].y * cospi(k * w * q[t].x / nTf);
+    ipT[i] = (float)(1.0 / (w * p));
+}
+
+// the (T, y) position of detector row `id` = p nrows + j and its footprint
+struct RowPos {
+    int p, j, lT, ly;
+    float dT, dy;
+};
 template <int W>
-__device__ __forceinline__ int es_start(float xc, int nf, double s) {
-    double u = (double)xc * s;
-    int64_t l = (int64_t)ceil(u - 0.5 * W);
-    l %= nf;
-    if (l < 0) l += nf;
-    return (int)l;
-}
-
-template <int W, bool PAIRED>
-__device__ __forceinline__ uint32_t point_bin(const GeomView &g, const Fine &F, const BinLayout &B, uint32_t pid) {
-    int p, j, k;
-    if (PAIRED) {
-        int j2, k2;
-        decode_pair(pid, g, p, j, k, j2, k2);
+__device__ __forceinline__ RowPos row_pos(const GeomView &g, bool raw, double invh, int T0,
+                                          const Fine &F, int id) {
+    RowPos r;
+    r.p = id / g.nrows;
+    r.j = id - r.p * g.nrows;
+    double T, y;
+    if (raw) {
+        const float qy = __ldg(g.qY + r.j);
+        T = (double)__fmul_rn(qy, __ldg(g.ct + r.p));
+        y = (double)__fmul_rn(-qy, __ldg(g.st + r.p));
     } else {
-        decode_pid(pid, g, p, j, k);
+        const double qy = odd_part(g.qY, r.j, g.nrows);
+        T = qy * (double)__ldg(g.ct + r.p);
+        y = -qy * (double)__ldg(g.st + r.p);
     }
-    float x, y, z;
-    point_xyz(g, p, j, k, x, y, z);
-    const int l1 = es_start<W>(z, F.nf1, F.s1), l2 = es_start<W>(y, F.nf2, F.s2), l3 = es_start<W>(x, F.nf3, F.s3);
-    return ((uint32_t)(l1 / B.b1) * (uint32_t)B.nb2 + (uint32_t)(l2 / B.b2)) * (uint32_t)B.nb3 +
-           (uint32_t)(l3 / B.b3);
+    r.lT = es_first<W>(T, invh, r.dT) - T0;
+    r.ly = wrap(es_first<W>(y, F.s2, r.dy), F.nf2);
+    return r;
+}
+template <int W>
+__global__ void __launch_bounds__(256) k_rows_count(GeomView g, bool raw, double invh,
+                                                    int T0, int nstart, Fine F, uint32_t *__restrict__ cnt) {
+    const int n = g.nproj * g.nrows;
+    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
+        const RowPos r = row_pos<W>(g, raw, invh, T0, F, id);
+        atomicAdd(cnt + (int64_t)r.ly * nstart + r.lT, 1u);
+    }
+}
+template <int W>
+__global__ void __launch_bounds__(256) k_rows_place(GeomView g, bool raw, double invh,
+                                                    int T0, int nstart, Fine F, uint32_t *__restrict__ cursor,
+                                                    int4 *__restrict__ pt, float2 *__restrict__ pd) {
+    const int n = g.nproj * g.nrows;
+    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
+        const RowPos r = row_pos<W>(g, raw, invh, T0, F, id);
+        const uint32_t at = atomicAdd(cursor + (int64_t)r.ly * nstart + r.lT, 1u);
+        pt[at] = make_int4(id, r.lT, r.ly, r.p);
+        pd[at] = make_float2(r.dT, r.dy);
+    }
 }
 
-// Consecutive point ids walk a projection row, so the lanes of a warp mostly
-// share a bin: one atomic per distinct bin in the warp.
-template <bool PAIRED>
-__device__ __forceinline__ uint32_t sort_ids(const GeomView &g) {
-    return (uint32_t)g.nproj * (PAIRED ? pairs_per_proj(g) : (uint32_t)g.nrows * (uint32_t)g.ncols);
+
+// ---------------------------------------------------------------------------
+// (z, x) <-> (T, X)
+// ---------------------------------------------------------------------------
+
+struct LatView {
+    const double *X;
+    double cg, sg, h;
+    int nc, nT, T0;
+};
+// footprint of node (line t, column k) in the (z, x) plane
+template <int W>
+__device__ __forceinline__ void node_pos(const LatView &L, const Fine &F, int t, int k, int &l1, int &l3, float &d1,
+                                         float &d3) {
+    const double X = L.X[k], T = (L.T0 + t) * L.h;
+    l3 = es_first<W>(X * L.cg + T * L.sg, F.s3, d3);
+    l1 = es_first<W>(T * L.cg - X * L.sg, F.s1, d1);
 }
 
-template <int W, bool PAIRED>
-__global__ void __launch_bounds__(256) k_bin_count(GeomView g, Fine F, BinLayout B, uint32_t *__restrict__ cnt) {
-    const uint32_t M = sort_ids<PAIRED>(g);
-    const int lane = threadIdx.x & 31;
+// Fine grid -> nodes.  A CTA owns 16 columns x 8 T lines; the threads of a
+// y chunk take (node, y) pairs with y fastest, so a tap is one contiguous read
+// of up to 16 y values (128 B) and neighbouring nodes find each other's taps in
+// L1.  Results go through shared memory to the node grid [T][y][X], X fastest.
+constexpr int kNodeK = 16, kNodeT = 8, kNodes = kNodeK * kNodeT, kNodeY = 16;
+template <int W>
+__global__ void __launch_bounds__(256) k_nodes_gather(LatView L, Fine F, const float2 *__restrict__ g, float2 *__restrict__ G,
+                                                      int pitch, int ktiles, int ychunk, uint32_t ydiv,
+                                                      int nchunk) {
+    __shared__ float w1[W][kNodes], w3[W][kNodes];
+    __shared__ int o1[W][kNodes], o3[W][kNodes];
+    __shared__ float2 st[kNodeY][kNodes + 1];
+    const int t0 = blockIdx.x / ktiles, k0 = (blockIdx.x - t0 * ktiles) * kNodeK;
+    const int tid = threadIdx.x;
+    {
+        // threads 0..127 the z side of a node, 128..255 the x side
+        const int n = tid & (kNodes - 1);
+        const int k = min(k0 + (n & (kNodeK - 1)), L.nc - 1), t = min(t0 * kNodeT + n / kNodeK, L.nT - 1);
+        int l1, l3;
+        float d1, d3;
+        node_pos<W>(L, F, t, k, l1, l3, d1, d3);
+        if (tid < kNodes) {
+            l1 = wrap(l1, F.nf1);
+#pragma unroll
+            for (int r = 0; r < W; ++r) {
+                int i = l1 + r; if (i >= F.nf1) i -= F.nf1;
+                o1[r][n] = i * F.nf3 * F.nf2;
+                w1[r][n] = es_weight<W>(d1, r, F.beta);
+            }
+        } else {
+            l3 = wrap(l3, F.nf3);
+#pragma unroll
+            for (int r = 0; r < W; ++r) {
+                int i = l3 + r; if (i >= F.nf3) i -= F.nf3;
+                o3[r][n] = i * F.nf2;
+                w3[r][n] = es_weight<W>(d3, r, F.beta);
+            }
+        }
+    }
+    for (int c = blockIdx.y; c < nchunk; c += gridDim.y) {
+        const int y0 = c * ychunk, ny = min(ychunk, F.nf2 - y0);
+        __syncthreads();
+        for (int e = tid; e < kNodes * ychunk; e += 256) {
+            const int n = (int)__umulhi((uint32_t)e, ydiv), y = e - n * ychunk;
+            if (y >= ny) continue;
+            const float2 *p = g + y0 + y;
+            float v3[W];
+            int q3[W];
+#pragma unroll
+            for (int r = 0; r < W; ++r) {
+                v3[r] = w3[r][n];
+                q3[r] = o3[r][n];
+            }
+            float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int r1 = 0; r1 < W; ++r1) {
+                const float2 *row = p + o1[r1][n];
+                const float u = w1[r1][n];
+                float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int r3 = 0; r3 < W; ++r3) s = __ffma2_rn(make_float2(v3[r3], v3[r3]), __ldg(row + q3[r3]), s);
+                acc = __ffma2_rn(make_float2(u, u), s, acc);
+            }
+            st[y][n] = acc;
+        }
+        __syncthreads();
+        for (int e = tid; e < kNodes * ny; e += 256) {
+            const int n = e & (kNodes - 1), y = e / kNodes;
+            const int k = k0 + (n & (kNodeK - 1)), t = t0 * kNodeT + n / kNodeK;
+            if (k < L.nc && t < L.nT) G[((int64_t)t * F.nf2 + y0 + y) * pitch + k] = st[y][n];
+        }
+    }
+}
+
+// Nodes -> fine grid (the transpose).  A CTA owns 4 x 4 (z, x) cells for all y,
+// a thread one y: it walks the nodes whose footprint meets the cells and adds
+// each into its 16 complex sums, held in registers, so no cell is written
+// twice and the order of the sum is fixed.  The nodes are found from the
+// lattice: the cells' box of footprint starts, turned into (X, T), bounds a
+// range of columns and lines; candidates are tested in parallel and the
+// accepted ones listed, with their 16 weights, in shared memory.  The box is
+// tried at every period of the fine grid that the lattice reaches.
+constexpr int kCell = 4;
+template <int W>
+__global__ void __launch_bounds__(256) k_nodes_spread(LatView L, Fine F, int reach1, int reach3, int xtiles,
+                                                      const float2 *__restrict__ Gt, float2 *__restrict__ g) {
+    extern __shared__ __align__(16) unsigned char nsm[];
+    const int cap = 2 * blockDim.x;
+    float4 *lw = reinterpret_cast<float4 *>(nsm);  // [cap][kCell]
+    int *ln = reinterpret_cast<int *>(lw + cap * kCell);
+    __shared__ int wsum[9];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int zt = blockIdx.x / xtiles, c1 = zt * kCell, c3 = (blockIdx.x - zt * xtiles) * kCell;
+    const int y = blockIdx.y * blockDim.x + tid;
+    const float2 *src = Gt + min(y, F.nf2 - 1);
+    float2 re[kCell][2], im[kCell][2];
+#pragma unroll
+    for (int i = 0; i < kCell; ++i) re[i][0] = re[i][1] = im[i][0] = im[i][1] = make_float2(0.f, 0.f);
+    int n = 0;  // listed nodes (the same in every thread)
+    auto flush = [&]() {
+        __syncthreads();
+#pragma unroll 4
+        for (int q = 0; q < n; ++q) {
+            const float2 v = __ldg(src + (int64_t)ln[q] * F.nf2);
+            const float2 vr = make_float2(v.x, v.x), vi = make_float2(v.y, v.y);
+#pragma unroll
+            for (int i = 0; i < kCell; ++i) {
+                const float4 t = lw[q * kCell + i];
+                re[i][0] = __ffma2_rn(make_float2(t.x, t.y), vr, re[i][0]);
+                re[i][1] = __ffma2_rn(make_float2(t.z, t.w), vr, re[i][1]);
+                im[i][0] = __ffma2_rn(make_float2(t.x, t.y), vi, im[i][0]);
+                im[i][1] = __ffma2_rn(make_float2(t.z, t.w), vi, im[i][1]);
+            }
+        }
+        __syncthreads();
+        n = 0;
+    };
+    const double dX = 2 * M_PI / L.nc;
+    // copies of the cells, one period apart, that the lattice reaches: the
+    // footprints lie in [-reach, reach] along each axis
+    const int m1 = (reach1 + c1 + kCell) / F.nf1, m3 = (reach3 + c3 + kCell) / F.nf3;
+    for (int b1 = c1 - m1 * F.nf1; b1 <= reach1; b1 += F.nf1)
+        for (int b3 = c3 - m3 * F.nf3; b3 <= reach3; b3 += F.nf3) {
+            // positions whose footprint starts in [b - W + 1, b + kCell - 1]
+            const double zlo = (b1 - W + 0.5 * W) / F.s1, zhi = (b1 + kCell - 1 + 0.5 * W) / F.s1;
+            const double xlo = (b3 - W + 0.5 * W) / F.s3, xhi = (b3 + kCell - 1 + 0.5 * W) / F.s3;
+            const double xm = 0.5 * (xlo + xhi), zm = 0.5 * (zlo + zhi), xr = 0.5 * (xhi - xlo), zr = 0.5 * (zhi - zlo);
+            const double Xm = xm * L.cg - zm * L.sg, Xr = xr * fabs(L.cg) + zr * fabs(L.sg);
+            const double Tm = xm * L.sg + zm * L.cg, Tr = xr * fabs(L.sg) + zr * fabs(L.cg);
+            // one column / line of margin for the rounding of the positions
+            const int ka = max(0, (int)floor((Xm - Xr + M_PI) / dX - 0.5) - 1);
+            const int kb = min(L.nc - 1, (int)ceil((Xm + Xr + M_PI) / dX - 0.5) + 1);
+            const int ta = max(0, (int)floor((Tm - Tr) / L.h) - L.T0 - 1);
+            const int tb = min(L.nT - 1, (int)ceil((Tm + Tr) / L.h) - L.T0 + 1);
+            if (ka > kb || ta > tb) continue;
+            const int nk = kb - ka + 1, cnt = nk * (tb - ta + 1);
+            for (int base = 0; base < cnt; base += blockDim.x) {
+                const int id = base + tid;
+                bool ok = false;
+                int e1 = 0, e3 = 0, node = 0;
+                float d1 = 0.f, d3 = 0.f;
+                if (id < cnt) {
+                    const int t = ta + id / nk, k = ka + id % nk;
+                    node_pos<W>(L, F, t, k, e1, e3, d1, d3);
+                    e1 = b1 - e1;  // tap of the box's first cell
+                    e3 = b3 - e3;
+                    ok = e1 > -kCell && e1 < W && e3 > -kCell && e3 < W;
+                    node = t * L.nc + k;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, ok);
+                if (lane == 0) wsum[warp] = __popc(m);
+                __syncthreads();
+                int at = n + __popc(m & ((1u << lane) - 1u)), tot = 0;
+                for (int v = 0; v < nwarps; ++v) {
+                    if (v == warp) at += tot;
+                    tot += wsum[v];
+                }
+                if (ok) {
+                    float u[kCell];
+#pragma unroll
+                    for (int i = 0; i < kCell; ++i) u[i] = es_tap<W>(d3, e3 + i, F.beta);
+#pragma unroll
+                    for (int i = 0; i < kCell; ++i) {
+                        const float s = es_tap<W>(d1, e1 + i, F.beta);
+                        lw[at * kCell + i] = make_float4(s * u[0], s * u[1], s * u[2], s * u[3]);
+                    }
+                    ln[at] = node;
+                }
+                n += tot;
+                __syncthreads();
+                if (n > cap - (int)blockDim.x) flush();
+            }
+        }
+    flush();
+    if (y >= F.nf2) return;
+#pragma unroll
+    for (int i = 0; i < kCell; ++i) {
+        if (c1 + i >= F.nf1) break;
+        float2 *o = g + ((int64_t)(c1 + i) * F.nf3 + c3) * F.nf2 + y;
+#pragma unroll
+        for (int r = 0; r < kCell; ++r) {
+            if (c3 + r >= F.nf3) break;
+            const float2 a = re[i][r / 2], b = im[i][r / 2];
+            o[r * F.nf2] = r & 1 ? make_float2(a.y, b.y) : make_float2(a.x, b.x);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// (T, y) <-> detector rows
+// ---------------------------------------------------------------------------
+
+// Nodes -> rows.  A CTA takes 32 rows, consecutive in cell order, and 64
+// columns; a warp one row at a time, two columns per lane, w^2 16-byte loads
+// of contiguous columns.  Rows of neighbouring cells share most of their taps,
+// which stay in L1.
+constexpr int kRowGroup = 32;
+template <int W>
+__global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nrow,
+                                                     const float2 *__restrict__ G, int nf2, int pitch, int nc, int groups,
+                                                     float beta, float2 *__restrict__ out) {
+    __shared__ float wT[kRowGroup][W], wy[kRowGroup][W];
+    __shared__ int4 info[kRowGroup];
+    const int kb = blockIdx.x / groups, base = (blockIdx.x - kb * groups) * kRowGroup, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 2 * kRowGroup) {
+        const int r = threadIdx.x & (kRowGroup - 1), q = base + r;
+        if (q < nrow) {
+            const float2 d = pd[q];
+            if (threadIdx.x < kRowGroup) {
+                info[r] = pt[q];
+#pragma unroll
+                for (int t = 0; t < W; ++t) wT[r][t] = es_weight<W>(d.x, t, beta);
+            } else {
+#pragma unroll
+                for (int t = 0; t < W; ++t) wy[r][t] = es_weight<W>(d.y, t, beta);
+            }
+        }
+    }
+    __syncthreads();
+    const int k = kb * 64 + 2 * lane;
+    if (k >= nc) return;
+    const int64_t line = (int64_t)nf2 * pitch;
+    for (int r = warp; r < kRowGroup && base + r < nrow; r += 8) {
+        const int4 I = info[r];
+        const float2 *p = G + I.y * line + k;
+        float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+#pragma unroll
+        for (int t2 = 0; t2 < W; ++t2) {
+            int yy = I.z + t2; if (yy >= nf2) yy -= nf2;
+            const float2 *q = p + (int64_t)yy * pitch;
+            float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll
+            for (int t1 = 0; t1 < W; ++t1) {
+                const float4 v = __ldg(reinterpret_cast<const float4 *>(q + t1 * line));
+                const float u = wT[r][t1];
+                s0 = __ffma2_rn(make_float2(u, u), make_float2(v.x, v.y), s0);
+                s1 = __ffma2_rn(make_float2(u, u), make_float2(v.z, v.w), s1);
+            }
+            const float u = wy[r][t2];
+            a0 = __ffma2_rn(make_float2(u, u), s0, a0);
+            a1 = __ffma2_rn(make_float2(u, u), s1, a1);
+        }
+        float2 *o = out + (int64_t)I.x * nc + k;
+        o[0] = a0;
+        if (k + 1 < nc) o[1] = a1;
+    }
+}
+
+// Rows -> nodes (the transpose).  A CTA owns 4 x 4 (T, y) cells, a thread one
+// column: 16 complex sums in registers over the rows whose footprint meets the
+// cells, which the cell order gives as W + 3 runs (one per y start).  Writes
+// the node grid as [T][X][y], y fastest, four y at a time.  With SYM a row's
+// value is the projection spectrum of sysmat, formed from F at q and at -q:
+// the strength conj(a) 2 P / N = (F(q) / 2 + 2 conj(a)^2 conj F(-q)) / N.
+template <int W, bool SYM>
+__global__ void __launch_bounds__(256) k_rows_spread(const uint32_t *__restrict__ start, const int4 *__restrict__ pt,
+                                                     const float2 *__restrict__ pd, int nstart, int nT, int ntile, int nf2,
+                                                     const float2 *__restrict__ src, int nr, int nc, float beta,
+                                                     const float2 *__restrict__ beam, float scale, float2 *__restrict__ Gt) {
+    extern __shared__ __align__(16) unsigned char rsm[];
+    const int cap = blockDim.x;
+    float4 *lw = reinterpret_cast<float4 *>(rsm);            // [cap][kCell] weights, T by y
+    int2 *lr = reinterpret_cast<int2 *>(lw + cap * kCell);   // row, mirrored row
+    float2 *lb = reinterpret_cast<float2 *>(lr + cap);       // 2 conj(a)^2 / N
+    constexpr int NR = W + kCell - 1;
+    __shared__ int beg[NR], pre[NR + 1];
+    const int tid = threadIdx.x;
+    const int c1 = (blockIdx.x % ntile) * kCell, c2 = (blockIdx.x / ntile) * kCell;
+    const int k = blockIdx.y * blockDim.x + tid;
+    const int kc = min(k, nc - 1);
+    if (tid < NR) {
+        const int ys = wrap(c2 - (W - 1) + tid, nf2);
+        const int lo = max(0, c1 - (W - 1)), hi = min(nstart - 1, c1 + kCell - 1);
+        const int64_t o = (int64_t)ys * nstart;
+        beg[tid] = (int)start[o + lo];
+        pre[tid + 1] = (int)(start[o + hi + 1] - start[o + lo]);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        pre[0] = 0;
+        for (int r = 0; r < NR; ++r) pre[r + 1] += pre[r];
+    }
+    __syncthreads();
+    const int total = pre[NR];
+    float2 re[kCell][2], im[kCell][2];
+#pragma unroll
+    for (int i = 0; i < kCell; ++i) re[i][0] = re[i][1] = im[i][0] = im[i][1] = make_float2(0.f, 0.f);
+    for (int base = 0; base < total; base += cap) {
+        const int n = min(cap, total - base);
+        if (tid < n) {
+            int r = 0;
+            while (base + tid >= pre[r + 1]) ++r;
+            const int at = beg[r] + base + tid - pre[r];
+            const int4 I = pt[at];
+            const float2 d = pd[at];
+            float u[kCell];
+#pragma unroll
+            for (int i = 0; i < kCell; ++i) u[i] = es_tap<W>(d.y, i + W - 1 - r, beta);
+#pragma unroll
+            for (int i = 0; i < kCell; ++i) {
+                const float s = es_tap<W>(d.x, c1 + i - I.y, beta);
+                lw[tid * kCell + i] = make_float4(s * u[0], s * u[1], s * u[2], s * u[3]);
+            }
+            const int j = I.x - I.w * nr;
+            lr[tid] = make_int2(I.x, I.w * nr + nr - 1 - j);
+            if (SYM) {
+                const float2 a = beam[I.w];  // conj(a)^2 = (ax^2 - ay^2) - 2 i ax ay
+                lb[tid] = make_float2(2 * scale * (a.x * a.x - a.y * a.y), -4 * scale * a.x * a.y);
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int q = 0; q < n; ++q) {
+            const int2 row = lr[q];
+            float2 v = __ldg(src + (int64_t)row.x * nc + kc);
+            if (SYM) {
+                const float2 m = __ldg(src + (int64_t)row.y * nc + nc - 1 - kc), b = lb[q];
+                v = make_float2(fmaf(b.x, m.x, fmaf(b.y, m.y, 0.5f * scale * v.x)),
+                                fmaf(b.y, m.x, fmaf(-b.x, m.y, 0.5f * scale * v.y)));
+            }
+            const float2 vr = make_float2(v.x, v.x), vi = make_float2(v.y, v.y);
+#pragma unroll
+            for (int i = 0; i < kCell; ++i) {
+                const float4 t = lw[q * kCell + i];
+                re[i][0] = __ffma2_rn(make_float2(t.x, t.y), vr, re[i][0]);
+                re[i][1] = __ffma2_rn(make_float2(t.z, t.w), vr, re[i][1]);
+                im[i][0] = __ffma2_rn(make_float2(t.x, t.y), vi, im[i][0]);
+                im[i][1] = __ffma2_rn(make_float2(t.z, t.w), vi, im[i][1]);
+            }
+        }
+        __syncthreads();
+    }
+    if (k >= nc) return;
+#pragma unroll
+    for (int i = 0; i < kCell; ++i) {
+        if (c1 + i >= nT) break;
+        float4 *o = reinterpret_cast<float4 *>(Gt + ((int64_t)(c1 + i) * nc + k) * nf2 + c2);
+        o[0] = make_float4(re[i][0].x, im[i][0].x, re[i][0].y, im[i][0].y);  // nf2 is even: pairs are whole
+        if (c2 + 2 < nf2) o[1] = make_float4(re[i][1].x, im[i][1].x, re[i][1].y, im[i][1].y);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// projection space: fftshift2 / ifftshift2, the beam factor and the mirrored
+// half of the spectrum, as one factor per detector pixel:
+//   proj = scale Re(c a t), spectrum input = proj conj(a t),
+//   t(m1, m2) = 2 cos(b1 + b2) e^{i pi (m1 / nr + m2 / nc)}, b from k_lat_tables
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ float2 twist(float4 r, float4 c, float2 a) {
+    const float f = 2.f * (r.x * c.x - r.y * c.y);
+    const float tr = r.z * c.z - r.w * c.w, ti = r.z * c.w + r.w * c.z;
+    return make_float2(f * (tr * a.x - ti * a.y), f * (tr * a.y + ti * a.x));
+}
+// one CTA row of blocks per detector row (blockIdx.y = projection * nr + row)
+__global__ void __launch_bounds__(256) k_proj_post(const float2 *__restrict__ P, int64_t nrow, int nr, int nc,
+                                                   const float4 *__restrict__ trow, const float4 *__restrict__ tcol,
+                                                   const float2 *__restrict__ beam, float scale, float *__restrict__ proj) {
+    const int e1 = (nr + 1) / 2, e2 = (nc + 1) / 2;
+    for (int64_t row = blockIdx.x; row < nrow; row += gridDim.x) {
+        const int p = (int)(row / nr), j = (int)(row - (int64_t)p * nr);
+        int js = j + e1; if (js >= nr) js -= nr;
+        const float2 a = __ldg(beam + p);
+        const float4 tr = __ldg(trow + js);
+        const float2 *src = P + ((int64_t)p * nr + js) * nc;
+        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+            int ks = k + e2; if (ks >= nc) ks -= nc;
+            const float2 t = twist(tr, __ldg(tcol + ks), a), c = src[ks];
+            proj[row * nc + k] = (c.x * t.x - c.y * t.y) * scale;
+        }
+    }
+}
+__global__ void __launch_bounds__(256) k_proj_pre(const float *__restrict__ proj, int64_t nrow, int nr, int nc,
+                                                  const float4 *__restrict__ trow, const float4 *__restrict__ tcol,
+                                                  const float2 *__restrict__ beam, float2 *__restrict__ P) {
+    const int d1 = nr / 2, d2 = nc / 2;
+    for (int64_t row = blockIdx.x; row < nrow; row += gridDim.x) {
+        const int p = (int)(row / nr), j = (int)(row - (int64_t)p * nr);
+        int js = j + d1; if (js >= nr) js -= nr;
+        const float2 a = __ldg(beam + p);
+        const float4 tr = __ldg(trow + j);
+        const float *src = proj + ((int64_t)p * nr + js) * nc;
+        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+            int ks = k + d2; if (ks >= nc) ks -= nc;
+            const float2 t = twist(tr, __ldg(tcol + k), a);
+            const float v = src[ks];
+            P[row * nc + k] = make_float2(v * t.x, -v * t.y);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// direct sysmat per point, for calls that may not allocate a lattice: w^3 taps
+// per point from the fine grid of W and atomics into the fine grid of U, at q
+// and at -q (float positions, so -q is not a lattice point)
+// ---------------------------------------------------------------------------
+
+template <int W>
+struct Taps {
+    float w1[W], w2[W], w3[W];
+    int l1, l2, l3;
+    __device__ __forceinline__ Taps(const Fine &F, float x, float y, float z) {
+        float d1, d2, d3;
+        l3 = wrap(es_first<W>(x, F.s3, d3), F.nf3);
+        l2 = wrap(es_first<W>(y, F.s2, d2), F.nf2);
+        l1 = wrap(es_first<W>(z, F.s1, d1), F.nf1);
+#pragma unroll
+        for (int t = 0; t < W; ++t) {
+            w1[t] = es_weight<W>(d1, t, F.beta);
+            w2[t] = es_weight<W>(d2, t, F.beta);
+            w3[t] = es_weight<W>(d3, t, F.beta);
+        }
+    }
+    template <class Fn>
+    __device__ __forceinline__ void each(const Fine &F, Fn &&fn) const {
+        for (int a = 0; a < W; ++a) {
+            int i1 = l1 + a; if (i1 >= F.nf1) i1 -= F.nf1;
+            for (int b = 0; b < W; ++b) {
+                int i3 = l3 + b; if (i3 >= F.nf3) i3 -= F.nf3;
+                const int64_t row = ((int64_t)i1 * F.nf3 + i3) * F.nf2;
+                const float u = w1[a] * w3[b];
+#pragma unroll
+                for (int c = 0; c < W; ++c) {
+                    int i2 = l2 + c; if (i2 >= F.nf2) i2 -= F.nf2;
+                    fn(row + i2, u * w2[c]);
+                }
+            }
+        }
+    }
+};
+template <int W>
+__global__ void __launch_bounds__(256) k_sysmat_points(GeomView g, const float2 *__restrict__ G, float2 *__restrict__ H,
+                                                       Fine F, float inv_scale) {
+    const uint32_t plane = (uint32_t)g.nrows * g.ncols, M = (uint32_t)g.nproj * plane;
     for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < M; pid += gridDim.x * blockDim.x) {
-        const uint32_t bin = point_bin<W, PAIRED>(g, F, B, pid);
-        const unsigned grp = __match_any_sync(__activemask(), bin);
-        if (lane == __ffs(grp) - 1) atomicAdd(cnt + bin, (uint32_t)__popc(grp));
+        const int p = (int)(pid / plane);
+        const uint32_t r = pid - (uint32_t)p * plane;
+        const int j = (int)(r / (uint32_t)g.ncols), k = (int)(r - (uint32_t)j * g.ncols);
+        float x, y, z;
+        point_xyz(g, p, j, k, x, y, z);
+        const float ax = 0.5f * __ldg(g.st + p), ay = -0.5f * __ldg(g.ct + p);
+        const Taps<W> tq(F, x, y, z), tm(F, -x, -y, -z);
+        float2 f = make_float2(0.f, 0.f), h = f;
+        tq.each(F, [&](int64_t i, float u) { const float2 v = __ldg(G + i); f.x = fmaf(u, v.x, f.x); f.y = fmaf(u, v.y, f.y); });
+        tm.each(F, [&](int64_t i, float u) { const float2 v = __ldg(G + i); h.x = fmaf(u, v.x, h.x); h.y = fmaf(u, v.y, h.y); });
+        // P = a F(q) + conj(a F(-q)); strengths conj(a) P at q, conj(a) conj(P) at -q
+        const float pr = (ax * f.x - ay * f.y + ax * h.x - ay * h.y) * inv_scale;
+        const float pi = (ax * f.y + ay * f.x - ax * h.y - ay * h.x) * inv_scale;
+        const float2 s = make_float2(ax * pr + ay * pi, ax * pi - ay * pr);
+        const float2 m = make_float2(ax * pr - ay * pi, -ax * pi - ay * pr);
+        tq.each(F, [&](int64_t i, float u) { atomicAdd(H + i, make_float2(u * s.x, u * s.y)); });
+        tm.each(F, [&](int64_t i, float u) { atomicAdd(H + i, make_float2(u * m.x, u * m.y)); });
     }
 }
 
-template <int W, bool PAIRED>
-__global__ void __launch_bounds__(256) k_bin_scatter(GeomView g, Fine F, BinLayout B, uint32_t *__restrict__ cursor,
-                                                     uint32_t *__restrict__ perm) {
-    const uint32_t M = sort_ids<PAIRED>(g);
-    const int lane = threadIdx.x & 31;
-    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < M; pid += gridDim.x * blockDim.x) {
-        const uint32_t bin = point_bin<W, PAIRED>(g, F, B, pid);
-        const unsigned grp = __match_any_sync(__activemask(), bin);
-        const int leader = __ffs(grp) - 1;
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(cursor + bin, (uint32_t)__popc(grp));
-        base = __shfl_sync(grp, base, leader);
-        perm[base + __popc(grp & ((1u << lane) - 1u))] = pid;
+// ---------------------------------------------------------------------------
+// host orchestration
+// ---------------------------------------------------------------------------
+
+static Fine fine_of(const NufftPlan &pl) {
+    Fine F;
+    F.nf1 = (int)pl.nf1; F.nf2 = (int)pl.nf2; F.nf3 = (int)pl.nf3;
+    F.s1 = (double)pl.nf1 / (2 * M_PI);
+    F.s2 = (double)pl.nf2 / (2 * M_PI);
+    F.s3 = (double)pl.nf3 / (2 * M_PI);
+    F.beta = pl.beta;
+    return F;
+}
+static unsigned volume_tiles(const Dims3 &v) { return (unsigned)(v.n1 * ((v.n2 + 31) / 32) * ((v.n3 + 31) / 32)); }
+static LatView lat_view(const Lattice &l, const Geom &g) {
+    return LatView{l.X, l.cg, l.sg, l.h, (int)g.ncols, l.nT, l.T0};
+}
+static void check_points(const Geom &g) {
+    if (g.npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "too many points in one geometry");
+}
+
+// width as a compile-time constant for a generic lambda
+template <class Fn>
+static void with_width(int w, Fn &&fn) {
+    switch (w) {
+        case 4: fn(std::integral_constant<int, 4>{}); break;
+        case 5: fn(std::integral_constant<int, 5>{}); break;
+        case 6: fn(std::integral_constant<int, 6>{}); break;
+        case 7: fn(std::integral_constant<int, 7>{}); break;
+        case 8: fn(std::integral_constant<int, 8>{}); break;
+        default: throw Error(ERR_ARG, "unsupported kernel width");
     }
+}
+
+void NufftPlan::pad_real(const float *x3, double sg, double cg, const float *ipT, cudaStream_t s) {
+    LAMINO_CUDA(cudaMemsetAsync(grid.p, 0, nf() * sizeof(float2), s));
+    const unsigned b = volume_tiles(vol);
+    k_pad<false><<<b, 256, 0, s>>>(x3, nullptr, (int)vol.n1, (int)vol.n2, (int)vol.n3, (float)sg, (float)cg, grid.p,
+                                   fine_of(*this), ip1.p, ip2.p, ip3.p, ipT);
+    LAMINO_LAUNCH("k_pad");
+}
+
+void NufftPlan::extract_real(float *y3, double sg, double cg, const float *ipT, float scale, bool accumulate,
+                             cudaStream_t s) {
+    const unsigned b = volume_tiles(vol);
+    k_extract<false><<<b, 256, 0, s>>>(grid.p, (int)vol.n1, (int)vol.n2, (int)vol.n3, (float)sg, (float)cg, y3, nullptr,
+                                       fine_of(*this), ip1.p, ip2.p, ip3.p, ipT, scale, accumulate ? 1 : 0);
+    LAMINO_LAUNCH("k_extract");
+}
+
+void NufftPlan::fft_fine(float2 *g, int sign, cudaStream_t s) {
+    LAMINO_CUFFT(cufftSetStream(fft3.h, s));
+    LAMINO_CUFFT(cufftExecC2C(fft3.h, (cufftComplex *)g, (cufftComplex *)g, sign < 0 ? CUFFT_FORWARD : CUFFT_INVERSE));
+}
+
+void NufftPlan::ensure_proj(const Geom &g) {
+    check_points(g);
+    if ((int64_t)pbuf.n < g.npts()) pbuf.alloc(g.npts());
+    if (f2_np != g.nproj || f2_nr != g.nrows || f2_nc != g.ncols) {
+        int n[2] = {(int)g.nrows, (int)g.ncols};
+        fft2.make(2, n, CUFFT_C2C, (int)g.nproj);
+        f2_np = g.nproj; f2_nr = g.nrows; f2_nc = g.ncols;
+    }
+}
+
+// Bin layouts were the tiles of a point-by-point spread; the limits on them
+// (that kernel's tile, two sets of three components and its staged points, in
+// 227 KB of shared memory) still define which layouts the entry point takes.
+void NufftPlan::set_bins(int c1, int c2, int c3) {
+    if (c1 <= 0 || c2 <= 0 || c3 <= 0) throw Error(ERR_ARG, "bin sizes must be positive");
+    if (c1 > 16) throw Error(ERR_ARG, "bin extent along n1 must be at most 16");
+    if (c2 > 4095 || c3 > 4095) throw Error(ERR_ARG, "bin extents along n2 and n3 must be below 4096");
+    const int64_t cells = (int64_t)(c1 + w - 1) * (c2 + w - 1) * (c3 + w - 1);
+    const int64_t rec = (16 * 3 + 24 * w + 4 + 15) / 16 * 16, tables = 4 * (8 * 16 + 17);
+    if ((48 * cells + 15) / 16 * 16 + 256 * rec > 227 * 1024 - tables)
+        throw Error(ERR_ARG, "bin tile too large for shared memory");
+    b1 = c1; b2 = c2; b3 = c3;
 }
 
 // exclusive scan of the bin counts (one CTA of 1024 threads, 4096 bins per pass)
@@ -457,904 +956,143 @@ __global__ void __launch_bounds__(1024) k_scan_offsets(const uint32_t *__restric
     if (threadIdx.x == 0) start[n] = carry_s;
 }
 
-// ---------------------------------------------------------------------------
-// binned spread / interpolation: one CTA per bin, the bin's tile of
-// (b + w - 1)^3 cells per component staged in shared memory
-
-struct BinOrigin {
-    int o1, o2, o3;
-};
-__device__ __forceinline__ BinOrigin bin_origin(const BinLayout &B, int bin) {
-    const int c3 = bin % B.nb3, r = bin / B.nb3;
-    const int c2 = r % B.nb2, c1 = r / B.nb2;
-    return BinOrigin{c1 * B.b1, c2 * B.b2, c3 * B.b3};
-}
-// fine-grid index of tile cell `cell` (wrapped)
-__device__ __forceinline__ int64_t tile_cell_index(const BinLayout &B, const BinOrigin &o, const Fine &F, int cell) {
-    const int i3 = cell % B.r3, r = cell / B.r3;
-    const int i2 = r % B.t2, i1 = r / B.t2;
-    const int g1 = (o.o1 + i1) % F.nf1, g2 = (o.o2 + i2) % F.nf2, g3 = (o.o3 + i3) % F.nf3;
-    return ((int64_t)g1 * F.nf2 + g2) * F.nf3 + g3;
-}
-
-template <int W, int NC>
-__device__ __forceinline__ void gather_tile(const float2 *tile, int tsz, const BinLayout &B, int a1, int a2, int a3,
-                                            const float *w1, const float *w2, const float *w3, float2 *out) {
-#pragma unroll
-    for (int c = 0; c < NC; ++c) out[c] = make_float2(0.f, 0.f);
-#pragma unroll 1
-    for (int t1 = 0; t1 < W; ++t1) {
-#pragma unroll
-        for (int t2 = 0; t2 < W; ++t2) {
-            const float2 *row = tile + ((a1 + t1) * B.t2 + a2 + t2) * B.r3 + a3;
-            const float k12 = w1[t1] * w2[t2];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                float rr = 0.f, ri = 0.f;
-#pragma unroll
-                for (int t3 = 0; t3 < W; ++t3) {
-                    const float2 v = row[c * tsz + t3];
-                    rr = fmaf(w3[t3], v.x, rr);
-                    ri = fmaf(w3[t3], v.y, ri);
-                }
-                out[c].x = fmaf(k12, rr, out[c].x);
-                out[c].y = fmaf(k12, ri, out[c].y);
-            }
-        }
-    }
-}
-
-// gather_tile for a pair: each tile value is read once and weighted for both
-// points (out: first point, same sums as gather_tile; outu: second point)
-template <int W, int NC>
-__device__ __forceinline__ void gather_tile_pair(const float2 *tile, int tsz, const BinLayout &B, int a1, int a2,
-                                                 int a3, const float (&w)[3][W], const float (&u)[3][W], float2 *out,
-                                                 float2 *outu) {
-#pragma unroll
-    for (int c = 0; c < NC; ++c) out[c] = outu[c] = make_float2(0.f, 0.f);
-#pragma unroll 1
-    for (int t1 = 0; t1 < W; ++t1) {
-        // the slab weights by selects, so that no weight array is indexed at run
-        // time (which would move the arrays to local memory)
-        float w1 = w[0][0], u1 = u[0][0];
-#pragma unroll
-        for (int r = 1; r < W; ++r) {
-            w1 = t1 == r ? w[0][r] : w1;
-            u1 = t1 == r ? u[0][r] : u1;
-        }
-#pragma unroll
-        for (int t2 = 0; t2 < W; ++t2) {
-            const float2 *row = tile + ((a1 + t1) * B.t2 + a2 + t2) * B.r3 + a3;
-            const float k12 = w1 * w[1][t2], m12 = u1 * u[1][t2];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                float rr = 0.f, ri = 0.f, sr = 0.f, si = 0.f;
-#pragma unroll
-                for (int t3 = 0; t3 < W; ++t3) {
-                    const float2 v = row[c * tsz + t3];
-                    rr = fmaf(w[2][t3], v.x, rr);
-                    ri = fmaf(w[2][t3], v.y, ri);
-                    sr = fmaf(u[2][t3], v.x, sr);
-                    si = fmaf(u[2][t3], v.y, si);
-                }
-                out[c].x = fmaf(k12, rr, out[c].x);
-                out[c].y = fmaf(k12, ri, out[c].y);
-                outu[c].x = fmaf(m12, sr, outu[c].x);
-                outu[c].y = fmaf(m12, si, outu[c].y);
-            }
-        }
-    }
-}
-
-// global-memory paths for a point outside its bin's tile (never taken when the
-// sort and the kernels agree on the taps); out of line to spare registers
-template <int W, int NC>
-__device__ __noinline__ void spread_point_global(float2 *H, int64_t NF, Fine F, float x, float y, float z,
-                                                 const float2 *str) {
-    spread_point<W, NC>(H, NF, F, x, y, z, str);
-}
-template <int W, int NC>
-__device__ __noinline__ void interp_point_global(const float2 *G, int64_t NF, Fine F, float x, float y, float z,
-                                                 float2 *out) {
-    interp_point<W, NC>(G, NF, F, x, y, z, out);
-}
-
-// taps of a point and its offset inside the bin's tile; false if the point lies
-// outside the bin (only possible if the sort and this kernel disagreed)
-template <int W>
-__device__ __forceinline__ bool point_taps(const GeomView &g, const Fine &F, const BinLayout &B, const BinOrigin &o,
-                                           int p, int j, int k, float *w1, float *w2, float *w3, int &a1, int &a2,
-                                           int &a3, float &x, float &y, float &z) {
-    point_xyz(g, p, j, k, x, y, z);
-    const int l3 = es_taps<W>(x, F.nf3, F.s3, F.beta, w3);
-    const int l2 = es_taps<W>(y, F.nf2, F.s2, F.beta, w2);
-    const int l1 = es_taps<W>(z, F.nf1, F.s1, F.beta, w1);
-    a1 = l1 - o.o1;
-    a2 = l2 - o.o2;
-    a3 = l3 - o.o3;
-    return (unsigned)a1 < (unsigned)B.b1 && (unsigned)a2 < (unsigned)B.b2 && (unsigned)a3 < (unsigned)B.b3;
-}
-
-struct RawStrength {
-    const float2 *c;
-    __device__ __forceinline__ void operator()(const GeomView &, int, int, int, uint32_t pid, float2 *s) const {
-        s[0] = c[pid];
-    }
-};
-// forward: P[fftshift2 position of (j, k)] = sum_i coeff_i(th) * v_i
-__device__ __forceinline__ float2 beam_combine(const GeomView &g, int p, const float2 *v) {
-    const float c0 = __ldg(g.coeff + p), c1 = __ldg(g.coeff + g.nproj + p), c2 = __ldg(g.coeff + 2 * g.nproj + p);
-    return make_float2(c0 * v[0].x + c1 * v[1].x + c2 * v[2].x, c0 * v[0].y + c1 * v[1].y + c2 * v[2].y);
-}
-__device__ __forceinline__ void forward_store(const GeomView &g, int p, int j, int k, float2 o, float2 *P) {
-    int js = j - g.nrows / 2; if (js < 0) js += g.nrows;
-    int ks = k - g.ncols / 2; if (ks < 0) ks += g.ncols;
-    P[((int64_t)p * g.nrows + js) * g.ncols + ks] = o;
-}
-struct RawSink {
-    float2 *c;
-    __device__ __forceinline__ void operator()(const GeomView &, int, int, int, uint32_t pid, const float2 *v) const {
-        c[pid] = v[0];
-    }
-};
-
-// A staged point: its offset in the bin's tile, its separable kernel weights and
-// its NC strengths.
-template <int W, int NC>
-struct PointRec {
-    int a1, a2, a3;
-    float w1[W], w2[W], w3[W];
-    float2 s[NC];
-};
-// A staged antipodal pair, laid out so that a visit reads each quantity of
-// both points with one load: per component the two strengths (s.x, s.y, g.x,
-// g.y), per tap the two weights (first, second point), and the first point's
-// tile offset packed as a1 | a2 << 8 | a3 << 20.
-template <int W, int NC>
-struct __align__(16) PairRec {
-    float4 sg[NC];
-    float2 w1[W], w2[W], w3[W];
-    int a;
-};
-constexpr int kStageChunk = 256;  // points staged per pass (threads of the staging CTAs)
-constexpr int kStagePairs = kStageChunk / 2;  // pairs staged per pass, two threads each
-constexpr size_t point_rec_bytes(int w, int nc) { return (size_t)((12 + 12 * w + 7) / 8 * 8 + 8 * nc); }
-constexpr size_t pair_rec_bytes(int w, int nc) { return (size_t)((16 * nc + 24 * w + 4 + 15) / 16 * 16); }
-// byte offset of the pair records after NC tiles of tsz cells (16-byte aligned)
-__host__ __device__ constexpr size_t pair_rec_offset(int64_t tsz, int nc) { return (size_t)((nc * tsz * 8 + 15) / 16 * 16); }
-static_assert(sizeof(PointRec<7, 3>) == point_rec_bytes(7, 3), "record layout");
-static_assert(sizeof(PointRec<8, 1>) == point_rec_bytes(8, 1), "record layout");
-static_assert(sizeof(PairRec<7, 3>) == pair_rec_bytes(7, 3), "record layout");
-static_assert(sizeof(PairRec<8, 3>) == pair_rec_bytes(8, 3), "record layout");
-static_assert(sizeof(PairRec<4, 3>) == pair_rec_bytes(4, 3), "record layout");
-
-// Records of a staged chunk in slab order.  Every CTA of the binned kernels
-// runs kStageChunk threads, one point each.  A point whose taps fit in the
-// bin's tile starts at tile slab a1 in [0, b1) (bkt = a1; -1 otherwise); its
-// record goes to position bstart[a1] + (its rank among the chunk's points with
-// that a1, in point order), so records are sorted by a1 and the sum into every
-// cell runs in a fixed order.  The ranks come from one ballot per slab start,
-// the offsets from a scan over warps and starts by warp 0.  Returns the
-// record position (-1 for bkt < 0); called by every thread of the CTA.
-constexpr int kMaxB1 = 16;                       // largest bin extent along n1
-constexpr int kStageWarps = kStageChunk / 32;
-__device__ __forceinline__ int place_slot(int bkt, int *wcnt, int *bstart, const BinLayout &B) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int rank = 0;
-    for (int b = 0; b < B.b1; ++b) {
-        const unsigned m = __ballot_sync(0xffffffffu, bkt == b);
-        if (bkt == b) rank = __popc(m & ((1u << lane) - 1u));
-        if (lane == 0) wcnt[warp * kMaxB1 + b] = __popc(m);
-    }
-    __syncthreads();
-    if (warp == 0) {
-        int tot = 0;
-        if (lane < B.b1)
-            for (int v = 0; v < kStageWarps; ++v) {
-                const int c = wcnt[v * kMaxB1 + lane];
-                wcnt[v * kMaxB1 + lane] = tot;
-                tot += c;
-            }
-        int incl = tot;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += u;
-        }
-        if (lane < B.b1) {
-            const int excl = incl - tot;
-            for (int v = 0; v < kStageWarps; ++v) wcnt[v * kMaxB1 + lane] += excl;
-            bstart[lane] = excl;
-            if (lane == B.b1 - 1) bstart[B.b1] = incl;
-        }
-    }
-    __syncthreads();
-    return bkt >= 0 ? wcnt[warp * kMaxB1 + bkt] + rank : -1;
-}
-
-// Spread the staged points into the tile without atomics: warp v owns the tile
-// slabs i1 = v, v + nwarps, ... and, slab by slab, applies the taps of the
-// points that reach the slab (those with a1 in [slab - w + 1, slab], one run
-// of the sorted records), its lanes covering a point's w x w (t2, t3) taps.
-// Each cell has one writer and its sum runs in record order.  The NR x NC
-// read-modify-writes of one point touch distinct cells, so their loads are
-// issued together, then the FMAs, then the stores.
-template <int W, int NC>
-__device__ __forceinline__ void spread_sorted(float2 *tile, int tsz, const BinLayout &B,
-                                              const PointRec<W, NC> *recs, const int *bstart) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    constexpr int NT = W * W;
-    constexpr int NR = (NT + 31) / 32;
-    int t2s[NR], t3s[NR], loff[NR];
-    bool act[NR];
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        const int q = lane + 32 * r;
-        act[r] = q < NT;
-        t2s[r] = act[r] ? q / W : 0;
-        t3s[r] = act[r] ? q - (q / W) * W : 0;
-        loff[r] = t2s[r] * B.r3 + t3s[r];
-    }
-    const int slab_stride = B.t2 * B.r3;
-    for (int slab = warp; slab < B.t1; slab += nwarps) {
-        const int lo = max(0, slab - (W - 1)), hi = min(B.b1 - 1, slab);
-        if (lo > hi) continue;
-        const int q1 = bstart[hi + 1];
-        float2 *srow = tile + slab * slab_stride;
-        for (int q = bstart[lo]; q < q1; ++q) {
-            const PointRec<W, NC> &pr = recs[q];
-            const float w1v = pr.w1[slab - pr.a1];
-            float2 *cell0 = srow + pr.a2 * B.r3 + pr.a3;
-            float wt[NR];
-            float2 v[NR][NC];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                wt[r] = w1v * (pr.w2[t2s[r]] * pr.w3[t3s[r]]);
-                if (act[r]) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) v[r][c] = cell0[loff[r] + c * tsz];
-                }
-            }
-            float2 sv[NC];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) sv[c] = pr.s[c];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                if (act[r]) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        v[r][c].x = fmaf(wt[r], sv[c].x, v[r][c].x);
-                        v[r][c].y = fmaf(wt[r], sv[c].y, v[r][c].y);
-                        cell0[loff[r] + c * tsz] = v[r][c];
-                    }
-                }
-            }
-        }
-    }
-}
-
-// spread_sorted for pair records: each tap adds the first point's term, then
-// the second's
-template <int W, int NC>
-__device__ __forceinline__ void spread_pairs_sorted(float2 *tile, int tsz, const BinLayout &B,
-                                                    const PairRec<W, NC> *recs, const int *bstart) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    constexpr int NT = W * W;
-    constexpr int NR = (NT + 31) / 32;
-    int t2s[NR], t3s[NR], loff[NR];
-    bool act[NR];
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        const int q = lane + 32 * r;
-        act[r] = q < NT;
-        t2s[r] = act[r] ? q / W : 0;
-        t3s[r] = act[r] ? q - (q / W) * W : 0;
-        loff[r] = t2s[r] * B.r3 + t3s[r];
-    }
-    const int slab_stride = B.t2 * B.r3;
-    for (int slab = warp; slab < B.t1; slab += nwarps) {
-        const int lo = max(0, slab - (W - 1)), hi = min(B.b1 - 1, slab);
-        if (lo > hi) continue;
-        const int q1 = bstart[hi + 1];
-        float2 *srow = tile + slab * slab_stride;
-        for (int q = bstart[lo]; q < q1; ++q) {
-            const PairRec<W, NC> &pr = recs[q];
-            const int a = pr.a;
-            const float2 w1v = pr.w1[slab - (a & 0xff)];
-            float2 *cell0 = srow + ((a >> 8) & 0xfff) * B.r3 + (a >> 20);
-            float wt[NR], ut[NR];
-            float2 v[NR][NC];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const float2 b2 = pr.w2[t2s[r]], b3 = pr.w3[t3s[r]];
-                wt[r] = w1v.x * (b2.x * b3.x);
-                ut[r] = w1v.y * (b2.y * b3.y);
-                if (act[r]) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) v[r][c] = cell0[loff[r] + c * tsz];
-                }
-            }
-            float4 sg[NC];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) sg[c] = pr.sg[c];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                if (act[r]) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        v[r][c].x = fmaf(wt[r], sg[c].x, v[r][c].x);
-                        v[r][c].y = fmaf(wt[r], sg[c].y, v[r][c].y);
-                        v[r][c].x = fmaf(ut[r], sg[c].z, v[r][c].x);
-                        v[r][c].y = fmaf(ut[r], sg[c].w, v[r][c].y);
-                        cell0[loff[r] + c * tsz] = v[r][c];
-                    }
-                }
-            }
-        }
-    }
-}
-
-template <int NC>
-__device__ __forceinline__ void flush_tile(const float2 *tile, int tsz, const BinLayout &B, const BinOrigin &o,
-                                           const Fine &F, float2 *H, int64_t NF) {
-    for (int cell = threadIdx.x; cell < tsz; cell += blockDim.x) {
-        const int64_t gi = tile_cell_index(B, o, F, cell);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const float2 v = tile[c * tsz + cell];
-            if (v.x != 0.f || v.y != 0.f) atomicAdd(H + c * NF + gi, v);
-        }
-    }
-}
-
-template <int W, int NC, class Str>
-__global__ void __launch_bounds__(kStageChunk, 2) k_spread_binned(GeomView g, const uint32_t *__restrict__ perm,
-                                                       const uint32_t *__restrict__ start, BinLayout B, Fine F,
-                                                       float2 *__restrict__ H, int64_t NF, Str str) {
-    extern __shared__ float2 tile[];
-    const int bin = blockIdx.x;
-    const uint32_t p0 = start[bin], p1 = start[bin + 1];
-    if (p0 == p1) return;
-    const BinOrigin o = bin_origin(B, bin);
-    const int tsz = (int)B.tile_cells();
-    PointRec<W, NC> *recs = reinterpret_cast<PointRec<W, NC> *>(tile + NC * tsz);
-    for (int i = threadIdx.x; i < NC * tsz; i += blockDim.x) tile[i] = make_float2(0.f, 0.f);
-    __shared__ int wcnt[kStageWarps * kMaxB1];
-    __shared__ int bstart[kMaxB1 + 1];
-    for (uint32_t base = p0; base < p1; base += kStageChunk) {
-        const int n = (int)min((uint32_t)kStageChunk, p1 - base);
-        const int t = threadIdx.x;  // one point per thread (blockDim.x == kStageChunk)
-        uint32_t pid = 0;
-        int p = 0, j = 0, k = 0, a1 = -1, a2 = 0, a3 = 0;
-        float x = 0.f, y = 0.f, z = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-        bool in = false;
-        if (t < n) {
-            pid = __ldg(perm + base + t);
-            decode_pid(pid, g, p, j, k);
-            point_xyz(g, p, j, k, x, y, z);
-            a3 = es_start<W>(x, F.nf3, F.s3, d3) - o.o3;
-            a2 = es_start<W>(y, F.nf2, F.s2, d2) - o.o2;
-            a1 = es_start<W>(z, F.nf1, F.s1, d1) - o.o1;
-            in = (unsigned)a1 < (unsigned)B.b1 && (unsigned)a2 < (unsigned)B.b2 && (unsigned)a3 < (unsigned)B.b3;
-        }
-        const int pos = place_slot(in ? a1 : -1, wcnt, bstart, B);
-        if (t < n) {
-            float2 s[NC];
-            str(g, p, j, k, pid, s);
-            if (in) {
-                PointRec<W, NC> &pr = recs[pos];
-                pr.a1 = a1;
-                pr.a2 = a2;
-                pr.a3 = a3;
-                es_weights<W>(d1, F.beta, pr.w1);
-                es_weights<W>(d2, F.beta, pr.w2);
-                es_weights<W>(d3, F.beta, pr.w3);
-#pragma unroll
-                for (int c = 0; c < NC; ++c) pr.s[c] = s[c];
-            } else {
-                spread_point_global<W, NC>(H, NF, F, x, y, z, s);
-            }
-        }
-        __syncthreads();
-        spread_sorted<W, NC>(tile, tsz, B, recs, bstart);
-        __syncthreads();
-    }
-    flush_tile<NC>(tile, tsz, B, o, F, H, NF);
-}
-
-// Both points of pair `pid`: the first point's position, tile offsets (a1 < 0 when
-// outside the bin) and tap offsets d, and the second point's position x2 = -x_{i'}
-// with its tap offsets e on the first point's footprint; `near` as es_offset_from.
-struct PairPos {
-    int p, j, k, j2, k2, a1, a2, a3;
-    float x, y, z, x2, y2, z2;
-    float d1, d2, d3, e1, e2, e3;
-    bool in, near, self;
-};
-template <int W>
-__device__ __forceinline__ void pair_positions(const GeomView &g, const Fine &F, const BinLayout &B,
-                                               const BinOrigin &o, uint32_t pid, PairPos &q) {
-    decode_pair(pid, g, q.p, q.j, q.k, q.j2, q.k2);
-    q.self = q.j2 == q.j && q.k2 == q.k;
-    point_xyz(g, q.p, q.j, q.k, q.x, q.y, q.z);
-    double l1, l2, l3;
-    q.a3 = es_start<W>(q.x, F.nf3, F.s3, q.d3, l3) - o.o3;
-    q.a2 = es_start<W>(q.y, F.nf2, F.s2, q.d2, l2) - o.o2;
-    q.a1 = es_start<W>(q.z, F.nf1, F.s1, q.d1, l1) - o.o1;
-    q.in = (unsigned)q.a1 < (unsigned)B.b1 && (unsigned)q.a2 < (unsigned)B.b2 && (unsigned)q.a3 < (unsigned)B.b3;
-    float xa, ya, za;
-    point_xyz(g, q.p, q.j2, q.k2, xa, ya, za);
-    q.x2 = -xa;
-    q.y2 = -ya;
-    q.z2 = -za;
-    q.near = es_offset_from<W>(q.x2, F.s3, l3, q.e3) && es_offset_from<W>(q.y2, F.s2, l2, q.e2) &&
-             es_offset_from<W>(q.z2, F.s1, l1, q.e1);
-}
-
-// Adjoint spread over antipodal pairs (see decode_pair): two threads stage a
-// pair, the even one its first point (offsets, weights, strengths
-// coeff_i(th) P), the odd one its second point -x_{i'} (weights on the first
-// point's footprint, strengths coeff_i(th) conj(P_{i'})); records are ranked
-// by the first point's slab and spread as k_spread_binned does.  A second
-// point whose own footprint starts more than one cell away (not the case for
-// the reference's symmetric detector grids) is spread through global memory.
-template <int W>
-__global__ void __launch_bounds__(kStageChunk, 2) k_spread_pairs(GeomView g, const uint32_t *__restrict__ perm,
-                                                      const uint32_t *__restrict__ start, BinLayout B, Fine F,
-                                                      float2 *__restrict__ H, int64_t NF,
-                                                      const float2 *__restrict__ Pf) {
-    extern __shared__ __align__(16) unsigned char psm[];
-    float2 *tile = reinterpret_cast<float2 *>(psm);
-    const int bin = blockIdx.x;
-    const uint32_t p0 = start[bin], p1 = start[bin + 1];
-    if (p0 == p1) return;
-    const BinOrigin o = bin_origin(B, bin);
-    const int tsz = (int)B.tile_cells();
-    PairRec<W, 3> *recs = reinterpret_cast<PairRec<W, 3> *>(psm + pair_rec_offset(tsz, 3));
-    for (int i = threadIdx.x; i < 3 * tsz; i += blockDim.x) tile[i] = make_float2(0.f, 0.f);
-    __shared__ int wcnt[kStageWarps * kMaxB1];
-    __shared__ int bstart[kMaxB1 + 1];
-    const bool second = (threadIdx.x & 1) != 0;
-    const int t = threadIdx.x >> 1;  // pair slot (blockDim.x == kStageChunk == 2 kStagePairs)
-    for (uint32_t base = p0; base < p1; base += kStagePairs) {
-        const int n = (int)min((uint32_t)kStagePairs, p1 - base);
-        int p = 0, j = 0, k = 0, j2 = 0, k2 = 0, a1 = -1, a2 = 0, a3 = 0;
-        float x = 0.f, y = 0.f, z = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-        bool in = false, near = true;
-        if (t < n) {
-            decode_pair(__ldg(perm + base + t), g, p, j, k, j2, k2);
-            point_xyz(g, p, j, k, x, y, z);
-            double l1, l2, l3;
-            a3 = es_start<W>(x, F.nf3, F.s3, d3, l3) - o.o3;
-            a2 = es_start<W>(y, F.nf2, F.s2, d2, l2) - o.o2;
-            a1 = es_start<W>(z, F.nf1, F.s1, d1, l1) - o.o1;
-            in = (unsigned)a1 < (unsigned)B.b1 && (unsigned)a2 < (unsigned)B.b2 && (unsigned)a3 < (unsigned)B.b3;
-            if (second) {
-                float xa, ya, za;
-                point_xyz(g, p, j2, k2, xa, ya, za);
-                x = -xa;
-                y = -ya;
-                z = -za;
-                near = es_offset_from<W>(x, F.s3, l3, d3) && es_offset_from<W>(y, F.s2, l2, d2) &&
-                       es_offset_from<W>(z, F.s1, l1, d1);
-            }
-        }
-        int pos = place_slot(in && !second ? a1 : -1, wcnt, bstart, B);
-        pos = __shfl_sync(0xffffffffu, pos, (threadIdx.x & 31) & ~1);
-        if (t < n) {
-            const int jj = second ? j2 : j, kk = second ? k2 : k;
-            int js = jj + (g.nrows + 1) / 2; if (js >= g.nrows) js -= g.nrows;
-            int ks = kk + (g.ncols + 1) / 2; if (ks >= g.ncols) ks -= g.ncols;
-            float2 c = Pf[((int64_t)p * g.nrows + js) * g.ncols + ks];
-            if (second) c = (j2 == j && k2 == k) ? make_float2(0.f, 0.f) : make_float2(c.x, -c.y);
-            float2 sv[3];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const float cq = __ldg(g.coeff + q * g.nproj + p);
-                sv[q] = make_float2(cq * c.x, cq * c.y);
-            }
-            if (in) {
-                // the even thread fills the first point's halves of the record,
-                // the odd thread the second point's
-                PairRec<W, 3> &pr = recs[pos];
-                const int h = second ? 1 : 0;
-                float *wx[3] = {&pr.w1[0].x + h, &pr.w2[0].x + h, &pr.w3[0].x + h};
-                float wt[3][W];
-                if (near) {
-                    es_weights<W>(d1, F.beta, wt[0]);
-                    es_weights<W>(d2, F.beta, wt[1]);
-                    es_weights<W>(d3, F.beta, wt[2]);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < W; ++q) wt[0][q] = wt[1][q] = wt[2][q] = 0.f;
-                    spread_point_global<W, 3>(H, NF, F, x, y, z, sv);
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) sv[q] = make_float2(0.f, 0.f);
-                }
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-#pragma unroll
-                    for (int q = 0; q < W; ++q) wx[d][2 * q] = wt[d][q];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    float *sq = &pr.sg[q].x + 2 * h;
-                    sq[0] = sv[q].x;
-                    sq[1] = sv[q].y;
-                }
-                if (!second) pr.a = a1 | (a2 << 8) | (a3 << 20);
-            } else {
-                spread_point_global<W, 3>(H, NF, F, x, y, z, sv);
-            }
-        }
-        __syncthreads();
-        spread_pairs_sorted<W, 3>(tile, tsz, B, recs, bstart);
-        __syncthreads();
-    }
-    flush_tile<3>(tile, tsz, B, o, F, H, NF);
-}
-
-// Interpolation: the CTA loads its bin's tile, each thread gathers one point's
-// w^3 taps from shared memory and hands the NC values to the sink.
-template <int W, int NC, class Sink>
-__global__ void __launch_bounds__(256) k_interp_binned(GeomView g, const uint32_t *__restrict__ perm,
-                                                       const uint32_t *__restrict__ start, BinLayout B, Fine F,
-                                                       const float2 *__restrict__ G, int64_t NF, Sink sink) {
-    extern __shared__ float2 tile[];
-    const int bin = blockIdx.x;
-    const uint32_t p0 = start[bin], p1 = start[bin + 1];
-    if (p0 == p1) return;
-    const BinOrigin o = bin_origin(B, bin);
-    const int tsz = (int)B.tile_cells();
-    for (int i = threadIdx.x; i < NC * tsz; i += blockDim.x) {
-        const int c = i / tsz, cell = i - c * tsz;
-        tile[i] = __ldg(G + c * NF + tile_cell_index(B, o, F, cell));
-    }
-    __syncthreads();
-    for (uint32_t i = p0 + threadIdx.x; i < p1; i += blockDim.x) {
-        const uint32_t pid = __ldg(perm + i);
-        int p, j, k;
-        decode_pid(pid, g, p, j, k);
-        float w1[W], w2[W], w3[W], x, y, z;
-        int a1, a2, a3;
-        float2 v[NC];
-        if (point_taps<W>(g, F, B, o, p, j, k, w1, w2, w3, a1, a2, a3, x, y, z))
-            gather_tile<W, NC>(tile, tsz, B, a1, a2, a3, w1, w2, w3, v);
-        else
-            interp_point_global<W, NC>(G, NF, F, x, y, z, v);
-        sink(g, p, j, k, pid, v);
-    }
-}
-
-// Forward interpolation over antipodal pairs: a thread per pair gathers both
-// points from the tile (each tile value read once, weighted for both).  The
-// fine grid is the transform of a real volume, so G(-m) = conj(G(m)) and the
-// value at the antipode x_{i'} is conj of the gather at x2 = -x_{i'}; each is
-// combined with the beam vector and stored at its detector position.
-template <int W>
-__global__ void __launch_bounds__(256) k_interp_pairs(GeomView g, const uint32_t *__restrict__ perm,
-                                                      const uint32_t *__restrict__ start, BinLayout B, Fine F,
-                                                      const float2 *__restrict__ G, int64_t NF, float2 *__restrict__ P) {
-    extern __shared__ float2 tile[];
-    const int bin = blockIdx.x;
-    const uint32_t p0 = start[bin], p1 = start[bin + 1];
-    if (p0 == p1) return;
-    const BinOrigin o = bin_origin(B, bin);
-    const int tsz = (int)B.tile_cells();
-    for (int i = threadIdx.x; i < 3 * tsz; i += blockDim.x) {
-        const int c = i / tsz, cell = i - c * tsz;
-        tile[i] = __ldg(G + c * NF + tile_cell_index(B, o, F, cell));
-    }
-    __syncthreads();
-    for (uint32_t i = p0 + threadIdx.x; i < p1; i += blockDim.x) {
-        PairPos q;
-        pair_positions<W>(g, F, B, o, __ldg(perm + i), q);
-        float w[3][W], u[3][W];
-        float2 v[3], vt[3];
-        if (q.in && q.near) {
-            es_weights<W>(q.d1, F.beta, w[0]);
-            es_weights<W>(q.d2, F.beta, w[1]);
-            es_weights<W>(q.d3, F.beta, w[2]);
-            es_weights<W>(q.e1, F.beta, u[0]);
-            es_weights<W>(q.e2, F.beta, u[1]);
-            es_weights<W>(q.e3, F.beta, u[2]);
-            gather_tile_pair<W, 3>(tile, tsz, B, q.a1, q.a2, q.a3, w, u, v, vt);
-        } else {
-            interp_point_global<W, 3>(G, NF, F, q.x, q.y, q.z, v);
-            interp_point_global<W, 3>(G, NF, F, q.x2, q.y2, q.z2, vt);
-        }
-        forward_store(g, q.p, q.j, q.k, beam_combine(g, q.p, v), P);
-        if (!q.self) {
-            const float2 b = beam_combine(g, q.p, vt);
-            forward_store(g, q.p, q.j2, q.k2, make_float2(b.x, -b.y), P);
-        }
-    }
-}
-
-// sysmat over antipodal pairs, binned (src/gradient.cpp:34-89): a thread per
-// pair gathers both points' 3 components from the input tile (the second as in
-// k_interp_pairs), forms both strengths c_i (sum_k c_k v_k) / (nrows ncols) and
-// stages one pair record; the records are spread into the output tile as the
-// adjoint's are.  The second point's record strength is formed from the gather
-// at x2 itself, without the conjugation: that is the conjugate of its true
-// strength, which is what the pair rule spreads at x2.
-template <int W>
-__global__ void __launch_bounds__(kStageChunk, 1) k_sysmat_pairs(GeomView g, const uint32_t *__restrict__ perm,
-                                                      const uint32_t *__restrict__ start, BinLayout B, Fine F,
-                                                      const float2 *__restrict__ G, float2 *__restrict__ H,
-                                                      int64_t NF, float inv_scale) {
-    extern __shared__ __align__(16) unsigned char psm[];
-    const int bin = blockIdx.x;
-    const uint32_t p0 = start[bin], p1 = start[bin + 1];
-    if (p0 == p1) return;
-    const BinOrigin o = bin_origin(B, bin);
-    const int tsz = (int)B.tile_cells();
-    float2 *gt = reinterpret_cast<float2 *>(psm), *ht = gt + 3 * tsz;
-    PairRec<W, 3> *recs = reinterpret_cast<PairRec<W, 3> *>(psm + pair_rec_offset(tsz, 6));
-    for (int i = threadIdx.x; i < 3 * tsz; i += blockDim.x) {
-        const int c = i / tsz, cell = i - c * tsz;
-        gt[i] = __ldg(G + c * NF + tile_cell_index(B, o, F, cell));
-        ht[i] = make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    __shared__ int wcnt[kStageWarps * kMaxB1];
-    __shared__ int bstart[kMaxB1 + 1];
-    const int t = threadIdx.x;  // one pair per thread (blockDim.x == kStageChunk)
-    for (uint32_t base = p0; base < p1; base += kStageChunk) {
-        const int n = (int)min((uint32_t)kStageChunk, p1 - base);
-        PairPos q;
-        q.in = false;
-        if (t < n) pair_positions<W>(g, F, B, o, __ldg(perm + base + t), q);
-        const int pos = place_slot(t < n && q.in ? q.a1 : -1, wcnt, bstart, B);
-        if (t < n) {
-            float w[3][W], u[3][W];
-            float2 v[3], vt[3];
-            es_weights<W>(q.d1, F.beta, w[0]);
-            es_weights<W>(q.d2, F.beta, w[1]);
-            es_weights<W>(q.d3, F.beta, w[2]);
-            if (q.near) {
-                es_weights<W>(q.e1, F.beta, u[0]);
-                es_weights<W>(q.e2, F.beta, u[1]);
-                es_weights<W>(q.e3, F.beta, u[2]);
-            } else {
-#pragma unroll
-                for (int r = 0; r < W; ++r) u[0][r] = u[1][r] = u[2][r] = 0.f;
-            }
-            if (q.in)
-                gather_tile_pair<W, 3>(gt, tsz, B, q.a1, q.a2, q.a3, w, u, v, vt);
-            else
-                interp_point_global<W, 3>(G, NF, F, q.x, q.y, q.z, v);
-            const bool far2 = !q.in || !q.near;  // second point through global memory
-            if (far2) interp_point_global<W, 3>(G, NF, F, q.x2, q.y2, q.z2, vt);
-            const float c0 = __ldg(g.coeff + q.p), c1 = __ldg(g.coeff + g.nproj + q.p),
-                        c2 = __ldg(g.coeff + 2 * g.nproj + q.p);
-            const float sr = (c0 * v[0].x + c1 * v[1].x + c2 * v[2].x) * inv_scale;
-            const float si = (c0 * v[0].y + c1 * v[1].y + c2 * v[2].y) * inv_scale;
-            float tr = (c0 * vt[0].x + c1 * vt[1].x + c2 * vt[2].x) * inv_scale;
-            float ti = (c0 * vt[0].y + c1 * vt[1].y + c2 * vt[2].y) * inv_scale;
-            if (q.self) tr = ti = 0.f;
-            const float2 sv[3] = {make_float2(c0 * sr, c0 * si), make_float2(c1 * sr, c1 * si),
-                                  make_float2(c2 * sr, c2 * si)};
-            const float2 gv[3] = {make_float2(c0 * tr, c0 * ti), make_float2(c1 * tr, c1 * ti),
-                                  make_float2(c2 * tr, c2 * ti)};
-            if (far2) spread_point_global<W, 3>(H, NF, F, q.x2, q.y2, q.z2, gv);
-            if (q.in) {
-                PairRec<W, 3> &pr = recs[pos];
-#pragma unroll
-                for (int r = 0; r < W; ++r) {
-                    pr.w1[r] = make_float2(w[0][r], u[0][r]);
-                    pr.w2[r] = make_float2(w[1][r], u[1][r]);
-                    pr.w3[r] = make_float2(w[2][r], u[2][r]);
-                }
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    pr.sg[c] = far2 ? make_float4(sv[c].x, sv[c].y, 0.f, 0.f)
-                                    : make_float4(sv[c].x, sv[c].y, gv[c].x, gv[c].y);
-                pr.a = q.a1 | (q.a2 << 8) | (q.a3 << 20);
-            } else {
-                spread_point_global<W, 3>(H, NF, F, q.x, q.y, q.z, sv);
-            }
-        }
-        __syncthreads();
-        spread_pairs_sorted<W, 3>(ht, tsz, B, recs, bstart);
-        __syncthreads();
-    }
-    flush_tile<3>(ht, tsz, B, o, F, H, NF);
-}
-
-// direct (unsorted) sysmat per point, for calls that may not allocate a sorted order:
-// sysmat points: v_k = N2(x_k)(pt), s = sum_k c_k v_k, spread c_i s / (nrows ncols) into H_i
-template <int W>
-__global__ void __launch_bounds__(256) k_sysmat_points(GeomView g, const float2 *__restrict__ G,
-                                                       float2 *__restrict__ H, int64_t NF, Fine F,
-                                                       float inv_scale) {
-    const uint32_t M = (uint32_t)g.nproj * g.nrows * g.ncols;
-    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < M; pid += gridDim.x * blockDim.x) {
-        int p, j, k;
-        decode_pid(pid, g, p, j, k);
-        float x, y, z;
-        point_xyz(g, p, j, k, x, y, z);
-        float2 v[3];
-        interp_point<W, 3>(G, NF, F, x, y, z, v);
-        float c0 = __ldg(g.coeff + p), c1 = __ldg(g.coeff + g.nproj + p), c2 = __ldg(g.coeff + 2 * g.nproj + p);
-        float sr = (c0 * v[0].x + c1 * v[1].x + c2 * v[2].x) * inv_scale;
-        float si = (c0 * v[0].y + c1 * v[1].y + c2 * v[2].y) * inv_scale;
-        float2 s[3] = {make_float2(c0 * sr, c0 * si), make_float2(c1 * sr, c1 * si), make_float2(c2 * sr, c2 * si)};
-        spread_point<W, 3>(H, NF, F, x, y, z, s);
-    }
-}
-
-// projection space: proj = Re(P[ifftshift2 position]) * scale
-__global__ void k_proj_post(const float2 *__restrict__ P, int np, int nr, int nc, float scale,
-                            float *__restrict__ proj) {
-    const int64_t M = (int64_t)np * nr * nc;
-    const int e1 = (nr + 1) / 2, e2 = (nc + 1) / 2;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M; i += (int64_t)gridDim.x * blockDim.x) {
-        int k = (int)(i % nc);
-        int64_t r = i / nc;
-        int j = (int)(r % nr);
-        int64_t p = r / nr;
-        int js = j + e1; if (js >= nr) js -= nr;
-        int ks = k + e2; if (ks >= nc) ks -= nc;
-        proj[i] = P[(p * nr + js) * nc + ks].x * scale;
-    }
-}
-
-// projection space: P = fftshift2(proj) as complex
-__global__ void k_proj_pre(const float *__restrict__ proj, int np, int nr, int nc, float2 *__restrict__ P) {
-    const int64_t M = (int64_t)np * nr * nc;
-    const int d1 = nr / 2, d2 = nc / 2;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M; i += (int64_t)gridDim.x * blockDim.x) {
-        int k = (int)(i % nc);
-        int64_t r = i / nc;
-        int j = (int)(r % nr);
-        int64_t p = r / nr;
-        int js = j + d1; if (js >= nr) js -= nr;
-        int ks = k + d2; if (ks >= nc) ks -= nc;
-        P[i] = make_float2(proj[(p * nr + js) * nc + ks], 0.f);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// host orchestration
-// ---------------------------------------------------------------------------
-
-static Fine fine_of(const NufftPlan &pl) {
-    Fine F;
-    F.nf1 = (int)pl.nf1; F.nf2 = (int)pl.nf2; F.nf3 = (int)pl.nf3;
-    F.s1 = (double)pl.nf1 / (2 * M_PI);
-    F.s2 = (double)pl.nf2 / (2 * M_PI);
-    F.s3 = (double)pl.nf3 / (2 * M_PI);
-    F.beta = pl.beta;
-    return F;
-}
-
-void NufftPlan::pad_real(const float *x3, int ncomp, cudaStream_t s) {
-    Fine F = fine_of(*this);
-    dim3 grid(grid_for(vol.size(), 256), ncomp);
-    k_pad_real<<<grid, 256, 0, s>>>(x3, (int)vol.n1, (int)vol.n2, (int)vol.n3, gin.p, F, ip1.p, ip2.p, ip3.p);
-    LAMINO_LAUNCH("k_pad_real");
-}
-
-void NufftPlan::pad_complex(const float2 *f, cudaStream_t s) {
-    Fine F = fine_of(*this);
-    k_pad_complex<<<grid_for(vol.size(), 256), 256, 0, s>>>(f, (int)vol.n1, (int)vol.n2, (int)vol.n3, gin.p, F,
-                                                              ip1.p, ip2.p, ip3.p);
-    LAMINO_LAUNCH("k_pad_complex");
-}
-
-// sign -1: gin -> gwork (type 2); sign +1: gwork in place (type 1)
-void NufftPlan::fft_fine(int sign, int ncomp, cudaStream_t s) {
-    LAMINO_CUFFT(cufftSetStream(fft3.h, s));
-    for (int c = 0; c < ncomp; ++c) {
-        if (sign < 0)
-            LAMINO_CUFFT(cufftExecC2C(fft3.h, (cufftComplex *)(gin.p + c * nf()),
-                                      (cufftComplex *)(gwork.p + c * nf()), CUFFT_FORWARD));
-        else
-            LAMINO_CUFFT(cufftExecC2C(fft3.h, (cufftComplex *)(gwork.p + c * nf()),
-                                      (cufftComplex *)(gwork.p + c * nf()), CUFFT_INVERSE));
-    }
-}
-
-void NufftPlan::extract_real(float *y3, int ncomp, float scale, bool accumulate, cudaStream_t s) {
-    Fine F = fine_of(*this);
-    dim3 grid(grid_for(vol.size(), 256), ncomp);
-    k_extract_real<<<grid, 256, 0, s>>>(gwork.p, (int)vol.n1, (int)vol.n2, (int)vol.n3, y3, F, ip1.p, ip2.p,
-                                        ip3.p, scale, accumulate ? 1 : 0);
-    LAMINO_LAUNCH("k_extract_real");
-}
-
-void NufftPlan::ensure_proj(const Geom &g, cudaStream_t s) {
-    (void)s;
-    if (g.npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "too many points in one geometry");
-    if ((int64_t)pbuf.n < g.npts()) pbuf.alloc(g.npts());
-    if (f2_np != g.nproj || f2_nr != g.nrows || f2_nc != g.ncols) {
-        int n[2] = {(int)g.nrows, (int)g.ncols};
-        fft2.make(2, n, CUFFT_C2C, (int)g.nproj);
-        f2_np = g.nproj; f2_nr = g.nrows; f2_nc = g.ncols;
-    }
-}
-
-// width as a compile-time constant for a generic lambda
-template <class Fn>
-static void with_width(int w, Fn &&fn) {
-    switch (w) {
-        case 4: fn(std::integral_constant<int, 4>{}); break;
-        case 5: fn(std::integral_constant<int, 5>{}); break;
-        case 6: fn(std::integral_constant<int, 6>{}); break;
-        case 7: fn(std::integral_constant<int, 7>{}); break;
-        case 8: fn(std::integral_constant<int, 8>{}); break;
-        default: throw Error(ERR_ARG, "unsupported kernel width");
-    }
-}
-
-void NufftPlan::set_bins(int b1, int b2, int b3) {
-    if (b1 <= 0 || b2 <= 0 || b3 <= 0) throw Error(ERR_ARG, "bin sizes must be positive");
-    if (b1 > kMaxB1) throw Error(ERR_ARG, "bin extent along n1 must be at most 16");
-    if (b2 > 4095 || b3 > 4095) throw Error(ERR_ARG, "bin extents along n2 and n3 must be below 4096");
-    BinLayout B;
-    B.b1 = b1; B.b2 = b2; B.b3 = b3;
-    B.nb1 = (int)((nf1 + b1 - 1) / b1);
-    B.nb2 = (int)((nf2 + b2 - 1) / b2);
-    B.nb3 = (int)((nf3 + b3 - 1) / b3);
-    B.t1 = b1 + w - 1; B.t2 = b2 + w - 1; B.t3 = b3 + w - 1;
-    auto smem_need = [&](const BinLayout &L) {  // the largest kernel: sysmat, two 3-component tiles
-        return (int64_t)pair_rec_offset(L.tile_cells(), 6) + kStageChunk * (int64_t)pair_rec_bytes(w, 3);
-    };
-    B.r3 = B.t3 + (((w - B.t3) % 16) + 16) % 16;  // conflict-free rows when they fit
-    // 227 KB per CTA, less the binned kernels' static slab-start tables
-    constexpr int64_t kSmemMax = 227 * 1024 - (int64_t)sizeof(int) * (kStageWarps * kMaxB1 + kMaxB1 + 1);
-    if (smem_need(B) > kSmemMax) B.r3 = B.t3;
-    if (B.nbins() > (int64_t)INT32_MAX - 1) throw Error(ERR_ARG, "too many bins");
-    if (smem_need(B) > kSmemMax) throw Error(ERR_ARG, "bin tile too large for shared memory");
-    bins = B;
-    drop_sorted();
-}
-
-const SortedPoints *NufftPlan::find_sorted(const Geom &g, bool paired) const {
-    for (const auto &sp : sorted)
-        if (sp->uid == g.uid && sp->paired == paired) return sp.get();
+const Lattice *NufftPlan::find_lattice(const Geom &g, bool raw) const {
+    for (const auto &l : lats)
+        if (l->uid == g.uid && l->raw == raw) return l.get();
     return nullptr;
 }
 
-const SortedPoints &NufftPlan::sort_points(const Geom &g, cudaStream_t s, bool paired) {
-    for (auto &sp : sorted)
-        if (sp->uid == g.uid && sp->paired == paired) {
-            sp->last_use = ++use_clock;
-            return *sp;
+const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
+    for (auto &l : lats)
+        if (l->uid == g.uid && l->raw == raw) {
+            l->last_use = ++use_clock;
+            return *l;
         }
-    if ((int)sorted.size() >= kMaxSorted) {
+    check_points(g);
+    if ((int)lats.size() >= kMaxLattices) {
         size_t lru = 0;
-        for (size_t i = 1; i < sorted.size(); ++i)
-            if (sorted[i]->last_use < sorted[lru]->last_use) lru = i;
-        sorted.erase(sorted.begin() + (long)lru);
+        for (size_t i = 1; i < lats.size(); ++i)
+            if (lats[i]->last_use < lats[lru]->last_use) lru = i;
+        lats.erase(lats.begin() + (long)lru);
     }
-    if (g.npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "too many points in one geometry");
-    auto sp = std::make_unique<SortedPoints>();
-    sp->uid = g.uid;
-    sp->paired = paired;
-    const int64_t nb = bins.nbins();
-    const int64_t ids = paired ? g.nproj * ((g.nrows * g.ncols + 1) / 2) : g.npts();
-    DevBuf<uint32_t> cnt(nb), cursor(nb);
-    sp->start.alloc(nb + 1);
-    sp->perm.alloc(ids);
-    LAMINO_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes(), s));
+    auto l = std::make_unique<Lattice>();
+    l->uid = g.uid;
+    l->raw = raw;
+    l->cg = g.cg;
+    l->sg = g.sg;
+    // twice the volume's extent along t, in cells over the period 2 pi
+    const double band = vol.n3 * std::fabs(l->sg) + vol.n1 * std::fabs(l->cg);
+    const int nTf = band > w ? 2 * (int)std::ceil(band - 1e-9) : 2 * w;  // (also for a NaN tilt)
+    l->h = 2 * M_PI / nTf;
+    // |T| <= pi up to float rounding: footprints start in [-nTf/2 - w/2, nTf/2 - w/2 + 1)
+    l->T0 = -nTf / 2 - (w + 1) / 2 - 1;
+    l->nT = nTf + w + 4;
+    l->nstart = l->nT - w + 1;
+    const int64_t np = g.nproj, nrow = np * g.nrows, cells = (int64_t)l->nstart * nf2;
+    if (cells > (int64_t)INT32_MAX - 1 || l->nT * g.ncols > (int64_t)INT32_MAX)
+        throw Error(ERR_ARG, "node grid too large");
+    // one allocation for all tables
+    size_t bytes = 0;
+    auto room = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t oX = room(g.ncols * sizeof(double)), oa = room(np * sizeof(float2)), otr = room(g.nrows * sizeof(float4)),
+                 otc = room(g.ncols * sizeof(float4)), oip = room(vol.n1 * vol.n3 * sizeof(float)),
+                 opt = room(nrow * sizeof(int4)), opd = room(nrow * sizeof(float2)),
+                 ost = room((cells + 1) * sizeof(uint32_t)), ocnt = room(cells * sizeof(uint32_t));
+    l->mem.alloc(bytes);
+    char *m0 = l->mem.p;
+    l->X = reinterpret_cast<double *>(m0 + oX);
+    l->a = reinterpret_cast<float2 *>(m0 + oa);
+    l->trow = reinterpret_cast<float4 *>(m0 + otr);
+    l->tcol = reinterpret_cast<float4 *>(m0 + otc);
+    l->ipT = reinterpret_cast<float *>(m0 + oip);
+    l->pt = reinterpret_cast<int4 *>(m0 + opt);
+    l->pd = reinterpret_cast<float2 *>(m0 + opd);
+    l->start = reinterpret_cast<uint32_t *>(m0 + ost);
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(m0 + ocnt);  // counts, then placement cursors
+    const int64_t need = (int64_t)l->nT * nf2 * node_pitch(g.ncols);
+    if ((int64_t)work.n < need) work.alloc(need);
+    LAMINO_CUDA(cudaMemsetAsync(cnt, 0, cells * sizeof(uint32_t), s));
     const Fine F = fine_of(*this);
     const GeomView gv = g.view();
-    const unsigned grid = grid_for(ids, 256, 148LL * 16 * 8);
+    const int64_t m = std::max(std::max(g.ncols, g.nrows), np);
+    k_lat_tables<<<(unsigned)((m + 127) / 128), 128, 0, s>>>(gv, raw, g.offX, g.offY, l->X, l->a, l->trow, l->tcol);
+    LAMINO_LAUNCH("k_lat_tables");
+    const int64_t modes = vol.n1 * vol.n3;
+    k_lat_deconv<<<(unsigned)((modes + 127) / 128), 128, 0, s>>>(quad.p, (int)vol.n1, (int)vol.n3, l->sg, l->cg, w, nTf,
+                                                                 l->ipT);
+    LAMINO_LAUNCH("k_lat_deconv");
+    const double invh = nTf / (2 * M_PI);
+    const unsigned grid_n = grid_for(nrow, 256);
     with_width(w, [&](auto WC) {
         constexpr int W = decltype(WC)::value;
-        auto count = paired ? k_bin_count<W, true> : k_bin_count<W, false>;
-        auto scatter = paired ? k_bin_scatter<W, true> : k_bin_scatter<W, false>;
-        count<<<grid, 256, 0, s>>>(gv, F, bins, cnt.p);
-        LAMINO_LAUNCH("k_bin_count");
-        k_scan_offsets<<<1, 1024, 0, s>>>(cnt.p, (int)nb, sp->start.p, cursor.p);
+        k_rows_count<W><<<grid_n, 256, 0, s>>>(gv, raw, invh, l->T0, l->nstart, F, cnt);
+        LAMINO_LAUNCH("k_rows_count");
+        k_scan_offsets<<<1, 1024, 0, s>>>(cnt, (int)cells, l->start, cnt);
         LAMINO_LAUNCH("k_scan_offsets");
-        scatter<<<grid, 256, 0, s>>>(gv, F, bins, cursor.p, sp->perm.p);
-        LAMINO_LAUNCH("k_bin_scatter");
+        k_rows_place<W><<<grid_n, 256, 0, s>>>(gv, raw, invh, l->T0, l->nstart, F, cnt, l->pt, l->pd);
+        LAMINO_LAUNCH("k_rows_place");
     });
-    sp->last_use = ++use_clock;
-    sorted.push_back(std::move(sp));
-    return *sorted.back();
+    l->last_use = ++use_clock;
+    lats.push_back(std::move(l));
+    return *lats.back();
+}
+
+void NufftPlan::nodes_to_rows(const Lattice &l, const Geom &g, float2 *rows, cudaStream_t s) {
+    const Fine F = fine_of(*this);
+    const LatView L = lat_view(l, g);
+    const int pitch = (int)node_pitch(g.ncols);
+    // y in equal chunks of at most 16; small node grids spread the chunks over CTAs
+    const int nchunk = (int)((nf2 + kNodeY - 1) / kNodeY), ychunk = (int)((nf2 + nchunk - 1) / nchunk);
+    const int ktiles = (int)((g.ncols + kNodeK - 1) / kNodeK);
+    dim3 b1((unsigned)(ktiles * ((l.nT + kNodeT - 1) / kNodeT)));
+    b1.y = (unsigned)std::min<int64_t>(nchunk, std::max<int64_t>(1, 148LL * 12 / b1.x));
+    const uint32_t ydiv = (uint32_t)((0x100000000ULL + ychunk - 1) / ychunk);
+    const int64_t nrow = g.nproj * g.nrows;
+    const int groups = (int)((nrow + kRowGroup - 1) / kRowGroup);
+    const unsigned b2 = (unsigned)(groups * ((g.ncols + 63) / 64));
+    with_width(w, [&](auto WC) {
+        constexpr int W = decltype(WC)::value;
+        k_nodes_gather<W><<<b1, 256, 0, s>>>(L, F, grid.p, work.p, pitch, ktiles, ychunk, ydiv, nchunk);
+        LAMINO_LAUNCH("k_nodes_gather");
+        k_rows_gather<W><<<b2, 256, 0, s>>>(l.pt, l.pd, (int)nrow, work.p, (int)nf2, pitch, (int)g.ncols, groups, beta,
+                                            rows);
+        LAMINO_LAUNCH("k_rows_gather");
+    });
+}
+
+void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *rows, bool symmetric, cudaStream_t s) {
+    const Fine F = fine_of(*this);
+    const LatView L = lat_view(l, g);
+    const int nc = (int)g.ncols;
+    const int kblocks = (nc + 255) / 256, bt = ((nc + kblocks - 1) / kblocks + 31) / 32 * 32;
+    const int ntile = (l.nT + kCell - 1) / kCell;
+    const dim3 b1((unsigned)(ntile * ((nf2 + kCell - 1) / kCell)), (unsigned)((nc + bt - 1) / bt));
+    const int smem1 = bt * (int)(kCell * sizeof(float4) + sizeof(int2) + sizeof(float2));
+    const int yb = (int)std::min<int64_t>(256, (nf2 + 31) / 32 * 32);
+    const int xtiles = (int)((nf3 + kCell - 1) / kCell);
+    const dim3 b2((unsigned)(xtiles * ((nf1 + kCell - 1) / kCell)), (unsigned)((nf2 + yb - 1) / yb));
+    // largest |footprint cell| of the nodes along z and x (a NaN tilt has none)
+    const double Tmax = std::max(-l.T0, l.T0 + l.nT) * l.h;
+    auto reach = [&](double c, double t, double sc) {
+        const double r = sc * (3.1416 * std::fabs(c) + Tmax * std::fabs(t)) + w + 1;
+        return r < 1e9 ? (int)r : 0;
+    };
+    const int reach1 = reach(l.sg, l.cg, F.s1), reach3 = reach(l.cg, l.sg, F.s3);
+    const int smem2 = 2 * yb * (int)(kCell * sizeof(float4) + sizeof(int));
+    const float scale = 1.0f / (float)(g.nrows * g.ncols);
+    with_width(w, [&](auto WC) {
+        constexpr int W = decltype(WC)::value;
+        auto rs = symmetric ? k_rows_spread<W, true> : k_rows_spread<W, false>;
+        rs<<<b1, bt, smem1, s>>>(l.start, l.pt, l.pd, l.nstart, l.nT, ntile, (int)nf2, rows, (int)g.nrows, nc, beta,
+                                 l.a, scale, work.p);
+        LAMINO_LAUNCH("k_rows_spread");
+        k_nodes_spread<W><<<b2, yb, smem2, s>>>(L, F, reach1, reach3, xtiles, work.p, grid.p);
+        LAMINO_LAUNCH("k_nodes_spread");
+    });
 }
 
 namespace {
@@ -1377,8 +1115,7 @@ double NufftPlan::autotune_bins(const std::vector<const Geom *> &gs, int objecti
         std::lock_guard<std::mutex> lk(g_bins_mu);
         auto it = g_bins_cache.find(key);
         if (it != g_bins_cache.end()) {
-            if (it->second[0] != bins.b1 || it->second[1] != bins.b2 || it->second[2] != bins.b3)
-                set_bins(it->second[0], it->second[1], it->second[2]);
+            b1 = it->second[0]; b2 = it->second[1]; b3 = it->second[2];
             return 0.0;
         }
     }
@@ -1394,176 +1131,116 @@ double NufftPlan::autotune_bins(const std::vector<const Geom *> &gs, int objecti
     cudaEvent_t e0, e1;
     LAMINO_CUDA(cudaEventCreate(&e0));
     LAMINO_CUDA(cudaEventCreate(&e1));
-    const std::array<int, 3> cands[] = {{4, 8, 16}, {8, 4, 16}, {4, 4, 16}, {2, 8, 16}, {8, 8, 8}, {4, 4, 8}, {16, 4, 8}};
-    double best = 1e300;
-    std::array<int, 3> bb{bins.b1, bins.b2, bins.b3};
-    for (const auto &c : cands) {
-        try {
-            set_bins(c[0], c[1], c[2]);
-        } catch (const Error &) {
-            continue;
-        }
-        float ms = 0.f;
-        if (objective == 0) {
-            LAMINO_CUDA(cudaEventRecord(e0, s));
-            adjoint(*gs[0], proj.p, y.p, false, s);  // sorts, then spreads
-            LAMINO_CUDA(cudaEventRecord(e1, s));
-        } else {
-            normal(gs, x.p, y.p, s);  // sorts
-            LAMINO_CUDA(cudaEventRecord(e0, s));
-            normal(gs, x.p, y.p, s);
-            LAMINO_CUDA(cudaEventRecord(e1, s));
-        }
-        LAMINO_CUDA(cudaEventSynchronize(e1));
-        LAMINO_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) {
-            best = ms;
-            bb = c;
-        }
-    }
+    float ms = 0.f;
+    LAMINO_CUDA(cudaEventRecord(e0, s));
+    if (objective == 0) adjoint(*gs[0], proj.p, y.p, false, s);
+    else normal(gs, x.p, y.p, s);
+    LAMINO_CUDA(cudaEventRecord(e1, s));
+    LAMINO_CUDA(cudaEventSynchronize(e1));
+    LAMINO_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    set_bins(bb[0], bb[1], bb[2]);
     std::lock_guard<std::mutex> lk(g_bins_mu);
-    g_bins_cache[key] = bb;
-    return best;
+    g_bins_cache[key] = {b1, b2, b3};
+    return ms;
 }
 
 void NufftPlan::forward(const Geom &g, const float *m3, float *proj, cudaStream_t s) {
-    ensure_proj(g, s);
-    const SortedPoints &sp = sort_points(g, s, true);
-    pad_real(m3, 3, s);
-    fft_fine(-1, 3, s);
-    const Fine F = fine_of(*this);
-    const GeomView gv = g.view();
-    const int smem = (int)(3 * bins.tile_cells() * sizeof(float2));
-    with_width(w, [&](auto WC) {
-        constexpr int W = decltype(WC)::value;
-        auto kern = k_interp_pairs<W>;
-        raise_smem_limit((const void *)kern, smem);
-        kern<<<(unsigned)bins.nbins(), 256, smem, s>>>(gv, sp.perm.p, sp.start.p, bins, F, gwork.p, nf(), pbuf.p);
-        LAMINO_LAUNCH("k_interp_pairs");
-    });
+    ensure_proj(g);
+    const Lattice &l = lattice(g, false, s);
+    pad_real(m3, l.sg, l.cg, l.ipT, s);
+    fft_fine(grid.p, -1, s);
+    nodes_to_rows(l, g, pbuf.p, s);
     LAMINO_CUFFT(cufftSetStream(fft2.h, s));
     LAMINO_CUFFT(cufftExecC2C(fft2.h, (cufftComplex *)pbuf.p, (cufftComplex *)pbuf.p, CUFFT_INVERSE));
-    float scale = 1.0f / (float)(g.nrows * g.ncols);
-    k_proj_post<<<grid_for(g.npts(), 256), 256, 0, s>>>(pbuf.p, (int)g.nproj, (int)g.nrows, (int)g.ncols, scale, proj);
+    const int64_t nrow = g.nproj * g.nrows;
+    k_proj_post<<<(unsigned)std::min<int64_t>(nrow, 148 * 64), 256, 0, s>>>(
+        pbuf.p, nrow, (int)g.nrows, (int)g.ncols, l.trow, l.tcol, l.a, 1.0f / (float)(g.nrows * g.ncols), proj);
     LAMINO_LAUNCH("k_proj_post");
 }
 
 void NufftPlan::adjoint(const Geom &g, const float *proj, float *m3, bool accumulate, cudaStream_t s) {
-    ensure_proj(g, s);
-    const SortedPoints &sp = sort_points(g, s, true);
-    k_proj_pre<<<grid_for(g.npts(), 256), 256, 0, s>>>(proj, (int)g.nproj, (int)g.nrows, (int)g.ncols, pbuf.p);
+    ensure_proj(g);
+    const Lattice &l = lattice(g, false, s);
+    const int64_t nrow = g.nproj * g.nrows;
+    k_proj_pre<<<(unsigned)std::min<int64_t>(nrow, 148 * 64), 256, 0, s>>>(proj, nrow, (int)g.nrows, (int)g.ncols, l.trow,
+                                                                          l.tcol, l.a, pbuf.p);
     LAMINO_LAUNCH("k_proj_pre");
     LAMINO_CUFFT(cufftSetStream(fft2.h, s));
     LAMINO_CUFFT(cufftExecC2C(fft2.h, (cufftComplex *)pbuf.p, (cufftComplex *)pbuf.p, CUFFT_FORWARD));
-    LAMINO_CUDA(cudaMemsetAsync(gwork.p, 0, gwork.bytes(), s));
-    const Fine F = fine_of(*this);
-    const GeomView gv = g.view();
-    const int smem = (int)(pair_rec_offset(bins.tile_cells(), 3) + kStagePairs * pair_rec_bytes(w, 3));
-    with_width(w, [&](auto WC) {
-        constexpr int W = decltype(WC)::value;
-        auto kern = k_spread_pairs<W>;
-        raise_smem_limit((const void *)kern, smem);
-        kern<<<(unsigned)bins.nbins(), kStageChunk, smem, s>>>(gv, sp.perm.p, sp.start.p, bins, F, gwork.p, nf(),
-                                                                pbuf.p);
-        LAMINO_LAUNCH("k_spread_pairs");
-    });
-    fft_fine(+1, 3, s);
-    extract_real(m3, 3, 1.0f / (float)(g.nrows * g.ncols), accumulate, s);
+    rows_to_nodes(l, g, pbuf.p, false, s);
+    fft_fine(grid.p, +1, s);
+    extract_real(m3, l.sg, l.cg, l.ipT, 1.0f / (float)(g.nrows * g.ncols), accumulate, s);
 }
 
-// sysmat of every geometry, accumulated into gin after the forward FFT of x;
-// `may_sort`: build missing point orders (allocates) or fall back to the direct kernel
-void NufftPlan::normal_points(const Geom *const *gs, int ng, bool may_sort, cudaStream_t s) {
-    const Fine F = fine_of(*this);
-    const int smem = (int)(pair_rec_offset(bins.tile_cells(), 6) + kStageChunk * pair_rec_bytes(w, 3));
-    for (int i = 0; i < ng; ++i) {
-        const Geom &g = *gs[i];
-        if (g.npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "too many points in one geometry");
-        const GeomView gv = g.view();
-        const float inv_scale = 1.0f / (float)(g.nrows * g.ncols);
-        const SortedPoints *sp = may_sort ? &sort_points(g, s, true) : find_sorted(g, true);
-        with_width(w, [&](auto WC) {
-            constexpr int W = decltype(WC)::value;
-            if (sp) {
-                auto kern = k_sysmat_pairs<W>;
-                raise_smem_limit((const void *)kern, smem);
-                kern<<<(unsigned)bins.nbins(), kStageChunk, smem, s>>>(gv, sp->perm.p, sp->start.p, bins, F, gwork.p,
-                                                                        gin.p, nf(), inv_scale);
-                LAMINO_LAUNCH("k_sysmat_pairs");
-            } else {
-                unsigned grid = grid_for(g.npts(), 256, 148LL * 16 * 8);
-                k_sysmat_points<W><<<grid, 256, 0, s>>>(gv, gwork.p, gin.p, nf(), F, inv_scale);
-                LAMINO_LAUNCH("k_sysmat_points");
-            }
-        });
+// one geometry's sysmat, (+)= into y3: over its lattice, or point by point without one
+void NufftPlan::normal_one(const Geom &g, const Lattice *l, const float *x3, float *y3, bool accumulate,
+                           cudaStream_t s) {
+    const double sg = l ? l->sg : (double)g.sg, cg = l ? l->cg : (double)g.cg;
+    const float *ipT = l ? l->ipT : nullptr;
+    pad_real(x3, sg, cg, ipT, s);
+    fft_fine(grid.p, -1, s);
+    if (l) {
+        nodes_to_rows(*l, g, pbuf.p, s);
+        rows_to_nodes(*l, g, pbuf.p, true, s);
+        fft_fine(grid.p, +1, s);
+        extract_real(y3, sg, cg, ipT, 1.0f, accumulate, s);
+        return;
     }
+    LAMINO_CUDA(cudaMemsetAsync(work.p, 0, nf() * sizeof(float2), s));
+    const Fine F = fine_of(*this);
+    with_width(w, [&](auto WC) {
+        constexpr int W = decltype(WC)::value;
+        k_sysmat_points<W><<<grid_for(g.npts(), 256, 148LL * 16 * 8), 256, 0, s>>>(
+            g.view(), grid.p, work.p, F, 1.0f / (float)(g.nrows * g.ncols));
+        LAMINO_LAUNCH("k_sysmat_points");
+    });
+    LAMINO_CUDA(cudaMemcpyAsync(grid.p, work.p, nf() * sizeof(float2), cudaMemcpyDeviceToDevice, s));
+    fft_fine(grid.p, +1, s);
+    extract_real(y3, sg, cg, nullptr, 1.0f, accumulate, s);
 }
 
 void NufftPlan::normal(const std::vector<const Geom *> &gs, const float *x3, float *y3, cudaStream_t s) {
     if (gs.empty()) throw Error(ERR_ARG, "normal operator needs at least one geometry");
-    for (const Geom *g : gs) sort_points(*g, s, true);  // before any work on the grids
-    normal_impl(gs.data(), (int)gs.size(), true, x3, y3, s);
+    for (const Geom *g : gs) {
+        if (!g) throw Error(ERR_ARG, "bad geometry");
+        check_points(*g);
+        if ((int64_t)pbuf.n < g->npts()) pbuf.alloc(g->npts());
+    }
+    for (const Geom *g : gs) lattice(*g, false, s);
+    for (size_t i = 0; i < gs.size(); ++i) normal_one(*gs[i], &lattice(*gs[i], false, s), x3, y3, i > 0, s);
 }
 
 void NufftPlan::normal_ptrs(const Geom *const *gs, int ng, const float *x3, float *y3, cudaStream_t s) {
     if (!gs || ng <= 0) throw Error(ERR_ARG, "normal operator needs at least one geometry");
-    normal_impl(gs, ng, false, x3, y3, s);
-}
-
-void NufftPlan::normal_impl(const Geom *const *gs, int ng, bool may_sort, const float *x3, float *y3,
-                            cudaStream_t s) {
     for (int i = 0; i < ng; ++i)
         if (!gs[i] || gs[i]->npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "bad geometry");
-    pad_real(x3, 3, s);
-    // forward fine-grid spectra go to gwork; the spread accumulates in gin (zeroed after its FFT)
-    fft_fine(-1, 3, s);
-    LAMINO_CUDA(cudaMemsetAsync(gin.p, 0, gin.bytes(), s));
-    normal_points(gs, ng, may_sort, s);
-    LAMINO_CUFFT(cufftSetStream(fft3.h, s));
-    for (int c = 0; c < 3; ++c)
-        LAMINO_CUFFT(cufftExecC2C(fft3.h, (cufftComplex *)(gin.p + c * nf()),
-                                  (cufftComplex *)(gwork.p + c * nf()), CUFFT_INVERSE));
-    extract_real(y3, 3, 1.0f, false, s);
-    LAMINO_CUDA(cudaMemsetAsync(gin.p, 0, gin.bytes(), s));
+    for (int i = 0; i < ng; ++i) {
+        const Lattice *l = find_lattice(*gs[i], false);
+        if (l && (int64_t)pbuf.n < gs[i]->npts()) l = nullptr;  // no row buffer from an earlier call
+        normal_one(*gs[i], l, x3, y3, i > 0, s);
+    }
 }
 
 void NufftPlan::type2(const Geom &g, const float2 *modes, float2 *c, cudaStream_t s) {
-    const SortedPoints &sp = sort_points(g, s);
-    pad_complex(modes, s);
-    fft_fine(-1, 1, s);
-    const Fine F = fine_of(*this);
-    const GeomView gv = g.view();
-    const int smem = (int)(bins.tile_cells() * sizeof(float2));
-    with_width(w, [&](auto WC) {
-        constexpr int W = decltype(WC)::value;
-        auto kern = k_interp_binned<W, 1, RawSink>;
-        raise_smem_limit((const void *)kern, smem);
-        kern<<<(unsigned)bins.nbins(), 256, smem, s>>>(gv, sp.perm.p, sp.start.p, bins, F, gwork.p, nf(), RawSink{c});
-        LAMINO_LAUNCH("k_interp_binned<raw>");
-    });
+    const Lattice &l = lattice(g, true, s);
+    LAMINO_CUDA(cudaMemsetAsync(grid.p, 0, nf() * sizeof(float2), s));
+    const unsigned b = volume_tiles(vol);
+    k_pad<true><<<b, 256, 0, s>>>(nullptr, modes, (int)vol.n1, (int)vol.n2, (int)vol.n3, 0.f, 0.f, grid.p, fine_of(*this),
+                                  ip1.p, ip2.p, ip3.p, l.ipT);
+    LAMINO_LAUNCH("k_pad");
+    fft_fine(grid.p, -1, s);
+    nodes_to_rows(l, g, c, s);
 }
 
 void NufftPlan::type1(const Geom &g, const float2 *c, float2 *modes, cudaStream_t s) {
-    const SortedPoints &sp = sort_points(g, s);
-    LAMINO_CUDA(cudaMemsetAsync(gwork.p, 0, nf() * sizeof(float2), s));
-    const Fine F = fine_of(*this);
-    const GeomView gv = g.view();
-    const int smem = (int)(bins.tile_cells() * sizeof(float2) + kStageChunk * point_rec_bytes(w, 1));
-    with_width(w, [&](auto WC) {
-        constexpr int W = decltype(WC)::value;
-        auto kern = k_spread_binned<W, 1, RawStrength>;
-        raise_smem_limit((const void *)kern, smem);
-        kern<<<(unsigned)bins.nbins(), kStageChunk, smem, s>>>(gv, sp.perm.p, sp.start.p, bins, F, gwork.p, nf(),
-                                                                RawStrength{c});
-        LAMINO_LAUNCH("k_spread_binned<raw>");
-    });
-    fft_fine(+1, 1, s);
-    k_extract_complex<<<grid_for(vol.size(), 256), 256, 0, s>>>(gwork.p, (int)vol.n1, (int)vol.n2, (int)vol.n3,
-                                                                  modes, F, ip1.p, ip2.p, ip3.p);
-    LAMINO_LAUNCH("k_extract_complex");
+    const Lattice &l = lattice(g, true, s);
+    rows_to_nodes(l, g, c, false, s);
+    fft_fine(grid.p, +1, s);
+    const unsigned b = volume_tiles(vol);
+    k_extract<true><<<b, 256, 0, s>>>(grid.p, (int)vol.n1, (int)vol.n2, (int)vol.n3, 0.f, 0.f, nullptr, modes,
+                                      fine_of(*this), ip1.p, ip2.p, ip3.p, l.ipT, 1.0f, 0);
+    LAMINO_LAUNCH("k_extract");
 }
 
 }  // namespace lamino

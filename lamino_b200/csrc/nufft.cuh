@@ -18,27 +18,28 @@ inline int es_width(double eps) {
 }
 int64_t next_smooth_even(int64_t n);
 
-// Partition of the fine grid into bins of b1 x b2 x b3 cells.  A point belongs
-// to the bin holding the first cell of its kernel footprint, so its w^3 taps
-// stay inside the bin's tile of (b + w - 1) cells per dimension, which one CTA
-// stages in shared memory.  Tile rows are r3 >= t3 cells apart with
-// r3 = w (mod 16): the w x w (t2, t3) taps that consecutive lanes take then fall
-// in distinct shared-memory banks.
-struct BinLayout {
-    int b1 = 8, b2 = 8, b3 = 8;
-    int nb1 = 0, nb2 = 0, nb3 = 0;
-    int t1 = 0, t2 = 0, t3 = 0, r3 = 0;
-    __host__ __device__ int64_t nbins() const { return (int64_t)nb1 * nb2 * nb3; }
-    __host__ __device__ int64_t tile_cells() const { return (int64_t)t1 * t2 * r3; }
-};
-
-// Point ids of one geometry grouped by bin (counting sort), with bin offsets.
-struct SortedPoints {
+// The points of one geometry as a lattice (see nufft.cu): every point is
+// X a(gamma) + (T, y)(theta, Y), X a column frequency, T = Y cos(theta) the
+// coordinate along the tilted axis normal to a and y.  The plane of columns and
+// T lines is a regular grid of nodes (nT lines, spacing h, first line T0); the
+// (T, y) positions of the detector rows are kept sorted by the grid cell their
+// kernel footprint starts in.
+struct Lattice {
     uint64_t uid = 0;
-    bool paired = false;     // ids of antipodal pairs (the adjoint), else of points
+    bool raw = false;        // the float frequencies as they are (raw transforms), else
+                             // their antisymmetric part (forward, adjoint, sysmat)
     uint64_t last_use = 0;
-    DevBuf<uint32_t> perm;   // npts
-    DevBuf<uint32_t> start;  // nbins + 1
+    double cg = 1, sg = 0, h = 0;
+    int nT = 0, T0 = 0;
+    int nstart = 0;          // footprint starts along T: nT - w + 1
+    DevBuf<char> mem;        // holds the tables below
+    double *X = nullptr;     // column frequencies
+    float *ipT = nullptr;    // 1 / p_T of every mode (k1, k3): deconvolution along T
+    float2 *a = nullptr;     // (sin - i cos) / 2 of every angle
+    float4 *trow = nullptr, *tcol = nullptr;  // twist factors of the projection-space transform
+    int4 *pt = nullptr;      // rows sorted by cell: row id (angle, detector row), T start, y start, angle
+    float2 *pd = nullptr;    // offsets of the T and y footprints from the row's position
+    uint32_t *start = nullptr;  // first row of each (y start, T start) cell
 };
 
 struct NufftPlan {
@@ -48,35 +49,33 @@ struct NufftPlan {
     float beta = 16.1f;
     double eps = 1.2e-6;
     DevBuf<float> ip1, ip2, ip3;   // 1 / p(k) per mode index along each dim
-    DevBuf<float2> gin;            // 3 fine grids: deconvolved modes (zero elsewhere)
-    DevBuf<float2> gwork;          // 3 fine grids: FFT outputs / spread accumulators
-    FftPlan fft3;                  // batched 3 x C2C 3-D on the fine grid
+    DevBuf<double2> quad;          // quadrature of the kernel's transform (node, weight x kernel)
+    DevBuf<float2> grid;           // fine grid [nf1][nf3][nf2] (n2 fastest)
+    DevBuf<float2> work;           // node grid, or the direct form's second fine grid
+    FftPlan fft3;                  // C2C 3-D on the fine grid
     // projection-space workspace (largest geometry seen), with its 2-D plan
     DevBuf<float2> pbuf;
     FftPlan fft2;
     int64_t f2_np = -1, f2_nr = -1, f2_nc = -1;
-    // bin-sorted point orders of the geometries used with this plan (bounded LRU)
-    BinLayout bins;
-    std::vector<std::unique_ptr<SortedPoints>> sorted;
+    // lattices of the geometries used with this plan (bounded LRU)
+    std::vector<std::unique_ptr<Lattice>> lats;
     uint64_t use_clock = 0;
-    static constexpr int kMaxSorted = 16;
+    static constexpr int kMaxLattices = 16;
+    int b1 = 4, b2 = 8, b3 = 16;   // bin layout of lamino_plan_set_bins (a hint, see set_bins)
 
     NufftPlan(Dims3 d, double eps);
     int64_t nf() const { return nf1 * nf2 * nf3; }
-    void ensure_proj(const Geom &g, cudaStream_t s);
-    // bin layout for b1 x b2 x b3 bins (drops cached point orders)
+    void ensure_proj(const Geom &g);
+    // accepts the layouts that a tile of (b + w - 1)^3 cells in shared memory
+    // allows; the lattice transforms choose their own tiles
     void set_bins(int b1, int b2, int b3);
-    // the geometry's bin-sorted order of points, or of antipodal point pairs
-    // (built on first use, then cached)
-    const SortedPoints &sort_points(const Geom &g, cudaStream_t s, bool paired = false);
-    const SortedPoints *find_sorted(const Geom &g, bool paired = false) const;
-    // time candidate bin layouts and keep the fastest for objective 0 (adjoint of
-    // the first geometry, including its sort: a setup pass) or 1 (the sum over
-    // the geometries of sysmat, sorted orders reused: a solver's operator);
-    // cached per (fine grid, width, objective, points) for the process.  Returns
-    // the best time in ms (0 when taken from the cache).
+    // the geometry's lattice (built on first use, then cached) with the node grid allocated
+    const Lattice &lattice(const Geom &g, bool raw, cudaStream_t s);
+    const Lattice *find_lattice(const Geom &g, bool raw) const;
+    // one pass of the adjoint (objective 0) or of the sum over the geometries of
+    // sysmat (objective 1) timed; cached per (fine grid, width, objective, points)
+    // for the process.  Returns its time in ms (0 when taken from the cache).
     double autotune_bins(const std::vector<const Geom *> &gs, int objective, cudaStream_t s);
-    void drop_sorted() { sorted.clear(); }
 
     // --- operators (device pointers; volumes are 3 contiguous components) ---
     // forward projection (src/projection.cpp:42-77)
@@ -85,19 +84,21 @@ struct NufftPlan {
     void adjoint(const Geom &g, const float *proj, float *m3, bool accumulate, cudaStream_t s);
     // sum over geometries of sysmat (src/gradient.cpp:34-89), NUFFT form
     void normal(const std::vector<const Geom *> &gs, const float *x3, float *y3, cudaStream_t s);
-    // same sum over geometries given as a pointer array (no host containers)
+    // same sum over geometries given as a pointer array, without any allocation
+    // (geometries whose lattice is not cached take the direct point kernel)
     void normal_ptrs(const Geom *const *gs, int ng, const float *x3, float *y3, cudaStream_t s);
     // raw transforms on one geometry (FINUFFT-level boundary, complex data)
     void type2(const Geom &g, const float2 *modes, float2 *c, cudaStream_t s);
     void type1(const Geom &g, const float2 *c, float2 *modes, cudaStream_t s);
 
     // internals
-    void normal_impl(const Geom *const *gs, int ng, bool may_sort, const float *x3, float *y3, cudaStream_t s);
-    void normal_points(const Geom *const *gs, int ng, bool may_sort, cudaStream_t s);
-    void pad_real(const float *x3, int ncomp, cudaStream_t s);
-    void pad_complex(const float2 *f, cudaStream_t s);
-    void fft_fine(int sign, int ncomp, cudaStream_t s);
-    void extract_real(float *y3, int ncomp, float scale, bool accumulate, cudaStream_t s);
+    void normal_one(const Geom &g, const Lattice *lat, const float *x3, float *y3, bool accumulate, cudaStream_t s);
+    void pad_real(const float *x3, double sg, double cg, const float *ipT, cudaStream_t s);
+    void extract_real(float *y3, double sg, double cg, const float *ipT, float scale, bool accumulate, cudaStream_t s);
+    void fft_fine(float2 *g, int sign, cudaStream_t s);
+    void nodes_to_rows(const Lattice &lat, const Geom &g, float2 *rows, cudaStream_t s);   // grid -> nodes -> rows
+    void rows_to_nodes(const Lattice &lat, const Geom &g, const float2 *rows, bool symmetric, cudaStream_t s);
+    int64_t node_pitch(int64_t ncols) const { return (ncols + 3) / 4 * 4; }
 };
 
 }  // namespace lamino
