@@ -26,10 +26,10 @@
 // 3.0e8 node values and 49 for 5.5e8 points, all of it contiguous along y or X,
 // in place of 343 taps per point from scattered tiles.
 // Measured on B200 against antipodal point pairs spread through 3-D tiles (the
-// form before): adjoint at that size 333.6 -> 38.2 ms, forward of 181 x 362^2
-// points from 362 x 44 x 362 19.5 -> 3.4 ms, sysmat of 2 x 91 x 309^2 points on
-// 180 x 16 x 180 20.3 -> 2.05 ms, and no sort of the points on the first call
-// (adjoint of a new geometry 346 -> 42 ms).
+// form before): adjoint at that size 333.5 -> 36.7 ms, forward of 181 x 362^2
+// points from 362 x 44 x 362 19.5 -> 2.9 ms, sysmat of 2 x 91 x 309^2 points on
+// 180 x 16 x 180 19.9 -> 1.29 ms, and no sort of the points on the first call
+// (adjoint of a new geometry 351 -> 41 ms).
 //
 // The three components need one complex transform, not three.  The beam vector
 // (sin g sin th, cos th, cos g sin th) spans two dimensions:
@@ -372,78 +372,173 @@ __device__ __forceinline__ void node_pos(const LatView &L, const Fine &F, int t,
     l1 = es_first<W>(T * L.cg - X * L.sg, F.s1, d1);
 }
 
-// Fine grid -> nodes.  A CTA owns 16 columns x 8 T lines; the threads of a
-// y chunk take (node, y) pairs with y fastest, so a tap is one contiguous read
-// of up to 16 y values (128 B) and neighbouring nodes find each other's taps in
-// L1.  Results go through shared memory to the node grid [T][y][X], X fastest.
-constexpr int kNodeK = 16, kNodeT = 8, kNodes = kNodeK * kNodeT, kNodeY = 16;
-template <int W>
-__global__ void __launch_bounds__(256) k_nodes_gather(LatView L, Fine F, const float2 *__restrict__ g, float2 *__restrict__ G,
-                                                      int pitch, int ktiles, int ychunk, uint32_t ydiv,
-                                                      int nchunk) {
-    __shared__ float w1[W][kNodes], w3[W][kNodes];
-    __shared__ int o1[W][kNodes], o3[W][kNodes];
-    __shared__ float2 st[kNodeY][kNodes + 1];
+// Fine grid -> nodes.  A CTA owns 128 nodes (16 columns x 8 T lines, or 8 x 16).
+// Per chunk of up to 16 y it stages the (z, x) box of cells that the nodes'
+// footprints cover in shared memory; a thread then takes two nodes, one T line
+// apart, and two y: the lattice keeps T lines at most one cell apart, so both
+// footprints lie in (W + 1)^2 cells, each read once (16 bytes) and weighted for
+// both nodes with the weights padded by zeros.  Results go through shared memory
+// to the node grid [T][y][X], X fastest.  Bound by shared-memory wavefronts:
+// 64 16-byte reads per four values where one node and one y at a time takes 196
+// of 8 bytes.  A box that does not fit (a detector far coarser than the fine
+// grid) is read from global memory tap by tap.
+// Measured (before: every tap from global memory, one node and one y per lane,
+// five wavefronts per tap where runs straddle lines): 362 x 1020 nodes x 90 y
+// 1314 -> 857 us; staging through registers instead of asynchronous copies 1267 us.
+constexpr int kNodes = 128, kNodeY = 16;
+__device__ __forceinline__ void copy16_async(void *smem, const void *global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global) : "memory");
+}
+template <int W, int kNodeK>
+__global__ void __launch_bounds__(256, 2) k_nodes_gather(LatView L, Fine F, const float2 *__restrict__ g,
+                                                         float2 *__restrict__ G, int pitch, int ktiles, int ychunk,
+                                                         uint32_t ydiv, int nchunk, int boxcap) {
+    constexpr int kNodeT = kNodes / kNodeK, kPairs = kNodes / 2;
+    extern __shared__ __align__(16) float2 box[];  // [cell][ychunk]; then the results [y][node], kNodes + 1 apart
+    __shared__ float w1[W + 2][kNodes], w3[W + 2][kNodes];  // weights between two zeros
+    __shared__ int n1[kNodes], n3[kNodes];
+    __shared__ int lo1, hi1, lo3, hi3;
     const int t0 = blockIdx.x / ktiles, k0 = (blockIdx.x - t0 * ktiles) * kNodeK;
     const int tid = threadIdx.x;
+    if (tid == 0) {
+        lo1 = lo3 = 0x7fffffff;
+        hi1 = hi3 = -0x7fffffff;
+    }
+    __syncthreads();
     {
         // threads 0..127 the z side of a node, 128..255 the x side
         const int n = tid & (kNodes - 1);
-        const int k = min(k0 + (n & (kNodeK - 1)), L.nc - 1), t = min(t0 * kNodeT + n / kNodeK, L.nT - 1);
+        const int k = min(k0 + n % kNodeK, L.nc - 1), t = min(t0 * kNodeT + n / kNodeK, L.nT - 1);
         int l1, l3;
         float d1, d3;
         node_pos<W>(L, F, t, k, l1, l3, d1, d3);
-        if (tid < kNodes) {
-            l1 = wrap(l1, F.nf1);
+        const bool z = tid < kNodes;
+        const int l = z ? l1 : l3;
+        (z ? n1 : n3)[n] = l;
+        atomicMin(z ? &lo1 : &lo3, __reduce_min_sync(0xffffffffu, l));
+        atomicMax(z ? &hi1 : &hi3, __reduce_max_sync(0xffffffffu, l));
+        float(*wt)[kNodes] = z ? w1 : w3;
+        wt[0][n] = wt[W + 1][n] = 0.f;
 #pragma unroll
-            for (int r = 0; r < W; ++r) {
-                int i = l1 + r; if (i >= F.nf1) i -= F.nf1;
-                o1[r][n] = i * F.nf3 * F.nf2;
-                w1[r][n] = es_weight<W>(d1, r, F.beta);
-            }
-        } else {
-            l3 = wrap(l3, F.nf3);
-#pragma unroll
-            for (int r = 0; r < W; ++r) {
-                int i = l3 + r; if (i >= F.nf3) i -= F.nf3;
-                o3[r][n] = i * F.nf2;
-                w3[r][n] = es_weight<W>(d3, r, F.beta);
-            }
-        }
+        for (int r = 0; r < W; ++r) wt[r + 1][n] = es_weight<W>(z ? d1 : d3, r, F.beta);
     }
+    __syncthreads();
+    const int B1 = hi1 - lo1 + W + 1, B3 = hi3 - lo3 + W + 1;
+    const int base1 = wrap(lo1, F.nf1), base3 = wrap(lo3, F.nf3);
+    const bool staged = (int64_t)B1 * B3 <= boxcap;
+    const int half = ychunk / 2;
     for (int c = blockIdx.y; c < nchunk; c += gridDim.y) {
         const int y0 = c * ychunk, ny = min(ychunk, F.nf2 - y0);
-        __syncthreads();
-        for (int e = tid; e < kNodes * ychunk; e += 256) {
-            const int n = (int)__umulhi((uint32_t)e, ydiv), y = e - n * ychunk;
-            if (y >= ny) continue;
-            const float2 *p = g + y0 + y;
-            float v3[W];
-            int q3[W];
-#pragma unroll
-            for (int r = 0; r < W; ++r) {
-                v3[r] = w3[r][n];
-                q3[r] = o3[r][n];
+        if (staged) {
+            // eight lanes per cell, two y per load (y0 and nf2 are even); 32 cells a pass
+            const int y = 2 * (tid & 7);
+            int r1 = 0, r3 = tid >> 3;
+            while (r3 >= B3) { r3 -= B3; ++r1; }
+            while (r1 < B1) {
+                int i1 = base1 + r1, i3 = base3 + r3;
+                while (i1 >= F.nf1) i1 -= F.nf1;
+                while (i3 >= F.nf3) i3 -= F.nf3;
+                if (y < ny) copy16_async(box + (r1 * B3 + r3) * ychunk + y, g + ((int64_t)i1 * F.nf3 + i3) * F.nf2 + y0 + y);
+                r3 += 32;
+                while (r3 >= B3) { r3 -= B3; ++r1; }
             }
-            float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int r1 = 0; r1 < W; ++r1) {
-                const float2 *row = p + o1[r1][n];
-                const float u = w1[r1][n];
-                float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int r3 = 0; r3 < W; ++r3) s = __ffma2_rn(make_float2(v3[r3], v3[r3]), __ldg(row + q3[r3]), s);
-                acc = __ffma2_rn(make_float2(u, u), s, acc);
-            }
-            st[y][n] = acc;
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        // (pair, y pair) items, at most two per thread; kept until the box is free
+        float4 va[2], vb[2];
+        int where[2];
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+            const int e = tid + 256 * it;
+            const int q = (int)__umulhi((uint32_t)e, ydiv), y = 2 * (e - q * half);
+            where[it] = -1;
+            if (q >= kPairs || y >= ny) continue;
+            const int a = q / kNodeK * 2 * kNodeK + q % kNodeK, b = a + kNodeK;  // nodes of the pair
+            where[it] = y * (kNodes + 1) + a;
+            float2 a0 = make_float2(0.f, 0.f), a1 = a0, b0 = a0, b1 = a0;
+            if (staged) {
+                const int s1 = min(n1[a], n1[b]), s3 = min(n3[a], n3[b]);
+                const float *wa1 = &w1[1 - (n1[a] - s1)][a], *wb1 = &w1[1 - (n1[b] - s1)][b];
+                const float *wa3 = &w3[1 - (n3[a] - s3)][a], *wb3 = &w3[1 - (n3[b] - s3)][b];
+                const float2 *p = box + ((s1 - lo1) * B3 + s3 - lo3) * ychunk + y;
+                float ua[W + 1], ub[W + 1];
+#pragma unroll
+                for (int r = 0; r <= W; ++r) {
+                    ua[r] = wa3[r * kNodes];
+                    ub[r] = wb3[r * kNodes];
+                }
+#pragma unroll
+                for (int r1 = 0; r1 <= W; ++r1) {
+                    const float2 *row = p + r1 * B3 * ychunk;
+                    float2 sa0 = make_float2(0.f, 0.f), sa1 = sa0, sb0 = sa0, sb1 = sa0;
+#pragma unroll
+                    for (int r3 = 0; r3 <= W; ++r3) {
+                        const float4 v = *reinterpret_cast<const float4 *>(row + r3 * ychunk);
+                        const float2 x = make_float2(v.x, v.y), z = make_float2(v.z, v.w);
+                        const float2 wa = make_float2(ua[r3], ua[r3]), wb = make_float2(ub[r3], ub[r3]);
+                        sa0 = __ffma2_rn(wa, x, sa0);
+                        sa1 = __ffma2_rn(wa, z, sa1);
+                        sb0 = __ffma2_rn(wb, x, sb0);
+                        sb1 = __ffma2_rn(wb, z, sb1);
+                    }
+                    const float fa = wa1[r1 * kNodes], fb = wb1[r1 * kNodes];
+                    a0 = __ffma2_rn(make_float2(fa, fa), sa0, a0);
+                    a1 = __ffma2_rn(make_float2(fa, fa), sa1, a1);
+                    b0 = __ffma2_rn(make_float2(fb, fb), sb0, b0);
+                    b1 = __ffma2_rn(make_float2(fb, fb), sb1, b1);
+                }
+            } else {
+                for (int m = 0; m < 2; ++m) {
+                    const int n = m ? b : a, l1 = wrap(n1[n], F.nf1), l3 = wrap(n3[n], F.nf3);
+                    float2 c0 = make_float2(0.f, 0.f), c1 = c0;
+                    for (int r1 = 0; r1 < W; ++r1) {
+                        int i1 = l1 + r1; if (i1 >= F.nf1) i1 -= F.nf1;
+                        const float2 *row = g + (int64_t)i1 * F.nf3 * F.nf2 + y0 + y;
+                        for (int r3 = 0; r3 < W; ++r3) {
+                            int i3 = l3 + r3; if (i3 >= F.nf3) i3 -= F.nf3;
+                            const float t = w1[r1 + 1][n] * w3[r3 + 1][n];
+                            const float4 v = __ldg(reinterpret_cast<const float4 *>(row + (int64_t)i3 * F.nf2));
+                            c0 = __ffma2_rn(make_float2(t, t), make_float2(v.x, v.y), c0);
+                            c1 = __ffma2_rn(make_float2(t, t), make_float2(v.z, v.w), c1);
+                        }
+                    }
+                    if (m) { b0 = c0; b1 = c1; } else { a0 = c0; a1 = c1; }
+                }
+            }
+            va[it] = make_float4(a0.x, a0.y, a1.x, a1.y);
+            vb[it] = make_float4(b0.x, b0.y, b1.x, b1.y);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < 2; ++it)
+            if (where[it] >= 0) {
+                float2 *o = box + where[it];
+                o[0] = make_float2(va[it].x, va[it].y);
+                o[kNodeK] = make_float2(vb[it].x, vb[it].y);
+                o[kNodes + 1] = make_float2(va[it].z, va[it].w);
+                o[kNodes + 1 + kNodeK] = make_float2(vb[it].z, vb[it].w);
+            }
         __syncthreads();
         for (int e = tid; e < kNodes * ny; e += 256) {
             const int n = e & (kNodes - 1), y = e / kNodes;
-            const int k = k0 + (n & (kNodeK - 1)), t = t0 * kNodeT + n / kNodeK;
-            if (k < L.nc && t < L.nT) G[((int64_t)t * F.nf2 + y0 + y) * pitch + k] = st[y][n];
+            const int k = k0 + n % kNodeK, t = t0 * kNodeT + n / kNodeK;
+            if (k < L.nc && t < L.nT) G[((int64_t)t * F.nf2 + y0 + y) * pitch + k] = box[y * (kNodes + 1) + n];
         }
+        __syncthreads();
     }
+}
+
+// 2-D tiles in strips of 8 along x, y within a strip: the source values that a
+// tile shares with its neighbours in both directions are then still in L2 (in
+// row order the README-size detector rows between two rows of tiles are 60 MB).
+constexpr int kStrip = 8;
+__host__ __device__ __forceinline__ int64_t strip_count(int64_t nx, int64_t ny) { return (nx + kStrip - 1) / kStrip * kStrip * ny; }
+__device__ __forceinline__ bool strip_order(int i, int nx, int ny, int &x, int &y) {
+    const int s = i / (kStrip * ny), r = i - s * (kStrip * ny);
+    y = r / kStrip;
+    x = s * kStrip + r - y * kStrip;
+    return x < nx && y < ny;
 }
 
 // Nodes -> fine grid (the transpose).  A CTA owns 4 x 4 (z, x) cells for all y,
@@ -456,7 +551,7 @@ __global__ void __launch_bounds__(256) k_nodes_gather(LatView L, Fine F, const f
 // tried at every period of the fine grid that the lattice reaches.
 constexpr int kCell = 4;
 template <int W>
-__global__ void __launch_bounds__(256) k_nodes_spread(LatView L, Fine F, int reach1, int reach3, int xtiles,
+__global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int reach1, int reach3, int xtiles,
                                                       const float2 *__restrict__ Gt, float2 *__restrict__ g) {
     extern __shared__ __align__(16) unsigned char nsm[];
     const int cap = 2 * blockDim.x;
@@ -464,7 +559,9 @@ __global__ void __launch_bounds__(256) k_nodes_spread(LatView L, Fine F, int rea
     int *ln = reinterpret_cast<int *>(lw + cap * kCell);
     __shared__ int wsum[9];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int zt = blockIdx.x / xtiles, c1 = zt * kCell, c3 = (blockIdx.x - zt * xtiles) * kCell;
+    int xt, zt;
+    if (!strip_order(blockIdx.x, xtiles, (F.nf1 + kCell - 1) / kCell, xt, zt)) return;
+    const int c1 = zt * kCell, c3 = xt * kCell;
     const int y = blockIdx.y * blockDim.x + tid;
     const float2 *src = Gt + min(y, F.nf2 - 1);
     float2 re[kCell][2], im[kCell][2];
@@ -620,34 +717,88 @@ __global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt
     }
 }
 
+// the run of rows (first, count) that start in y cell c2 - (W - 1) + r and whose
+// footprint meets T cells [c1, c1 + kCell)
+template <int W>
+__device__ __forceinline__ int2 tile_run(const uint32_t *__restrict__ start, int nstart, int nf2, int c1, int c2, int r) {
+    const int lo = max(0, c1 - (W - 1)), hi = min(nstart - 1, c1 + kCell - 1);
+    const uint32_t *o = start + (int64_t)wrap(c2 - (W - 1) + r, nf2) * nstart;
+    return make_int2((int)o[lo], (int)(o[hi + 1] - o[lo]));
+}
+// work items of k_rows_spread: (tile, first row of the segment, sign bit set if
+// the tile has several segments); empty tiles get one item, which stores zeros.
+// Tiles are taken in strips (strip_order).
+template <int W>
+__global__ void __launch_bounds__(128) k_tile_items(const uint32_t *__restrict__ start, int nstart, int nf2, int ntile,
+                                                    int ntiles, int seg, int *__restrict__ nitem, int2 *__restrict__ items) {
+    int tx, ty;
+    if (!strip_order(blockIdx.x * blockDim.x + threadIdx.x, ntile, ntiles / ntile, tx, ty)) return;
+    const int t = ty * ntile + tx, c1 = tx * kCell, c2 = ty * kCell;
+    int n = 0;
+    for (int r = 0; r < W + kCell - 1; ++r) n += tile_run<W>(start, nstart, nf2, c1, c2, r).y;
+    const int m = max(1, (n + seg - 1) / seg), at = atomicAdd(nitem, m);
+    for (int i = 0; i < m; ++i) items[at + i] = make_int2(t, (i * seg) | (m > 1 ? (int)0x80000000 : 0));
+}
+__global__ void __launch_bounds__(256) k_tiles_zero(const int *__restrict__ nitem, const int2 *__restrict__ items, int nT,
+                                                    int ntile, int nf2, int nc, float2 *__restrict__ Gt) {
+    const int n = __ldg(nitem);
+    for (int q = blockIdx.x; q < n; q += gridDim.x) {
+        const int2 item = __ldg(items + q);
+        if (item.y != (int)0x80000000) continue;  // first segment of several
+        const int ty = item.x / ntile, c1 = (item.x - ty * ntile) * kCell, c2 = ty * kCell;
+        for (int e = threadIdx.x; e < 2 * kCell * nc; e += blockDim.x) {
+            const int h = e & 1, i = (e >> 1) & (kCell - 1), k = e >> 3;
+            if (c1 + i < nT && c2 + 2 * h < nf2)
+                *reinterpret_cast<float4 *>(Gt + ((int64_t)(c1 + i) * nc + k) * nf2 + c2 + 2 * h) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
 // Rows -> nodes (the transpose).  A CTA owns 4 x 4 (T, y) cells, a thread one
 // column: 16 complex sums in registers over the rows whose footprint meets the
 // cells, which the cell order gives as W + 3 runs (one per y start).  Writes
 // the node grid as [T][X][y], y fastest, four y at a time.  With SYM a row's
 // value is the projection spectrum of sysmat, formed from F at q and at -q:
 // the strength conj(a) 2 P / N = (F(q) / 2 + 2 conj(a)^2 conj F(-q)) / N.
+//
+// Every projection passes through the origin, so the tiles there meet many
+// times the average of about 200 rows (all angles x 8 rows), and the walk over
+// a tile's rows is serial in its CTA.  The rows of a tile are therefore cut into
+// segments (k_tile_items, once per lattice); tiles of one segment are stored,
+// the others zeroed first and added to with vector atomics.
+// Measured (before: one CTA per tile, 256 threads of one column, tiles in row
+// order): 60 x 154^2 rows 186 -> 31 us, 2 x 91 x 309^2 (SYM) 1090 -> 340 us,
+// 361 x 1233^2 8.1 -> 6.7 ms.
+constexpr int kCols = 2;   // columns per thread
+constexpr int kAhead = 4;  // rows in flight per thread
 template <int W, bool SYM>
-__global__ void __launch_bounds__(256) k_rows_spread(const uint32_t *__restrict__ start, const int4 *__restrict__ pt,
-                                                     const float2 *__restrict__ pd, int nstart, int nT, int ntile, int nf2,
+__global__ void __launch_bounds__(128) k_rows_spread(const int *__restrict__ nitem, const int2 *__restrict__ items,
+                                                     int seg, const uint32_t *__restrict__ start,
+                                                     const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nstart,
+                                                     int nT, int ntile, int nf2,
                                                      const float2 *__restrict__ src, int nr, int nc, float beta,
                                                      const float2 *__restrict__ beam, float scale, float2 *__restrict__ Gt) {
     extern __shared__ __align__(16) unsigned char rsm[];
-    const int cap = blockDim.x;
-    float4 *lw = reinterpret_cast<float4 *>(rsm);            // [cap][kCell] weights, T by y
-    int2 *lr = reinterpret_cast<int2 *>(lw + cap * kCell);   // row, mirrored row
-    float2 *lb = reinterpret_cast<float2 *>(lr + cap);       // 2 conj(a)^2 / N
+    const int cap = blockDim.x;  // rows listed at a time
+    float4 *lw = reinterpret_cast<float4 *>(rsm);            // [row][kCell] weights, T by y
+    uint2 *lr = reinterpret_cast<uint2 *>(lw + (cap + 2 * kAhead) * kCell);  // row's first value, mirrored row's last
+    float2 *lb = reinterpret_cast<float2 *>(lr + cap + 2 * kAhead);          // 2 conj(a)^2 / N
     constexpr int NR = W + kCell - 1;
     __shared__ int beg[NR], pre[NR + 1];
-    const int tid = threadIdx.x;
-    const int c1 = (blockIdx.x % ntile) * kCell, c2 = (blockIdx.x / ntile) * kCell;
-    const int k = blockIdx.y * blockDim.x + tid;
-    const int kc = min(k, nc - 1);
+    if ((int)blockIdx.x >= __ldg(nitem)) return;
+    const int2 item = __ldg(items + blockIdx.x);
+    const int tid = threadIdx.x, ty = item.x / ntile;
+    const int c1 = (item.x - ty * ntile) * kCell, c2 = ty * kCell;
+    const int first = item.y & 0x7fffffff;
+    const bool shared_tile = item.y < 0;
+    const int k0 = blockIdx.y * kCols * blockDim.x + tid;
+    int kc[kCols];
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) kc[c] = min(k0 + c * (int)blockDim.x, nc - 1);
     if (tid < NR) {
-        const int ys = wrap(c2 - (W - 1) + tid, nf2);
-        const int lo = max(0, c1 - (W - 1)), hi = min(nstart - 1, c1 + kCell - 1);
-        const int64_t o = (int64_t)ys * nstart;
-        beg[tid] = (int)start[o + lo];
-        pre[tid + 1] = (int)(start[o + hi + 1] - start[o + lo]);
+        const int2 r = tile_run<W>(start, nstart, nf2, c1, c2, tid);
+        beg[tid] = r.x;
+        pre[tid + 1] = r.y;
     }
     __syncthreads();
     if (tid == 0) {
@@ -655,62 +806,102 @@ __global__ void __launch_bounds__(256) k_rows_spread(const uint32_t *__restrict_
         for (int r = 0; r < NR; ++r) pre[r + 1] += pre[r];
     }
     __syncthreads();
-    const int total = pre[NR];
-    float2 re[kCell][2], im[kCell][2];
+    const int total = min(pre[NR], first + seg);
+    float2 re[kCols][kCell][2], im[kCols][kCell][2];
 #pragma unroll
-    for (int i = 0; i < kCell; ++i) re[i][0] = re[i][1] = im[i][0] = im[i][1] = make_float2(0.f, 0.f);
-    for (int base = 0; base < total; base += cap) {
+    for (int c = 0; c < kCols; ++c)
+#pragma unroll
+        for (int i = 0; i < kCell; ++i) re[c][i][0] = re[c][i][1] = im[c][i][0] = im[c][i][1] = make_float2(0.f, 0.f);
+    for (int base = first; base < total; base += cap) {
         const int n = min(cap, total - base);
-        if (tid < n) {
+        // the last row is listed again, with weights of zero, up to 2 kAhead times:
+        // the loop below takes kAhead rows at a time and fetches as many beyond
+        for (int e = tid; e < n + 2 * kAhead; e += cap) {
+            const int q = min(e, n - 1);
             int r = 0;
-            while (base + tid >= pre[r + 1]) ++r;
-            const int at = beg[r] + base + tid - pre[r];
+            while (base + q >= pre[r + 1]) ++r;
+            const int at = beg[r] + base + q - pre[r];
             const int4 I = pt[at];
             const float2 d = pd[at];
+            const float on = e < n ? 1.f : 0.f;
             float u[kCell];
 #pragma unroll
-            for (int i = 0; i < kCell; ++i) u[i] = es_tap<W>(d.y, i + W - 1 - r, beta);
+            for (int i = 0; i < kCell; ++i) u[i] = on * es_tap<W>(d.y, i + W - 1 - r, beta);
 #pragma unroll
             for (int i = 0; i < kCell; ++i) {
                 const float s = es_tap<W>(d.x, c1 + i - I.y, beta);
-                lw[tid * kCell + i] = make_float4(s * u[0], s * u[1], s * u[2], s * u[3]);
+                lw[e * kCell + i] = make_float4(s * u[0], s * u[1], s * u[2], s * u[3]);
             }
             const int j = I.x - I.w * nr;
-            lr[tid] = make_int2(I.x, I.w * nr + nr - 1 - j);
+            lr[e] = make_uint2((uint32_t)I.x * nc, (uint32_t)(I.w * nr + nr - 1 - j) * nc + nc - 1);
             if (SYM) {
                 const float2 a = beam[I.w];  // conj(a)^2 = (ax^2 - ay^2) - 2 i ax ay
-                lb[tid] = make_float2(2 * scale * (a.x * a.x - a.y * a.y), -4 * scale * a.x * a.y);
+                lb[e] = make_float2(2 * scale * (a.x * a.x - a.y * a.y), -4 * scale * a.x * a.y);
             }
         }
         __syncthreads();
-#pragma unroll 4
-        for (int q = 0; q < n; ++q) {
-            const int2 row = lr[q];
-            float2 v = __ldg(src + (int64_t)row.x * nc + kc);
-            if (SYM) {
-                const float2 m = __ldg(src + (int64_t)row.y * nc + nc - 1 - kc), b = lb[q];
-                v = make_float2(fmaf(b.x, m.x, fmaf(b.y, m.y, 0.5f * scale * v.x)),
-                                fmaf(b.y, m.x, fmaf(-b.x, m.y, 0.5f * scale * v.y)));
-            }
-            const float2 vr = make_float2(v.x, v.x), vi = make_float2(v.y, v.y);
+        // values of the next kAhead rows are in flight while a row is added
+        float2 v[kAhead][kCols], m[kAhead][kCols];
+        auto fetch = [&](int q, float2 (&a)[kCols], float2 (&b)[kCols]) {
+            const uint2 row = lr[q];
 #pragma unroll
-            for (int i = 0; i < kCell; ++i) {
-                const float4 t = lw[q * kCell + i];
-                re[i][0] = __ffma2_rn(make_float2(t.x, t.y), vr, re[i][0]);
-                re[i][1] = __ffma2_rn(make_float2(t.z, t.w), vr, re[i][1]);
-                im[i][0] = __ffma2_rn(make_float2(t.x, t.y), vi, im[i][0]);
-                im[i][1] = __ffma2_rn(make_float2(t.z, t.w), vi, im[i][1]);
+            for (int c = 0; c < kCols; ++c) {
+                a[c] = __ldg(src + row.x + kc[c]);
+                if (SYM) b[c] = __ldg(src + row.y - kc[c]);
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) fetch(u, v[u], m[u]);
+        for (int q0 = 0; q0 < n; q0 += kAhead) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int q = q0 + u;
+                float2 x[kCols];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) {
+                    x[c] = v[u][c];
+                    if (SYM) {
+                        const float2 b = lb[q];
+                        x[c] = make_float2(fmaf(b.x, m[u][c].x, fmaf(b.y, m[u][c].y, 0.5f * scale * x[c].x)),
+                                           fmaf(b.y, m[u][c].x, fmaf(-b.x, m[u][c].y, 0.5f * scale * x[c].y)));
+                    }
+                }
+                fetch(q + kAhead, v[u], m[u]);
+#pragma unroll
+                for (int i = 0; i < kCell; ++i) {
+                    const float4 t = lw[q * kCell + i];
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) {
+                        const float2 vr = make_float2(x[c].x, x[c].x), vi = make_float2(x[c].y, x[c].y);
+                        re[c][i][0] = __ffma2_rn(make_float2(t.x, t.y), vr, re[c][i][0]);
+                        re[c][i][1] = __ffma2_rn(make_float2(t.z, t.w), vr, re[c][i][1]);
+                        im[c][i][0] = __ffma2_rn(make_float2(t.x, t.y), vi, im[c][i][0]);
+                        im[c][i][1] = __ffma2_rn(make_float2(t.z, t.w), vi, im[c][i][1]);
+                    }
+                }
             }
         }
         __syncthreads();
     }
-    if (k >= nc) return;
 #pragma unroll
-    for (int i = 0; i < kCell; ++i) {
-        if (c1 + i >= nT) break;
-        float4 *o = reinterpret_cast<float4 *>(Gt + ((int64_t)(c1 + i) * nc + k) * nf2 + c2);
-        o[0] = make_float4(re[i][0].x, im[i][0].x, re[i][0].y, im[i][0].y);  // nf2 is even: pairs are whole
-        if (c2 + 2 < nf2) o[1] = make_float4(re[i][1].x, im[i][1].x, re[i][1].y, im[i][1].y);
+    for (int c = 0; c < kCols; ++c) {
+        const int k = k0 + c * (int)blockDim.x;
+        if (k >= nc) break;
+#pragma unroll
+        for (int i = 0; i < kCell; ++i) {
+            if (c1 + i >= nT) break;
+            float4 *o = reinterpret_cast<float4 *>(Gt + ((int64_t)(c1 + i) * nc + k) * nf2 + c2);
+            const float2(&r)[2] = re[c][i], (&m)[2] = im[c][i];
+            const float4 v0 = make_float4(r[0].x, m[0].x, r[0].y, m[0].y);  // nf2 is even: pairs are whole
+            const float4 v1 = make_float4(r[1].x, m[1].x, r[1].y, m[1].y);
+            if (shared_tile) {
+                atomicAdd(o, v0);
+                if (c2 + 2 < nf2) atomicAdd(o + 1, v1);
+            } else {
+                o[0] = v0;
+                if (c2 + 2 < nf2) o[1] = v1;
+            }
+        }
     }
 }
 
@@ -982,7 +1173,10 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->sg = g.sg;
     // twice the volume's extent along t, in cells over the period 2 pi
     const double band = vol.n3 * std::fabs(l->sg) + vol.n1 * std::fabs(l->cg);
-    const int nTf = band > w ? 2 * (int)std::ceil(band - 1e-9) : 2 * w;  // (also for a NaN tilt)
+    int nTf = band > w ? 2 * (int)std::ceil(band - 1e-9) : 2 * w;  // (also for a NaN tilt)
+    // and no T line more than one cell of the fine grid from the next (k_nodes_gather)
+    const double near = std::max(nf1 * std::fabs(l->cg), nf3 * std::fabs(l->sg));
+    if (near > nTf) nTf = 2 * (int)std::ceil(0.5 * near);
     l->h = 2 * M_PI / nTf;
     // |T| <= pi up to float rounding: footprints start in [-nTf/2 - w/2, nTf/2 - w/2 + 1)
     l->T0 = -nTf / 2 - (w + 1) / 2 - 1;
@@ -991,6 +1185,16 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     const int64_t np = g.nproj, nrow = np * g.nrows, cells = (int64_t)l->nstart * nf2;
     if (cells > (int64_t)INT32_MAX - 1 || l->nT * g.ncols > (int64_t)INT32_MAX)
         throw Error(ERR_ARG, "node grid too large");
+    // Segments of k_rows_spread: 256 rows, fewer where that would leave less than
+    // about 16 CTAs per SM (a row meets 6 to 9 tiles).
+    l->ntile = (l->nT + kCell - 1) / kCell;
+    const int64_t ntiles = (int64_t)l->ntile * ((nf2 + kCell - 1) / kCell);
+    l->seg = (int)std::min<int64_t>(256, std::max<int64_t>(32, nrow * 6 * ((g.ncols + 255) / 256) / (148 * 16) / 32 * 32));
+    const int64_t meet = (w + kCell - 2) / kCell + 1;  // tiles a footprint meets along one axis, at most
+    const int64_t max_items = ntiles + nrow * meet * meet / l->seg + 1;
+    if (max_items > (int64_t)INT32_MAX || nrow * meet * meet > (int64_t)INT32_MAX)
+        throw Error(ERR_ARG, "too many detector rows in one geometry");
+    l->max_items = (int)max_items;
     // one allocation for all tables
     size_t bytes = 0;
     auto room = [&](size_t n) {
@@ -1001,7 +1205,8 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     const size_t oX = room(g.ncols * sizeof(double)), oa = room(np * sizeof(float2)), otr = room(g.nrows * sizeof(float4)),
                  otc = room(g.ncols * sizeof(float4)), oip = room(vol.n1 * vol.n3 * sizeof(float)),
                  opt = room(nrow * sizeof(int4)), opd = room(nrow * sizeof(float2)),
-                 ost = room((cells + 1) * sizeof(uint32_t)), ocnt = room(cells * sizeof(uint32_t));
+                 ost = room((cells + 1) * sizeof(uint32_t)), ocnt = room(cells * sizeof(uint32_t)),
+                 oni = room(sizeof(int)), oit = room(l->max_items * sizeof(int2));
     l->mem.alloc(bytes);
     char *m0 = l->mem.p;
     l->X = reinterpret_cast<double *>(m0 + oX);
@@ -1012,10 +1217,12 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->pt = reinterpret_cast<int4 *>(m0 + opt);
     l->pd = reinterpret_cast<float2 *>(m0 + opd);
     l->start = reinterpret_cast<uint32_t *>(m0 + ost);
+    l->nitem = reinterpret_cast<int *>(m0 + oni);
+    l->items = reinterpret_cast<int2 *>(m0 + oit);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(m0 + ocnt);  // counts, then placement cursors
     const int64_t need = (int64_t)l->nT * nf2 * node_pitch(g.ncols);
     if ((int64_t)work.n < need) work.alloc(need);
-    LAMINO_CUDA(cudaMemsetAsync(cnt, 0, cells * sizeof(uint32_t), s));
+    LAMINO_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(reinterpret_cast<char *>(l->items) - reinterpret_cast<char *>(cnt)), s));
     const Fine F = fine_of(*this);
     const GeomView gv = g.view();
     const int64_t m = std::max(std::max(g.ncols, g.nrows), np);
@@ -1035,6 +1242,9 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
         LAMINO_LAUNCH("k_scan_offsets");
         k_rows_place<W><<<grid_n, 256, 0, s>>>(gv, raw, invh, l->T0, l->nstart, F, cnt, l->pt, l->pd);
         LAMINO_LAUNCH("k_rows_place");
+        k_tile_items<W><<<(unsigned)((strip_count(l->ntile, ntiles / l->ntile) + 127) / 128), 128, 0, s>>>(l->start, l->nstart, (int)nf2, l->ntile, (int)ntiles,
+                                                                         l->seg, l->nitem, l->items);
+        LAMINO_LAUNCH("k_tile_items");
     });
     l->last_use = ++use_clock;
     lats.push_back(std::move(l));
@@ -1045,18 +1255,37 @@ void NufftPlan::nodes_to_rows(const Lattice &l, const Geom &g, float2 *rows, cud
     const Fine F = fine_of(*this);
     const LatView L = lat_view(l, g);
     const int pitch = (int)node_pitch(g.ncols);
-    // y in equal chunks of at most 16; small node grids spread the chunks over CTAs
-    const int nchunk = (int)((nf2 + kNodeY - 1) / kNodeY), ychunk = (int)((nf2 + nchunk - 1) / nchunk);
-    const int ktiles = (int)((g.ncols + kNodeK - 1) / kNodeK);
-    dim3 b1((unsigned)(ktiles * ((l.nT + kNodeT - 1) / kNodeT)));
+    // The box of cells under a tile of nodes, one cell of slack on either side, for
+    // 16 x 8 and 8 x 16 tiles (columns are 1.2 to 2 cells apart, T lines 0.7 to 1):
+    // the smaller box is staged, with 16 y where two CTAs then fit an SM, else with
+    // fewer.
+    auto box_cells = [&](int K) {
+        const double ek = (double)(std::min<int64_t>(K, g.ncols) - 1) * 2 * M_PI / g.ncols, et = (kNodes / K - 1) * l.h;
+        return std::ceil(F.s1 * (ek * std::fabs(l.sg) + et * std::fabs(l.cg)) + w + 3) *
+               std::ceil(F.s3 * (ek * std::fabs(l.cg) + et * std::fabs(l.sg)) + w + 3);
+    };
+    const int K = box_cells(16) <= box_cells(8) ? 16 : 8;
+    const double cells = box_cells(K);
+    constexpr double kBoxBytes = 100 * 1024;
+    // y in even chunks of at most 16; small node grids spread the chunks over CTAs
+    int nchunk = (int)((nf2 + kNodeY - 1) / kNodeY), ychunk = (int)((nf2 + nchunk - 1) / nchunk + 1) / 2 * 2;
+    if (cells * 4 * sizeof(float2) <= kBoxBytes)
+        while (cells * ychunk * sizeof(float2) > kBoxBytes) ychunk -= 2;
+    nchunk = (int)((nf2 + ychunk - 1) / ychunk);
+    const int boxcap = cells * ychunk * sizeof(float2) <= kBoxBytes ? (int)cells : 0;
+    const int smem = (int)(std::max(boxcap, kNodes + 1) * ychunk * sizeof(float2));
+    const int ktiles = (int)((g.ncols + K - 1) / K);
+    dim3 b1((unsigned)(ktiles * ((l.nT + kNodes / K - 1) / (kNodes / K))));
     b1.y = (unsigned)std::min<int64_t>(nchunk, std::max<int64_t>(1, 148LL * 12 / b1.x));
-    const uint32_t ydiv = (uint32_t)((0x100000000ULL + ychunk - 1) / ychunk);
+    const uint32_t ydiv = (uint32_t)((0x100000000ULL + ychunk / 2 - 1) / (ychunk / 2));
     const int64_t nrow = g.nproj * g.nrows;
     const int groups = (int)((nrow + kRowGroup - 1) / kRowGroup);
     const unsigned b2 = (unsigned)(groups * ((g.ncols + 63) / 64));
     with_width(w, [&](auto WC) {
         constexpr int W = decltype(WC)::value;
-        k_nodes_gather<W><<<b1, 256, 0, s>>>(L, F, grid.p, work.p, pitch, ktiles, ychunk, ydiv, nchunk);
+        auto ng = K == 16 ? k_nodes_gather<W, 16> : k_nodes_gather<W, 8>;
+        raise_smem_limit((const void *)ng, smem);
+        ng<<<b1, 256, smem, s>>>(L, F, grid.p, work.p, pitch, ktiles, ychunk, ydiv, nchunk, boxcap);
         LAMINO_LAUNCH("k_nodes_gather");
         k_rows_gather<W><<<b2, 256, 0, s>>>(l.pt, l.pd, (int)nrow, work.p, (int)nf2, pitch, (int)g.ncols, groups, beta,
                                             rows);
@@ -1068,13 +1297,15 @@ void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *row
     const Fine F = fine_of(*this);
     const LatView L = lat_view(l, g);
     const int nc = (int)g.ncols;
-    const int kblocks = (nc + 255) / 256, bt = ((nc + kblocks - 1) / kblocks + 31) / 32 * 32;
-    const int ntile = (l.nT + kCell - 1) / kCell;
-    const dim3 b1((unsigned)(ntile * ((nf2 + kCell - 1) / kCell)), (unsigned)((nc + bt - 1) / bt));
-    const int smem1 = bt * (int)(kCell * sizeof(float4) + sizeof(int2) + sizeof(float2));
+    // 32 to 128 threads of two columns each: the width that pads the columns least
+    int bt = 128;
+    for (int b : {96, 64, 32})
+        if ((nc + kCols * b - 1) / (kCols * b) * b < (nc + kCols * bt - 1) / (kCols * bt) * bt) bt = b;
+    const dim3 b1((unsigned)l.max_items, (unsigned)((nc + kCols * bt - 1) / (kCols * bt)));
+    const int smem1 = (bt + 2 * kAhead) * (int)(kCell * sizeof(float4) + sizeof(uint2) + sizeof(float2));
     const int yb = (int)std::min<int64_t>(256, (nf2 + 31) / 32 * 32);
     const int xtiles = (int)((nf3 + kCell - 1) / kCell);
-    const dim3 b2((unsigned)(xtiles * ((nf1 + kCell - 1) / kCell)), (unsigned)((nf2 + yb - 1) / yb));
+    const dim3 b2((unsigned)strip_count(xtiles, (nf1 + kCell - 1) / kCell), (unsigned)((nf2 + yb - 1) / yb));
     // largest |footprint cell| of the nodes along z and x (a NaN tilt has none)
     const double Tmax = std::max(-l.T0, l.T0 + l.nT) * l.h;
     auto reach = [&](double c, double t, double sc) {
@@ -1087,7 +1318,10 @@ void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *row
     with_width(w, [&](auto WC) {
         constexpr int W = decltype(WC)::value;
         auto rs = symmetric ? k_rows_spread<W, true> : k_rows_spread<W, false>;
-        rs<<<b1, bt, smem1, s>>>(l.start, l.pt, l.pd, l.nstart, l.nT, ntile, (int)nf2, rows, (int)g.nrows, nc, beta,
+        k_tiles_zero<<<(unsigned)std::min(l.max_items, 148 * 8), 256, 0, s>>>(l.nitem, l.items, l.nT, l.ntile, (int)nf2, nc,
+                                                                              work.p);
+        LAMINO_LAUNCH("k_tiles_zero");
+        rs<<<b1, bt, smem1, s>>>(l.nitem, l.items, l.seg, l.start, l.pt, l.pd, l.nstart, l.nT, l.ntile, (int)nf2, rows, (int)g.nrows, nc, beta,
                                  l.a, scale, work.p);
         LAMINO_LAUNCH("k_rows_spread");
         k_nodes_spread<W><<<b2, yb, smem2, s>>>(L, F, reach1, reach3, xtiles, work.p, grid.p);

@@ -40,6 +40,9 @@ struct Lattice {
     int4 *pt = nullptr;      // rows sorted by cell: row id (angle, detector row), T start, y start, angle
     float2 *pd = nullptr;    // offsets of the T and y footprints from the row's position
     uint32_t *start = nullptr;  // first row of each (y start, T start) cell
+    int ntile = 0, seg = 0, max_items = 0;  // rows -> nodes: tiles along T, rows per work item, bound on the items
+    int *nitem = nullptr;    // number of work items
+    int2 *items = nullptr;
 };
 
 struct NufftPlan {
@@ -98,7 +101,8 @@ struct NufftPlan {
     void fft_fine(float2 *g, int sign, cudaStream_t s);
     void nodes_to_rows(const Lattice &lat, const Geom &g, float2 *rows, cudaStream_t s);   // grid -> nodes -> rows
     void rows_to_nodes(const Lattice &lat, const Geom &g, const float2 *rows, bool symmetric, cudaStream_t s);
-    int64_t node_pitch(int64_t ncols) const { return (ncols + 3) / 4 * 4; }
+    // whole 128-byte lines, so that a run of columns never straddles one
+    int64_t node_pitch(int64_t ncols) const { return (ncols + 15) / 16 * 16; }
 };
 
 }  // namespace lamino
