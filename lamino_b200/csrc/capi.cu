@@ -536,7 +536,7 @@ int lamino_ramp_precond(const float *r3, int64_t n1, int64_t n2, int64_t n3, flo
     Dims3 d = dims_of(n1, n2, n3);
     In<float> ri(r3, 3 * d.size(), S(stream));
     Out<float> o(z3, 3 * d.size(), S(stream));
-    RampPrecond M(d);
+    RampPrecond M(d, S(stream));
     M.apply3(ri.d, o.d, S(stream));
     o.finish(S(stream));
     LAMINO_CUDA(cudaStreamSynchronize(S(stream)));

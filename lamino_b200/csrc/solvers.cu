@@ -559,8 +559,7 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_ramp_cols(float2 *__restrict_
 #pragma unroll
                     for (int r = 0; r < RC_ROWS; ++r) {
                         const float2 x = buf[(r - u + RC_ROWS) % RC_ROWS];
-                        acc[r].x = fmaf(g, x.x, acc[r].x);
-                        acc[r].y = fmaf(g, x.y, acc[r].y);
+                        acc[r] = __ffma2_rn(make_float2(g, g), x, acc[r]);
                     }
                 }
             }
@@ -703,55 +702,81 @@ __global__ void __launch_bounds__(256, FIXED ? 5 : 4) k_blue_c2r(const float2 *_
     blue_convolve<FIXED>(rows, F, V, tw, sm, M);
 }
 
-// chirp w_n = e^{i pi n^2 / N}, the convolution kernels' spectra in DIF position
-// order (forward: v; inverse: conj v; both / M) and the M-point twiddles, in FP64
-static void blue_tables(int N, int M, std::vector<float2> &chirp, std::vector<float2> &vf, std::vector<float2> &vi,
-                        std::vector<float2> &tw) {
-    std::vector<double> wc(N), ws(N);
-    for (int64_t n = 0; n < N; ++n) {
-        const double a = M_PI * (double)((n * n) % (2 * (int64_t)N)) / (double)N;
-        wc[n] = std::cos(a);
-        ws[n] = std::sin(a);
+// The tables of a size, built on the device in FP64 (on the host their sums, M^2
+// and n2^2 n3 / 2 terms, took 11 ms at 721 x 71 x 721, five times the apply).
+
+// filter value f(k2, k3), in the reference's float operations, with the
+// 1 / (n2 n3) of the c2r folded in
+__device__ __forceinline__ float ramp_filter(int j, int i, int n2, int n3, float scale) {
+    const float x = __fdiv_rn((float)i, (float)n3);
+    const float y = __fdiv_rn((float)(j <= n2 / 2 ? j : j - n2), (float)n2);
+    return __fmul_rn(__fsqrt_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y))), scale);
+}
+// conv: G[d][k3] = sum_k2 f(k2, k3) cos(2 pi k2 d / n2) (n2 <= kRampConvMaxN2), else f itself
+__global__ void __launch_bounds__(128) k_ramp_table(int n2, int n3, int h3, float scale, bool conv,
+                                                    float *__restrict__ out) {
+    __shared__ double cs[kRampConvMaxN2];
+    if (conv) {
+        for (int t = threadIdx.x; t < n2; t += blockDim.x) cs[t] = cospi(2.0 * t / n2);
+        __syncthreads();
     }
-    chirp.resize(N);
-    for (int n = 0; n < N; ++n) chirp[n] = make_float2((float)wc[n], (float)ws[n]);
-    std::vector<double> vr(M, 0.0), vim(M, 0.0);
-    for (int m = 0; m < N; ++m) {
-        vr[m] = wc[m];
-        vim[m] = ws[m];
-        if (m > 0) {
-            vr[M - m] = wc[m];
-            vim[M - m] = ws[m];
+    const int64_t n = (int64_t)n2 * h3;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int d = (int)(e / h3), i = (int)(e - (int64_t)d * h3);
+        if (!conv) {
+            out[e] = ramp_filter(d, i, n2, n3, scale);
+            continue;
         }
-    }
-    std::vector<double> cs(M), sn(M);
-    for (int e = 0; e < M; ++e) {
-        cs[e] = std::cos(-2.0 * M_PI * e / M);
-        sn[e] = std::sin(-2.0 * M_PI * e / M);
-    }
-    const std::vector<int> pos = fft_positions(M, fft_schedule(M, true));
-    vf.assign(M, make_float2(0.f, 0.f));
-    vi.assign(M, make_float2(0.f, 0.f));
-    std::vector<double> Fr(M), Fi(M);
-    for (int k = 0; k < M; ++k) {
-        double re = 0.0, im = 0.0;
-        for (int m = 0; m < M; ++m) {
-            if (vr[m] == 0.0 && vim[m] == 0.0) continue;
-            const int e = (int)(((int64_t)k * m) % M);
-            re += vr[m] * cs[e] - vim[m] * sn[e];
-            im += vr[m] * sn[e] + vim[m] * cs[e];
+        double acc = 0.0;
+        for (int j = 0, t = 0; j < n2; ++j) {
+            acc += (double)ramp_filter(j, i, n2, n3, scale) * cs[t];
+            t += d;
+            if (t >= n2) t -= n2;
         }
-        Fr[k] = re;
-        Fi[k] = im;
+        out[e] = (float)acc;
     }
-    for (int k = 0; k < M; ++k) {
-        // transform of conj v at k = conj(transform of v at -k)
-        const int km = (M - k) % M;
-        vf[pos[k]] = make_float2((float)(Fr[k] / M), (float)(Fi[k] / M));
-        vi[pos[k]] = make_float2((float)(Fr[km] / M), (float)(-Fi[km] / M));
+}
+// chirp w_n = e^{i pi n^2 / N}, the M-point twiddles and, in double for
+// k_blue_spectra, w and cos(2 pi e / M)
+__global__ void k_blue_tables(int N, int M, float2 *__restrict__ chirp, float2 *__restrict__ tw, double2 *__restrict__ w,
+                              double *__restrict__ cs) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double s, c;
+    if (i < N) {
+        sincospi((double)(((long long)i * i) % (2LL * N)) / N, &s, &c);
+        w[i] = make_double2(c, s);
+        chirp[i] = make_float2((float)c, (float)s);
     }
-    tw.resize(M);
-    for (int e = 0; e < M; ++e) tw[e] = make_float2((float)cs[e], (float)sn[e]);
+    if (i < M) {
+        sincospi(2.0 * i / M, &s, &c);
+        cs[i] = c;
+        tw[i] = make_float2((float)c, (float)-s);
+    }
+}
+// the convolution kernel's spectrum, V_k = w_0 + 2 sum_{0 < m < N} w_m cos(2 pi k m / M)
+// (v is even, so V is), over M, in DIF position order, and its conjugate (the
+// spectrum of conj v); one warp per k
+__global__ void __launch_bounds__(256) k_blue_spectra(int N, int M, const double2 *__restrict__ w,
+                                                      const double *__restrict__ cs, const int *__restrict__ pos,
+                                                      float2 *__restrict__ vf, float2 *__restrict__ vi) {
+    const int k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (k >= M) return;
+    double re = 0.0, im = 0.0;
+    for (int m = 1 + lane; m < N; m += 32) {
+        const double c = cs[(int)(((long long)k * m) % M)];
+        re += w[m].x * c;
+        im += w[m].y * c;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        re += __shfl_down_sync(0xffffffffu, re, o);
+        im += __shfl_down_sync(0xffffffffu, im, o);
+    }
+    if (lane) return;
+    re = (w[0].x + 2.0 * re) / M;
+    im = (w[0].y + 2.0 * im) / M;
+    vf[pos[k]] = make_float2((float)re, (float)im);
+    vi[pos[k]] = make_float2((float)re, (float)-im);
 }
 
 // largest prime factor of n
@@ -784,64 +809,61 @@ static FftLen blue_len(int M, const float2 *tw_dev) {
     return F;
 }
 
-RampPrecond::RampPrecond(Dims3 dd) : d(dd) {
-    int64_t n2 = d.n2, n3 = d.n3, h3 = n3 / 2 + 1;
-    std::vector<float> xf(h3), yf(n2), f(n2 * h3);
-    for (int64_t i = 0; i < h3; ++i) xf[i] = (float)i / (float)n3;
-    for (int64_t i = 0; i < n2; ++i) yf[i] = (i <= n2 / 2) ? (float)i / (float)n2 : (float)(i - n2) / (float)n2;
-    // the 1/(n2 n3) normalisation of the c2r is folded into the filter
-    float scale = (float)(1.0 / (double)(n2 * n3));
-    for (int64_t j = 0; j < n2; ++j)
-        for (int64_t i = 0; i < h3; ++i) f[j * h3 + i] = std::sqrt(xf[i] * xf[i] + yf[j] * yf[j]) * scale;
+RampPrecond::RampPrecond(Dims3 dd, cudaStream_t s) : d(dd) {
+    const int64_t n2 = d.n2, n3 = d.n3, h3 = n3 / 2 + 1;
     spec.alloc(3 * d.n1 * n2 * h3);
     cols = n2 <= kRampConvMaxN2 && 3 * d.n1 <= 65535;
-    if (cols) {
-        // G[dd * h3 + k3] = sum_k2 f(k2, k3) cos(2 pi k2 dd / n2), in double
-        std::vector<double> cs(n2);
-        for (int64_t t = 0; t < n2; ++t) cs[t] = std::cos(2.0 * M_PI * (double)t / (double)n2);
-        std::vector<float> g(n2 * h3);
-        for (int64_t dd2 = 0; dd2 < n2; ++dd2)
-            for (int64_t i = 0; i < h3; ++i) {
-                double acc = 0.0;
-                for (int64_t j = 0; j < n2; ++j) acc += (double)f[j * h3 + i] * cs[(j * dd2) % n2];
-                g[dd2 * h3 + i] = (float)acc;
-            }
-        filt.alloc(n2 * h3);
-        upload(filt.p, g.data(), g.size());
-        const bool fixed = n3 >= 365 && n3 <= kBlueHalf;
-        const int64_t mrt = next_smooth_even(2 * n3 - 1);
-        blue = fixed || (n3 >= 128 && largest_prime_factor(n3) > 7 && mrt <= kBlueMaxM);
-        blue_fixed = fixed;
-        if (blue) {
-            const int M = fixed ? kBlueM : (int)mrt;
-            std::vector<float2> hc, hvf, hvi, htw;
-            blue_tables((int)n3, M, hc, hvf, hvi, htw);
-            chirp.alloc(hc.size());
-            upload(chirp.p, hc.data(), hc.size());
-            vfwd.alloc(hvf.size());
-            upload(vfwd.p, hvf.data(), hvf.size());
-            vinv.alloc(hvi.size());
-            upload(vinv.p, hvi.data(), hvi.size());
-            tw.alloc(htw.size());
-            upload(tw.p, htw.data(), htw.size());
-            blue_f = blue_len(M, tw.p);
-            raise_smem_limit((const void *)k_blue_r2c<true>, (int)(3 * (kBlueM + kBlueHalf) * sizeof(float2)));
-            raise_smem_limit((const void *)k_blue_c2r<true>, (int)(3 * kBlueM * sizeof(float2)));
-            raise_smem_limit((const void *)k_blue_r2c<false>, (int)(3 * (M + M / 2) * sizeof(float2)));
-            raise_smem_limit((const void *)k_blue_c2r<false>, (int)(3 * M * sizeof(float2)));
-        } else {
-            int n[1] = {(int)n3};
-            r2c.make(1, n, CUFFT_R2C, (int)(3 * d.n1 * n2));
-            c2r.make(1, n, CUFFT_C2R, (int)(3 * d.n1 * n2));
-        }
-        raise_smem_limit((const void *)k_ramp_cols, (int)(n2 * RC_KB * (2 * sizeof(float2) + sizeof(float))));
+    const bool fixed = n3 >= 365 && n3 <= kBlueHalf;
+    const int64_t mrt = next_smooth_even(2 * n3 - 1);
+    blue_fixed = cols && fixed;
+    blue = cols && (fixed || (n3 >= 128 && largest_prime_factor(n3) > 7 && mrt <= kBlueMaxM));
+    const int M = !blue ? 0 : (fixed ? kBlueM : (int)mrt), N = blue ? (int)n3 : 0;
+    // one allocation for all tables
+    size_t bytes = 0;
+    auto room = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t of = room(n2 * h3 * sizeof(float)), oc = room(N * sizeof(float2)), ot = room(M * sizeof(float2)),
+                 ovf = room(M * sizeof(float2)), ovi = room(M * sizeof(float2)), ow = room(N * sizeof(double2)),
+                 ocs = room(M * sizeof(double)), op = room(M * sizeof(int));
+    tables.alloc(bytes);
+    char *m0 = tables.p;
+    filt = reinterpret_cast<float *>(m0 + of);
+    chirp = reinterpret_cast<float2 *>(m0 + oc);
+    tw = reinterpret_cast<float2 *>(m0 + ot);
+    vfwd = reinterpret_cast<float2 *>(m0 + ovf);
+    vinv = reinterpret_cast<float2 *>(m0 + ovi);
+    const float scale = (float)(1.0 / (double)(n2 * n3));
+    k_ramp_table<<<grid_for(n2 * h3, 128), 128, 0, s>>>((int)n2, (int)n3, (int)h3, scale, cols, filt);
+    LAMINO_LAUNCH("k_ramp_table");
+    if (blue) {
+        const std::vector<int> hpos = fft_positions(M, fft_schedule(M, true));
+        int *pos = reinterpret_cast<int *>(m0 + op);
+        LAMINO_CUDA(cudaMemcpyAsync(pos, hpos.data(), M * sizeof(int), cudaMemcpyHostToDevice, s));
+        double2 *w = reinterpret_cast<double2 *>(m0 + ow);
+        double *cs = reinterpret_cast<double *>(m0 + ocs);
+        k_blue_tables<<<(unsigned)((std::max(M, N) + 127) / 128), 128, 0, s>>>(N, M, chirp, tw, w, cs);
+        LAMINO_LAUNCH("k_blue_tables");
+        k_blue_spectra<<<(unsigned)((M + 7) / 8), 256, 0, s>>>(N, M, w, cs, pos, vfwd, vinv);
+        LAMINO_LAUNCH("k_blue_spectra");
+        LAMINO_CUDA(cudaStreamSynchronize(s));  // hpos goes out of scope
+        blue_f = blue_len(M, tw);
+        raise_smem_limit((const void *)k_blue_r2c<true>, (int)(3 * (kBlueM + kBlueHalf) * sizeof(float2)));
+        raise_smem_limit((const void *)k_blue_c2r<true>, (int)(3 * kBlueM * sizeof(float2)));
+        raise_smem_limit((const void *)k_blue_r2c<false>, (int)(3 * (M + M / 2) * sizeof(float2)));
+        raise_smem_limit((const void *)k_blue_c2r<false>, (int)(3 * M * sizeof(float2)));
+    } else if (cols) {
+        int n[1] = {(int)n3};
+        r2c.make(1, n, CUFFT_R2C, (int)(3 * d.n1 * n2));
+        c2r.make(1, n, CUFFT_C2R, (int)(3 * d.n1 * n2));
     } else {
-        filt.alloc(n2 * h3);
-        upload(filt.p, f.data(), f.size());
         int n[2] = {(int)n2, (int)n3};
         r2c.make(2, n, CUFFT_R2C, (int)(3 * d.n1));
         c2r.make(2, n, CUFFT_C2R, (int)(3 * d.n1));
     }
+    if (cols) raise_smem_limit((const void *)k_ramp_cols, (int)(n2 * RC_KB * (2 * sizeof(float2) + sizeof(float))));
 }
 
 void RampPrecond::apply3(const float *r3, float *z3, cudaStream_t s) {
@@ -851,11 +873,11 @@ void RampPrecond::apply3(const float *r3, float *z3, cudaStream_t s) {
     const int M = blue_f.n;
     if (blue && blue_fixed) {
         k_blue_r2c<true><<<gblue, 256, 3 * (kBlueM + kBlueHalf) * sizeof(float2), s>>>(
-            r3, nrows, (int)d.n3, chirp.p, vfwd.p, tw.p, blue_f, spec.p);
+            r3, nrows, (int)d.n3, chirp, vfwd, tw, blue_f, spec.p);
         LAMINO_LAUNCH("k_blue_r2c");
     } else if (blue) {
-        k_blue_r2c<false><<<gblue, 256, 3 * (M + M / 2) * sizeof(float2), s>>>(r3, nrows, (int)d.n3, chirp.p,
-                                                                              vfwd.p, tw.p, blue_f, spec.p);
+        k_blue_r2c<false><<<gblue, 256, 3 * (M + M / 2) * sizeof(float2), s>>>(r3, nrows, (int)d.n3, chirp,
+                                                                              vfwd, tw, blue_f, spec.p);
         LAMINO_LAUNCH("k_blue_r2c");
     } else {
         LAMINO_CUFFT(cufftSetStream(r2c.h, s));
@@ -864,19 +886,19 @@ void RampPrecond::apply3(const float *r3, float *z3, cudaStream_t s) {
     if (cols) {
         const dim3 grid((unsigned)((h3 + RC_KB - 1) / RC_KB), (unsigned)(3 * d.n1));
         const int smem = (int)(d.n2 * RC_KB * (2 * sizeof(float2) + sizeof(float)));
-        k_ramp_cols<<<grid, RC_WARPS * 32, smem, s>>>(spec.p, filt.p, (int)d.n2, (int)h3);
+        k_ramp_cols<<<grid, RC_WARPS * 32, smem, s>>>(spec.p, filt, (int)d.n2, (int)h3);
         LAMINO_LAUNCH("k_ramp_cols");
     } else {
-        k_filter_mul<<<grid_for(3 * d.n1 * plane, 256), 256, 0, s>>>(spec.p, filt.p, plane, 3 * d.n1 * plane);
+        k_filter_mul<<<grid_for(3 * d.n1 * plane, 256), 256, 0, s>>>(spec.p, filt, plane, 3 * d.n1 * plane);
         LAMINO_LAUNCH("k_filter_mul");
     }
     if (blue && blue_fixed) {
-        k_blue_c2r<true><<<gblue, 256, 3 * kBlueM * sizeof(float2), s>>>(spec.p, nrows, (int)d.n3, chirp.p,
-                                                                         vinv.p, tw.p, blue_f, z3);
+        k_blue_c2r<true><<<gblue, 256, 3 * kBlueM * sizeof(float2), s>>>(spec.p, nrows, (int)d.n3, chirp,
+                                                                         vinv, tw, blue_f, z3);
         LAMINO_LAUNCH("k_blue_c2r");
     } else if (blue) {
-        k_blue_c2r<false><<<gblue, 256, 3 * M * sizeof(float2), s>>>(spec.p, nrows, (int)d.n3, chirp.p, vinv.p,
-                                                                     tw.p, blue_f, z3);
+        k_blue_c2r<false><<<gblue, 256, 3 * M * sizeof(float2), s>>>(spec.p, nrows, (int)d.n3, chirp, vinv,
+                                                                     tw, blue_f, z3);
         LAMINO_LAUNCH("k_blue_c2r");
     } else {
         LAMINO_CUFFT(cufftSetStream(c2r.h, s));
@@ -901,7 +923,7 @@ __global__ void k_cg_dir(float *__restrict__ p, const float *__restrict__ z, flo
 }
 
 CgStats cgsolver(const OpFn &A, const float *y3, float *x3, Dims3 d, int max_iter, float tol, cudaStream_t s) {
-    CgWork w(d);
+    CgWork w(d, s);
     CgStats st = cgsolver(A, y3, x3, w, max_iter, tol, s);
     LAMINO_CUDA(cudaStreamSynchronize(s));
     return st;
@@ -950,7 +972,7 @@ CgStats cgsolver(const OpFn &A, const float *y3, float *x3, CgWork &w, int max_i
 
 CgStats cgsolver_refined(const OpFn &A_hi, const OpFn &A_lo, const float *y3, float *x3, Dims3 d, int inner,
                          int refinements, float tol, cudaStream_t s) {
-    CgWork w(d);
+    CgWork w(d, s);
     CgStats st = cgsolver_refined(A_hi, A_lo, y3, x3, w, inner, refinements, tol, s);
     LAMINO_CUDA(cudaStreamSynchronize(s));
     return st;
@@ -1005,7 +1027,7 @@ int split_bregman_refined(const OpFn &A, const OpFn &A_lo, int refinements, cons
         laplacian_axpy(out, mu, u, d, st);
     };
     Reducer red(8);
-    CgWork work(d);
+    CgWork work(d, s);
     int it = 0;
     for (; it < outer_max; ++it) {
         sb_rhs(yT3, dd.p, bb.p, mu, d, rhs.p, s);

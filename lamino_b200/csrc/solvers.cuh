@@ -50,13 +50,15 @@ struct RampPrecond {
     Dims3 d;
     FftPlan r2c, c2r;
     DevBuf<float2> spec;
-    DevBuf<float> filt;  // the filter (2-D path) or the n2 convolution kernels (column path)
+    DevBuf<char> tables;    // holds the tables below
+    float *filt = nullptr;  // the filter (2-D path) or the n2 convolution kernels (column path)
     bool cols = false;   // 1-D transforms along n3 and a circulant convolution along n2
     bool blue = false;        // (with cols) the n3 transforms as Bluestein convolutions
     bool blue_fixed = false;  // of length 1458 on the compile-time pipeline (else runtime M)
-    DevBuf<float2> chirp, vfwd, vinv, tw;  // Bluestein tables: chirp, kernel spectra, twiddles
+    float2 *chirp = nullptr, *vfwd = nullptr, *vinv = nullptr, *tw = nullptr;  // Bluestein tables: chirp, kernel
+                                                                               // spectra, twiddles
     FftLen blue_f{};                       // schedule of the Bluestein length M
-    explicit RampPrecond(Dims3 d);
+    RampPrecond(Dims3 d, cudaStream_t s);  // the tables are built on s
     void apply3(const float *r3, float *z3, cudaStream_t s);  // all 3 components
 };
 
@@ -71,8 +73,8 @@ struct CgWork {
     DevBuf<float> r, p, z, Ap, e1, e2;  // e1, e2: refinement residual / correction
     RampPrecond M;
     Reducer red;
-    explicit CgWork(Dims3 dd)
-        : d(dd), r(3 * dd.size()), p(3 * dd.size()), z(3 * dd.size()), Ap(3 * dd.size()), M(dd), red(4) {}
+    CgWork(Dims3 dd, cudaStream_t s)
+        : d(dd), r(3 * dd.size()), p(3 * dd.size()), z(3 * dd.size()), Ap(3 * dd.size()), M(dd, s), red(4) {}
 };
 
 // src/conjgrad.cpp:37-117.  x3 holds x0 on entry and the solution on exit.
