@@ -64,10 +64,30 @@ inline cudaStream_t &alloc_stream() {
     static thread_local cudaStream_t s = nullptr;
     return s;
 }
+// Pool of the calling thread's stream-ordered allocations (null: the device's
+// default pool).
+inline cudaMemPool_t &alloc_pool() {
+    static thread_local cudaMemPool_t p = nullptr;
+    return p;
+}
+// This library's own pool on the current device, for the buffers of one driver
+// call (nothing that outlives the call may be allocated from it): it keeps up to
+// kCallPoolKeep bytes between calls, which are given back to the device when an
+// allocation of this library fails.  Null if the device has no pools.
+constexpr uint64_t kCallPoolKeep = 4ull << 30;
+cudaMemPool_t call_pool();
+void trim_call_pool();
 struct AllocStreamScope {
     cudaStream_t prev;
-    explicit AllocStreamScope(cudaStream_t s) : prev(alloc_stream()) { alloc_stream() = s; }
-    ~AllocStreamScope() { alloc_stream() = prev; }
+    cudaMemPool_t prev_pool;
+    explicit AllocStreamScope(cudaStream_t s, cudaMemPool_t pool = nullptr) : prev(alloc_stream()), prev_pool(alloc_pool()) {
+        alloc_stream() = s;
+        alloc_pool() = pool;
+    }
+    ~AllocStreamScope() {
+        alloc_stream() = prev;
+        alloc_pool() = prev_pool;
+    }
     AllocStreamScope(const AllocStreamScope &) = delete;
     AllocStreamScope &operator=(const AllocStreamScope &) = delete;
 };
@@ -100,9 +120,23 @@ struct DevBuf {
         release();
         if (!count) return;
         as = alloc_stream();
-        if (as) LAMINO_CUDA(cudaMallocAsync((void **)&p, count * sizeof(T), as));
-        else LAMINO_CUDA(cudaMalloc((void **)&p, count * sizeof(T)));
+        cudaError_t e = get(count * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            trim_call_pool();
+            e = get(count * sizeof(T));
+        }
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();
+        }
+        LAMINO_CUDA(e);
         n = count;
+    }
+    cudaError_t get(size_t bytes) {
+        if (as && alloc_pool()) return cudaMallocFromPoolAsync((void **)&p, bytes, alloc_pool(), as);
+        if (as) return cudaMallocAsync((void **)&p, bytes, as);
+        return cudaMalloc((void **)&p, bytes);
     }
     void release() {
         if (p) {

@@ -5,6 +5,8 @@
 // with warp-shuffle trees instead of the reference's serial float sums.
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -12,6 +14,44 @@
 #include "solvers.cuh"
 
 namespace lamino {
+
+namespace {
+std::mutex g_pool_mu;
+std::map<int, cudaMemPool_t> g_pools;
+}  // namespace
+
+cudaMemPool_t call_pool() {
+    int dev = 0, has = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&has, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !has) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    cudaMemPool_t &p = g_pools[dev];
+    uint64_t keep = kCallPoolKeep;
+    // (the attribute call also tells a pool that a device reset took away)
+    if (p && cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) return p;
+    cudaGetLastError();
+    p = nullptr;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+    }
+    return p;
+}
+void trim_call_pool() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pools.find(dev);
+    if (it != g_pools.end() && it->second && cudaMemPoolTrimTo(it->second, 0) != cudaSuccess) cudaGetLastError();
+}
 
 // ---------------------------------------------------------------------------
 // reductions
@@ -811,14 +851,13 @@ static FftLen blue_len(int M, const float2 *tw_dev) {
 
 RampPrecond::RampPrecond(Dims3 dd, cudaStream_t s) : d(dd) {
     const int64_t n2 = d.n2, n3 = d.n3, h3 = n3 / 2 + 1;
-    spec.alloc(3 * d.n1 * n2 * h3);
     cols = n2 <= kRampConvMaxN2 && 3 * d.n1 <= 65535;
     const bool fixed = n3 >= 365 && n3 <= kBlueHalf;
     const int64_t mrt = next_smooth_even(2 * n3 - 1);
     blue_fixed = cols && fixed;
     blue = cols && (fixed || (n3 >= 128 && largest_prime_factor(n3) > 7 && mrt <= kBlueMaxM));
     const int M = !blue ? 0 : (fixed ? kBlueM : (int)mrt), N = blue ? (int)n3 : 0;
-    // one allocation for all tables
+    // one allocation for the tables and the spectra
     size_t bytes = 0;
     auto room = [&](size_t n) {
         const size_t at = bytes;
@@ -827,9 +866,11 @@ RampPrecond::RampPrecond(Dims3 dd, cudaStream_t s) : d(dd) {
     };
     const size_t of = room(n2 * h3 * sizeof(float)), oc = room(N * sizeof(float2)), ot = room(M * sizeof(float2)),
                  ovf = room(M * sizeof(float2)), ovi = room(M * sizeof(float2)), ow = room(N * sizeof(double2)),
-                 ocs = room(M * sizeof(double)), op = room(M * sizeof(int));
-    tables.alloc(bytes);
-    char *m0 = tables.p;
+                 ocs = room(M * sizeof(double)), op = room(M * sizeof(int)),
+                 os = room(3 * d.n1 * n2 * h3 * sizeof(float2));
+    mem.alloc(bytes);
+    char *m0 = mem.p;
+    spec = reinterpret_cast<float2 *>(m0 + os);
     filt = reinterpret_cast<float *>(m0 + of);
     chirp = reinterpret_cast<float2 *>(m0 + oc);
     tw = reinterpret_cast<float2 *>(m0 + ot);
@@ -873,36 +914,36 @@ void RampPrecond::apply3(const float *r3, float *z3, cudaStream_t s) {
     const int M = blue_f.n;
     if (blue && blue_fixed) {
         k_blue_r2c<true><<<gblue, 256, 3 * (kBlueM + kBlueHalf) * sizeof(float2), s>>>(
-            r3, nrows, (int)d.n3, chirp, vfwd, tw, blue_f, spec.p);
+            r3, nrows, (int)d.n3, chirp, vfwd, tw, blue_f, spec);
         LAMINO_LAUNCH("k_blue_r2c");
     } else if (blue) {
         k_blue_r2c<false><<<gblue, 256, 3 * (M + M / 2) * sizeof(float2), s>>>(r3, nrows, (int)d.n3, chirp,
-                                                                              vfwd, tw, blue_f, spec.p);
+                                                                              vfwd, tw, blue_f, spec);
         LAMINO_LAUNCH("k_blue_r2c");
     } else {
         LAMINO_CUFFT(cufftSetStream(r2c.h, s));
-        LAMINO_CUFFT(cufftExecR2C(r2c.h, const_cast<float *>(r3), (cufftComplex *)spec.p));
+        LAMINO_CUFFT(cufftExecR2C(r2c.h, const_cast<float *>(r3), (cufftComplex *)spec));
     }
     if (cols) {
         const dim3 grid((unsigned)((h3 + RC_KB - 1) / RC_KB), (unsigned)(3 * d.n1));
         const int smem = (int)(d.n2 * RC_KB * (2 * sizeof(float2) + sizeof(float)));
-        k_ramp_cols<<<grid, RC_WARPS * 32, smem, s>>>(spec.p, filt, (int)d.n2, (int)h3);
+        k_ramp_cols<<<grid, RC_WARPS * 32, smem, s>>>(spec, filt, (int)d.n2, (int)h3);
         LAMINO_LAUNCH("k_ramp_cols");
     } else {
-        k_filter_mul<<<grid_for(3 * d.n1 * plane, 256), 256, 0, s>>>(spec.p, filt, plane, 3 * d.n1 * plane);
+        k_filter_mul<<<grid_for(3 * d.n1 * plane, 256), 256, 0, s>>>(spec, filt, plane, 3 * d.n1 * plane);
         LAMINO_LAUNCH("k_filter_mul");
     }
     if (blue && blue_fixed) {
-        k_blue_c2r<true><<<gblue, 256, 3 * kBlueM * sizeof(float2), s>>>(spec.p, nrows, (int)d.n3, chirp,
+        k_blue_c2r<true><<<gblue, 256, 3 * kBlueM * sizeof(float2), s>>>(spec, nrows, (int)d.n3, chirp,
                                                                          vinv, tw, blue_f, z3);
         LAMINO_LAUNCH("k_blue_c2r");
     } else if (blue) {
-        k_blue_c2r<false><<<gblue, 256, 3 * M * sizeof(float2), s>>>(spec.p, nrows, (int)d.n3, chirp, vinv,
+        k_blue_c2r<false><<<gblue, 256, 3 * M * sizeof(float2), s>>>(spec, nrows, (int)d.n3, chirp, vinv,
                                                                      tw, blue_f, z3);
         LAMINO_LAUNCH("k_blue_c2r");
     } else {
         LAMINO_CUFFT(cufftSetStream(c2r.h, s));
-        LAMINO_CUFFT(cufftExecC2R(c2r.h, (cufftComplex *)spec.p, z3));
+        LAMINO_CUFFT(cufftExecC2R(c2r.h, (cufftComplex *)spec, z3));
     }
 }
 

@@ -49,8 +49,8 @@ void sb_shrink(const float *x3, float *d9, float *b9, float lam, float mu, Dims3
 struct RampPrecond {
     Dims3 d;
     FftPlan r2c, c2r;
-    DevBuf<float2> spec;
-    DevBuf<char> tables;    // holds the tables below
+    DevBuf<char> mem;       // holds the spectra and the tables below
+    float2 *spec = nullptr;
     float *filt = nullptr;  // the filter (2-D path) or the n2 convolution kernels (column path)
     bool cols = false;   // 1-D transforms along n3 and a circulant convolution along n2
     bool blue = false;        // (with cols) the n3 transforms as Bluestein convolutions
