@@ -176,8 +176,7 @@ void MbirJob::prepare() {
 
     t_setup_ = now_s();
 
-    // normal operator sum_gamma sysmat; MBIR3 also needs one operator per gamma
-    // for its loss, and then the sum is formed from their spectra
+    // normal operator sum_gamma sysmat; MBIR3 keeps each gamma's spectra for its loss
     const bool mixed = prm.op_kind == OP_TOEPLITZ_MIXED;
     if (prm.op_kind == OP_NUFFT) {
         NufftPlan *pl = plan_.get();
@@ -194,12 +193,7 @@ void MbirJob::prepare() {
         plan_.reset();  // the fine grids are only needed for the setup adjoints
         int prec = prm.op_kind == OP_TOEPLITZ_FP16 ? PREC_FP16 : (mixed ? PREC_MIXED : PREC_FP32);
         if (method == 3) {
-            for (const Geom *g : gptr_) {
-                Tg_.emplace_back(new Toeplitz({g}, od, PREC_FP32, s));
-                Tg_.back()->drop_work();  // kept for its spectra (loss quadratic forms, the sum)
-                parts_.push_back(Tg_.back().get());
-            }
-            T_.reset(new Toeplitz(parts_, prec, s));
+            T_.reset(new Toeplitz(Toeplitz::PerDataset{}, gptr_, od, prec, s));  // the loss needs each dataset's form
         } else {
             T_.reset(new Toeplitz(gptr_, od, prec, s));
         }
@@ -226,38 +220,47 @@ void MbirJob::prepare() {
     red.fetch(1, s);
     const double yTy = red.h[0];
     const float ng = (float)gptr_.size();
-    // gradient: sum_gamma (sysmat x - yT) + qGGMRF (src/mbir3.cpp:91-103), one graph per input
-    gGrad_.reset(new GraphedOp(
-        [this, ng, n, V](const float *xx, float *g, cudaStream_t st) {
-            A_raw_(xx, g, st);
-            k_axpy_scalar<<<grid_for(n, 256), 256, 0, st>>>(g, -ng, yT_.p, n);
-            LAMINO_LAUNCH("k_axpy_scalar");
-            for (int i = 0; i < 3; ++i) qggmrf_add(g + i * V, xx + i * V, od_, prm_.sigma, prm_.p, st);
-        },
-        graphs));
-    GradFn grad = [this](const float *xx, float *g, cudaStream_t st) {
-        (*gGrad_)(xx, g, st);
-        ++extra_applies_;
-    };
+    // gradient: sum_gamma (sysmat x - yT) + qGGMRF (src/mbir3.cpp:91-103) and, with
+    // slots, the loss terms of the same volume; one graph per input.
     // loss (src/mbir3.cpp:108-116): sum over gamma and component of
     // sqrt(x_i . S_g x_i - 2 x_i . yT_i + yTy).  Toeplitz forms get every
-    // x_i . S_g x_i from one forward half-spectrum of x (Parseval); the NUFFT
-    // form applies each S_g.  The terms land in the caller's (zeroed) device
-    // slots; the graph is keyed by (input, slot) pointers.
+    // x_i . S_g x_i from one forward half-spectrum of x (Parseval), which is also
+    // the product's; the NUFFT form applies each S_g.  The terms land in the
+    // caller's (zeroed) device slots; the graphs are keyed by (input, slot) pointers
+    // and, for the gradient, its slots are the same in every call.
     const int ngi = (int)gptr_.size();
     if (!T_) Sx_.alloc(n);
+    auto data_terms = [this, ngi, V](const float *xx, double *acc, cudaStream_t st) {
+        for (int i = 0; i < 3; ++i) vec_dot(xx + i * V, yT_.p + i * V, V, acc + 3 * ngi + i, st);
+    };
+    auto prior = [this, ng, n, V](const float *xx, float *g, cudaStream_t st) {
+        k_axpy_scalar<<<grid_for(n, 256), 256, 0, st>>>(g, -ng, yT_.p, n);
+        LAMINO_LAUNCH("k_axpy_scalar");
+        for (int i = 0; i < 3; ++i) qggmrf_add(g + i * V, xx + i * V, od_, prm_.sigma, prm_.p, st);
+    };
+    gGrad_.reset(new GraphedOp(
+        [this, data_terms, prior](const float *xx, float *g, cudaStream_t st) {
+            if (T_) {
+                T_->dataset_forms(xx, grad_slots_, st, g);
+                data_terms(xx, grad_slots_, st);
+            } else {
+                A_raw_(xx, g, st);
+            }
+            prior(xx, g, st);
+        },
+        graphs));
     gLoss_.reset(new GraphedOp(
-        [this, ngi, V](const float *xx, float *slot, cudaStream_t st) {
+        [this, ngi, V, data_terms](const float *xx, float *slot, cudaStream_t st) {
             double *acc = reinterpret_cast<double *>(slot);
             if (T_) {
-                T_->quadforms(xx, parts_, acc, st);
+                T_->dataset_forms(xx, acc, st);
             } else {
                 for (int q = 0; q < ngi; ++q) {
                     Ag_[q](xx, Sx_.p, st);
                     for (int i = 0; i < 3; ++i) vec_dot(xx + i * V, Sx_.p + i * V, V, acc + 3 * q + i, st);
                 }
             }
-            for (int i = 0; i < 3; ++i) vec_dot(xx + i * V, yT_.p + i * V, V, acc + 3 * ngi + i, st);
+            data_terms(xx, acc, st);
         },
         graphs));
     LossTerms loss;
@@ -271,6 +274,13 @@ void MbirJob::prepare() {
         for (int q = 0; q < ngi; ++q)
             for (int i = 0; i < 3; ++i) e += std::sqrt(h[3 * q + i] - 2.0 * h[3 * ngi + i] + yTy);
         return e;
+    };
+    GradFn grad = [this, loss](const float *xx, float *g, double *acc, cudaStream_t st) {
+        if (grad_slots_ && grad_slots_ != acc) throw Error(ERR_STATE, "gradient called with other slots");
+        grad_slots_ = acc;
+        (*gGrad_)(xx, g, st);
+        ++extra_applies_;
+        if (!T_) loss.enqueue(xx, acc, st);
     };
     float lip = prm.mu;
     if (!(lip > 0.f)) {  // estimate: 30 power iterations of sum_gamma sysmat (qGGMRF curvature neglected)

@@ -100,8 +100,7 @@ class MbirJob {
     std::vector<const Geom *> gptr_;
     DevBuf<float> yT_, x_, Sx_;
     std::unique_ptr<Toeplitz> T_;
-    std::vector<std::unique_ptr<Toeplitz>> Tg_;
-    std::vector<const Toeplitz *> parts_;
+    double *grad_slots_ = nullptr;  // loss slots of the gradient's volume
     OpFn A_raw_, A_lo_raw_;
     std::vector<OpFn> Ag_;
     std::unique_ptr<GraphedOp> gA_, gA_lo_, gGrad_, gLoss_;

@@ -1127,11 +1127,10 @@ void NagSolve::enqueue() {
     tnew_ = 0.5 * (std::sqrt(std::pow(t_, 4) + 4 * std::pow(t_, 2)) - std::pow(t_, 2));
     k_extrap<<<grid_for(n, 256), 256, 0, s_>>>(y_.p, x_, xold_.p, beta, n);
     LAMINO_LAUNCH("k_extrap");
-    grad_(y_.p, g_.p, s_);
-    vec_lin2(x_, 1.f, y_.p, -step_, g_.p, n, s_);
     red_.zero(2 * M + 9, s_);
+    grad_(y_.p, g_.p, red_.d + M, s_);
+    vec_lin2(x_, 1.f, y_.p, -step_, g_.p, n, s_);
     loss_.enqueue(x_, red_.d, s_);
-    loss_.enqueue(y_.p, red_.d + M, s_);
     vec_sqdist3(g_.p, nullptr, V, gsl, s_);
     vec_sqdist3(x_, xold_.p, V, gsl + 3, s_);
     vec_sqdist3(x_, nullptr, V, gsl + 6, s_);

@@ -97,7 +97,9 @@ int split_bregman(const OpFn &A, const float *yT3, float *x3, Dims3 d, float lam
                   int inner_max, float tol, float xtol, cudaStream_t s);
 
 // src/nagopt.cpp:116-209 (vector form); grad and loss are closures.
-using GradFn = std::function<void(const float *x3, float *g3, cudaStream_t)>;
+// grad(x, g, acc): the gradient at x into g and the loss terms of x, added into the
+// (zeroed) device doubles acc as LossTerms::enqueue does.
+using GradFn = std::function<void(const float *x3, float *g3, double *acc, cudaStream_t)>;
 // A loss split so that several evaluations share one host read: enqueue(x, acc)
 // adds the loss's nterms partial sums of x into device doubles acc[0..nterms)
 // (zeroed by the caller) without reading them; value(terms) forms the loss from

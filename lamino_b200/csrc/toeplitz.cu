@@ -77,6 +77,7 @@ __device__ __forceinline__ float dirichlet(double s, int n, double inv_n) {
 }
 
 // One thread per cell with d_z = m1 in [0, n1); writes T[d] and its mirror T[-d].
+template <int NP>  // 6 pairs 00, 11, 22, 01, 02, 12, or 3: sin^2, cos^2, sin cos of the angles
 __global__ void __launch_bounds__(256) k_toeplitz_kernel(
     float *__restrict__ T, int64_t L1, int64_t L2, int64_t L3, int n1, int n2, int n3,
     const TGam *__restrict__ gams, int ngam, const TProj *__restrict__ projs) {
@@ -89,28 +90,28 @@ __global__ void __launch_bounds__(256) k_toeplitz_kernel(
         int64_t r = idx / nx;
         int dy = (int)(r % ny) - (n2 - 1);
         int dz = (int)(r / ny);
-        double acc[6] = {0, 0, 0, 0, 0, 0};
+        double acc[NP] = {};
         for (int gi = 0; gi < ngam; ++gi) {
             const TGam G = gams[gi];
             double Da = (double)dirichlet((double)dx * G.cg - (double)dz * G.sg, G.ncols, G.inv_ncols) * G.inv_scale;
             double u = (double)dx * G.sg + (double)dz * G.cg;
             // per-dataset sums over the projections in float (|terms| <= nrows), then FP64
-            float part[6] = {0, 0, 0, 0, 0, 0};
+            float part[NP] = {};
             for (int p = 0; p < G.np; ++p) {
                 const TProj P = projs[G.p0 + p];
                 const float Db = dirichlet(P.ct * u - (double)dy * P.st, G.nrows, G.inv_nrows);
 #pragma unroll
-                for (int q = 0; q < 6; ++q) part[q] = fmaf(P.w[q], Db, part[q]);
+                for (int q = 0; q < NP; ++q) part[q] = fmaf(P.w[q], Db, part[q]);
             }
 #pragma unroll
-            for (int q = 0; q < 6; ++q) acc[q] = fma(Da, (double)part[q], acc[q]);
+            for (int q = 0; q < NP; ++q) acc[q] = fma(Da, (double)part[q], acc[q]);
         }
         int64_t m1 = dz, m2 = dy < 0 ? dy + L2 : dy, m3 = dx < 0 ? dx + L3 : dx;
         int64_t c0 = (m1 * L2 + m2) * L3 + m3;
         int64_t mm1 = (L1 - m1) % L1, mm2 = (L2 - m2) % L2, mm3 = (L3 - m3) % L3;
         int64_t c1 = (mm1 * L2 + mm2) * L3 + mm3;
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
+        for (int q = 0; q < NP; ++q) {
             T[q * LS + c0] = (float)acc[q];
             T[q * LS + c1] = (float)acc[q];
         }
@@ -121,9 +122,10 @@ __global__ void __launch_bounds__(256) k_toeplitz_kernel(
 // spectra in apply order
 // ---------------------------------------------------------------------------
 
-// K[(pen * 6 + q) * L1 + p1] = Re(S[(nat1[p1] * L2 + nat2[p2]) * L3h + k3]) * norm, pen = p2 * L3h + k3
+// K[(pen * np + q) * L1 + p1] = Re(S[(nat1[p1] * L2 + nat2[p2]) * L3h + k3]) * norm, pen = p2 * L3h + k3
 __global__ void k_take_real_perm(const float2 *__restrict__ S, int L1, int L2, int L3h, const int *__restrict__ nat1,
-                                 const int *__restrict__ nat2, int q, float norm, float *__restrict__ K) {
+                                 const int *__restrict__ nat2, int np, int q, float norm,
+                                 float *__restrict__ K) {
     const int64_t total = (int64_t)L1 * L2 * L3h;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int p1 = (int)(i % L1);
@@ -131,7 +133,7 @@ __global__ void k_take_real_perm(const float2 *__restrict__ S, int L1, int L2, i
         int k3 = (int)(pen % L3h);
         int p2 = (int)(pen / L3h);
         float v = S[((int64_t)nat1[p1] * L2 + nat2[p2]) * L3h + k3].x * norm;
-        K[(pen * 6 + q) * L1 + p1] = v;
+        K[(pen * np + q) * L1 + p1] = v;
     }
 }
 
@@ -1339,26 +1341,14 @@ static std::vector<int> two_stage_schedule(int L) {
     }
 }
 
-// B: one (p2, k3) pencil of the 3 components along n1: DIF (zero-padded), 3x3
-// symmetric multiply with the spectra (same position order), undo, first n1 kept.
-// In place on xa.  N1: compile-time L1 or 0.  At L1 = 1458, five CTAs of 256
-// threads per SM (48 registers, 35 KB of shared memory each); four otherwise.
-template <bool HALF, int N1>
-__global__ void __launch_bounds__(pencil_threads(N1), 4) k_pencil(float2 *__restrict__ xa, int n1, int n1p, int L2, int L3h, FftLen F1,
-                                                const float2 *__restrict__ tw1, const float *__restrict__ K,
-                                                const __half *__restrict__ Kh, const float *__restrict__ kscale) {
-    extern __shared__ float2 sm[];
-    const int64_t pen = blockIdx.x;
+// the zero-padded forward transform of a pencil's three components into shared
+// memory (DIF position order; ends synchronised), and its undo into the first n1
+// values in place
+template <int N1>
+__device__ __forceinline__ void pencil_forward(float2 *pv, int64_t cs, int n1, const FftLen &F1,
+                                               const float2 *__restrict__ tw1, float2 *sm) {
     const int L1 = N1 ? N1 : F1.n;
     const int half = L1 / 2;
-    const int64_t cs = (int64_t)L2 * L3h * n1p;  // component stride in xa
-    float2 *pv = xa + pen * n1p;
-    // the pencil's 6 spectra (one contiguous range) start moving into L2 while
-    // the forward transform runs, so the multiply does not wait on HBM
-    if (threadIdx.x == 0) {
-        if constexpr (HALF) prefetch_l2(Kh + pen * 6 * L1, (size_t)6 * L1 * sizeof(__half));
-        else prefetch_l2(K + pen * 6 * L1, (size_t)6 * L1 * sizeof(float));
-    }
     if constexpr (N1 == 1458) {
         p1458_forward(PencilRows{pv, cs, n1}, tw1, sm);
     } else if constexpr (TwoStage<N1>::on) {
@@ -1393,6 +1383,51 @@ __global__ void __launch_bounds__(pencil_threads(N1), 4) k_pencil(float2 *__rest
         __syncthreads();
         fft_fwd_any<N1, 1>(sm, 3, L1, F1, threadIdx.x, blockDim.x);
     }
+}
+template <int N1>
+__device__ __forceinline__ void pencil_inverse(float2 *pv, int64_t cs, int n1, const FftLen &F1,
+                                               const float2 *__restrict__ tw1, float2 *sm) {
+    const int L1 = N1 ? N1 : F1.n;
+    const int half = L1 / 2;
+    if constexpr (N1 == 1458) {
+        p1458_inverse(PencilRows{pv, cs, n1}, tw1, sm);
+    } else if constexpr (TwoStage<N1>::on) {
+        p2s_inverse<TwoStage<N1>::A, TwoStage<N1>::B>(PencilRows{pv, cs, n1}, tw1, sm);
+    } else if constexpr (N1 != 0) {
+        ct_inverse<N1, CtSched<N1>::ns - 1, 2>(sm, 3, N1, tw1, threadIdx.x, blockDim.x);
+        fftlead_store<CtSched<N1>::r[1]>(PencilRows{pv, cs, n1}, tw1, sm, N1, N1, threadIdx.x, blockDim.x);
+    } else if (F1.ns >= 2) {
+        fft_inverse(sm, 3, L1, F1, 2, threadIdx.x, blockDim.x);
+        fftlead_any<true>(PencilRows{pv, cs, n1}, F1, sm, L1, threadIdx.x, blockDim.x);
+    } else {
+        fft_inv_any<N1, 1>(sm, 3, L1, F1, threadIdx.x, blockDim.x);
+        for (int t = threadIdx.x; t < 3 * n1; t += blockDim.x) {
+            int c = t / n1, i1 = t - c * n1;
+            pv[c * cs + i1] = c_add(sm[c * L1 + i1], c_mulc(sm[c * L1 + i1 + half], __ldg(tw1 + i1)));
+        }
+    }
+}
+
+// B: one (p2, k3) pencil of the 3 components along n1: DIF (zero-padded), 3x3
+// symmetric multiply with the spectra (same position order), undo, first n1 kept.
+// In place on xa.  N1: compile-time L1 or 0.  At L1 = 1458, five CTAs of 256
+// threads per SM (48 registers, 35 KB of shared memory each); four otherwise.
+template <bool HALF, int N1>
+__global__ void __launch_bounds__(pencil_threads(N1), 4) k_pencil(float2 *__restrict__ xa, int n1, int n1p, int L2, int L3h, FftLen F1,
+                                                const float2 *__restrict__ tw1, const float *__restrict__ K,
+                                                const __half *__restrict__ Kh, const float *__restrict__ kscale) {
+    extern __shared__ float2 sm[];
+    const int64_t pen = blockIdx.x;
+    const int L1 = N1 ? N1 : F1.n;
+    const int64_t cs = (int64_t)L2 * L3h * n1p;  // component stride in xa
+    float2 *pv = xa + pen * n1p;
+    // the pencil's 6 spectra (one contiguous range) start moving into L2 while
+    // the forward transform runs, so the multiply does not wait on HBM
+    if (threadIdx.x == 0) {
+        if constexpr (HALF) prefetch_l2(Kh + pen * 6 * L1, (size_t)6 * L1 * sizeof(__half));
+        else prefetch_l2(K + pen * 6 * L1, (size_t)6 * L1 * sizeof(float));
+    }
+    pencil_forward<N1>(pv, cs, n1, F1, tw1, sm);
     const float sc = HALF ? kscale[pen] : 1.f;
     // two adjacent positions per thread (L1 is even): 8-byte spectrum loads and
     // 16-byte shared accesses; KU pairs whose 6 spectra are in flight together
@@ -1438,23 +1473,7 @@ __global__ void __launch_bounds__(pencil_threads(N1), 4) k_pencil(float2 *__rest
         }
     }
     __syncthreads();
-    if constexpr (N1 == 1458) {
-        p1458_inverse(PencilRows{pv, cs, n1}, tw1, sm);
-    } else if constexpr (TwoStage<N1>::on) {
-        p2s_inverse<TwoStage<N1>::A, TwoStage<N1>::B>(PencilRows{pv, cs, n1}, tw1, sm);
-    } else if constexpr (N1 != 0) {
-        ct_inverse<N1, CtSched<N1>::ns - 1, 2>(sm, 3, N1, tw1, threadIdx.x, blockDim.x);
-        fftlead_store<CtSched<N1>::r[1]>(PencilRows{pv, cs, n1}, tw1, sm, N1, N1, threadIdx.x, blockDim.x);
-    } else if (F1.ns >= 2) {
-        fft_inverse(sm, 3, L1, F1, 2, threadIdx.x, blockDim.x);
-        fftlead_any<true>(PencilRows{pv, cs, n1}, F1, sm, L1, threadIdx.x, blockDim.x);
-    } else {
-        fft_inv_any<N1, 1>(sm, 3, L1, F1, threadIdx.x, blockDim.x);
-        for (int t = threadIdx.x; t < 3 * n1; t += blockDim.x) {
-            int c = t / n1, i1 = t - c * n1;
-            pv[c * cs + i1] = c_add(sm[c * L1 + i1], c_mulc(sm[c * L1 + i1 + half], __ldg(tw1 + i1)));
-        }
-    }
+    pencil_inverse<N1>(pv, cs, n1, F1, tw1, sm);
 }
 
 // Quadratic forms x_i . (S_g x)_i of up to kMaxQuadSets operators S_g sharing
@@ -1474,32 +1493,14 @@ __global__ void __launch_bounds__(pencil_threads(N1)) k_pencil_quad(const float2
     __shared__ float red[8][3 * kMaxQuadSets];
     const int64_t pen = blockIdx.x;
     const int L1 = N1 ? N1 : F1.n;
-    const int half = L1 / 2;
     const int64_t cs = (int64_t)L2 * L3h * n1p;
-    const float2 *pv = xa + pen * n1p;
-    if constexpr (N1 == 1458) {
-        p1458_forward(PencilRows{const_cast<float2 *>(pv), cs, n1}, tw1, sm);  // reads only
-    } else if constexpr (TwoStage<N1>::on) {
-        p2s_forward<TwoStage<N1>::A, TwoStage<N1>::B>(PencilRows{const_cast<float2 *>(pv), cs, n1}, tw1, sm);
-    } else if constexpr (N1 != 0) {
-        fftlead_load<CtSched<N1>::r[1]>(PencilRows{const_cast<float2 *>(pv), cs, n1}, tw1, sm, N1, N1,
-                                        threadIdx.x, blockDim.x);
-        __syncthreads();
-        ct_forward<N1, 2>(sm, 3, N1, tw1, threadIdx.x, blockDim.x);
-    } else if (F1.ns >= 2) {
-        fftlead_any<false>(PencilRows{const_cast<float2 *>(pv), cs, n1}, F1, sm, L1, threadIdx.x, blockDim.x);
-        __syncthreads();
-        fft_forward(sm, 3, L1, F1, 2, threadIdx.x, blockDim.x);
-    } else {
-        for (int t = threadIdx.x; t < 3 * half; t += blockDim.x) {
-            int c = t / half, i1 = t - c * half;
-            float2 v = i1 < n1 ? pv[c * cs + i1] : make_float2(0.f, 0.f);
-            sm[c * L1 + i1] = v;
-            sm[c * L1 + i1 + half] = c_mul(v, __ldg(tw1 + i1));
-        }
-        __syncthreads();
-        fft_fwd_any<N1, 1>(sm, 3, L1, F1, threadIdx.x, blockDim.x);
+    float2 *pv = const_cast<float2 *>(xa) + pen * n1p;  // read only here
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int g = 0; g < kMaxQuadSets; ++g)
+            if (g < ng) prefetch_l2(ks.K[g] + pen * 6 * L1, (size_t)6 * L1 * sizeof(float));
     }
+    pencil_forward<N1>(pv, cs, n1, F1, tw1, sm);
     float part[kMaxQuadSets][3];
 #pragma unroll
     for (int g = 0; g < kMaxQuadSets; ++g) part[g][0] = part[g][1] = part[g][2] = 0.f;
@@ -1540,6 +1541,141 @@ __global__ void __launch_bounds__(pencil_threads(N1)) k_pencil_quad(const float2
         const int k3 = (int)(pen % L3h);
         const double wk = (k3 == 0 || k3 == L3h - 1) ? 1.0 : 2.0;
         atomicAdd(acc + threadIdx.x, wk * t);
+    }
+}
+
+// The pencil step over the datasets' own spectra.  One dataset's kernel has three
+// independent spectra, not six: its beam vectors are (sin g sin th, cos th,
+// cos g sin th), so with S = sin g x_0 + cos g x_2 and C = x_1
+//     y_0 = sin g t,  y_1 = u,  y_2 = cos g t,  t = SS S + SC C,  u = SC S + CC C,
+// SS, CC, SC the spectra of D_a sum_th D_b (sin^2, cos^2, sin cos).  K: [pencil][3]
+// [p1] of every dataset.  Writes the datasets' sum in place (apply) and, with
+// part, each dataset's quadratic forms x_i . (S_g x)_i of the pencil (Parseval,
+// as k_pencil_quad) to part[pencil][g][i]; the reconstruction step with two
+// datasets gets the product and the loss of one volume from one pass that reads
+// as many spectra as the product alone did.
+// Measured at 270 x 32 x 270 (embedding 540 x 64 x 540) with two datasets: 193 us
+// on average over products, forms and both at once, where k_pencil takes 183 us
+// and k_pencil_quad, which reads 12 spectra and adds every pencil's sums to the
+// same six doubles by atomics, 296 us.
+constexpr int kMaxTilts = 4;
+struct Tilts {
+    const float *K[kMaxTilts];
+    float sg[kMaxTilts], cg[kMaxTilts];
+};
+template <int N1>
+__global__ void __launch_bounds__(pencil_threads(N1), pencil_threads(N1) == 256 ? 3 : 4) k_pencil_tilts(float2 *__restrict__ xa, int n1, int n1p, int L2,
+                                                                      int L3h, FftLen F1, const float2 *__restrict__ tw1,
+                                                                      Tilts T, int ng, bool apply,
+                                                                      double *__restrict__ part) {
+    extern __shared__ __align__(16) float2 sm[];
+    __shared__ float red[8][3 * kMaxTilts];
+    const int64_t pen = blockIdx.x;
+    const int L1 = N1 ? N1 : F1.n;
+    const int64_t cs = (int64_t)L2 * L3h * n1p;
+    float2 *pv = xa + pen * n1p;
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int g = 0; g < kMaxTilts; ++g)
+            if (g < ng) prefetch_l2(T.K[g] + pen * 3 * L1, (size_t)3 * L1 * sizeof(float));
+    }
+    pencil_forward<N1>(pv, cs, n1, F1, tw1, sm);
+    float q[kMaxTilts][3];
+#pragma unroll
+    for (int g = 0; g < kMaxTilts; ++g) q[g][0] = q[g][1] = q[g][2] = 0.f;
+    // two adjacent positions per thread (L1 is even)
+    const int L1h = L1 / 2;
+    for (int pp = threadIdx.x; pp < L1h; pp += blockDim.x) {
+        float2 k[kMaxTilts][3];
+#pragma unroll
+        for (int g = 0; g < kMaxTilts; ++g)
+            if (g < ng) {
+                const float2 *Kp = reinterpret_cast<const float2 *>(T.K[g] + pen * 3 * L1) + pp;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) k[g][i] = __ldg(Kp + i * L1h);
+            }
+        float4 *s0 = reinterpret_cast<float4 *>(sm) + pp, *s1 = reinterpret_cast<float4 *>(sm + L1) + pp,
+               *s2 = reinterpret_cast<float4 *>(sm + 2 * L1) + pp;
+        const float4 a = *s0, b = *s1, c = *s2;
+        float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0, y2 = y0;
+#pragma unroll
+        for (int g = 0; g < kMaxTilts; ++g)
+            if (g < ng) {
+                const float sg = T.sg[g], cg = T.cg[g];
+                const float2 ss = k[g][0], cc = k[g][1], sc = k[g][2];
+                const float4 S = make_float4(sg * a.x + cg * c.x, sg * a.y + cg * c.y, sg * a.z + cg * c.z, sg * a.w + cg * c.w);
+                const float4 t = make_float4(ss.x * S.x + sc.x * b.x, ss.x * S.y + sc.x * b.y, ss.y * S.z + sc.y * b.z,
+                                             ss.y * S.w + sc.y * b.w);
+                const float4 u = make_float4(sc.x * S.x + cc.x * b.x, sc.x * S.y + cc.x * b.y, sc.y * S.z + cc.y * b.z,
+                                             sc.y * S.w + cc.y * b.w);
+                q[g][0] += sg * (a.x * t.x + a.y * t.y + a.z * t.z + a.w * t.w);
+                q[g][1] += b.x * u.x + b.y * u.y + b.z * u.z + b.w * u.w;
+                q[g][2] += cg * (c.x * t.x + c.y * t.y + c.z * t.z + c.w * t.w);
+                y0.x += sg * t.x; y0.y += sg * t.y; y0.z += sg * t.z; y0.w += sg * t.w;
+                y1.x += u.x; y1.y += u.y; y1.z += u.z; y1.w += u.w;
+                y2.x += cg * t.x; y2.y += cg * t.y; y2.z += cg * t.z; y2.w += cg * t.w;
+            }
+        if (apply) {
+            *s0 = y0;
+            *s1 = y1;
+            *s2 = y2;
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (part) {
+#pragma unroll
+        for (int g = 0; g < kMaxTilts; ++g)
+            if (g < ng)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    float v = q[g][i];
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                    if (lane == 0) red[warp][g * 3 + i] = v;
+                }
+    }
+    __syncthreads();
+    if (part && (int)threadIdx.x < 3 * ng) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += (double)red[w][threadIdx.x];
+        const int k3 = (int)(pen % L3h);
+        part[pen * 3 * ng + threadIdx.x] = (k3 == 0 || k3 == L3h - 1) ? t : 2.0 * t;
+    }
+    if (apply) pencil_inverse<N1>(pv, cs, n1, F1, tw1, sm);
+}
+// acc[i] += sum over the pencils of part[pencil][i], in a fixed order; one CTA per i
+__global__ void __launch_bounds__(512) k_sum_pencils(const double *__restrict__ part, int64_t npen, int n,
+                                                     double *__restrict__ acc) {
+    __shared__ double red[16];
+    double t = 0.0;
+    for (int64_t p = threadIdx.x; p < npen; p += blockDim.x) t += part[p * n + blockIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        t = 0.0;
+        for (int w = 0; w < 16; ++w) t += red[w];
+        acc[blockIdx.x] += t;
+    }
+}
+// the six pair spectra of the datasets' sum from their three each
+__global__ void k_sum_tilts(const float *__restrict__ K3, int64_t set, int ng, const float *__restrict__ sc, int L1,
+                            int64_t n, float *__restrict__ K) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t pen = i / L1, p = i - pen * L1;
+        float k[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int g = 0; g < ng; ++g) {
+            const float *s = K3 + g * set + pen * 3 * L1 + p;
+            const float ss = s[0], cc = s[L1], sx = s[2 * L1], sg = sc[2 * g], cg = sc[2 * g + 1];
+            k[0] += sg * sg * ss;
+            k[1] += cc;
+            k[2] += cg * cg * ss;
+            k[3] += sg * sx;
+            k[4] += sg * cg * ss;
+            k[5] += cg * sx;
+        }
+        for (int q = 0; q < 6; ++q) K[(pen * 6 + q) * L1 + p] = k[q];
     }
 }
 
@@ -1714,11 +1850,6 @@ std::vector<int> fft_positions(int n, const std::vector<int> &radix) {
     return pos;
 }
 
-__global__ void k_add_into(float *a, const float *b, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        a[i] += b[i];
-}
-
 // The dynamic shared-memory limit is a per-function attribute shared by every
 // operator (and host thread) of the process on a device: it is only ever raised,
 // under a lock, so an operator built concurrently for a smaller volume cannot
@@ -1849,9 +1980,9 @@ void Toeplitz::init_tables(Dims3 d, int prec) {
     r2_ = r2;
 }
 
-Toeplitz::Toeplitz(const std::vector<const Geom *> &gs, Dims3 d, int prec, cudaStream_t s) : vol(d), precision(prec) {
-    if (gs.empty()) throw Error(ERR_ARG, "Toeplitz operator needs at least one geometry");
-    init_tables(d, prec);
+// Spectra of np pair kernels summed over gs, in apply order: `out` holds np per pencil.
+void Toeplitz::build_spectra(const std::vector<const Geom *> &gs, int np, float *out, cudaStream_t s) {
+    const Dims3 d = vol;
     std::vector<int> nat1(L1), nat2(L2);
     {
         std::vector<int> p1 = fft_positions((int)L1, r1_), p2 = fft_positions((int)L2, r2_);
@@ -1881,11 +2012,15 @@ Toeplitz::Toeplitz(const std::vector<const Geom *> &gs, Dims3 d, int prec, cudaS
         for (int64_t i = 0; i < g->nproj; ++i) {
             double th = (double)g->theta[i];
             double c[3] = {std::sin(gm) * std::sin(th), std::cos(th), std::cos(gm) * std::sin(th)};
-            TProj P;
+            TProj P{};
             P.ct = std::cos(th);
             P.st = std::sin(th);
-            P.w[0] = (float)(c[0] * c[0]); P.w[1] = (float)(c[1] * c[1]); P.w[2] = (float)(c[2] * c[2]);
-            P.w[3] = (float)(c[0] * c[1]); P.w[4] = (float)(c[0] * c[2]); P.w[5] = (float)(c[1] * c[2]);
+            if (np == 3) {
+                P.w[0] = (float)(P.st * P.st); P.w[1] = (float)(P.ct * P.ct); P.w[2] = (float)(P.st * P.ct);
+            } else {
+                P.w[0] = (float)(c[0] * c[0]); P.w[1] = (float)(c[1] * c[1]); P.w[2] = (float)(c[2] * c[2]);
+                P.w[3] = (float)(c[0] * c[1]); P.w[4] = (float)(c[0] * c[2]); P.w[5] = (float)(c[1] * c[2]);
+            }
             hp.push_back(P);
         }
     }
@@ -1894,12 +2029,13 @@ Toeplitz::Toeplitz(const std::vector<const Geom *> &gs, Dims3 d, int prec, cudaS
     LAMINO_CUDA(cudaMemcpyAsync(dg.p, hg.data(), hg.size() * sizeof(TGam), cudaMemcpyHostToDevice, s));
     LAMINO_CUDA(cudaMemcpyAsync(dp.p, hp.data(), hp.size() * sizeof(TProj), cudaMemcpyHostToDevice, s));
 
-    // kernel on the embedding grid, 6 pairs
-    DevBuf<float> T(6 * Lsize());
+    // kernel on the embedding grid
+    DevBuf<float> T(np * Lsize());
     LAMINO_CUDA(cudaMemsetAsync(T.p, 0, T.bytes(), s));
     int64_t cells = d.n1 * (2 * d.n2 - 1) * (2 * d.n3 - 1);
-    k_toeplitz_kernel<<<grid_for(cells, 256, 148LL * 64), 256, 0, s>>>(
-        T.p, L1, L2, L3, (int)d.n1, (int)d.n2, (int)d.n3, dg.p, (int)hg.size(), dp.p);
+    auto kern = np == 3 ? k_toeplitz_kernel<3> : k_toeplitz_kernel<6>;
+    kern<<<grid_for(cells, 256, 148LL * 64), 256, 0, s>>>(T.p, L1, L2, L3, (int)d.n1, (int)d.n2, (int)d.n3, dg.p,
+                                                          (int)hg.size(), dp.p);
     LAMINO_LAUNCH("k_toeplitz_kernel");
 
     // one-off uniform R2C per pair (cuFFT), real part stored in apply order
@@ -1908,35 +2044,45 @@ Toeplitz::Toeplitz(const std::vector<const Geom *> &gs, Dims3 d, int prec, cudaS
     r2c.make(3, n, CUFFT_R2C, 1);
     LAMINO_CUFFT(cufftSetStream(r2c.h, s));
     DevBuf<float2> spec(Ssize());
-    K.alloc(6 * Ssize());
     float norm = (float)(1.0 / ((double)L1 * L2 * L3));
-    for (int q = 0; q < 6; ++q) {
+    for (int q = 0; q < np; ++q) {
         LAMINO_CUFFT(cufftExecR2C(r2c.h, T.p + q * Lsize(), (cufftComplex *)spec.p));
         k_take_real_perm<<<grid_for(Ssize(), 256), 256, 0, s>>>(spec.p, (int)L1, (int)L2, (int)L3h, dnat1.p,
-                                                                 dnat2.p, q, norm, K.p);
+                                                                 dnat2.p, np, q, norm, out);
         LAMINO_LAUNCH("k_take_real_perm");
     }
-    T.release();
-    spec.release();
+    LAMINO_CUDA(cudaStreamSynchronize(s));  // the tables and buffers above go out of scope
+}
+
+Toeplitz::Toeplitz(const std::vector<const Geom *> &gs, Dims3 d, int prec, cudaStream_t s) : vol(d), precision(prec) {
+    if (gs.empty()) throw Error(ERR_ARG, "Toeplitz operator needs at least one geometry");
+    init_tables(d, prec);
+    K.alloc(6 * Ssize());
+    build_spectra(gs, 6, K.p, s);
     finish(s);
 }
 
-// Sum of operators over disjoint geometry sets: the kernel is linear in the
-// geometry, so its spectra add.
-Toeplitz::Toeplitz(const std::vector<const Toeplitz *> &parts, int prec, cudaStream_t s)
-    : vol(parts.empty() ? Dims3{0, 0, 0} : parts[0]->vol), precision(prec) {
-    if (parts.empty()) throw Error(ERR_ARG, "Toeplitz sum needs at least one operator");
-    for (const Toeplitz *t : parts) {
-        if (!t || !t->has_fp32()) throw Error(ERR_ARG, "Toeplitz sum needs operators with FP32 spectra");
-        if (t->vol.n1 != vol.n1 || t->vol.n2 != vol.n2 || t->vol.n3 != vol.n3)
-            throw Error(ERR_ARG, "Toeplitz sum needs operators of one volume size");
+Toeplitz::Toeplitz(PerDataset, const std::vector<const Geom *> &gs, Dims3 d, int prec, cudaStream_t s)
+    : vol(d), precision(prec) {
+    if (gs.empty()) throw Error(ERR_ARG, "Toeplitz operator needs at least one geometry");
+    init_tables(d, prec);
+    const int ng = (int)gs.size();
+    K3.alloc(ng * 3 * Ssize());
+    for (int g = 0; g < ng; ++g) {
+        tilt_sc.push_back((float)std::sin((double)gs[g]->gamma));
+        tilt_sc.push_back((float)std::cos((double)gs[g]->gamma));
+        build_spectra({gs[g]}, 3, K3.p + g * 3 * Ssize(), s);
     }
-    init_tables(vol, prec);
-    K.alloc(6 * Ssize());
-    LAMINO_CUDA(cudaMemcpyAsync(K.p, parts[0]->K.p, K.bytes(), cudaMemcpyDeviceToDevice, s));
-    for (size_t i = 1; i < parts.size(); ++i) {
-        k_add_into<<<grid_for(6 * Ssize(), 256), 256, 0, s>>>(K.p, parts[i]->K.p, 6 * Ssize());
-        LAMINO_LAUNCH("k_add_into");
+    qpart.alloc(L2 * L3h * 3 * std::min(ng, kMaxTilts));
+    // the sum's own spectra where a product over the datasets' would read more
+    // (3 per dataset against 6), or where they are wanted in half precision
+    if (ng > 2 || prec != PREC_FP32) {
+        DevBuf<float> sc(tilt_sc.size());
+        upload(sc.p, tilt_sc.data(), tilt_sc.size());
+        K.alloc(6 * Ssize());
+        k_sum_tilts<<<grid_for(Ssize(), 256), 256, 0, s>>>(K3.p, 3 * Ssize(), ng, sc.p, (int)L1, Ssize(), K.p);
+        LAMINO_LAUNCH("k_sum_tilts");
+        LAMINO_CUDA(cudaStreamSynchronize(s));
     }
     finish(s);
 }
@@ -1978,6 +2124,11 @@ void Toeplitz::finish(cudaStream_t s) {
     attr((const void *)k_pencil<true, 1458>, smem_pen);
     attr((const void *)k_pencil_quad<0>, smem_pen);
     attr((const void *)k_pencil_quad<1458>, smem_pen);
+    if (K3.p)
+        for (const void *f : {(const void *)k_pencil_tilts<0>, (const void *)k_pencil_tilts<1458>,
+                              (const void *)k_pencil_tilts<750>, (const void *)k_pencil_tilts<540>,
+                              (const void *)k_pencil_tilts<360>, (const void *)k_pencil_tilts<180>})
+            attr(f, smem_pen);
     for (const void *f : {(const void *)k_pencil<false, 750>, (const void *)k_pencil<true, 750>,
                           (const void *)k_pencil_quad<750>, (const void *)k_pencil<false, 540>,
                           (const void *)k_pencil<true, 540>, (const void *)k_pencil_quad<540>,
@@ -1992,7 +2143,7 @@ Toeplitz::~Toeplitz() {
 }
 
 size_t Toeplitz::device_bytes() const {
-    return K.bytes() + Kh.bytes() + Kscale.bytes() + z1.bytes() + xa.bytes() + tw1.bytes() + tw2.bytes() +
+    return K.bytes() + K3.bytes() + qpart.bytes() + Kh.bytes() + Kscale.bytes() + z1.bytes() + xa.bytes() + tw1.bytes() + tw2.bytes() +
            tw3.bytes() + twh3.bytes() + pos3.bytes();
 }
 
@@ -2132,7 +2283,81 @@ static void raise_rows_smem(int bytes) {
 #undef LAMINO_ROWS_ATTR
 }
 
+// the pencil step over datasets [g0, g0 + ng) (k_pencil_tilts)
+void Toeplitz::launch_tilts(int g0, int ng, bool apply, bool forms, cudaStream_t s) {
+    Tilts T{};
+    for (int g = 0; g < ng; ++g) {
+        T.K[g] = K3.p + (g0 + g) * 3 * Ssize();
+        T.sg[g] = tilt_sc[2 * (g0 + g)];
+        T.cg[g] = tilt_sc[2 * (g0 + g) + 1];
+    }
+    const unsigned gpen = (unsigned)(L2 * L3h);
+    const int smem_pen = 3 * (int)L1 * (int)sizeof(float2);
+    switch (ct1) {
+#define LAMINO_TILTS(N)                                                                                              \
+    case N:                                                                                                          \
+        k_pencil_tilts<N><<<gpen, pencil_threads(N), smem_pen, s>>>(xa.p, (int)vol.n1, (int)n1p, (int)L2, (int)L3h, f1, \
+                                                                    tw1.p, T, ng, apply, forms ? qpart.p : nullptr); \
+        break;
+        LAMINO_TILTS(1458)
+        LAMINO_TILTS(750)
+        LAMINO_TILTS(540)
+        LAMINO_TILTS(360)
+        LAMINO_TILTS(180)
+        LAMINO_TILTS(0)
+#undef LAMINO_TILTS
+        default: throw Error(ERR_STATE, "no pencil kernel for this length");
+    }
+    LAMINO_LAUNCH("k_pencil_tilts");
+}
+
+// n3 and n2 transforms of x into xa
+void Toeplitz::forward_spectra(const float *x3, cudaStream_t s) {
+    if (!z1.p || !xa.p) throw Error(ERR_STATE, "Toeplitz operator has no work buffers");
+    const int64_t nrows = 3 * vol.n1 * vol.n2;
+    const dim3 gd2((unsigned)((vol.n1 + D2_IB - 1) / D2_IB), (unsigned)((L3h + kb2 - 1) / kb2), 3);
+    launch_r2c(ct3, (unsigned)((nrows + rows1 - 1) / rows1), rows1, rows1 * (int)L3h * (int)sizeof(float2), s, x3, nrows,
+               (int)vol.n3, f3, pos3.p, twh3.p, z1.p);
+    LAMINO_LAUNCH("k_r2c_rows");
+    launch_dim2_fwd(ct2, gd2, kb2, d2_smem_values((int)L2, kb2) * (int)sizeof(float2), s, z1.p, (int)vol.n1, (int)vol.n2,
+                    (int)L3h, (int)n1p, f2, tw2.p, xa.p);
+    LAMINO_LAUNCH("k_dim2_fwd");
+}
+// the inverses, xa into y
+void Toeplitz::inverse_spectra(float *y3, cudaStream_t s) {
+    const int64_t nrows = 3 * vol.n1 * vol.n2;
+    const dim3 gd2((unsigned)((vol.n1 + D2_IB - 1) / D2_IB), (unsigned)((L3h + kb2 - 1) / kb2), 3);
+    launch_dim2_inv(ct2, gd2, kb2, d2_smem_values((int)L2, kb2) * (int)sizeof(float2), s, xa.p, (int)vol.n1, (int)vol.n2,
+                    (int)L3h, (int)n1p, f2, tw2.p, z1.p);
+    LAMINO_LAUNCH("k_dim2_inv");
+    launch_c2r(ct3, (unsigned)((nrows + rows1 - 1) / rows1), rows1, rows1 * (int)L3h * (int)sizeof(float2), s, z1.p, nrows,
+               (int)vol.n3, f3, pos3.p, twh3.p, y3);
+    LAMINO_LAUNCH("k_c2r_rows");
+}
+
+void Toeplitz::dataset_forms(const float *x3, double *acc, cudaStream_t s, float *y3) {
+    const int ng = (int)tilt_sc.size() / 2;
+    if (!K3.p) throw Error(ERR_STATE, "operator without per-dataset spectra");
+    const bool fused = y3 && ng <= kMaxTilts && precision != PREC_FP16;
+    if (y3 && !fused) apply(x3, y3, s);
+    forward_spectra(x3, s);
+    for (int g0 = 0; g0 < ng; g0 += kMaxTilts) {
+        const int m = std::min(kMaxTilts, ng - g0);
+        launch_tilts(g0, m, fused, true, s);
+        k_sum_pencils<<<3 * m, 512, 0, s>>>(qpart.p, L2 * L3h, 3 * m, acc + 3 * g0);
+        LAMINO_LAUNCH("k_sum_pencils");
+    }
+    if (fused) inverse_spectra(y3, s);
+}
+
 void Toeplitz::apply(const float *x3, float *y3, cudaStream_t s, bool low) {
+    const bool h = precision == PREC_FP16 || (precision == PREC_MIXED && low);
+    if (!h && !K.p) {  // at most two datasets, by their own spectra
+        forward_spectra(x3, s);
+        launch_tilts(0, (int)tilt_sc.size() / 2, true, false, s);
+        inverse_spectra(y3, s);
+        return;
+    }
     if (!z1.p || !xa.p) throw Error(ERR_STATE, "Toeplitz operator has no work buffers");
     const bool prof = profiling && (size_t)(nprof + 1) * (NSTAGE + 1) <= ev.size();
     cudaEvent_t *E = prof ? &ev[(size_t)nprof * (NSTAGE + 1)] : nullptr;
@@ -2151,7 +2376,6 @@ void Toeplitz::apply(const float *x3, float *y3, cudaStream_t s, bool low) {
     launch_dim2_fwd(ct2, gd2, kb2, smem_d2, s, z1.p, n1, n2, l3h, np1, f2, tw2.p, xa.p);
     LAMINO_LAUNCH("k_dim2_fwd");
     if (prof) LAMINO_CUDA(cudaEventRecord(E[2], s));
-    const bool h = precision == PREC_FP16 || (precision == PREC_MIXED && low);
     if (h) launch_pencil<true>(ct1, gpen, smem_pen, s, xa.p, n1, np1, l2, l3h, f1, tw1.p, nullptr, Kh.p, Kscale.p);
     else launch_pencil<false>(ct1, gpen, smem_pen, s, xa.p, n1, np1, l2, l3h, f1, tw1.p, K.p, nullptr, nullptr);
     LAMINO_LAUNCH("k_pencil");
@@ -2176,18 +2400,10 @@ void Toeplitz::quadforms(const float *x3, const std::vector<const Toeplitz *> &p
         if (t->vol.n1 != vol.n1 || t->vol.n2 != vol.n2 || t->vol.n3 != vol.n3)
             throw Error(ERR_ARG, "quadratic forms need operators of this volume size");
     }
-    const int64_t nrows = 3 * vol.n1 * vol.n2;
-    const unsigned grows = (unsigned)((nrows + rows1 - 1) / rows1);
-    const int smem_rows = rows1 * (int)L3h * (int)sizeof(float2);
-    const int smem_d2 = d2_smem_values((int)L2, kb2) * (int)sizeof(float2);
     const int smem_pen = 3 * (int)L1 * (int)sizeof(float2);
-    const dim3 gd2((unsigned)((vol.n1 + D2_IB - 1) / D2_IB), (unsigned)((L3h + kb2 - 1) / kb2), 3);
-    const int n1 = (int)vol.n1, n2 = (int)vol.n2, n3 = (int)vol.n3, l2 = (int)L2, l3h = (int)L3h, np1 = (int)n1p;
+    const int n1 = (int)vol.n1, l2 = (int)L2, l3h = (int)L3h, np1 = (int)n1p;
     const unsigned gpen = (unsigned)(L2 * L3h);
-    launch_r2c(ct3, grows, rows1, smem_rows, s, x3, nrows, n3, f3, pos3.p, twh3.p, z1.p);
-    LAMINO_LAUNCH("k_r2c_rows");
-    launch_dim2_fwd(ct2, gd2, kb2, smem_d2, s, z1.p, n1, n2, l3h, np1, f2, tw2.p, xa.p);
-    LAMINO_LAUNCH("k_dim2_fwd");
+    forward_spectra(x3, s);
     for (size_t g0 = 0; g0 < parts.size(); g0 += kMaxQuadSets) {
         QuadSets qs{};
         const int ng = (int)std::min<size_t>(kMaxQuadSets, parts.size() - g0);
@@ -2229,7 +2445,7 @@ std::map<std::array<int64_t, 4>, std::pair<int, int>> g_shape_cache;
 }  // namespace
 
 double Toeplitz::autotune(cudaStream_t s) {
-    const std::array<int64_t, 4> key{L1, L2, L3, (int64_t)precision};
+    const std::array<int64_t, 4> key{L1, L2, L3, (int64_t)precision + (K.p || Kh.p ? 0 : 16)};
     {
         std::lock_guard<std::mutex> lk(g_shape_mu);
         auto it = g_shape_cache.find(key);
@@ -2277,11 +2493,6 @@ double Toeplitz::autotune(cudaStream_t s) {
     std::lock_guard<std::mutex> lk(g_shape_mu);
     g_shape_cache[key] = {br, bk};
     return best;
-}
-
-void Toeplitz::drop_work() {
-    z1.release();
-    xa.release();
 }
 
 }  // namespace lamino

@@ -24,6 +24,12 @@ struct Toeplitz {
     // spectra in apply order: [(p2 * L3h + k3) * 6 + q][p1], p = DIF position of k
     DevBuf<float> K;             // fp32 storage
     DevBuf<__half> Kh;           // fp16 storage variant
+    // per-dataset form: [(p2 * L3h + k3) * 3 + q][p1] of every dataset (sin^2, cos^2
+    // and sin cos of its angles; see k_pencil_tilts), the sines and cosines of the
+    // datasets' gammas, and the pencils' partial quadratic forms
+    DevBuf<float> K3;
+    std::vector<float> tilt_sc;  // sin, cos of each gamma
+    DevBuf<double> qpart;
     DevBuf<float> Kscale;        // power-of-two scale per (p2, k3) pencil of Kh
     // FFT schedules and twiddles: dim 1 (length L1), dim 2 (L2), dim 3 (packed, M3)
     FftLen f1, f2, f3;
@@ -47,12 +53,17 @@ struct Toeplitz {
     std::vector<int> r1_, r2_;  // radix schedules of L1 and L2
     void init_tables(Dims3 d, int precision);
     void finish(cudaStream_t s);  // FP16 spectra, intermediates, launch shapes
+    void build_spectra(const std::vector<const Geom *> &gs, int np, float *out, cudaStream_t s);
+    void launch_tilts(int g0, int ng, bool apply, bool forms, cudaStream_t s);
+    void forward_spectra(const float *x3, cudaStream_t s);
+    void inverse_spectra(float *y3, cudaStream_t s);
 
   public:
 
     Toeplitz(const std::vector<const Geom *> &gs, Dims3 d, int precision, cudaStream_t s);
-    // the operator of the union of the parts' geometries, from their FP32 spectra
-    Toeplitz(const std::vector<const Toeplitz *> &parts, int precision, cudaStream_t s);
+    // the same operator that keeps each dataset's spectra, for dataset_forms
+    struct PerDataset {};
+    Toeplitz(PerDataset, const std::vector<const Geom *> &gs, Dims3 d, int precision, cudaStream_t s);
     ~Toeplitz();
     int64_t Lsize() const { return L1 * L2 * L3; }
     int64_t Ssize() const { return L1 * L2 * L3h; }
@@ -62,8 +73,10 @@ struct Toeplitz {
     // spectra, this volume size): one forward half-spectrum of x with this
     // operator's buffers, no inverse transform.  acc: device doubles.
     void quadforms(const float *x3, const std::vector<const Toeplitz *> &parts, double *acc, cudaStream_t s);
-    // free the work buffers of an operator kept only for its spectra
-    void drop_work();
+    // (PerDataset) acc[3 g + i] += x_i . (S_g x)_i for every dataset g, from one
+    // forward half-spectrum of x; with y3 also y = sum_g S_g x, in the same pass
+    // where the FP32 spectra of at most four datasets allow it
+    void dataset_forms(const float *x3, double *acc, cudaStream_t s, float *y3 = nullptr);
     // launch shape: rows per CTA of the n3 kernels, k3 values per CTA of the n2 kernels
     void set_shape(int rows, int kb);
     // time the valid launch shapes on this operator and keep the fastest; the
