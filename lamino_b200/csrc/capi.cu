@@ -490,7 +490,7 @@ int lamino_qggmrf(float *g, const float *x, int64_t n1, int64_t n2, int64_t n3, 
     Dims3 d = dims_of(n1, n2, n3);
     In<float> xi(x, d.size(), S(stream));
     Out<float> go(g, d.size(), S(stream), true);
-    qggmrf_add(go.d, xi.d, d, sigma, p, S(stream));
+    qggmrf_add(go.d, xi.d, d, 1, sigma, p, S(stream));
     go.finish(S(stream));
     API_END
 }

@@ -233,10 +233,10 @@ void MbirJob::prepare() {
     auto data_terms = [this, ngi, V](const float *xx, double *acc, cudaStream_t st) {
         for (int i = 0; i < 3; ++i) vec_dot(xx + i * V, yT_.p + i * V, V, acc + 3 * ngi + i, st);
     };
-    auto prior = [this, ng, n, V](const float *xx, float *g, cudaStream_t st) {
+    auto prior = [this, ng, n](const float *xx, float *g, cudaStream_t st) {
         k_axpy_scalar<<<grid_for(n, 256), 256, 0, st>>>(g, -ng, yT_.p, n);
         LAMINO_LAUNCH("k_axpy_scalar");
-        for (int i = 0; i < 3; ++i) qggmrf_add(g + i * V, xx + i * V, od_, prm_.sigma, prm_.p, st);
+        qggmrf_add(g, xx, od_, 3, prm_.sigma, prm_.p, st);
     };
     gGrad_.reset(new GraphedOp(
         [this, data_terms, prior](const float *xx, float *g, cudaStream_t st) {

@@ -227,13 +227,48 @@ struct QgConst {
     float inv_sq;      // 1 / sigma^q
     float at_zero;     // q / (sigma^q C)
 };
+// x^q for x > 0 as 2^(q log2 x): x = 2^e m with m in [1/sqrt 2, sqrt 2),
+// log2 m = f P(f), f = m - 1, and 2^z = Q(z) on [-1/2, 1/2], P and Q polynomials of
+// degree 8 and 6 fitted to the functions in the largest error (4e-8 and 2e-9;
+// Lawson's reweighted least squares); the product q e is kept to twice float
+// precision, so the result's error is that of a float: 2.9e-8 rms and at most
+// 1.1e-7 relative over x in [1e-9, 1e4], q in [-0.3, 0.9] (against double;
+// rounding alone has 2.5e-8 rms).  powf takes x that is not a normal number and
+// results near the ends of the float range.
+__device__ __forceinline__ float pow_pos(float x, float q) {
+    const int b = __float_as_int(x);
+    const int e = (b - 0x3f3504f3) >> 23;
+    const float f = __int_as_float(b - (e << 23)) - 1.0f;
+    float p = 0.12926264f;
+    p = fmaf(p, f, -0.20893306f);
+    p = fmaf(p, f, 0.21521251f);
+    p = fmaf(p, f, -0.2386758f);
+    p = fmaf(p, f, 0.28793907f);
+    p = fmaf(p, f, -0.36071625f);
+    p = fmaf(p, f, 0.48091027f);
+    p = fmaf(p, f, -0.7213472f);
+    p = fmaf(p, f, 1.442695f);
+    const float ef = (float)e, ph = q * ef, low = fmaf(q, f * p, fmaf(q, ef, -ph));
+    const float t = ph + low, rm = t + 12582912.0f;  // 1.5 * 2^23: the sum's low bits are rint(t)
+    const float z = (ph - (rm - 12582912.0f)) + low;
+    float v = 0.00015478018f;
+    v = fmaf(v, z, 0.0013400431f);
+    v = fmaf(v, z, 0.009617995f);
+    v = fmaf(v, z, 0.05550327f);
+    v = fmaf(v, z, 0.24022652f);
+    v = fmaf(v, z, 0.6931472f);
+    v = fmaf(v, z, 1.0f);
+    if ((unsigned)b - 0x00800000u < 0x7f000000u && fabsf(t) < 120.0f)
+        return __int_as_float(__float_as_int(v) + (__float_as_int(rm) << 23));
+    return powf(x, q);
+}
 __device__ __forceinline__ float d_potential(float delta, const QgConst &k) {
     const float C = 0.001f;
     const float ad = fabsf(delta);
     if (!(ad > 0.f)) return k.at_zero;
-    const float t1 = powf(ad, k.qmp) * k.inv_sqp;
+    const float t1 = pow_pos(ad, k.qmp) * k.inv_sqp;
     const float t3 = C + t1;
-    const float r = 1.0f / t3;
+    const float r = __fdividef(1.0f, t3);
     const float a = delta * r * k.inv_sq;
     return a * (2.0f - k.qmp * t1 * r);
 }
@@ -245,51 +280,60 @@ __device__ __forceinline__ float d_potential(float delta, const QgConst &k) {
 // so the 13 "forward" directions (dx = +1, and dx = 0 with (dy, dz) after
 // (0, 0)) give every pair: the owner c keeps rho'(x[c+d] - x[c]) for its own
 // sum and leaves the other side's term in shared memory.  A CTA owns a tile of
-// QG_TJ x QG_TK columns (j, k) and marches through a run of planes i; its
+// TJ x QG_TK columns (j, k) and marches through a run of planes i; its
 // threads cover the tile plus a one-column halo, whose pairs reach into the
 // tile.  The 26 terms of every voxel are added in the reference's order (dx,
 // dy, dz from -1 to 1), as a direct 26-neighbour loop would add them.
-constexpr int QG_TJ = 12, QG_TK = 32;  // 476 threads, 42 KB of shared memory
-constexpr int QG_HJ = QG_TJ + 2, QG_HK = QG_TK + 2, QG_THREADS = QG_HJ * QG_HK;
+// Tiles start at the first interior column, and their height divides the interior
+// rows with the least halo (TJ: 14 rows for 44 thick, 10 for 22 and 32, 8 for 10).
+// Bound by instruction issue (13 powers per voxel).  Measured at 362 x 44 x 362,
+// sigma 1000, p 1.2: 262 us; 424 with powf, IEEE division and tiles of 12 from the
+// border in two waves of CTAs.
+constexpr int QG_TK = 32, QG_HK = QG_TK + 2;
+__host__ __device__ constexpr int qg_threads(int TJ) { return (TJ + 2) * QG_HK; }  // 340, 408, 476, 544 threads
+__host__ __device__ constexpr int qg_ctas(int TJ) { return TJ <= 8 ? 4 : TJ <= 12 ? 3 : 2; }  // resident per SM
 
-__global__ void __launch_bounds__(QG_THREADS) k_qggmrf_pairs(float *__restrict__ g, const float *__restrict__ x,
-                                                             int n1, int n2, int n3, QgConst kq) {
+template <int TJ>
+__global__ void __launch_bounds__(qg_threads(TJ), qg_ctas(TJ)) k_qggmrf_pairs(float *__restrict__ g, const float *__restrict__ x,
+                                                             int n1, int n2, int n3, int ncomp, QgConst kq) {
+    constexpr int QG_THREADS = qg_threads(TJ);
     __shared__ float q9[2][9][QG_THREADS];  // other-side terms of the dx = +1 pairs, planes i - 1 and i
     __shared__ float q4[4][QG_THREADS];     // other-side terms of the dx = 0 forward pairs, plane i
     const int t = threadIdx.x;
     const int tx = t % QG_HK, ty = t / QG_HK;
-    const int k = blockIdx.x * QG_TK - 1 + tx, j = blockIdx.y * QG_TJ - 1 + ty;
-    const bool col = j >= 0 && j < n2 && k >= 0 && k < n3;
-    const bool fin = tx >= 1 && tx <= QG_TK && ty >= 1 && ty <= QG_TJ && j >= 1 && j <= n2 - 2 && k >= 1 &&
-                     k <= n3 - 2;
+    const int k = blockIdx.x * QG_TK + tx, j = blockIdx.y * TJ + ty;
+    const bool col = j < n2 && k < n3;
+    const bool fin = tx >= 1 && tx <= QG_TK && ty >= 1 && ty <= TJ && j <= n2 - 2 && k <= n3 - 2;
     const int64_t sj = n3, si = (int64_t)n2 * n3;
-    const PlaneRun pr(n1);
+    // the components' runs of planes follow one another along z
+    const int runs = (int)gridDim.z / ncomp, comp = (int)blockIdx.z / runs, run = (int)blockIdx.z - comp * runs;
+    const int per = (n1 + runs - 1) / runs, z0 = run * per, z1 = min(n1, z0 + per);
+    x += comp * si * n1;
+    g += comp * si * n1;
     float p9[9], p4[4];
     // own derivatives of plane i's forward pairs; other sides into shared memory
+    // (neighbours beyond the volume are read at the border instead: no interior
+    // voxel uses their pairs)
+    const int ym = j > 0 ? -(int)sj : 0, yp = j < n2 - 1 ? (int)sj : 0, zm = k > 0 ? -1 : 0, zp = k < n3 - 1 ? 1 : 0;
     auto pairs = [&](int i, int buf, bool with4) {
         if (!col || i < 0 || i >= n1) return;
-        const int64_t c = i * si + j * sj + k;
-        const float u = x[c];
+        const float *xc = x + (i * si + j * sj + k);
+        const float u = xc[0];
         if (i + 1 < n1) {
+            const float *xn = xc + si;
 #pragma unroll
-            for (int dy = -1; dy < 2; ++dy)
-#pragma unroll
-                for (int dz = -1; dz < 2; ++dz) {
-                    const int e = (dy + 1) * 3 + (dz + 1);
-                    if (j + dy < 0 || j + dy >= n2 || k + dz < 0 || k + dz >= n3) continue;
-                    const float delta = x[c + si + dy * sj + dz] - u;
-                    const float pv = d_potential(delta, kq);
-                    p9[e] = pv;
-                    q9[buf][e][t] = !(fabsf(delta) > 0.f) ? kq.at_zero : -pv;
-                }
+            for (int e = 0; e < 9; ++e) {
+                const float delta = xn[(e / 3 == 0 ? ym : e / 3 == 1 ? 0 : yp) + (e % 3 == 0 ? zm : e % 3 == 1 ? 0 : zp)] - u;
+                const float pv = d_potential(delta, kq);
+                p9[e] = pv;
+                q9[buf][e][t] = !(fabsf(delta) > 0.f) ? kq.at_zero : -pv;
+            }
         }
         if (with4) {
-            const int dys[4] = {0, 1, 1, 1}, dzs[4] = {1, -1, 0, 1};
+            const int off[4] = {zp, yp + zm, yp, yp + zp};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int dy = dys[e], dz = dzs[e];
-                if (j + dy >= n2 || k + dz < 0 || k + dz >= n3) continue;
-                const float delta = x[c + dy * sj + dz] - u;
+                const float delta = xc[off[e]] - u;
                 const float pv = d_potential(delta, kq);
                 p4[e] = pv;
                 q4[e][t] = !(fabsf(delta) > 0.f) ? kq.at_zero : -pv;
@@ -297,8 +341,8 @@ __global__ void __launch_bounds__(QG_THREADS) k_qggmrf_pairs(float *__restrict__
         }
     };
     int buf = 0;
-    pairs(pr.z0 - 1, buf, false);  // plane z0 - 1's dx = +1 pairs feed plane z0
-    for (int i = pr.z0; i < pr.z1; ++i) {
+    pairs(z0 - 1, buf, false);  // plane z0 - 1's dx = +1 pairs feed plane z0
+    for (int i = z0; i < z1; ++i) {
         buf ^= 1;
         pairs(i, buf, true);
         __syncthreads();
@@ -332,7 +376,7 @@ __global__ void __launch_bounds__(QG_THREADS) k_qggmrf_pairs(float *__restrict__
     }
 }
 
-void qggmrf_add(float *g, const float *x, Dims3 d, float sigma, float p, cudaStream_t s) {
+void qggmrf_add(float *g, const float *x, Dims3 d, int ncomp, float sigma, float p, cudaStream_t s) {
     if (d.n1 < 3 || d.n2 < 3 || d.n3 < 3) return;  // no interior voxels
     float sigma_q = std::pow(sigma, 2.0f);
     float sigma_qp = std::pow(sigma, 2.0f - p);
@@ -341,11 +385,20 @@ void qggmrf_add(float *g, const float *x, Dims3 d, float sigma, float p, cudaStr
     kq.inv_sqp = (float)(1.0 / (double)sigma_qp);
     kq.inv_sq = (float)(1.0 / (double)sigma_q);
     kq.at_zero = (float)(2.0 / ((double)sigma_q * 0.001));
-    if (d.n2 > (int64_t)65535 * QG_TJ) throw Error(ERR_ARG, "n2 too large for the qGGMRF kernel");
-    const int64_t gx = (d.n3 + QG_TK - 1) / QG_TK, gy = (d.n2 + QG_TJ - 1) / QG_TJ;
-    const int64_t gz = std::max<int64_t>(1, std::min<int64_t>({d.n1, 65535, 148LL * 6 / (gx * gy) + 1}));
-    k_qggmrf_pairs<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), QG_THREADS, 0, s>>>(g, x, (int)d.n1, (int)d.n2,
-                                                                                        (int)d.n3, kq);
+    // tile height: the fewest rows formed, halos included
+    int TJ = 8;
+    for (int t : {10, 12, 14})
+        if ((d.n2 - 2 + t - 1) / t * (t + 2) <= (d.n2 - 2 + TJ - 1) / TJ * (TJ + 2)) TJ = t;
+    if (d.n2 - 2 > (int64_t)65535 * TJ) throw Error(ERR_ARG, "n2 too large for the qGGMRF kernel");
+    const int64_t gx = (d.n3 - 2 + QG_TK - 1) / QG_TK, gy = (d.n2 - 2 + TJ - 1) / TJ;
+    // runs of planes: six waves of CTAs (with two, the CTAs at the border leave
+    // the last one uneven: 316 against 274 us), a run not shorter than 4 planes,
+    // as its first plane's pairs are also formed by the run before
+    const int64_t cols = gx * gy * ncomp, resident = 148LL * qg_ctas(TJ);
+    const int64_t runs = std::max<int64_t>(1, std::min<int64_t>({(d.n1 + 3) / 4, 65535 / ncomp, 6 * resident / cols}));
+    auto kern = TJ == 8 ? k_qggmrf_pairs<8> : TJ == 10 ? k_qggmrf_pairs<10> : TJ == 12 ? k_qggmrf_pairs<12> : k_qggmrf_pairs<14>;
+    kern<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)(runs * ncomp)), qg_threads(TJ), 0, s>>>(
+        g, x, (int)d.n1, (int)d.n2, (int)d.n3, ncomp, kq);
     LAMINO_LAUNCH("k_qggmrf_pairs");
 }
 

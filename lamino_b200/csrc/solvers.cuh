@@ -36,7 +36,8 @@ void vec_sqdist3(const float *x, const float *y, int64_t V, double *out3, cudaSt
 void vec_max(const float *x, int64_t n, double *out, cudaStream_t s);
 
 // ---- regularisers / finite differences (one component of dims d) ----
-void qggmrf_add(float *g, const float *x, Dims3 d, float sigma, float p, cudaStream_t s);
+// ncomp components of dims d each, one after another
+void qggmrf_add(float *g, const float *x, Dims3 d, int ncomp, float sigma, float p, cudaStream_t s);
 void grad_u(const float *u, Dims3 d, float *out3, cudaStream_t s);
 void divergence(const float *du3, Dims3 d, float *out, cudaStream_t s);
 void laplacian_axpy(float *y, float mu, const float *u, Dims3 d, cudaStream_t s);  // y += mu*lap(u)
