@@ -386,10 +386,9 @@ __device__ __forceinline__ void fft_inverse(float2 *data, int P, int ps, const F
 
 // ---- compile-time schedules for the lengths of the common problem sizes ----
 // (729 = packed n3 transform and 1458 = n1 transform of a 721-voxel axis; 144 =
-// n2 transform of a 71-voxel axis; 180, 360 = n1 transforms of the 90- and
-// 180-voxel lateral axes of 64- and 128-wide reconstructions; 20, 48, 64, 90 =
-// n2 transforms of their 10- to 44-voxel thickness axes; 540 and 750 run in two
-// register stages instead).
+// n2 transform of a 71-voxel axis; 20, 48, 64, 90 = n2 transforms of the 10- to
+// 44-voxel thickness axes of 64- to 256-wide reconstructions, whose n1 transforms
+// of 180, 360, 540 and 750 run in two register stages instead).
 // Each equals the runtime schedule fft_schedule(N, true), so the DIF output
 // positions are the same either way.  Other lengths use the runtime path above.
 constexpr int CT_MAX_STAGES = 6;
@@ -412,16 +411,6 @@ template <>
 struct CtSched<144> {
     static constexpr int ns = 3;
     static constexpr int r[CT_MAX_STAGES] = {2, 8, 9, 0, 0, 0};
-};
-template <>
-struct CtSched<180> {
-    static constexpr int ns = 4;
-    static constexpr int r[CT_MAX_STAGES] = {2, 2, 9, 5, 0, 0};
-};
-template <>
-struct CtSched<360> {
-    static constexpr int ns = 4;
-    static constexpr int r[CT_MAX_STAGES] = {2, 4, 9, 5, 0, 0};
 };
 // n2 transforms of the 10-, 22-, 32- and 44-voxel thickness axes
 template <>

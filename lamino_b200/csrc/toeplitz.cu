@@ -229,6 +229,19 @@ __device__ __forceinline__ void rows729_store(const float2 *__restrict__ sm, int
 // ---- register DFTs of composite lengths (two-stage row and pencil transforms) ----
 // cos / sin of 2 pi m / R for the composite register DFTs (R = 15, 18, 25)
 __host__ __device__ constexpr float wr_c(int R, int m) {
+    if (R == 10) {
+        constexpr float t[10] = {
+        1.0f, 0.8090169943749475f, 0.30901699437494745f, -0.30901699437494734f, -0.8090169943749473f,
+        -1.0f, -0.8090169943749476f, -0.30901699437494756f, 0.30901699437494723f, 0.8090169943749473f};
+        return t[m];
+    }
+    if (R == 12) {
+        constexpr float t[12] = {
+        1.0f, 0.8660254037844387f, 0.5000000000000001f, 0.0f, -0.4999999999999998f,
+        -0.8660254037844387f, -1.0f, -0.8660254037844388f, -0.5000000000000004f, 0.0f,
+        0.5000000000000001f, 0.8660254037844384f};
+        return t[m];
+    }
     if (R == 18) {
         constexpr float t[18] = {
         1.0f, 0.9396926207859084f, 0.766044443118978f, 0.5000000000000001f, 0.17364817766693041f,
@@ -258,6 +271,19 @@ __host__ __device__ constexpr float wr_c(int R, int m) {
     return 1.f;
 }
 __host__ __device__ constexpr float wr_s(int R, int m) {
+    if (R == 10) {
+        constexpr float t[10] = {
+        0.0f, 0.5877852522924731f, 0.9510565162951535f, 0.9510565162951536f, 0.5877852522924732f,
+        0.0f, -0.587785252292473f, -0.9510565162951535f, -0.9510565162951536f, -0.5877852522924734f};
+        return t[m];
+    }
+    if (R == 12) {
+        constexpr float t[12] = {
+        0.0f, 0.49999999999999994f, 0.8660254037844386f, 1.0f, 0.8660254037844387f,
+        0.49999999999999994f, 0.0f, -0.4999999999999997f, -0.8660254037844384f, -1.0f,
+        -0.8660254037844386f, -0.5000000000000004f};
+        return t[m];
+    }
     if (R == 18) {
         constexpr float t[18] = {
         0.0f, 0.3420201433256687f, 0.6427876096865393f, 0.8660254037844386f, 0.984807753012208f,
@@ -322,6 +348,8 @@ __device__ __forceinline__ void dft_reg(float2 (&v)[R]) {
     else if constexpr (R == 25) dft_cs<5, 5, INV>(v);
     else if constexpr (R == 15) dft_cs<3, 5, INV>(v);
     else if constexpr (R == 18) dft_cs<2, 9, INV>(v);
+    else if constexpr (R == 12) dft_cs<3, 4, INV>(v);
+    else if constexpr (R == 10) dft_cs<2, 5, INV>(v);
     else dft_small<R, INV>(v);
 }
 
@@ -1235,14 +1263,20 @@ __device__ __forceinline__ void p1458_inverse(const PencilRows &rows, const floa
 // forms its A-point DFT, multiplies output k by w^{n (2k + h)} and stores it at
 // position A B h + n + B k; lane m < A then runs the B-point DFT of block m in
 // place.  DIF positions: fft_positions(L, {2, A, B}).
+// Its threads take the items of a stage in a row (unit (h, c) major: 6 B in the
+// stage over A values, 6 A in the other), so that all lanes but the last few work;
+// a warp per (c, h) left 14 to 17 of 32 idle at 540.  Pencil at the padded sizes of
+// the batched mix, before -> after: 540 186 -> 129 us (270 x 32 x 270), 750 433 ->
+// 338 us (362 x 44 x 362); 360 and 180, then shared-memory schedules, 68 -> 47 us
+// (180 x 22 x 180) and 14 -> 12 us (90 x 10 x 90).
 template <int A, int B>
 __device__ __forceinline__ void p2s_forward(const PencilRows &rows, const float2 *__restrict__ tw,
                                             float2 *__restrict__ sm) {
     constexpr int M = A * B, L = 2 * M;
-    const int w = threadIdx.x >> 5, n = threadIdx.x & 31;
-    const int c = w >> 1, h = w & 1;
-    float2 *half = sm + c * L + h * M;
-    if (n < B) {
+    const int t = threadIdx.x;
+    if (t < 6 * B) {
+        const int u = t / B, n = t - u * B, h = u / 3, c = u - 3 * h;
+        float2 *half = sm + c * L + h * M;
         float2 v[A];
 #pragma unroll
         for (int j = 0; j < A; ++j) v[j] = rows.get(c, n + B * j);
@@ -1256,8 +1290,8 @@ __device__ __forceinline__ void p2s_forward(const PencilRows &rows, const float2
         for (int k = 0; k < A; ++k) half[n + B * k] = v[k];
     }
     __syncthreads();
-    if (n < A) {
-        float2 *row = half + B * n;
+    if (t < 6 * A) {
+        float2 *row = sm + B * t;  // the blocks of B positions follow one another
         float2 v[B];
 #pragma unroll
         for (int j = 0; j < B; ++j) v[j] = row[j];
@@ -1267,18 +1301,13 @@ __device__ __forceinline__ void p2s_forward(const PencilRows &rows, const float2
     }
     __syncthreads();
 }
-
-// Its inverse and the pruned store of the first n1 values (the caller
-// synchronises after writing the spectrum).
 template <int A, int B>
 __device__ __forceinline__ void p2s_inverse(const PencilRows &rows, const float2 *__restrict__ tw,
                                             float2 *__restrict__ sm) {
     constexpr int M = A * B, L = 2 * M;
-    const int w = threadIdx.x >> 5, n = threadIdx.x & 31;
-    const int c = w >> 1, h = w & 1;
-    float2 *half = sm + c * L + h * M;
-    if (n < A) {
-        float2 *row = half + B * n;
+    const int t = threadIdx.x;
+    if (t < 6 * A) {
+        float2 *row = sm + B * t;
         float2 v[B];
 #pragma unroll
         for (int k = 0; k < B; ++k) v[k] = row[k];
@@ -1287,8 +1316,11 @@ __device__ __forceinline__ void p2s_inverse(const PencilRows &rows, const float2
         for (int j = 0; j < B; ++j) row[j] = v[j];
     }
     __syncthreads();
+    const int u = t / B, n = t - u * B, h = u / 3, c = u - 3 * h;
+    const bool on = t < 6 * B;
+    float2 *half = sm + c * L + h * M;
     float2 v[A];
-    if (n < B) {
+    if (on) {
 #pragma unroll
         for (int k = 0; k < A; ++k) v[k] = half[n + B * k];
         twiddle_lin<A, true>(tw, 2 * n, L, h ? __ldg(tw + n) : make_float2(1.f, 0.f), v);
@@ -1299,7 +1331,7 @@ __device__ __forceinline__ void p2s_inverse(const PencilRows &rows, const float2
         }
     }
     __syncthreads();
-    if (h == 0 && n < B) {
+    if (on && h == 0) {
         const float2 *other = half + M;
 #pragma unroll
         for (int j = 0; j < A; ++j) {
@@ -1326,17 +1358,30 @@ struct TwoStage<540> {
     static constexpr bool on = true;
     static constexpr int A = 15, B = 18;
 };
-// (360 as 12 x 15 and 180 as 9 x 10 were slower than their compile-time
-// shared-memory schedules: too few lanes busy per warp)
-// threads of a pencil CTA: six warps for the register-stage lengths, 256 otherwise
+template <>
+struct TwoStage<360> {
+    static constexpr bool on = true;
+    static constexpr int A = 12, B = 15;
+};
+template <>
+struct TwoStage<180> {
+    static constexpr bool on = true;
+    static constexpr int A = 9, B = 10;
+};
+// threads of a pencil CTA and the CTAs per SM its registers are held to
 __host__ __device__ constexpr int pencil_threads(int L) {
-    return (L == 1458 || L == 750 || L == 540) ? P1458_THREADS : 256;
+    return L == 1458 ? P1458_THREADS : L == 750 ? 160 : L == 540 ? 128 : L == 360 ? 96 : L == 180 ? 64 : 256;
+}
+__host__ __device__ constexpr int pencil_ctas(int L) {
+    return L == 750 ? 5 : L == 540 ? 6 : L == 360 ? 8 : L == 180 ? 12 : 4;
 }
 // the register-stage schedule (2, A, B) of an n1 length, empty when it has none
 static std::vector<int> two_stage_schedule(int L) {
     switch (L) {
         case 750: return {2, TwoStage<750>::A, TwoStage<750>::B};
         case 540: return {2, TwoStage<540>::A, TwoStage<540>::B};
+        case 360: return {2, TwoStage<360>::A, TwoStage<360>::B};
+        case 180: return {2, TwoStage<180>::A, TwoStage<180>::B};
         default: return {};
     }
 }
@@ -1353,10 +1398,6 @@ __device__ __forceinline__ void pencil_forward(float2 *pv, int64_t cs, int n1, c
         p1458_forward(PencilRows{pv, cs, n1}, tw1, sm);
     } else if constexpr (TwoStage<N1>::on) {
         p2s_forward<TwoStage<N1>::A, TwoStage<N1>::B>(PencilRows{pv, cs, n1}, tw1, sm);
-    } else if constexpr (N1 != 0) {  // compile-time schedule: lead stages in registers, the rest fixed
-        fftlead_load<CtSched<N1>::r[1]>(PencilRows{pv, cs, n1}, tw1, sm, N1, N1, threadIdx.x, blockDim.x);
-        __syncthreads();
-        ct_forward<N1, 2>(sm, 3, N1, tw1, threadIdx.x, blockDim.x);
     } else if (F1.ns >= 2) {  // runtime length: the outer stages in registers as well
         fftlead_any<false>(PencilRows{pv, cs, n1}, F1, sm, L1, threadIdx.x, blockDim.x);
         __syncthreads();
@@ -1393,9 +1434,6 @@ __device__ __forceinline__ void pencil_inverse(float2 *pv, int64_t cs, int n1, c
         p1458_inverse(PencilRows{pv, cs, n1}, tw1, sm);
     } else if constexpr (TwoStage<N1>::on) {
         p2s_inverse<TwoStage<N1>::A, TwoStage<N1>::B>(PencilRows{pv, cs, n1}, tw1, sm);
-    } else if constexpr (N1 != 0) {
-        ct_inverse<N1, CtSched<N1>::ns - 1, 2>(sm, 3, N1, tw1, threadIdx.x, blockDim.x);
-        fftlead_store<CtSched<N1>::r[1]>(PencilRows{pv, cs, n1}, tw1, sm, N1, N1, threadIdx.x, blockDim.x);
     } else if (F1.ns >= 2) {
         fft_inverse(sm, 3, L1, F1, 2, threadIdx.x, blockDim.x);
         fftlead_any<true>(PencilRows{pv, cs, n1}, F1, sm, L1, threadIdx.x, blockDim.x);
@@ -1413,7 +1451,7 @@ __device__ __forceinline__ void pencil_inverse(float2 *pv, int64_t cs, int n1, c
 // In place on xa.  N1: compile-time L1 or 0.  At L1 = 1458, five CTAs of 256
 // threads per SM (48 registers, 35 KB of shared memory each); four otherwise.
 template <bool HALF, int N1>
-__global__ void __launch_bounds__(pencil_threads(N1), 4) k_pencil(float2 *__restrict__ xa, int n1, int n1p, int L2, int L3h, FftLen F1,
+__global__ void __launch_bounds__(pencil_threads(N1), pencil_ctas(N1)) k_pencil(float2 *__restrict__ xa, int n1, int n1p, int L2, int L3h, FftLen F1,
                                                 const float2 *__restrict__ tw1, const float *__restrict__ K,
                                                 const __half *__restrict__ Kh, const float *__restrict__ kscale) {
     extern __shared__ float2 sm[];
@@ -1431,7 +1469,7 @@ __global__ void __launch_bounds__(pencil_threads(N1), 4) k_pencil(float2 *__rest
     const float sc = HALF ? kscale[pen] : 1.f;
     // two adjacent positions per thread (L1 is even): 8-byte spectrum loads and
     // 16-byte shared accesses; KU pairs whose 6 spectra are in flight together
-    constexpr int KU = 2;
+    constexpr int KU = TwoStage<N1>::on && (N1 / 2 + pencil_threads(N1) - 1) / pencil_threads(N1) == 3 ? 3 : 2;
     const int L1h = L1 / 2;
     for (int q0 = threadIdx.x; q0 < L1h; q0 += KU * blockDim.x) {
         float2 kv[KU][6];
@@ -1564,12 +1602,12 @@ struct Tilts {
     float sg[kMaxTilts], cg[kMaxTilts];
 };
 template <int N1>
-__global__ void __launch_bounds__(pencil_threads(N1), pencil_threads(N1) == 256 ? 3 : 4) k_pencil_tilts(float2 *__restrict__ xa, int n1, int n1p, int L2,
+__global__ void __launch_bounds__(pencil_threads(N1), N1 ? pencil_ctas(N1) : 3) k_pencil_tilts(float2 *__restrict__ xa, int n1, int n1p, int L2,
                                                                       int L3h, FftLen F1, const float2 *__restrict__ tw1,
                                                                       Tilts T, int ng, bool apply,
                                                                       double *__restrict__ part) {
     extern __shared__ __align__(16) float2 sm[];
-    __shared__ float red[8][3 * kMaxTilts];
+    __shared__ float red[8][3 * kMaxTilts];  // (at most eight warps)
     const int64_t pen = blockIdx.x;
     const int L1 = N1 ? N1 : F1.n;
     const int64_t cs = (int64_t)L2 * L3h * n1p;
@@ -1923,13 +1961,6 @@ static bool ct_row_matches(int M, const std::vector<int> &r) {
         default: return false;
     }
 }
-static bool ct_schedule_matches(int L, const std::vector<int> &r) {  // n1 (pencil) lengths
-    switch (L) {
-        case 360: return ct_equal<360>(r);
-        case 180: return ct_equal<180>(r);
-        default: return false;
-    }
-}
 static bool ct_dim2_matches(int L, const std::vector<int> &r) {  // n2 lengths
     switch (L) {
         case 90: return ct_equal<90>(r);
@@ -2109,7 +2140,7 @@ void Toeplitz::finish(cudaStream_t s) {
     while (kb2 > 1 && d2_smem_values((int)L2, kb2) * (int64_t)sizeof(float2) > 160 * 1024) kb2 /= 2;
     if (d2_smem_values((int)L2, kb2) * (int64_t)sizeof(float2) > 200 * 1024)
         throw Error(ERR_ARG, "n2 too large for the n2-pass kernels");
-    ct1 = (L1 == 1458 || !two_stage_schedule((int)L1).empty() || ct_schedule_matches((int)L1, r1_)) ? (int)L1 : 0;
+    ct1 = (L1 == 1458 || !two_stage_schedule((int)L1).empty()) ? (int)L1 : 0;
     ct2 = (L2 == 144 || ct_dim2_matches((int)L2, r2_)) ? (int)L2 : 0;
     ct3 = (warp_rows((int)M3) || ct_row_matches((int)M3, fft_schedule((int)M3, false))) ? (int)M3 : 0;
     const int smem_rows = rows1 * (int)L3h * (int)sizeof(float2);
@@ -2188,8 +2219,8 @@ void Toeplitz::stage_bytes(int64_t *b) const {
     b[4] = Z + 3 * V * 4;                               // read z1, write y
 }
 
-// the pencil kernel of the operator's n1 length: compile-time schedules for the
-// lengths in CtSched (ct1), the runtime one otherwise (ct1 = 0)
+// the pencil kernel of the operator's n1 length: register stages for 1458 and the
+// TwoStage lengths (ct1), the runtime schedule otherwise (ct1 = 0)
 template <bool HALF>
 static void launch_pencil(int ct1, unsigned grid, int smem, cudaStream_t s, float2 *xa, int n1, int np1, int l2,
                           int l3h, const FftLen &f1, const float2 *tw1, const float *K, const __half *Kh,
