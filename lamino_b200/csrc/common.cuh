@@ -176,14 +176,17 @@ struct FftPlan {
         valid = false;
         work.release();
     }
-    // contiguous batched transform of rank 1-3 (cufftPlanMany with default layouts)
-    void make(int rank, int *n, cufftType type, int batch) {
+    // contiguous batched transform of rank 1-3 (cufftPlanMany with default layouts);
+    // stride > 0: 1-D transforms of elements `stride` apart, one after another
+    void make(int rank, int *n, cufftType type, int batch, int stride = 0) {
         reset();
         LAMINO_CUFFT(cufftCreate(&h));
         valid = true;
         LAMINO_CUFFT(cufftSetAutoAllocation(h, 0));
         size_t ws = 0;
-        LAMINO_CUFFT(cufftMakePlanMany(h, rank, n, nullptr, 1, 0, nullptr, 1, 0, type, batch, &ws));
+        int *embed = stride ? n : nullptr;
+        LAMINO_CUFFT(cufftMakePlanMany(h, rank, n, embed, stride ? stride : 1, stride ? 1 : 0, embed, stride ? stride : 1,
+                                       stride ? 1 : 0, type, batch, &ws));
         work.alloc(ws > 0 ? ws : 16);
         LAMINO_CUFFT(cufftSetWorkArea(h, work.p));
     }

@@ -26,10 +26,10 @@
 // 3.0e8 node values and 49 for 5.5e8 points, all of it contiguous along y or X,
 // in place of 343 taps per point from scattered tiles.
 // Measured on B200 against antipodal point pairs spread through 3-D tiles (the
-// form before): adjoint at that size 333.5 -> 36.7 ms, forward of 181 x 362^2
-// points from 362 x 44 x 362 19.5 -> 2.9 ms, sysmat of 2 x 91 x 309^2 points on
+// form before): adjoint at that size 333.5 -> 26.6 ms, forward of 181 x 362^2
+// points from 362 x 44 x 362 19.5 -> 2.45 ms, sysmat of 2 x 91 x 309^2 points on
 // 180 x 16 x 180 19.9 -> 1.29 ms, and no sort of the points on the first call
-// (adjoint of a new geometry 351 -> 41 ms).
+// (adjoint of a new geometry 351 -> 31 ms).
 //
 // The three components need one complex transform, not three.  The beam vector
 // (sin g sin th, cos th, cos g sin th) spans two dimensions:
@@ -126,8 +126,19 @@ NufftPlan::NufftPlan(Dims3 d, double eps_) : vol(d), eps(eps_) {
     // node grids are 0.9 to 1.2 fine grids for the detectors and volumes that the
     // MBIR drivers pad together
     work.alloc(nf() + nf() / 4);
+    // Modes fill the n1 planes [0, (n1 + 1) / 2) and the last n1 / 2 of the fine
+    // grid: with the transform along n1 last (type 2) or first (type 1) the other
+    // planes skip their 2-D transforms, half the passes along n3 and n2 (1458 x 1458
+    // x 144: 6.1 -> 4.5 ms).  Grids below 64 MB stay with one 3-D transform: they are
+    // bound by launches.
+    split3 = nf() >= (8 << 20);
     int n[3] = {(int)nf1, (int)nf3, (int)nf2};
-    fft3.make(3, n, CUFFT_C2C, 1);
+    if (split3) {
+        fft3.make(2, n + 1, CUFFT_C2C, (int)(d.n1 - d.n1 / 2));
+        fft3n1.make(1, n, CUFFT_C2C, (int)(nf3 * nf2), (int)(nf3 * nf2));
+    } else {
+        fft3.make(3, n, CUFFT_C2C, 1);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -306,6 +317,11 @@ __global__ void k_lat_deconv(const double2 *__restrict__ quad, int n1, int n3, d
     ipT[i] = (float)(1.0 / (w * p));
 }
 
+// place of a detector row where first halves are stored first (Lattice::half)
+__device__ __forceinline__ int64_t half_row(int p, int j, int np, int nr) {
+    const int jh = (nr + 1) / 2;
+    return j < jh ? (int64_t)p * jh + j : (int64_t)np * jh + (int64_t)p * (nr - jh) + (j - jh);
+}
 // the (T, y) position of detector row `id` = p nrows + j and its footprint
 struct RowPos {
     int p, j, lT, ly;
@@ -342,13 +358,13 @@ __global__ void __launch_bounds__(256) k_rows_count(GeomView g, bool raw, double
 }
 template <int W>
 __global__ void __launch_bounds__(256) k_rows_place(GeomView g, bool raw, double invh,
-                                                    int T0, int nstart, Fine F, uint32_t *__restrict__ cursor,
+                                                    bool half, int T0, int nstart, Fine F, uint32_t *__restrict__ cursor,
                                                     int4 *__restrict__ pt, float2 *__restrict__ pd) {
     const int n = g.nproj * g.nrows;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
         const RowPos r = row_pos<W>(g, raw, invh, T0, F, id);
         const uint32_t at = atomicAdd(cursor + (int64_t)r.ly * nstart + r.lT, 1u);
-        pt[at] = make_int4(id, r.lT, r.ly, r.p);
+        pt[at] = make_int4(half ? (int)half_row(r.p, r.j, g.nproj, g.nrows) : id, r.lT, r.ly, id);
         pd[at] = make_float2(r.dT, r.dy);
     }
 }
@@ -759,7 +775,8 @@ __global__ void __launch_bounds__(256) k_tiles_zero(const int *__restrict__ nite
 // cells, which the cell order gives as W + 3 runs (one per y start).  Writes
 // the node grid as [T][X][y], y fastest, four y at a time.  With SYM a row's
 // value is the projection spectrum of sysmat, formed from F at q and at -q:
-// the strength conj(a) 2 P / N = (F(q) / 2 + 2 conj(a)^2 conj F(-q)) / N.
+// the strength conj(a) 2 P / N = (F(q) / 2 + 2 conj(a)^2 conj F(-q)) / N.  With
+// HALF the source holds P of the first half of the rows (Lattice::half).
 //
 // Every projection passes through the origin, so the tiles there meet many
 // times the average of about 200 rows (all angles x 8 rows), and the walk over
@@ -768,21 +785,23 @@ __global__ void __launch_bounds__(256) k_tiles_zero(const int *__restrict__ nite
 // the others zeroed first and added to with vector atomics.
 // Measured (before: one CTA per tile, 256 threads of one column, tiles in row
 // order): 60 x 154^2 rows 186 -> 31 us, 2 x 91 x 309^2 (SYM) 1090 -> 340 us,
-// 361 x 1233^2 8.1 -> 6.7 ms.
+// 361 x 1233^2 8.1 -> 6.9 ms.
 constexpr int kCols = 2;   // columns per thread
 constexpr int kAhead = 4;  // rows in flight per thread
-template <int W, bool SYM>
-__global__ void __launch_bounds__(128) k_rows_spread(const int *__restrict__ nitem, const int2 *__restrict__ items,
+template <int W, int SRC>
+__global__ void __launch_bounds__(128, 4) k_rows_spread(const int *__restrict__ nitem, const int2 *__restrict__ items,
                                                      int seg, const uint32_t *__restrict__ start,
                                                      const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nstart,
                                                      int nT, int ntile, int nf2,
                                                      const float2 *__restrict__ src, int nr, int nc, float beta,
-                                                     const float2 *__restrict__ beam, float scale, float2 *__restrict__ Gt) {
+                                                     const float2 *__restrict__ beam, int np, bool half, float scale,
+                                                     float2 *__restrict__ Gt) {
+    constexpr bool SYM = SRC == NufftPlan::ROWS_SYSMAT, HALF = SRC == NufftPlan::ROWS_HALF;
     extern __shared__ __align__(16) unsigned char rsm[];
     const int cap = blockDim.x;  // rows listed at a time
     float4 *lw = reinterpret_cast<float4 *>(rsm);            // [row][kCell] weights, T by y
     uint2 *lr = reinterpret_cast<uint2 *>(lw + (cap + 2 * kAhead) * kCell);  // row's first value, mirrored row's last
-    float2 *lb = reinterpret_cast<float2 *>(lr + cap + 2 * kAhead);          // 2 conj(a)^2 / N
+    float4 *lb = reinterpret_cast<float4 *>(lr + cap + 2 * kAhead);          // factors of the row's value
     constexpr int NR = W + kCell - 1;
     __shared__ int beg[NR], pre[NR + 1];
     if ((int)blockIdx.x >= __ldg(nitem)) return;
@@ -832,11 +851,18 @@ __global__ void __launch_bounds__(128) k_rows_spread(const int *__restrict__ nit
                 const float s = es_tap<W>(d.x, c1 + i - I.y, beta);
                 lw[e * kCell + i] = make_float4(s * u[0], s * u[1], s * u[2], s * u[3]);
             }
-            const int j = I.x - I.w * nr;
-            lr[e] = make_uint2((uint32_t)I.x * nc, (uint32_t)(I.w * nr + nr - 1 - j) * nc + nc - 1);
-            if (SYM) {
-                const float2 a = beam[I.w];  // conj(a)^2 = (ax^2 - ay^2) - 2 i ax ay
-                lb[e] = make_float2(2 * scale * (a.x * a.x - a.y * a.y), -4 * scale * a.x * a.y);
+            const int p = I.w / nr, j = I.w - p * nr;
+            const uint32_t mirror = (uint32_t)(half ? half_row(p, nr - 1 - j, np, nr) : p * nr + nr - 1 - j) * nc + nc - 1;
+            lr[e] = make_uint2((uint32_t)I.x * nc, mirror);
+            if (SYM) {  // conj(a)^2 = (ax^2 - ay^2) - 2 i ax ay
+                const float2 a = beam[p];
+                lb[e] = make_float4(2 * scale * (a.x * a.x - a.y * a.y), -4 * scale * a.x * a.y, 0.f, 0.f);
+            }
+            if (HALF) {  // conj(a) v, or conj(a) conj(v) of the mirrored value for a second-half row
+                const float2 a = beam[p];
+                const bool second = j >= (nr + 1) / 2;
+                lb[e] = second ? make_float4(a.x, -a.y, -a.y, -a.x) : make_float4(a.x, a.y, -a.y, a.x);
+                if (second) lr[e].x = mirror | 0x80000000u;
             }
         }
         __syncthreads();
@@ -846,7 +872,8 @@ __global__ void __launch_bounds__(128) k_rows_spread(const int *__restrict__ nit
             const uint2 row = lr[q];
 #pragma unroll
             for (int c = 0; c < kCols; ++c) {
-                a[c] = __ldg(src + row.x + kc[c]);
+                if (HALF) a[c] = __ldg(src + (int64_t)(row.x & 0x7fffffffu) + ((int)row.x < 0 ? -kc[c] : kc[c]));
+                else a[c] = __ldg(src + row.x + kc[c]);
                 if (SYM) b[c] = __ldg(src + row.y - kc[c]);
             }
         };
@@ -860,8 +887,12 @@ __global__ void __launch_bounds__(128) k_rows_spread(const int *__restrict__ nit
 #pragma unroll
                 for (int c = 0; c < kCols; ++c) {
                     x[c] = v[u][c];
+                    if (HALF) {
+                        const float4 b = lb[q];
+                        x[c] = make_float2(b.x * x[c].x + b.y * x[c].y, b.z * x[c].x + b.w * x[c].y);
+                    }
                     if (SYM) {
-                        const float2 b = lb[q];
+                        const float4 b = lb[q];
                         x[c] = make_float2(fmaf(b.x, m[u][c].x, fmaf(b.y, m[u][c].y, 0.5f * scale * x[c].x)),
                                            fmaf(b.y, m[u][c].x, fmaf(-b.x, m[u][c].y, 0.5f * scale * x[c].y)));
                     }
@@ -954,6 +985,158 @@ __global__ void __launch_bounds__(256) k_proj_pre(const float *__restrict__ proj
     }
 }
 
+// The same with half the transforms (Lattice::half).  With the phases e^{-i pi m / n}
+// of a half-sample frequency offset, P(j, k) is the transform of a real array g, so
+// P(nr-1-j, nc-1-k) = conj P(j, k): along the rows' index two real columns are
+// transformed as one complex one, the half j < jh of the rows is separated from the
+// pairs, and only those rows are transformed along the columns.
+// g = 2 cos(b1 + b2) proj.  Pairs are stored z[projection, pair][m1], so that both
+// transforms are of contiguous data (the library's strided one took 1.5 times as
+// long); the kernels between transpose 32 x 32 tiles through shared memory.
+__device__ __forceinline__ float2 cmul(float2 a, float cr, float ci) {
+    return make_float2(a.x * cr - a.y * ci, a.x * ci + a.y * cr);
+}
+// CTA -> projection, first row and first pair of its tile
+__device__ __forceinline__ void half_tile(int rows, int nch, int64_t t, int &p, int &r0, int &c0) {
+    const int tc = (nch + 31) / 32, tr = (rows + 31) / 32;
+    const int64_t q = t / tc;
+    c0 = (int)(t - q * tc) * 32;
+    p = (int)(q / tr);
+    r0 = (int)(q - (int64_t)p * tr) * 32;
+}
+__global__ void __launch_bounds__(256) k_half_pre(const float *__restrict__ proj, int nr, int nc,
+                                                  const float4 *__restrict__ trow, const float4 *__restrict__ tcol,
+                                                  float2 *__restrict__ z) {
+    __shared__ float2 tile[32][33];
+    const int d1 = nr / 2, d2 = nc / 2, nch = (nc + 1) / 2;
+    int p, r0, c0;
+    half_tile(nr, nch, blockIdx.x, p, r0, c0);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int c = c0 + tx;
+    if (c < nch)
+        for (int r = ty; r < 32 && r0 + r < nr; r += 8) {
+            const int m1 = r0 + r;
+            int js = m1 + d1; if (js >= nr) js -= nr;
+            const float4 tr = __ldg(trow + m1);
+            const float *src = proj + ((int64_t)p * nr + js) * nc;
+            float f[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int m2 = 2 * c + h;
+                int ks = m2 + d2; if (ks >= nc) ks -= nc;
+                const float4 tc = __ldg(tcol + min(m2, nc - 1));
+                f[h] = m2 < nc ? src[ks] * 2.f * (tr.x * tc.x - tr.y * tc.y) : 0.f;
+            }
+            tile[r][tx] = cmul(make_float2(f[0], f[1]), tr.z, -tr.w);
+        }
+    __syncthreads();
+    const int m1 = r0 + tx;
+    if (m1 < nr)
+        for (int q = ty; q < 32 && c0 + q < nch; q += 8) z[((int64_t)p * nch + c0 + q) * nr + m1] = tile[tx][q];
+}
+__global__ void __launch_bounds__(256) k_half_unpack(const float2 *__restrict__ z, int nr, int nc,
+                                                     const float4 *__restrict__ tcol, float2 *__restrict__ S) {
+    __shared__ float2 tile[2][32][33];
+    const int nch = (nc + 1) / 2, jh = (nr + 1) / 2;
+    int p, r0, c0;
+    half_tile(jh, nch, blockIdx.x, p, r0, c0);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    if (r0 + tx < jh)
+        for (int q = ty; q < 32 && c0 + q < nch; q += 8) {
+            const float2 *row = z + ((int64_t)p * nch + c0 + q) * nr;
+            tile[0][q][tx] = row[r0 + tx];
+            tile[1][q][tx] = row[nr - 1 - r0 - tx];
+        }
+    __syncthreads();
+    const int c = c0 + tx;
+    if (c >= nch) return;
+    const float4 t0 = __ldg(tcol + 2 * c), t1 = __ldg(tcol + min(2 * c + 1, nc - 1));
+    for (int r = ty; r < 32 && r0 + r < jh; r += 8) {
+        const float2 a = tile[0][tx][r], b = tile[1][tx][r];
+        float2 *o = S + ((int64_t)p * jh + r0 + r) * nc + 2 * c;
+        o[0] = cmul(make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y)), t0.z, -t0.w);
+        if (2 * c + 1 < nc) o[1] = cmul(make_float2(0.5f * (a.y + b.y), -0.5f * (a.x - b.x)), t1.z, -t1.w);
+    }
+}
+// first-half rows P = a F(j, k) + conj(a F(nr-1-j, nc-1-k)), in place: a thread takes
+// columns k and nc-1-k of a row, the only ones that read what it overwrites
+__global__ void __launch_bounds__(256) k_half_combine(float2 *__restrict__ F, int np, int nr, int nc,
+                                                      const float2 *__restrict__ beam) {
+    const int jh = (nr + 1) / 2;
+    for (int64_t row = blockIdx.x; row < (int64_t)np * jh; row += gridDim.x) {
+        const int p = (int)(row / jh), j = (int)(row - (int64_t)p * jh);
+        const float2 a = __ldg(beam + p);
+        float2 *f = F + row * nc;
+        const float2 *m = F + half_row(p, nr - 1 - j, np, nr) * nc;
+        for (int k = threadIdx.x; k < (nc + 1) / 2; k += blockDim.x) {
+            const int k2 = nc - 1 - k;
+            const float2 u = cmul(f[k], a.x, a.y), u2 = cmul(f[k2], a.x, a.y), v = cmul(m[k], a.x, a.y),
+                         v2 = cmul(m[k2], a.x, a.y);
+            f[k] = make_float2(u.x + v2.x, u.y - v2.y);
+            f[k2] = make_float2(u2.x + v.x, u2.y - v.y);
+        }
+    }
+}
+__global__ void __launch_bounds__(256) k_half_pack(const float2 *__restrict__ S, int nr, int nc,
+                                                   const float4 *__restrict__ tcol, float2 *__restrict__ z) {
+    __shared__ float2 tile[2][32][33];
+    const int nch = (nc + 1) / 2, jh = (nr + 1) / 2;
+    int p, r0, c0;
+    half_tile(jh, nch, blockIdx.x, p, r0, c0);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int c = c0 + tx;
+    if (c < nch) {
+        const float4 t0 = __ldg(tcol + 2 * c), t1 = __ldg(tcol + min(2 * c + 1, nc - 1));
+        for (int r = ty; r < 32 && r0 + r < jh; r += 8) {
+            const float2 *s = S + ((int64_t)p * jh + r0 + r) * nc + 2 * c;
+            const float2 a = cmul(s[0], t0.z, t0.w);
+            const float2 b = 2 * c + 1 < nc ? cmul(s[1], t1.z, t1.w) : make_float2(0.f, 0.f);
+            tile[0][r][tx] = make_float2(a.x - b.y, a.y + b.x);  // a + i b
+            tile[1][r][tx] = make_float2(a.x + b.y, b.x - a.y);  // conj a + i conj b
+        }
+    }
+    __syncthreads();
+    const int j = r0 + tx;
+    if (j < jh)
+        for (int q = ty; q < 32 && c0 + q < nch; q += 8) {
+            float2 *row = z + ((int64_t)p * nch + c0 + q) * nr;
+            row[j] = tile[0][tx][q];
+            if (nr - 1 - j != j) row[nr - 1 - j] = tile[1][tx][q];
+        }
+}
+__global__ void __launch_bounds__(256) k_half_post(const float2 *__restrict__ z, int nr, int nc,
+                                                   const float4 *__restrict__ trow, const float4 *__restrict__ tcol,
+                                                   float scale, float *__restrict__ proj) {
+    __shared__ float2 tile[32][33];
+    const int d1 = nr / 2, d2 = nc / 2, nch = (nc + 1) / 2;
+    int p, r0, c0;
+    half_tile(nr, nch, blockIdx.x, p, r0, c0);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    if (r0 + tx < nr) {
+        const float4 tr = __ldg(trow + r0 + tx);
+        for (int q = ty; q < 32 && c0 + q < nch; q += 8)
+            tile[q][tx] = cmul(z[((int64_t)p * nch + c0 + q) * nr + r0 + tx], tr.z, tr.w);
+    }
+    __syncthreads();
+    const int c = c0 + tx;
+    if (c >= nch) return;
+    for (int r = ty; r < 32 && r0 + r < nr; r += 8) {
+        const int m1 = r0 + r;
+        int js = m1 + d1; if (js >= nr) js -= nr;
+        const float4 tr = __ldg(trow + m1);
+        const float2 v = tile[tx][r];
+        float *o = proj + ((int64_t)p * nr + js) * nc;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m2 = 2 * c + h;
+            if (m2 >= nc) break;
+            int ks = m2 + d2; if (ks >= nc) ks -= nc;
+            const float4 tc = __ldg(tcol + m2);
+            o[ks] = (h ? v.y : v.x) * (tr.x * tc.x - tr.y * tc.y) * scale;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // direct sysmat per point, for calls that may not allocate a lattice: w^3 taps
 // per point from the fine grid of W and atomics into the fine grid of U, at q
@@ -1022,6 +1205,8 @@ __global__ void __launch_bounds__(256) k_sysmat_points(GeomView g, const float2 
 // host orchestration
 // ---------------------------------------------------------------------------
 
+constexpr int64_t kHalfPrime = 13;  // see halved()
+
 static Fine fine_of(const NufftPlan &pl) {
     Fine F;
     F.nf1 = (int)pl.nf1; F.nf2 = (int)pl.nf2; F.nf3 = (int)pl.nf3;
@@ -1068,19 +1253,110 @@ void NufftPlan::extract_real(float *y3, double sg, double cg, const float *ipT, 
     LAMINO_LAUNCH("k_extract");
 }
 
-void NufftPlan::fft_fine(float2 *g, int sign, cudaStream_t s) {
-    LAMINO_CUFFT(cufftSetStream(fft3.h, s));
-    LAMINO_CUFFT(cufftExecC2C(fft3.h, (cufftComplex *)g, (cufftComplex *)g, sign < 0 ? CUFFT_FORWARD : CUFFT_INVERSE));
+static void exec_c2c(const FftPlan &p, float2 *a, int sign, cudaStream_t s) {
+    LAMINO_CUFFT(cufftSetStream(p.h, s));
+    LAMINO_CUFFT(cufftExecC2C(p.h, (cufftComplex *)a, (cufftComplex *)a, sign < 0 ? CUFFT_FORWARD : CUFFT_INVERSE));
 }
+
+void NufftPlan::fft_fine(float2 *g, int sign, cudaStream_t s) {
+    if (!split3) {
+        exec_c2c(fft3, g, sign, s);
+        return;
+    }
+    const int64_t plane = nf3 * nf2, keep = vol.n1 - vol.n1 / 2;
+    if (sign > 0) exec_c2c(fft3n1, g, sign, s);
+    exec_c2c(fft3, g, sign, s);
+    exec_c2c(fft3, g + (nf1 - keep) * plane, sign, s);
+    if (sign < 0) exec_c2c(fft3n1, g, sign, s);
+}
+
+// the larger of the primes of n
+static int64_t largest_prime(int64_t n) {
+    int64_t p = 1;
+    for (int64_t q = 2; q * q <= n; ++q)
+        while (n % q == 0) {
+            p = q;
+            n /= q;
+        }
+    return n > 1 ? std::max(p, n) : p;
+}
+// Whether a geometry's detector transforms are halved: where a side has a large
+// prime the transforms are convolutions of twice the length and bound by
+// arithmetic, and half of them pay for the extra pass over memory.  Measured,
+// adjoint / forward of 60 projections, 2-D transform against halved: 618^2 2.15 / 2.05
+// against 1.48 / 1.44 ms, 724^2 1.96 / 1.91 against 1.42 / 1.46; 433^2 0.94 / 0.84
+// against 0.77 / 0.67.  With primes up to 13 only it is within 5 % either way (154^2
+// 0.305 / 0.315 against 0.320 / 0.332, 480^2 0.767 / 0.700 against 0.754 / 0.680), and the
+// 2-D transform has three launches fewer.
+static bool halved(const Geom &g) { return std::max(largest_prime(g.nrows), largest_prime(g.ncols)) > kHalfPrime; }
 
 void NufftPlan::ensure_proj(const Geom &g) {
     check_points(g);
-    if ((int64_t)pbuf.n < g.npts()) pbuf.alloc(g.npts());
+    const bool half = halved(g);
+    const int64_t need = half ? g.nproj * ((g.nrows + 1) / 2 * g.ncols + (g.ncols + 1) / 2 * g.nrows) : g.npts();
+    if ((int64_t)pbuf.n < need) pbuf.alloc(need);
     if (f2_np != g.nproj || f2_nr != g.nrows || f2_nc != g.ncols) {
         int n[2] = {(int)g.nrows, (int)g.ncols};
-        fft2.make(2, n, CUFFT_C2C, (int)g.nproj);
+        f2_np = -1;
+        if (half) {
+            const int pairs = (int)(g.nproj * ((g.ncols + 1) / 2));
+            fft2.make(1, n + 1, CUFFT_C2C, (int)(g.nproj * ((g.nrows + 1) / 2)));
+            fft2n.make(1, n, CUFFT_C2C, pairs);
+        } else {
+            fft2n.reset();
+            fft2.make(2, n, CUFFT_C2C, (int)g.nproj);
+        }
         f2_np = g.nproj; f2_nr = g.nrows; f2_nc = g.ncols;
     }
+}
+
+static unsigned half_tiles(const Geom &g, int rows) {
+    return (unsigned)(g.nproj * ((rows + 31) / 32) * (((g.ncols + 1) / 2 + 31) / 32));
+}
+
+// rows (pbuf) -> projections: the beam factors, the detector transform, real part
+void NufftPlan::rows_to_proj(const Lattice &l, const Geom &g, float *proj, cudaStream_t s) {
+    const int64_t nrow = g.nproj * g.nrows;
+    const int nr = (int)g.nrows, nc = (int)g.ncols;
+    const float scale = 1.0f / (float)(g.nrows * g.ncols);
+    const unsigned grid = (unsigned)std::min<int64_t>(nrow, 148 * 64);
+    if (!l.half) {
+        exec_c2c(fft2, pbuf.p, +1, s);
+        k_proj_post<<<grid, 256, 0, s>>>(pbuf.p, nrow, nr, nc, l.trow, l.tcol, l.a, scale, proj);
+        LAMINO_LAUNCH("k_proj_post");
+        return;
+    }
+    const int jh = (nr + 1) / 2, np = (int)g.nproj;
+    float2 *z = pbuf.p + (int64_t)np * jh * nc;
+    k_half_combine<<<grid, 256, 0, s>>>(pbuf.p, np, nr, nc, l.a);
+    LAMINO_LAUNCH("k_half_combine");
+    exec_c2c(fft2, pbuf.p, +1, s);
+    k_half_pack<<<half_tiles(g, jh), 256, 0, s>>>(pbuf.p, nr, nc, l.tcol, z);
+    LAMINO_LAUNCH("k_half_pack");
+    exec_c2c(fft2n, z, +1, s);
+    k_half_post<<<half_tiles(g, nr), 256, 0, s>>>(z, nr, nc, l.trow, l.tcol, scale, proj);
+    LAMINO_LAUNCH("k_half_post");
+}
+
+// projections -> rows (pbuf), the transpose
+void NufftPlan::proj_to_rows(const Lattice &l, const Geom &g, const float *proj, cudaStream_t s) {
+    const int64_t nrow = g.nproj * g.nrows;
+    const int nr = (int)g.nrows, nc = (int)g.ncols;
+    const unsigned grid = (unsigned)std::min<int64_t>(nrow, 148 * 64);
+    if (!l.half) {
+        k_proj_pre<<<grid, 256, 0, s>>>(proj, nrow, nr, nc, l.trow, l.tcol, l.a, pbuf.p);
+        LAMINO_LAUNCH("k_proj_pre");
+        exec_c2c(fft2, pbuf.p, -1, s);
+        return;
+    }
+    const int jh = (nr + 1) / 2, np = (int)g.nproj;
+    float2 *z = pbuf.p + (int64_t)np * jh * nc;
+    k_half_pre<<<half_tiles(g, nr), 256, 0, s>>>(proj, nr, nc, l.trow, l.tcol, z);
+    LAMINO_LAUNCH("k_half_pre");
+    exec_c2c(fft2n, z, -1, s);
+    k_half_unpack<<<half_tiles(g, jh), 256, 0, s>>>(z, nr, nc, l.tcol, pbuf.p);
+    LAMINO_LAUNCH("k_half_unpack");
+    exec_c2c(fft2, pbuf.p, -1, s);
 }
 
 // Bin layouts were the tiles of a point-by-point spread; the limits on them
@@ -1169,6 +1445,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     auto l = std::make_unique<Lattice>();
     l->uid = g.uid;
     l->raw = raw;
+    l->half = !raw && halved(g);
     l->cg = g.cg;
     l->sg = g.sg;
     // twice the volume's extent along t, in cells over the period 2 pi
@@ -1240,7 +1517,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
         LAMINO_LAUNCH("k_rows_count");
         k_scan_offsets<<<1, 1024, 0, s>>>(cnt, (int)cells, l->start, cnt);
         LAMINO_LAUNCH("k_scan_offsets");
-        k_rows_place<W><<<grid_n, 256, 0, s>>>(gv, raw, invh, l->T0, l->nstart, F, cnt, l->pt, l->pd);
+        k_rows_place<W><<<grid_n, 256, 0, s>>>(gv, raw, invh, l->half, l->T0, l->nstart, F, cnt, l->pt, l->pd);
         LAMINO_LAUNCH("k_rows_place");
         k_tile_items<W><<<(unsigned)((strip_count(l->ntile, ntiles / l->ntile) + 127) / 128), 128, 0, s>>>(l->start, l->nstart, (int)nf2, l->ntile, (int)ntiles,
                                                                          l->seg, l->nitem, l->items);
@@ -1293,7 +1570,7 @@ void NufftPlan::nodes_to_rows(const Lattice &l, const Geom &g, float2 *rows, cud
     });
 }
 
-void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *rows, bool symmetric, cudaStream_t s) {
+void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *rows, RowSource from, cudaStream_t s) {
     const Fine F = fine_of(*this);
     const LatView L = lat_view(l, g);
     const int nc = (int)g.ncols;
@@ -1302,7 +1579,7 @@ void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *row
     for (int b : {96, 64, 32})
         if ((nc + kCols * b - 1) / (kCols * b) * b < (nc + kCols * bt - 1) / (kCols * bt) * bt) bt = b;
     const dim3 b1((unsigned)l.max_items, (unsigned)((nc + kCols * bt - 1) / (kCols * bt)));
-    const int smem1 = (bt + 2 * kAhead) * (int)(kCell * sizeof(float4) + sizeof(uint2) + sizeof(float2));
+    const int smem1 = (bt + 2 * kAhead) * (int)(kCell * sizeof(float4) + sizeof(uint2) + sizeof(float4));
     const int yb = (int)std::min<int64_t>(256, (nf2 + 31) / 32 * 32);
     const int xtiles = (int)((nf3 + kCell - 1) / kCell);
     const dim3 b2((unsigned)strip_count(xtiles, (nf1 + kCell - 1) / kCell), (unsigned)((nf2 + yb - 1) / yb));
@@ -1317,12 +1594,13 @@ void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *row
     const float scale = 1.0f / (float)(g.nrows * g.ncols);
     with_width(w, [&](auto WC) {
         constexpr int W = decltype(WC)::value;
-        auto rs = symmetric ? k_rows_spread<W, true> : k_rows_spread<W, false>;
+        auto rs = from == ROWS_SYSMAT ? k_rows_spread<W, ROWS_SYSMAT>
+                  : from == ROWS_HALF ? k_rows_spread<W, ROWS_HALF> : k_rows_spread<W, ROWS_PLAIN>;
         k_tiles_zero<<<(unsigned)std::min(l.max_items, 148 * 8), 256, 0, s>>>(l.nitem, l.items, l.nT, l.ntile, (int)nf2, nc,
                                                                               work.p);
         LAMINO_LAUNCH("k_tiles_zero");
         rs<<<b1, bt, smem1, s>>>(l.nitem, l.items, l.seg, l.start, l.pt, l.pd, l.nstart, l.nT, l.ntile, (int)nf2, rows, (int)g.nrows, nc, beta,
-                                 l.a, scale, work.p);
+                                 l.a, (int)g.nproj, l.half, scale, work.p);
         LAMINO_LAUNCH("k_rows_spread");
         k_nodes_spread<W><<<b2, yb, smem2, s>>>(L, F, reach1, reach3, xtiles, work.p, grid.p);
         LAMINO_LAUNCH("k_nodes_spread");
@@ -1385,24 +1663,14 @@ void NufftPlan::forward(const Geom &g, const float *m3, float *proj, cudaStream_
     pad_real(m3, l.sg, l.cg, l.ipT, s);
     fft_fine(grid.p, -1, s);
     nodes_to_rows(l, g, pbuf.p, s);
-    LAMINO_CUFFT(cufftSetStream(fft2.h, s));
-    LAMINO_CUFFT(cufftExecC2C(fft2.h, (cufftComplex *)pbuf.p, (cufftComplex *)pbuf.p, CUFFT_INVERSE));
-    const int64_t nrow = g.nproj * g.nrows;
-    k_proj_post<<<(unsigned)std::min<int64_t>(nrow, 148 * 64), 256, 0, s>>>(
-        pbuf.p, nrow, (int)g.nrows, (int)g.ncols, l.trow, l.tcol, l.a, 1.0f / (float)(g.nrows * g.ncols), proj);
-    LAMINO_LAUNCH("k_proj_post");
+    rows_to_proj(l, g, proj, s);
 }
 
 void NufftPlan::adjoint(const Geom &g, const float *proj, float *m3, bool accumulate, cudaStream_t s) {
     ensure_proj(g);
     const Lattice &l = lattice(g, false, s);
-    const int64_t nrow = g.nproj * g.nrows;
-    k_proj_pre<<<(unsigned)std::min<int64_t>(nrow, 148 * 64), 256, 0, s>>>(proj, nrow, (int)g.nrows, (int)g.ncols, l.trow,
-                                                                          l.tcol, l.a, pbuf.p);
-    LAMINO_LAUNCH("k_proj_pre");
-    LAMINO_CUFFT(cufftSetStream(fft2.h, s));
-    LAMINO_CUFFT(cufftExecC2C(fft2.h, (cufftComplex *)pbuf.p, (cufftComplex *)pbuf.p, CUFFT_FORWARD));
-    rows_to_nodes(l, g, pbuf.p, false, s);
+    proj_to_rows(l, g, proj, s);
+    rows_to_nodes(l, g, pbuf.p, l.half ? ROWS_HALF : ROWS_PLAIN, s);
     fft_fine(grid.p, +1, s);
     extract_real(m3, l.sg, l.cg, l.ipT, 1.0f / (float)(g.nrows * g.ncols), accumulate, s);
 }
@@ -1416,7 +1684,7 @@ void NufftPlan::normal_one(const Geom &g, const Lattice *l, const float *x3, flo
     fft_fine(grid.p, -1, s);
     if (l) {
         nodes_to_rows(*l, g, pbuf.p, s);
-        rows_to_nodes(*l, g, pbuf.p, true, s);
+        rows_to_nodes(*l, g, pbuf.p, ROWS_SYSMAT, s);
         fft_fine(grid.p, +1, s);
         extract_real(y3, sg, cg, ipT, 1.0f, accumulate, s);
         return;
@@ -1469,7 +1737,7 @@ void NufftPlan::type2(const Geom &g, const float2 *modes, float2 *c, cudaStream_
 
 void NufftPlan::type1(const Geom &g, const float2 *c, float2 *modes, cudaStream_t s) {
     const Lattice &l = lattice(g, true, s);
-    rows_to_nodes(l, g, c, false, s);
+    rows_to_nodes(l, g, c, ROWS_PLAIN, s);
     fft_fine(grid.p, +1, s);
     const unsigned b = volume_tiles(vol);
     k_extract<true><<<b, 256, 0, s>>>(grid.p, (int)vol.n1, (int)vol.n2, (int)vol.n3, 0.f, 0.f, nullptr, modes,

@@ -29,6 +29,11 @@ struct Lattice {
     bool raw = false;        // the float frequencies as they are (raw transforms), else
                              // their antisymmetric part (forward, adjoint, sysmat)
     uint64_t last_use = 0;
+    // The projection spectra of real images are symmetric, so the detector transform
+    // needs only the first half of the rows: two real columns travel as one
+    // complex one.  Rows are then stored first halves of all projections first,
+    // and the second halves are read as mirrored conjugates.
+    bool half = false;
     double cg = 1, sg = 0, h = 0;
     int nT = 0, T0 = 0;
     int nstart = 0;          // footprint starts along T: nT - w + 1
@@ -37,7 +42,7 @@ struct Lattice {
     float *ipT = nullptr;    // 1 / p_T of every mode (k1, k3): deconvolution along T
     float2 *a = nullptr;     // (sin - i cos) / 2 of every angle
     float4 *trow = nullptr, *tcol = nullptr;  // twist factors of the projection-space transform
-    int4 *pt = nullptr;      // rows sorted by cell: row id (angle, detector row), T start, y start, angle
+    int4 *pt = nullptr;      // rows sorted by cell: place among the stored rows, T start, y start, id (angle, row)
     float2 *pd = nullptr;    // offsets of the T and y footprints from the row's position
     uint32_t *start = nullptr;  // first row of each (y start, T start) cell
     int ntile = 0, seg = 0, max_items = 0;  // rows -> nodes: tiles along T, rows per work item, bound on the items
@@ -55,10 +60,13 @@ struct NufftPlan {
     DevBuf<double2> quad;          // quadrature of the kernel's transform (node, weight x kernel)
     DevBuf<float2> grid;           // fine grid [nf1][nf3][nf2] (n2 fastest)
     DevBuf<float2> work;           // node grid, or the direct form's second fine grid
-    FftPlan fft3;                  // C2C 3-D on the fine grid
+    FftPlan fft3;                  // C2C 3-D on the fine grid; or, split, its planes of n1 ...
+    FftPlan fft3n1;                // ... and the transform along n1
+    bool split3 = false;           // only the planes that hold modes run their 2-D transforms
     // projection-space workspace (largest geometry seen), with its 2-D plan
     DevBuf<float2> pbuf;
-    FftPlan fft2;
+    FftPlan fft2;                  // 2-D; or, halved (Lattice::half), along the detector rows ...
+    FftPlan fft2n;                 // ... and along the columns, two real ones at a time
     int64_t f2_np = -1, f2_nr = -1, f2_nc = -1;
     // lattices of the geometries used with this plan (bounded LRU)
     std::vector<std::unique_ptr<Lattice>> lats;
@@ -69,6 +77,9 @@ struct NufftPlan {
     NufftPlan(Dims3 d, double eps);
     int64_t nf() const { return nf1 * nf2 * nf3; }
     void ensure_proj(const Geom &g);
+    // projection space <-> rows (see Lattice::half): proj is read / written
+    void rows_to_proj(const Lattice &lat, const Geom &g, float *proj, cudaStream_t s);
+    void proj_to_rows(const Lattice &lat, const Geom &g, const float *proj, cudaStream_t s);
     // accepts the layouts that a tile of (b + w - 1)^3 cells in shared memory
     // allows; the lattice transforms choose their own tiles
     void set_bins(int b1, int b2, int b3);
@@ -100,7 +111,8 @@ struct NufftPlan {
     void extract_real(float *y3, double sg, double cg, const float *ipT, float scale, bool accumulate, cudaStream_t s);
     void fft_fine(float2 *g, int sign, cudaStream_t s);
     void nodes_to_rows(const Lattice &lat, const Geom &g, float2 *rows, cudaStream_t s);   // grid -> nodes -> rows
-    void rows_to_nodes(const Lattice &lat, const Geom &g, const float2 *rows, bool symmetric, cudaStream_t s);
+    enum RowSource { ROWS_PLAIN, ROWS_SYSMAT, ROWS_HALF };  // see k_rows_spread
+    void rows_to_nodes(const Lattice &lat, const Geom &g, const float2 *rows, RowSource from, cudaStream_t s);
     // whole 128-byte lines, so that a run of columns never straddles one
     int64_t node_pitch(int64_t ncols) const { return (ncols + 15) / 16 * 16; }
 };
