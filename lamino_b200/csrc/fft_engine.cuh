@@ -434,25 +434,6 @@ struct CtSched<90> {
     static constexpr int r[CT_MAX_STAGES] = {2, 9, 5, 0, 0, 0};
 };
 
-// Schedules of the packed row transforms (no zero-padded lead stage): the
-// packed half lengths 90 and 180 of the 180- and 360-long n3 embeddings (270
-// and 375 run in two register stages).  Each equals fft_schedule(N, false).
-template <int N>
-struct CtRowSched {
-    static constexpr int ns = 0;
-    static constexpr int r[CT_MAX_STAGES] = {0, 0, 0, 0, 0, 0};
-};
-template <>
-struct CtRowSched<90> {
-    static constexpr int ns = 3;
-    static constexpr int r[CT_MAX_STAGES] = {2, 9, 5, 0, 0, 0};
-};
-template <>
-struct CtRowSched<180> {
-    static constexpr int ns = 3;
-    static constexpr int r[CT_MAX_STAGES] = {4, 9, 5, 0, 0, 0};
-};
-
 // block size before stage s of schedule SC (length N)
 template <int N, class SC>
 __host__ __device__ constexpr int ct_block(int s) {

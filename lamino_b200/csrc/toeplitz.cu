@@ -62,18 +62,18 @@ __device__ __forceinline__ float sinpi_half(float x) {
 // D_n(s) = sin(pi s) / sin(pi s / n), with the 0/0 limit n (-1)^{m (n-1)} at s = m n.
 // inv_n = 1/n in double: s / n only feeds the fractional part f2 (s is an exact
 // multiple of n only at s = 0, where the product is exact too).
+// Rounding to an integer is the addition of 1.5 2^52 (|s| < 2^51), whose low word
+// also gives the parity: double additions run at half the float rate, where rint
+// and the conversions to a 64-bit integer made up most of the kernel (2 x 150
+// angles at 270 x 32 x 270: 6.0 -> 5.3 ms).
 __device__ __forceinline__ float dirichlet(double s, int n, double inv_n) {
-    double m1 = rint(s);
-    double f1 = s - m1;
-    double q = s * inv_n;
-    double m2 = rint(q);
-    double f2 = q - m2;
-    long long i1 = (long long)m1, i2 = (long long)m2;
-    if (f2 == 0.0) return ((i2 * (long long)(n - 1)) & 1LL) ? -(float)n : (float)n;
-    float num = sinpi_half((float)f1);
-    float den = sinpi_half((float)f2);
-    float r = __fdividef(num, den);
-    return ((i1 + i2) & 1LL) ? -r : r;
+    constexpr double kRound = 6755399441055744.0;
+    const double r1 = s + kRound, q = s * inv_n, r2 = q + kRound;
+    const float f1 = (float)(s - (r1 - kRound)), f2 = (float)(q - (r2 - kRound));
+    const int i1 = __double2loint(r1), i2 = __double2loint(r2);
+    if (f2 == 0.f) return (i2 & (n - 1) & 1) ? -(float)n : (float)n;
+    const float r = __fdividef(sinpi_half(f1), sinpi_half(f2));
+    return ((i1 + i2) & 1) ? -r : r;
 }
 
 // One thread per cell with d_z = m1 in [0, n1); writes T[d] and its mirror T[-d].
@@ -379,8 +379,8 @@ __device__ __forceinline__ void twiddle_lin(const float2 *__restrict__ tw, int e
 }
 
 // Rows of M3 = 729 as 27 x 27 (schedule 27, 27; positions
-// fft_positions(729, {27, 27})): one warp per row, lanes 0..26 busy.  The first
-// stage (27-point DFTs over the packed values n + 27 j, twiddles w729^{n k})
+// fft_positions(729, {27, 27})): one warp per row, lanes 0..26 busy (27 threads per
+// row without idle lanes took 3 % longer).  The first stage (27-point DFTs over the packed values n + 27 j, twiddles w729^{n k})
 // runs between the global rows and shared memory, the second (a 27-point DFT
 // per block of 27 positions) in place in shared memory; the inverses mirror
 // them.  Each value makes one trip through shared memory between the stages.
@@ -442,8 +442,11 @@ __device__ __forceinline__ void rows27_store(const float2 *__restrict__ sm, int 
 }
 
 // Rows of M3 = A B in the same two register stages (schedule A, B; positions
-// fft_positions(M3, {A, B})): one warp per row; lane n < B takes the packed
-// values n + B j (j < A), lane b < A the B-point block b.
+// fft_positions(M3, {A, B})): thread n < B of a row takes the packed values
+// n + B j (j < A), thread b < A the B-point block b; rows follow one another
+// without idle lanes (a warp per row left up to 17 of 32 idle).  r2c / c2r, before ->
+// after: 270 x 32 x 270 39 / 45 -> 33 / 38 us, 362 x 44 x 362 87 / 98 -> 78 / 86;
+// 180 and 90, then shared-memory schedules, 18.9 / 18.5 -> 14.8 / 15.8 (180 x 22 x 180).
 template <int M3>
 struct RowTwo {
     static constexpr bool on = false;
@@ -459,12 +462,22 @@ struct RowTwo<270> {
     static constexpr bool on = true;
     static constexpr int A = 15, B = 18;
 };
+template <>
+struct RowTwo<180> {
+    static constexpr bool on = true;
+    static constexpr int A = 12, B = 15;
+};
+template <>
+struct RowTwo<90> {
+    static constexpr bool on = true;
+    static constexpr int A = 9, B = 10;
+};
 
 template <int A, int B>
 __device__ __forceinline__ void rows2s_load(const float *__restrict__ xb, int nr, int n3,
                                             const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps) {
-    const int r = threadIdx.x >> 5, n = threadIdx.x & 31;
-    if (r < nr && n < B) {
+    const int r = threadIdx.x / B, n = threadIdx.x - B * r;
+    if (r < nr) {
         const float *xr = xb + (int64_t)r * n3;
         float2 v[A];
 #pragma unroll
@@ -484,8 +497,8 @@ __device__ __forceinline__ void rows2s_load(const float *__restrict__ xb, int nr
 
 template <int A, int B, bool INV>
 __device__ __forceinline__ void rows2s_mid(float2 *__restrict__ sm, int nr, int ps) {
-    const int r = threadIdx.x >> 5, b = threadIdx.x & 31;
-    if (r < nr && b < A) {
+    const int r = threadIdx.x / A, b = threadIdx.x - A * r;
+    if (r < nr) {
         float2 *row = sm + r * ps + B * b;
         float2 v[B];
 #pragma unroll
@@ -500,8 +513,8 @@ __device__ __forceinline__ void rows2s_mid(float2 *__restrict__ sm, int nr, int 
 template <int A, int B>
 __device__ __forceinline__ void rows2s_store(const float2 *__restrict__ sm, int nr, int ps, int n3,
                                              const float2 *__restrict__ tw3, float *__restrict__ yb) {
-    const int r = threadIdx.x >> 5, n = threadIdx.x & 31;
-    if (r < nr && n < B) {
+    const int r = threadIdx.x / B, n = threadIdx.x - B * r;
+    if (r < nr) {
         const float2 *sp = sm + r * ps + n;
         float2 v[A];
 #pragma unroll
@@ -527,10 +540,14 @@ __device__ __forceinline__ int row_pos(const int *__restrict__ pos3, int k) {
     else return __ldg(pos3 + k);
 }
 
-// rows with a warp per row: 729 and the two-register-stage lengths
-__host__ __device__ constexpr bool warp_rows(int M3) { return M3 == 729 || M3 == 375 || M3 == 270; }
-// threads of a rows CTA of R rows: one warp per row where the lengths run in registers
-__host__ __device__ constexpr int rows_threads(int M3, int R) { return warp_rows(M3) && R <= 8 ? 32 * R : 256; }
+// threads per row of the lengths that run in registers (0: the others; 729 a warp)
+__host__ __device__ constexpr int row_items(int M3) {
+    return M3 == 729 ? 32 : M3 == 375 ? 25 : M3 == 270 ? 18 : M3 == 180 ? 15 : M3 == 90 ? 10 : 0;
+}
+// threads of a rows CTA of R rows (at most 8 where the length runs in registers)
+__host__ __device__ constexpr int rows_threads(int M3, int R) {
+    return row_items(M3) && R <= 8 ? (row_items(M3) * R + 31) / 32 * 32 : 256;
+}
 
 // The first stage of a runtime-length row transform (radix R0 over the whole
 // packed row of M3, m0 = M3 / R0 offsets) in registers on the way in and its
@@ -613,7 +630,7 @@ __device__ __forceinline__ void rowslead_any(const FftLen &F3, const float *xb, 
 // A1: real rows along n3 (zero-padded to L3) -> half spectrum k3 in [0, M3], via the
 // packed-complex M3-point DIF and the even/odd split.  N3: compile-time M3 or 0.
 template <int N3>
-__global__ void __launch_bounds__(256, warp_rows(N3) ? 3 : 4) k_r2c_rows(const float *__restrict__ x, int64_t nrows, int n3, FftLen F3,
+__global__ void __launch_bounds__(256, row_items(N3) ? 3 : 4) k_r2c_rows(const float *__restrict__ x, int64_t nrows, int n3, FftLen F3,
                                                   const int *__restrict__ pos3, const float2 *__restrict__ twh,
                                                   int R, float2 *__restrict__ z1) {
     extern __shared__ float2 sm[];
@@ -627,10 +644,6 @@ __global__ void __launch_bounds__(256, warp_rows(N3) ? 3 : 4) k_r2c_rows(const f
     } else if constexpr (RowTwo<N3>::on) {
         rows2s_load<RowTwo<N3>::A, RowTwo<N3>::B>(x + row0 * n3, nr, n3, F3.tw, sm, ps);
         rows2s_mid<RowTwo<N3>::A, RowTwo<N3>::B, false>(sm, nr, ps);
-    } else if constexpr (N3 != 0) {  // compile-time schedule: the first stage in registers
-        rowslead_load<CtRowSched<N3>::r[0]>(x + row0 * n3, nr, n3, N3, F3.tw, sm, ps, threadIdx.x, blockDim.x);
-        __syncthreads();
-        ct_forward<N3, 1, CtRowSched<N3>>(sm, nr, ps, F3.tw, threadIdx.x, blockDim.x);
     } else if (F3.ns >= 1) {  // runtime length: the first stage in registers as well
         rowslead_any<false>(F3, x + row0 * n3, nullptr, sm, nullptr, nr, n3, ps, threadIdx.x, blockDim.x);
         __syncthreads();
@@ -1833,10 +1846,6 @@ __global__ void __launch_bounds__(256) k_c2r_rows(const float2 *__restrict__ z1,
         rows2s_mid<RowTwo<N3>::A, RowTwo<N3>::B, true>(sm, nr, ps);
         rows2s_store<RowTwo<N3>::A, RowTwo<N3>::B>(sm, nr, ps, n3, F3.tw, y + row0 * n3);
         return;
-    } else if constexpr (N3 != 0) {
-        ct_inverse<N3, CtRowSched<N3>::ns - 1, 1, CtRowSched<N3>>(sm, nr, ps, F3.tw, threadIdx.x, blockDim.x);
-        rowslead_store<CtRowSched<N3>::r[0]>(sm, nr, ps, n3, N3, F3.tw, y + row0 * n3, threadIdx.x, blockDim.x);
-        return;
     }
     if (F3.ns >= 1) {
         fft_inverse(sm, nr, ps, F3, 1, threadIdx.x, blockDim.x);
@@ -1947,20 +1956,6 @@ static bool ct_equal(const std::vector<int> &r) {
         if (r[i] != CtSched<N>::r[i]) return false;
     return true;
 }
-template <int N>
-static bool ct_row_equal(const std::vector<int> &r) {
-    if ((int)r.size() != CtRowSched<N>::ns) return false;
-    for (int i = 0; i < CtRowSched<N>::ns; ++i)
-        if (r[i] != CtRowSched<N>::r[i]) return false;
-    return true;
-}
-static bool ct_row_matches(int M, const std::vector<int> &r) {
-    switch (M) {
-        case 180: return ct_row_equal<180>(r);
-        case 90: return ct_row_equal<90>(r);
-        default: return false;
-    }
-}
 static bool ct_dim2_matches(int L, const std::vector<int> &r) {  // n2 lengths
     switch (L) {
         case 90: return ct_equal<90>(r);
@@ -1990,6 +1985,8 @@ void Toeplitz::init_tables(Dims3 d, int prec) {
     f3 = make_len((int)M3, false, tw3, &r3);
     if (M3 == 729) r3 = {27, 27};  // the compile-time rows (rows27_load / rows27_mid)
     if (M3 == 375) r3 = {RowTwo<375>::A, RowTwo<375>::B};  // two register stages (rows2s_*)
+    if (M3 == 180) r3 = {RowTwo<180>::A, RowTwo<180>::B};
+    if (M3 == 90) r3 = {RowTwo<90>::A, RowTwo<90>::B};
     if (M3 == 270) r3 = {RowTwo<270>::A, RowTwo<270>::B};
     {
         std::vector<float2> h(M3 + 1);
@@ -2142,7 +2139,7 @@ void Toeplitz::finish(cudaStream_t s) {
         throw Error(ERR_ARG, "n2 too large for the n2-pass kernels");
     ct1 = (L1 == 1458 || !two_stage_schedule((int)L1).empty()) ? (int)L1 : 0;
     ct2 = (L2 == 144 || ct_dim2_matches((int)L2, r2_)) ? (int)L2 : 0;
-    ct3 = (warp_rows((int)M3) || ct_row_matches((int)M3, fft_schedule((int)M3, false))) ? (int)M3 : 0;
+    ct3 = row_items((int)M3) ? (int)M3 : 0;
     const int smem_rows = rows1 * (int)L3h * (int)sizeof(float2);
     const int smem_d2 = d2_smem_values((int)L2, kb2) * (int)sizeof(float2);
     const int smem_pen = 3 * (int)L1 * (int)sizeof(float2);
@@ -2278,7 +2275,7 @@ static void raise_d2_smem(int bytes) {
 }
 
 // the row kernels of the operator's packed n3 length (ct3: compile-time 729 or
-// a CtRowSched length, 0 = runtime schedule)
+// a RowTwo length, 0 = runtime schedule)
 #define LAMINO_ROW_LENGTHS(X) X(729) X(375) X(270) X(180) X(90) X(0)
 static void launch_r2c(int ct3, unsigned grid, int rows, int smem, cudaStream_t s, const float *x, int64_t nrows,
                        int n3, const FftLen &f3, const int *pos3, const float2 *twh3, float2 *z1) {
@@ -2460,7 +2457,7 @@ void Toeplitz::quadforms(const float *x3, const std::vector<const Toeplitz *> &p
 
 void Toeplitz::set_shape(int rows, int kb) {
     if (rows < 1 || kb < 1) throw Error(ERR_ARG, "launch shape values must be positive");
-    if (warp_rows(ct3) && rows > 8) throw Error(ERR_ARG, "rows of this length run one warp per row, at most 8 per CTA");
+    if (row_items(ct3) && rows > 8) throw Error(ERR_ARG, "rows of this length run at most 8 per CTA");
     const int64_t smem_rows = (int64_t)rows * L3h * (int64_t)sizeof(float2);
     const int64_t smem_d2 = (int64_t)d2_smem_values((int)L2, kb) * (int64_t)sizeof(float2);
     if (smem_rows > 200 * 1024 || smem_d2 > 200 * 1024) throw Error(ERR_ARG, "launch shape exceeds shared memory");
