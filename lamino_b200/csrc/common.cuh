@@ -50,6 +50,29 @@ inline unsigned grid_for(int64_t n, int block, int64_t cap = 148LL * 64) {
     return (unsigned)g;
 }
 
+// Launches that overlap the end of the kernel before them in the stream
+// (programmatic dependent launch): launch_after() lets the kernel's CTAs start once
+// every CTA of the one before has called allow_next(); the kernel reads and writes
+// nothing of earlier kernels before wait_previous(), which returns when they have
+// completed and their writes are visible.  A kernel of either kind may come before
+// or after.  What is gained is the launch latency between short kernels.
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    LAMINO_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+}
+
 // Raise a kernel's dynamic shared-memory limit to at least `bytes` (never
 // lowers it; safe from several host threads).
 void raise_smem_limit(const void *kernel, int bytes);

@@ -634,6 +634,8 @@ __global__ void __launch_bounds__(256, row_items(N3) ? 3 : 4) k_r2c_rows(const f
                                                   const int *__restrict__ pos3, const float2 *__restrict__ twh,
                                                   int R, float2 *__restrict__ z1) {
     extern __shared__ float2 sm[];
+    allow_next();
+    wait_previous();
     const int M3 = N3 ? N3 : F3.n;
     const int ps = M3 + 1;
     const int64_t row0 = (int64_t)blockIdx.x * R;
@@ -1078,6 +1080,8 @@ __global__ void __launch_bounds__(288, 4) k_dim2_fwd(const float2 *__restrict__ 
                                                   FftLen F2, const float2 *__restrict__ tw2, int KB,
                                                   float2 *__restrict__ xa) {
     extern __shared__ float2 sm[];
+    allow_next();
+    wait_previous();
     const int i1b = blockIdx.x * D2_IB, k3b = blockIdx.y * KB, c = blockIdx.z;
     const int nk = min(KB, L3h - k3b);
     const int L2 = N2 ? N2 : F2.n;
@@ -1468,6 +1472,7 @@ __global__ void __launch_bounds__(pencil_threads(N1), pencil_ctas(N1)) k_pencil(
                                                 const float2 *__restrict__ tw1, const float *__restrict__ K,
                                                 const __half *__restrict__ Kh, const float *__restrict__ kscale) {
     extern __shared__ float2 sm[];
+    allow_next();
     const int64_t pen = blockIdx.x;
     const int L1 = N1 ? N1 : F1.n;
     const int64_t cs = (int64_t)L2 * L3h * n1p;  // component stride in xa
@@ -1478,6 +1483,7 @@ __global__ void __launch_bounds__(pencil_threads(N1), pencil_ctas(N1)) k_pencil(
         if constexpr (HALF) prefetch_l2(Kh + pen * 6 * L1, (size_t)6 * L1 * sizeof(__half));
         else prefetch_l2(K + pen * 6 * L1, (size_t)6 * L1 * sizeof(float));
     }
+    wait_previous();
     pencil_forward<N1>(pv, cs, n1, F1, tw1, sm);
     const float sc = HALF ? kscale[pen] : 1.f;
     // two adjacent positions per thread (L1 is even): 8-byte spectrum loads and
@@ -1551,6 +1557,8 @@ __global__ void __launch_bounds__(pencil_threads(N1)) k_pencil_quad(const float2
         for (int g = 0; g < kMaxQuadSets; ++g)
             if (g < ng) prefetch_l2(ks.K[g] + pen * 6 * L1, (size_t)6 * L1 * sizeof(float));
     }
+    allow_next();
+    wait_previous();
     pencil_forward<N1>(pv, cs, n1, F1, tw1, sm);
     float part[kMaxQuadSets][3];
 #pragma unroll
@@ -1630,6 +1638,8 @@ __global__ void __launch_bounds__(pencil_threads(N1), N1 ? pencil_ctas(N1) : 3) 
         for (int g = 0; g < kMaxTilts; ++g)
             if (g < ng) prefetch_l2(T.K[g] + pen * 3 * L1, (size_t)3 * L1 * sizeof(float));
     }
+    allow_next();
+    wait_previous();
     pencil_forward<N1>(pv, cs, n1, F1, tw1, sm);
     float q[kMaxTilts][3];
 #pragma unroll
@@ -1736,6 +1746,8 @@ __global__ void __launch_bounds__(288, 4) k_dim2_inv(const float2 *__restrict__ 
                                                   FftLen F2, const float2 *__restrict__ tw2, int KB,
                                                   float2 *__restrict__ z1) {
     extern __shared__ float2 sm[];
+    allow_next();
+    wait_previous();
     const int i1b = blockIdx.x * D2_IB, k3b = blockIdx.y * KB, c = blockIdx.z;
     const int nk = min(KB, L3h - k3b);
     const int L2 = N2 ? N2 : F2.n;
@@ -1809,6 +1821,8 @@ __global__ void __launch_bounds__(256) k_c2r_rows(const float2 *__restrict__ z1,
                                                   const int *__restrict__ pos3, const float2 *__restrict__ twh, int R,
                                                   float *__restrict__ y) {
     extern __shared__ float2 sm[];
+    allow_next();
+    wait_previous();
     const int M3 = N3 ? N3 : F3.n;
     const int ps = M3 + 1;
     const int64_t row0 = (int64_t)blockIdx.x * R;
@@ -2225,7 +2239,7 @@ static void launch_pencil(int ct1, unsigned grid, int smem, cudaStream_t s, floa
     switch (ct1) {
 #define LAMINO_PENCIL(N)                                                                                       \
     case N:                                                                                                    \
-        k_pencil<HALF, N><<<grid, pencil_threads(N), smem, s>>>(xa, n1, np1, l2, l3h, f1, tw1, K, \
+        launch_after(k_pencil<HALF, N>, grid, pencil_threads(N), smem, s, xa, n1, np1, l2, l3h, f1, tw1, K, \
                                                                               Kh, ksc);                        \
         break;
         LAMINO_PENCIL(1458)
@@ -2247,7 +2261,7 @@ static void launch_dim2_fwd(int ct2, dim3 grid, int kb, int smem, cudaStream_t s
     switch (ct2) {
 #define LAMINO_D2F(N)                                                                                           \
     case N:                                                                                                     \
-        k_dim2_fwd<N><<<grid, N == 0 ? 256 : d2_threads(N, kb), smem, s>>>(z1, n1, n2, l3h, np1, f2, tw2, kb, xa); \
+        launch_after(k_dim2_fwd<N>, grid, N == 0 ? 256 : d2_threads(N, kb), smem, s, z1, n1, n2, l3h, np1, f2, tw2, kb, xa); \
         break;
         LAMINO_D2_LENGTHS(LAMINO_D2F)
 #undef LAMINO_D2F
@@ -2259,7 +2273,7 @@ static void launch_dim2_inv(int ct2, dim3 grid, int kb, int smem, cudaStream_t s
     switch (ct2) {
 #define LAMINO_D2I(N)                                                                                           \
     case N:                                                                                                     \
-        k_dim2_inv<N><<<grid, N == 0 ? 256 : d2_threads(N, kb), smem, s>>>(xa, n1, n2, l3h, np1, f2, tw2, kb, z1); \
+        launch_after(k_dim2_inv<N>, grid, N == 0 ? 256 : d2_threads(N, kb), smem, s, xa, n1, n2, l3h, np1, f2, tw2, kb, z1); \
         break;
         LAMINO_D2_LENGTHS(LAMINO_D2I)
 #undef LAMINO_D2I
@@ -2282,7 +2296,7 @@ static void launch_r2c(int ct3, unsigned grid, int rows, int smem, cudaStream_t 
     switch (ct3) {
 #define LAMINO_R2C(N)                                                                                         \
     case N:                                                                                                   \
-        k_r2c_rows<N><<<grid, rows_threads(N == 0 ? 1 : N, rows), smem, s>>>(x, nrows, n3, f3, pos3, twh3, rows, \
+        launch_after(k_r2c_rows<N>, grid, rows_threads(N == 0 ? 1 : N, rows), smem, s, x, nrows, n3, f3, pos3, twh3, rows, \
                                                                              z1);                             \
         break;
         LAMINO_ROW_LENGTHS(LAMINO_R2C)
@@ -2295,7 +2309,7 @@ static void launch_c2r(int ct3, unsigned grid, int rows, int smem, cudaStream_t 
     switch (ct3) {
 #define LAMINO_C2R(N)                                                                                         \
     case N:                                                                                                   \
-        k_c2r_rows<N><<<grid, rows_threads(N == 0 ? 1 : N, rows), smem, s>>>(z1, nrows, n3, f3, pos3, twh3, rows, \
+        launch_after(k_c2r_rows<N>, grid, rows_threads(N == 0 ? 1 : N, rows), smem, s, z1, nrows, n3, f3, pos3, twh3, rows, \
                                                                              y);                              \
         break;
         LAMINO_ROW_LENGTHS(LAMINO_C2R)
@@ -2324,7 +2338,7 @@ void Toeplitz::launch_tilts(int g0, int ng, bool apply, bool forms, cudaStream_t
     switch (ct1) {
 #define LAMINO_TILTS(N)                                                                                              \
     case N:                                                                                                          \
-        k_pencil_tilts<N><<<gpen, pencil_threads(N), smem_pen, s>>>(xa.p, (int)vol.n1, (int)n1p, (int)L2, (int)L3h, f1, \
+        launch_after(k_pencil_tilts<N>, gpen, pencil_threads(N), smem_pen, s, xa.p, (int)vol.n1, (int)n1p, (int)L2, (int)L3h, f1, \
                                                                     tw1.p, T, ng, apply, forms ? qpart.p : nullptr); \
         break;
         LAMINO_TILTS(1458)
@@ -2439,7 +2453,7 @@ void Toeplitz::quadforms(const float *x3, const std::vector<const Toeplitz *> &p
         switch (ct1) {
 #define LAMINO_QUAD(N)                                                                                          \
     case N:                                                                                                     \
-        k_pencil_quad<N><<<gpen, pencil_threads(N), smem_pen, s>>>(xa.p, n1, np1, l2, l3h, f1,    \
+        launch_after(k_pencil_quad<N>, gpen, pencil_threads(N), smem_pen, s, xa.p, n1, np1, l2, l3h, f1,    \
                                                                               tw1.p, qs, ng, acc + 3 * g0); \
         break;
             LAMINO_QUAD(1458)
