@@ -174,7 +174,7 @@ constexpr int LD_BATCH = 8;
 // way out (k_c2r_rows).  Item (r, n) holds the packed values n + 81 j of row r.
 constexpr int R729_OFS = 81;
 
-__device__ __forceinline__ void rows729_load(const float *__restrict__ xb, int nr, int n3,
+__device__ __forceinline__ void rows729_load(const float *xb, int nr, int n3,
                                              const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps,
                                              int tid, int nth) {
     for (int t = tid; t < nr * R729_OFS; t += nth) {
@@ -384,7 +384,7 @@ __device__ __forceinline__ void twiddle_lin(const float2 *__restrict__ tw, int e
 // runs between the global rows and shared memory, the second (a 27-point DFT
 // per block of 27 positions) in place in shared memory; the inverses mirror
 // them.  Each value makes one trip through shared memory between the stages.
-__device__ __forceinline__ void rows27_load(const float *__restrict__ xb, int nr, int n3,
+__device__ __forceinline__ void rows27_load(const float *xb, int nr, int n3,
                                             const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps) {
     const int r = threadIdx.x >> 5, n = threadIdx.x & 31;
     if (r < nr && n < 27) {
@@ -474,7 +474,7 @@ struct RowTwo<90> {
 };
 
 template <int A, int B>
-__device__ __forceinline__ void rows2s_load(const float *__restrict__ xb, int nr, int n3,
+__device__ __forceinline__ void rows2s_load(const float *xb, int nr, int n3,
                                             const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps) {
     const int r = threadIdx.x / B, n = threadIdx.x - B * r;
     if (r < nr) {
@@ -553,7 +553,7 @@ __host__ __device__ constexpr int rows_threads(int M3, int R) {
 // packed row of M3, m0 = M3 / R0 offsets) in registers on the way in and its
 // inverse on the way out, as rows729_load / rows729_store for other lengths.
 template <int R0>
-__device__ __forceinline__ void rowslead_load(const float *__restrict__ xb, int nr, int n3, int M3,
+__device__ __forceinline__ void rowslead_load(const float *xb, int nr, int n3, int M3,
                                               const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps,
                                               int tid, int nth) {
     const int m0 = M3 / R0;
@@ -630,7 +630,7 @@ __device__ __forceinline__ void rowslead_any(const FftLen &F3, const float *xb, 
 // A1: real rows along n3 (zero-padded to L3) -> half spectrum k3 in [0, M3], via the
 // packed-complex M3-point DIF and the even/odd split.  N3: compile-time M3 or 0.
 template <int N3>
-__global__ void __launch_bounds__(256, row_items(N3) ? 3 : 4) k_r2c_rows(const float *__restrict__ x, int64_t nrows, int n3, FftLen F3,
+__global__ void __launch_bounds__(256, row_items(N3) ? 3 : 4) k_r2c_rows(const float *x, int64_t nrows, int n3, FftLen F3,
                                                   const int *__restrict__ pos3, const float2 *__restrict__ twh,
                                                   int R, float2 *__restrict__ z1) {
     extern __shared__ float2 sm[];
@@ -722,7 +722,7 @@ __host__ __device__ constexpr int d2_threads(int L2, int KB) {
     return (L2 == 144 && KB <= 4) ? D2_144_OFS * D2_IB * KB : 256;
 }
 
-__device__ __forceinline__ void dim2_144_load(const float2 *__restrict__ z1, int n1, int n2, int L3h, int c, int i1b,
+__device__ __forceinline__ void dim2_144_load(const float2 *z1, int n1, int n2, int L3h, int c, int i1b,
                                               int k3b, int nk, int KB, int ps, const float2 *__restrict__ tw2,
                                               float2 *__restrict__ sm, int tid, int nth) {
     const int total = D2_IB * D2_144_OFS * KB;
@@ -821,7 +821,7 @@ __device__ __forceinline__ void dim2_144_tail_store(const float2 *__restrict__ s
 }
 
 // its inverse: the transposing load from xa and the inverse radix-9 stage
-__device__ __forceinline__ void dim2_144_tail_load(const float2 *__restrict__ xa, int L3h, int n1p, int c, int i1b,
+__device__ __forceinline__ void dim2_144_tail_load(const float2 *xa, int L3h, int n1p, int c, int i1b,
                                                    int k3b, int nk, int KB, float2 *__restrict__ sm, int tid,
                                                    int nth) {
     const int64_t pstride = (int64_t)L3h * n1p;
@@ -864,7 +864,7 @@ __device__ __forceinline__ void dim2_144_tail_load(const float2 *__restrict__ xa
 // ii fastest, so 8 lanes write one 64-byte i1 run), and their inverses mirror
 // them (d2f_tail_load, d2f_store).
 template <int R1, int R2>
-__device__ __forceinline__ void d2f_load(const float2 *__restrict__ z1, int n1, int n2, int L3h, int c, int i1b,
+__device__ __forceinline__ void d2f_load(const float2 *z1, int n1, int n2, int L3h, int c, int i1b,
                                          int k3b, int nk, int KB, int ps, const float2 *__restrict__ tw2,
                                          float2 *__restrict__ sm, int tid, int nth) {
     constexpr int M = R1 * R2;
@@ -924,7 +924,7 @@ __device__ __forceinline__ void d2f_tail_store(const float2 *__restrict__ sm, in
 }
 
 template <int R1, int R2>
-__device__ __forceinline__ void d2f_tail_load(const float2 *__restrict__ xa, int L3h, int n1p, int c, int i1b,
+__device__ __forceinline__ void d2f_tail_load(const float2 *xa, int L3h, int n1p, int c, int i1b,
                                               int k3b, int nk, int KB, int ps, float2 *__restrict__ sm, int tid,
                                               int nth) {
     constexpr int L = 2 * R1 * R2;
@@ -986,7 +986,7 @@ __device__ __forceinline__ void d2f_store(const float2 *__restrict__ sm, int n1,
 // kk fastest, holds the values i2 = n + m1 j of tile pencil ii * KB + kk,
 // m1 = L2 / (2 R1); the stages from 2 on run in shared memory.
 template <int R1>
-__device__ __forceinline__ void dim2lead_load(const float2 *__restrict__ z1, int n1, int n2, int L3h, int c, int i1b,
+__device__ __forceinline__ void dim2lead_load(const float2 *z1, int n1, int n2, int L3h, int c, int i1b,
                                               int k3b, int nk, int KB, int ps, int L2,
                                               const float2 *__restrict__ tw2, float2 *__restrict__ sm, int tid,
                                               int nth) {
@@ -1076,7 +1076,7 @@ __device__ __forceinline__ void dim2lead_store(const float2 *__restrict__ sm, in
 
 // A2: columns along n2 (zero-padded to L2) -> pencil-major xa[((c L2 + p2) L3h + k3) n1p + i1]
 template <int N2>
-__global__ void __launch_bounds__(288, 4) k_dim2_fwd(const float2 *__restrict__ z1, int n1, int n2, int L3h, int n1p,
+__global__ void __launch_bounds__(288, 4) k_dim2_fwd(const float2 *z1, int n1, int n2, int L3h, int n1p,
                                                   FftLen F2, const float2 *__restrict__ tw2, int KB,
                                                   float2 *__restrict__ xa) {
     extern __shared__ float2 sm[];
@@ -1543,7 +1543,7 @@ struct QuadSets {
 };
 
 template <int N1>
-__global__ void __launch_bounds__(pencil_threads(N1)) k_pencil_quad(const float2 *__restrict__ xa, int n1, int n1p, int L2, int L3h,
+__global__ void __launch_bounds__(pencil_threads(N1)) k_pencil_quad(const float2 *xa, int n1, int n1p, int L2, int L3h,
                                                      FftLen F1, const float2 *__restrict__ tw1, QuadSets ks, int ng,
                                                      double *__restrict__ acc) {
     extern __shared__ float2 sm[];
@@ -1742,7 +1742,7 @@ __global__ void k_sum_tilts(const float *__restrict__ K3, int64_t set, int ng, c
 
 // C2: undo along k2 (positions -> natural), first n2 rows kept, back into z1 rows
 template <int N2>
-__global__ void __launch_bounds__(288, 4) k_dim2_inv(const float2 *__restrict__ xa, int n1, int n2, int L3h, int n1p,
+__global__ void __launch_bounds__(288, 4) k_dim2_inv(const float2 *xa, int n1, int n2, int L3h, int n1p,
                                                   FftLen F2, const float2 *__restrict__ tw2, int KB,
                                                   float2 *__restrict__ z1) {
     extern __shared__ float2 sm[];
@@ -1817,7 +1817,7 @@ __global__ void __launch_bounds__(288, 4) k_dim2_inv(const float2 *__restrict__ 
 // C1: half spectrum k3 in [0, M3] -> real rows (first n3 kept), the inverse of A1
 // returning L3 x (unnormalised; the 1/(L1 L2 L3) lives in the spectra).
 template <int N3>
-__global__ void __launch_bounds__(256) k_c2r_rows(const float2 *__restrict__ z1, int64_t nrows, int n3, FftLen F3,
+__global__ void __launch_bounds__(256) k_c2r_rows(const float2 *z1, int64_t nrows, int n3, FftLen F3,
                                                   const int *__restrict__ pos3, const float2 *__restrict__ twh, int R,
                                                   float *__restrict__ y) {
     extern __shared__ float2 sm[];
