@@ -374,10 +374,12 @@ __global__ void __launch_bounds__(256) k_rows_place(GeomView g, bool raw, double
 // (z, x) <-> (T, X)
 // ---------------------------------------------------------------------------
 
+// the lattice's columns first .. first + nc - 1 of ncols (Lattice::ncc at a time)
 struct LatView {
     const double *X;
     double cg, sg, h;
     int nc, nT, T0;
+    int first, ncols;
 };
 // footprint of node (line t, column k) in the (z, x) plane
 template <int W>
@@ -571,7 +573,7 @@ __device__ __forceinline__ bool strip_order(int i, int nx, int ny, int &x, int &
 constexpr int kCell = 4;
 template <int W>
 __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int reach1, int reach3, int xtiles,
-                                                      const float2 *Gt, float2 *__restrict__ g) {
+                                                      const float2 *Gt, float2 *g) {
     extern __shared__ __align__(16) unsigned char nsm[];
     allow_next();
     const int cap = 2 * blockDim.x;
@@ -607,7 +609,7 @@ __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int 
         __syncthreads();
         n = 0;
     };
-    const double dX = 2 * M_PI / L.nc;
+    const double dX = 2 * M_PI / L.ncols;
     // copies of the cells, one period apart, that the lattice reaches: the
     // footprints lie in [-reach, reach] along each axis
     const int m1 = (reach1 + c1 + kCell) / F.nf1, m3 = (reach3 + c3 + kCell) / F.nf3;
@@ -620,8 +622,8 @@ __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int 
             const double Xm = xm * L.cg - zm * L.sg, Xr = xr * fabs(L.cg) + zr * fabs(L.sg);
             const double Tm = xm * L.sg + zm * L.cg, Tr = xr * fabs(L.sg) + zr * fabs(L.cg);
             // one column / line of margin for the rounding of the positions
-            const int ka = max(0, (int)floor((Xm - Xr + M_PI) / dX - 0.5) - 1);
-            const int kb = min(L.nc - 1, (int)ceil((Xm + Xr + M_PI) / dX - 0.5) + 1);
+            const int ka = max(0, (int)floor((Xm - Xr + M_PI) / dX - 0.5) - 1 - L.first);
+            const int kb = min(L.nc - 1, (int)ceil((Xm + Xr + M_PI) / dX - 0.5) + 1 - L.first);
             const int ta = max(0, (int)floor((Tm - Tr) / L.h) - L.T0 - 1);
             const int tb = min(L.nT - 1, (int)ceil((Tm + Tr) / L.h) - L.T0 + 1);
             if (ka > kb || ta > tb) continue;
@@ -673,7 +675,9 @@ __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int 
         for (int r = 0; r < kCell; ++r) {
             if (c3 + r >= F.nf3) break;
             const float2 a = re[i][r / 2], b = im[i][r / 2];
-            o[r * F.nf2] = r & 1 ? make_float2(a.y, b.y) : make_float2(a.x, b.x);
+            float2 v = r & 1 ? make_float2(a.y, b.y) : make_float2(a.x, b.x);
+            if (L.first) v = make_float2(v.x + o[r * F.nf2].x, v.y + o[r * F.nf2].y);
+            o[r * F.nf2] = v;
         }
     }
 }
@@ -689,8 +693,8 @@ __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int 
 constexpr int kRowGroup = 32;
 template <int W>
 __global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nrow,
-                                                     const float2 *__restrict__ G, int nf2, int pitch, int nc, int groups,
-                                                     float beta, float2 *__restrict__ out) {
+                                                     const float2 *__restrict__ G, int nf2, int pitch, int nc, int ncols,
+                                                     int groups, float beta, float2 *__restrict__ out) {
     __shared__ float wT[kRowGroup][W], wy[kRowGroup][W];
     __shared__ int4 info[kRowGroup];
     const int kb = blockIdx.x / groups, base = (blockIdx.x - kb * groups) * kRowGroup, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -732,7 +736,7 @@ __global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt
             a0 = __ffma2_rn(make_float2(u, u), s0, a0);
             a1 = __ffma2_rn(make_float2(u, u), s1, a1);
         }
-        float2 *o = out + (int64_t)I.x * nc + k;
+        float2 *o = out + (int64_t)I.x * ncols + k;
         o[0] = a0;
         if (k + 1 < nc) o[1] = a1;
     }
@@ -799,7 +803,7 @@ __global__ void __launch_bounds__(128, 4) k_rows_spread(const int *__restrict__ 
                                                      int seg, const uint32_t *__restrict__ start,
                                                      const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nstart,
                                                      int nT, int ntile, int nf2,
-                                                     const float2 *src, int nr, int nc, float beta,
+                                                     const float2 *src, int nr, int nc, int kfirst, int ncols, float beta,
                                                      const float2 *__restrict__ beam, int np, bool half, float scale,
                                                      float2 *__restrict__ Gt) {
     constexpr bool SYM = SRC == NufftPlan::ROWS_SYSMAT, HALF = SRC == NufftPlan::ROWS_HALF;
@@ -859,8 +863,8 @@ __global__ void __launch_bounds__(128, 4) k_rows_spread(const int *__restrict__ 
                 lw[e * kCell + i] = make_float4(s * u[0], s * u[1], s * u[2], s * u[3]);
             }
             const int p = I.w / nr, j = I.w - p * nr;
-            const uint32_t mirror = (uint32_t)(half ? half_row(p, nr - 1 - j, np, nr) : p * nr + nr - 1 - j) * nc + nc - 1;
-            lr[e] = make_uint2((uint32_t)I.x * nc, mirror);
+            const uint32_t mirror = (uint32_t)(half ? half_row(p, nr - 1 - j, np, nr) : p * nr + nr - 1 - j) * ncols + ncols - 1 - kfirst;
+            lr[e] = make_uint2((uint32_t)I.x * ncols + kfirst, mirror);
             if (SYM) {  // conj(a)^2 = (ax^2 - ay^2) - 2 i ax ay
                 const float2 a = beam[p];
                 lb[e] = make_float4(2 * scale * (a.x * a.x - a.y * a.y), -4 * scale * a.x * a.y, 0.f, 0.f);
@@ -1226,8 +1230,9 @@ static Fine fine_of(const NufftPlan &pl) {
     return F;
 }
 static unsigned volume_tiles(const Dims3 &v) { return (unsigned)(v.n1 * ((v.n2 + 31) / 32) * ((v.n3 + 31) / 32)); }
-static LatView lat_view(const Lattice &l, const Geom &g) {
-    return LatView{l.X, l.cg, l.sg, l.h, (int)g.ncols, l.nT, l.T0};
+static LatView lat_view(const Lattice &l, const Geom &g, int64_t first) {
+    return LatView{l.X + first, l.cg, l.sg, l.h, (int)std::min<int64_t>(l.ncc, g.ncols - first), l.nT, l.T0, (int)first,
+                   (int)g.ncols};
 }
 static void check_points(const Geom &g) {
     if (g.npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "too many points in one geometry");
@@ -1469,8 +1474,13 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->nT = nTf + w + 4;
     l->nstart = l->nT - w + 1;
     const int64_t np = g.nproj, nrow = np * g.nrows, cells = (int64_t)l->nstart * nf2;
-    if (cells > (int64_t)INT32_MAX - 1 || l->nT * g.ncols > (int64_t)INT32_MAX)
-        throw Error(ERR_ARG, "node grid too large");
+    if (cells > (int64_t)INT32_MAX - 1) throw Error(ERR_ARG, "node grid too large");
+    // Columns at a time: a wide detector over a thin volume has far more nodes than
+    // fine-grid cells (2400 T lines x 4096 y x 2048 columns for 16 x 2048 x 2048 at 35
+    // degrees: 161 GB), and the columns don't meet before the fine grid.  16 GiB hold
+    // the 955 x 1458 x 1233 nodes of the largest usual case at once.
+    constexpr int64_t kNodeBytes = 16LL << 30;
+    l->ncc = (int)std::min(g.ncols, std::max<int64_t>(64, kNodeBytes / (l->nT * nf2 * (int64_t)sizeof(float2)) / 64 * 64));
     // Segments of k_rows_spread: 256 rows, fewer where that would leave less than
     // about 16 CTAs per SM (a row meets 6 to 9 tiles).
     l->ntile = (l->nT + kCell - 1) / kCell;
@@ -1478,8 +1488,6 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->seg = (int)std::min<int64_t>(256, std::max<int64_t>(32, nrow * 6 * ((g.ncols + 255) / 256) / (148 * 16) / 32 * 32));
     const int64_t meet = (w + kCell - 2) / kCell + 1;  // tiles a footprint meets along one axis, at most
     const int64_t max_items = ntiles + nrow * meet * meet / l->seg + 1;
-    if (max_items > (int64_t)INT32_MAX || nrow * meet * meet > (int64_t)INT32_MAX)
-        throw Error(ERR_ARG, "too many detector rows in one geometry");
     l->max_items = (int)max_items;
     // one allocation for all tables
     size_t bytes = 0;
@@ -1506,7 +1514,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->nitem = reinterpret_cast<int *>(m0 + oni);
     l->items = reinterpret_cast<int2 *>(m0 + oit);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(m0 + ocnt);  // counts, then placement cursors
-    const int64_t need = (int64_t)l->nT * nf2 * node_pitch(g.ncols);
+    const int64_t need = (int64_t)l->nT * nf2 * node_pitch(l->ncc);
     if ((int64_t)work.n < need) work.alloc(need);
     LAMINO_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(reinterpret_cast<char *>(l->items) - reinterpret_cast<char *>(cnt)), s));
     const Fine F = fine_of(*this);
@@ -1539,8 +1547,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
 
 void NufftPlan::nodes_to_rows(const Lattice &l, const Geom &g, float2 *rows, cudaStream_t s) {
     const Fine F = fine_of(*this);
-    const LatView L = lat_view(l, g);
-    const int pitch = (int)node_pitch(g.ncols);
+    const int pitch = (int)node_pitch(l.ncc);
     // The box of cells under a tile of nodes, one cell of slack on either side, for
     // 16 x 8 and 8 x 16 tiles (columns are 1.2 to 2 cells apart, T lines 0.7 to 1):
     // the smaller box is staged, with 16 y where two CTAs then fit an SM, else with
@@ -1560,29 +1567,30 @@ void NufftPlan::nodes_to_rows(const Lattice &l, const Geom &g, float2 *rows, cud
     nchunk = (int)((nf2 + ychunk - 1) / ychunk);
     const int boxcap = cells * ychunk * sizeof(float2) <= kBoxBytes ? (int)cells : 0;
     const int smem = (int)(std::max(boxcap, kNodes + 1) * ychunk * sizeof(float2));
-    const int ktiles = (int)((g.ncols + K - 1) / K);
+    const int ktiles = (l.ncc + K - 1) / K;
     dim3 b1((unsigned)(ktiles * ((l.nT + kNodes / K - 1) / (kNodes / K))));
     b1.y = (unsigned)std::min<int64_t>(nchunk, std::max<int64_t>(1, 148LL * 12 / b1.x));
     const uint32_t ydiv = (uint32_t)((0x100000000ULL + ychunk / 2 - 1) / (ychunk / 2));
     const int64_t nrow = g.nproj * g.nrows;
     const int groups = (int)((nrow + kRowGroup - 1) / kRowGroup);
-    const unsigned b2 = (unsigned)(groups * ((g.ncols + 63) / 64));
     with_width(w, [&](auto WC) {
         constexpr int W = decltype(WC)::value;
         auto ng = K == 16 ? k_nodes_gather<W, 16> : k_nodes_gather<W, 8>;
         raise_smem_limit((const void *)ng, smem);
-        ng<<<b1, 256, smem, s>>>(L, F, grid.p, work.p, pitch, ktiles, ychunk, ydiv, nchunk, boxcap);
-        LAMINO_LAUNCH("k_nodes_gather");
-        k_rows_gather<W><<<b2, 256, 0, s>>>(l.pt, l.pd, (int)nrow, work.p, (int)nf2, pitch, (int)g.ncols, groups, beta,
-                                            rows);
-        LAMINO_LAUNCH("k_rows_gather");
+        for (int64_t k0 = 0; k0 < g.ncols; k0 += l.ncc) {
+            const LatView L = lat_view(l, g, k0);
+            ng<<<b1, 256, smem, s>>>(L, F, grid.p, work.p, pitch, ktiles, ychunk, ydiv, nchunk, boxcap);
+            LAMINO_LAUNCH("k_nodes_gather");
+            k_rows_gather<W><<<(unsigned)groups * ((L.nc + 63) / 64), 256, 0, s>>>(
+                l.pt, l.pd, (int)nrow, work.p, (int)nf2, pitch, L.nc, L.ncols, groups, beta, rows + k0);
+            LAMINO_LAUNCH("k_rows_gather");
+        }
     });
 }
 
 void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *rows, RowSource from, cudaStream_t s) {
     const Fine F = fine_of(*this);
-    const LatView L = lat_view(l, g);
-    const int nc = (int)g.ncols;
+    const int nc = l.ncc;
     // 32 to 128 threads of two columns each: the width that pads the columns least
     int bt = 128;
     for (int b : {96, 64, 32})
@@ -1605,14 +1613,18 @@ void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *row
         constexpr int W = decltype(WC)::value;
         auto rs = from == ROWS_SYSMAT ? k_rows_spread<W, ROWS_SYSMAT>
                   : from == ROWS_HALF ? k_rows_spread<W, ROWS_HALF> : k_rows_spread<W, ROWS_PLAIN>;
-        k_tiles_zero<<<(unsigned)std::min(l.max_items, 148 * 8), 256, 0, s>>>(l.nitem, l.items, l.nT, l.ntile, (int)nf2, nc,
-                                                                              work.p);
-        LAMINO_LAUNCH("k_tiles_zero");
-        launch_after(rs, b1, bt, smem1, s, l.nitem, l.items, l.seg, l.start, l.pt, l.pd, l.nstart, l.nT, l.ntile, (int)nf2, rows, (int)g.nrows, nc, beta,
-                                 l.a, (int)g.nproj, l.half, scale, work.p);
-        LAMINO_LAUNCH("k_rows_spread");
-        launch_after(k_nodes_spread<W>, b2, yb, smem2, s, L, F, reach1, reach3, xtiles, work.p, grid.p);
-        LAMINO_LAUNCH("k_nodes_spread");
+        for (int64_t k0 = 0; k0 < g.ncols; k0 += l.ncc) {
+            const LatView L = lat_view(l, g, k0);
+            k_tiles_zero<<<(unsigned)std::min(l.max_items, 148 * 8), 256, 0, s>>>(l.nitem, l.items, l.nT, l.ntile, (int)nf2,
+                                                                                  L.nc, work.p);
+            LAMINO_LAUNCH("k_tiles_zero");
+            launch_after(rs, b1, bt, smem1, s, l.nitem, l.items, l.seg, l.start, l.pt, l.pd, l.nstart, l.nT, l.ntile,
+                         (int)nf2, rows, (int)g.nrows, L.nc, L.first, L.ncols, beta, l.a, (int)g.nproj, l.half, scale,
+                         work.p);
+            LAMINO_LAUNCH("k_rows_spread");
+            launch_after(k_nodes_spread<W>, b2, yb, smem2, s, L, F, reach1, reach3, xtiles, work.p, grid.p);
+            LAMINO_LAUNCH("k_nodes_spread");
+        }
     });
 }
 

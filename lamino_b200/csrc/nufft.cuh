@@ -37,6 +37,7 @@ struct Lattice {
     double cg = 1, sg = 0, h = 0;
     int nT = 0, T0 = 0;
     int nstart = 0;          // footprint starts along T: nT - w + 1
+    int ncc = 0;             // columns of the node grid at a time
     DevBuf<char> mem;        // holds the tables below
     double *X = nullptr;     // column frequencies
     float *ipT = nullptr;    // 1 / p_T of every mode (k1, k3): deconvolution along T
