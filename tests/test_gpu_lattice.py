@@ -31,6 +31,7 @@ CASES = [
     ((11, 6, 9), 4, 18, 20, 0.7, 1e-4),
     ((11, 6, 9), 4, 18, 20, 0.7, 1e-5),
     ((11, 6, 9), 4, 18, 20, 0.7, 1e-7),
+    ((103, 101, 105), 3, 16, 21, 0.6, 1.2e-6),  # over 8 million cells: the split fine-grid transform
 ]
 
 
