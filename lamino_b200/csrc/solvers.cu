@@ -273,6 +273,49 @@ __device__ __forceinline__ float d_potential(float delta, const QgConst &k) {
     return a * (2.0f - k.qmp * t1 * r);
 }
 
+// d_potential of two differences at once, operation by operation the same with the
+// arithmetic packed in pairs.  Differences outside pow_pos's range go one by one.
+__device__ __forceinline__ float2 d_potential2(float2 delta, const QgConst &k) {
+    auto both = [](float v) { return make_float2(v, v); };
+    const float ax = fabsf(delta.x), ay = fabsf(delta.y);
+    const int bx = __float_as_int(ax), by = __float_as_int(ay);
+    const int ex = (bx - 0x3f3504f3) >> 23, ey = (by - 0x3f3504f3) >> 23;
+    const float2 f = __fadd2_rn(make_float2(__int_as_float(bx - (ex << 23)), __int_as_float(by - (ey << 23))), both(-1.0f));
+    float2 p = both(0.12926264f);
+    p = __ffma2_rn(p, f, both(-0.20893306f));
+    p = __ffma2_rn(p, f, both(0.21521251f));
+    p = __ffma2_rn(p, f, both(-0.2386758f));
+    p = __ffma2_rn(p, f, both(0.28793907f));
+    p = __ffma2_rn(p, f, both(-0.36071625f));
+    p = __ffma2_rn(p, f, both(0.48091027f));
+    p = __ffma2_rn(p, f, both(-0.7213472f));
+    p = __ffma2_rn(p, f, both(1.442695f));
+    const float2 q = both(k.qmp), ef = make_float2((float)ex, (float)ey);
+    const float2 nph = __fmul2_rn(both(-k.qmp), ef);  // -q e
+    const float2 low = __ffma2_rn(q, __fmul2_rn(f, p), __ffma2_rn(q, ef, nph));
+    const float2 t = __ffma2_rn(nph, both(-1.0f), low), rm = __fadd2_rn(t, both(12582912.0f));
+    const float2 z = __ffma2_rn(__fadd2_rn(nph, __fadd2_rn(rm, both(-12582912.0f))), both(-1.0f), low);
+    float2 v = both(0.00015478018f);
+    v = __ffma2_rn(v, z, both(0.0013400431f));
+    v = __ffma2_rn(v, z, both(0.009617995f));
+    v = __ffma2_rn(v, z, both(0.05550327f));
+    v = __ffma2_rn(v, z, both(0.24022652f));
+    v = __ffma2_rn(v, z, both(0.6931472f));
+    v = __ffma2_rn(v, z, both(1.0f));
+    const bool zx = !(ax > 0.f), zy = !(ay > 0.f);
+    if ((zx || ((unsigned)bx - 0x00800000u < 0x7f000000u && fabsf(t.x) < 120.0f)) &&
+        (zy || ((unsigned)by - 0x00800000u < 0x7f000000u && fabsf(t.y) < 120.0f))) {
+        const float2 w = make_float2(__int_as_float(__float_as_int(v.x) + (__float_as_int(rm.x) << 23)),
+                                     __int_as_float(__float_as_int(v.y) + (__float_as_int(rm.y) << 23)));
+        const float2 t1 = __fmul2_rn(w, both(k.inv_sqp)), t3 = __fadd2_rn(both(0.001f), t1);
+        const float2 r = make_float2(__fdividef(1.0f, t3.x), __fdividef(1.0f, t3.y));
+        const float2 a = __fmul2_rn(__fmul2_rn(delta, r), both(k.inv_sq));
+        const float2 o = __fmul2_rn(a, __ffma2_rn(__fmul2_rn(both(-k.qmp), t1), r, both(2.0f)));
+        return make_float2(zx ? k.at_zero : o.x, zy ? k.at_zero : o.y);
+    }
+    return make_float2(d_potential(delta.x, k), d_potential(delta.y, k));
+}
+
 // qGGMRF gradient: g[interior] += sum over the 26 neighbours of w_d rho'(x[c+d] -
 // x[c]) (src/qggmrf.cpp:60-95), with each neighbour pair's derivative evaluated
 // once.  rho'(-delta) = -rho'(delta) exactly in float for delta != 0 (the sign only
@@ -286,12 +329,14 @@ __device__ __forceinline__ float d_potential(float delta, const QgConst &k) {
 // dy, dz from -1 to 1), as a direct 26-neighbour loop would add them.
 // Tiles start at the first interior column, and their height divides the interior
 // rows with the least halo (TJ: 14 rows for 44 thick, 10 for 22 and 32, 8 for 10).
-// Bound by instruction issue (13 powers per voxel).  Measured at 362 x 44 x 362,
-// sigma 1000, p 1.2: 262 us; 424 with powf, IEEE division and tiles of 12 from the
-// border in two waves of CTAs.
+// Bound by instruction issue (13 powers per voxel), so pairs are evaluated two at a
+// time with packed arithmetic.  Measured at 362 x 44 x 362, sigma 1000, p 1.2:
+// 243 us; 262 one pair at a time; 424 with powf, IEEE division and tiles of 12 from
+// the border in two waves of CTAs.  The registers of the packed form cost the tiles of 8
+// and 12 rows a resident CTA (without that, spills: 90 x 10 x 90 16.5 against 14.5 us).
 constexpr int QG_TK = 32, QG_HK = QG_TK + 2;
 __host__ __device__ constexpr int qg_threads(int TJ) { return (TJ + 2) * QG_HK; }  // 340, 408, 476, 544 threads
-__host__ __device__ constexpr int qg_ctas(int TJ) { return TJ <= 8 ? 4 : TJ <= 12 ? 3 : 2; }  // resident per SM
+__host__ __device__ constexpr int qg_ctas(int TJ) { return TJ <= 10 ? 3 : 2; }  // resident per SM
 
 template <int TJ>
 __global__ void __launch_bounds__(qg_threads(TJ), qg_ctas(TJ)) k_qggmrf_pairs(float *__restrict__ g, const float *__restrict__ x,
@@ -321,22 +366,31 @@ __global__ void __launch_bounds__(qg_threads(TJ), qg_ctas(TJ)) k_qggmrf_pairs(fl
         const float u = xc[0];
         if (i + 1 < n1) {
             const float *xn = xc + si;
-#pragma unroll
-            for (int e = 0; e < 9; ++e) {
-                const float delta = xn[(e / 3 == 0 ? ym : e / 3 == 1 ? 0 : yp) + (e % 3 == 0 ? zm : e % 3 == 1 ? 0 : zp)] - u;
-                const float pv = d_potential(delta, kq);
+            auto diff = [&](int e) {
+                return xn[(e / 3 == 0 ? ym : e / 3 == 1 ? 0 : yp) + (e % 3 == 0 ? zm : e % 3 == 1 ? 0 : zp)] - u;
+            };
+            auto keep = [&](int e, float delta, float pv) {
                 p9[e] = pv;
                 q9[buf][e][t] = !(fabsf(delta) > 0.f) ? kq.at_zero : -pv;
+            };
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const float2 delta = make_float2(diff(e), diff(e + 1)), pv = d_potential2(delta, kq);
+                keep(e, delta.x, pv.x);
+                keep(e + 1, delta.y, pv.y);
             }
+            const float delta = diff(8);
+            keep(8, delta, d_potential(delta, kq));
         }
         if (with4) {
             const int off[4] = {zp, yp + zm, yp, yp + zp};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float delta = xc[off[e]] - u;
-                const float pv = d_potential(delta, kq);
-                p4[e] = pv;
-                q4[e][t] = !(fabsf(delta) > 0.f) ? kq.at_zero : -pv;
+            for (int e = 0; e < 4; e += 2) {
+                const float2 delta = make_float2(xc[off[e]] - u, xc[off[e + 1]] - u), pv = d_potential2(delta, kq);
+                p4[e] = pv.x;
+                p4[e + 1] = pv.y;
+                q4[e][t] = !(fabsf(delta.x) > 0.f) ? kq.at_zero : -pv.x;
+                q4[e + 1][t] = !(fabsf(delta.y) > 0.f) ? kq.at_zero : -pv.y;
             }
         }
     };
