@@ -711,9 +711,9 @@ def fp32_peak_tflops(torch) -> float:
 def nufft_measure(torch, L, scale: str, warmup: int, steps: int, bins=None):
     """The plain NUFFT form of the operator at a bench scale: forward and adjoint
     projection of one gamma dataset and the sum-over-gamma sysmat (interp ->
-    weight -> spread per point), CUDA-event timed with inputs in HBM, with the
-    FP32 rate of the taps.  The first call of each geometry includes its bin
-    sort (cached afterwards)."""
+    weight -> spread), CUDA-event timed with inputs in HBM, with the
+    FP32 rate of the detector points' taps.  The first call of each geometry
+    includes its lattice tables (cached afterwards)."""
     import numpy as np
     dims, nproj, det = SCALES[scale]
     rng = np.random.default_rng(2026)
@@ -739,7 +739,7 @@ def nufft_measure(torch, L, scale: str, warmup: int, steps: int, bins=None):
         return e0.elapsed_time(e1) / k
 
     t_sort = time.perf_counter()
-    L.adjoint(proj, pgs[0], dims, plan=plan)  # includes the bin sort of pgs[0]
+    L.adjoint(proj, pgs[0], dims, plan=plan)  # includes the tables of pgs[0]
     torch.cuda.synchronize()
     t_sort = time.perf_counter() - t_sort
     k = max(1, steps)
@@ -748,8 +748,9 @@ def nufft_measure(torch, L, scale: str, warmup: int, steps: int, bins=None):
     ms_sys = timed(lambda: L.sysmat(x, pgs, plan=plan), k)
     M = nproj * det * det
     w = 7
-    # one spread or one interpolation: 3 components x w^3 taps x 2 FMA (real weight x complex) per point
-    flop_pass = 3 * w ** 3 * 2 * 2 * M
+    # one spread or one interpolation between detector rows and the (T, X) lines of the
+    # lattice: w^2 taps x 2 FMA (real weight x complex) per point
+    flop_pass = w ** 2 * 2 * 2 * M
     peak = fp32_peak_tflops(torch)
     rate = {"adjoint": flop_pass / (ms_adj / 1e3) / 1e12, "forward": flop_pass / (ms_fwd / 1e3) / 1e12,
             "sysmat": 2 * len(pgs) * flop_pass / (ms_sys / 1e3) / 1e12}
@@ -760,7 +761,8 @@ def nufft_measure(torch, L, scale: str, warmup: int, steps: int, bins=None):
             "fp32_tflops": rate, "fp32_peak_tflops": peak,
             "fp32_frac": {kk: v / peak for kk, v in rate.items()},
             "fp32_peak_source": "nominal: SMs x 128 FP32 lanes x 2 FLOP x max SM clock",
-            "flop_count": "4116 FLOP per point per spread or interpolation (343 taps x 3 components x 2 FMA)"}
+            "flop_count": "196 FLOP per point per spread or interpolation (49 taps x 2 FMA of one complex value; "
+                          "the lattice lines' own 49 taps are not counted)"}
 
 
 def run_nufft_form(args):
