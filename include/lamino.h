@@ -62,18 +62,18 @@ int lamino_geom_destroy(lamino_geom_t g);
  */
 int lamino_plan_create(int64_t n1, int64_t n2, int64_t n3, double eps, lamino_plan_t *out);
 int lamino_plan_destroy(lamino_plan_t p);
-/* Fine-grid bins of b1 x b2 x b3 cells for the plan's spreading and
- * interpolation (each bin's tile of (b + w - 1)^3 cells per component is staged
- * in shared memory); default 4 x 8 x 16.  Drops the plan's cached point orders.
+/* Fine-grid bins of b1 x b2 x b3 cells, a hint (default 4 x 8 x 16): the present
+ * kernels follow the detector points' lattice and need no bins, so results and
+ * times do not depend on them.  Layouts whose tiles of (b + w - 1)^3 cells per
+ * component exceed shared memory are refused, as before.
  * No reference counterpart (FINUFFT's opts.gpu_binsize* play this role in
  * cuFINUFFT). */
 int lamino_plan_set_bins(lamino_plan_t p, int b1, int b2, int b3);
-/* Autotuner: times candidate bin layouts on the given geometries and keeps the
- * fastest for objective 0 (adjoint of geoms[0] including its bin sort, a setup
- * pass) or 1 (sum over geoms of sysmat with cached sorts, a solver's operator).
- * The choice is cached per fine grid, kernel width, objective and point count
- * for the process.  bins[3] (may be NULL) receives the layout, *best_ms (may be
- * NULL) its time (0 when taken from the cache). */
+/* Times the plan's operator on the given geometries for objective 0 (adjoint of
+ * geoms[0], a setup pass) or 1 (sum over geoms of sysmat, a solver's operator).
+ * Cached per fine grid, kernel width, objective and point count for the process.
+ * bins[3] (may be NULL) receives the plan's bin layout, *best_ms (may be
+ * NULL) the time (0 when taken from the cache). */
 int lamino_plan_autotune(lamino_plan_t p, const lamino_geom_t *geoms, int ngeom, int objective, int *bins,
                          double *best_ms, void *stream);
 /* Type 2, iflag -1: c[j] = sum_k modes[k] e^{-i k.x_j} (include/nufft.h:52-64).
@@ -226,7 +226,7 @@ typedef struct {
     double eps;
     int refinements;
     int use_graphs; /* replay each solver iteration's operator work as a CUDA graph (non-default streams) */
-    int autotune;   /* pick launch shapes / bin layouts by timing (cached per size) */
+    int autotune;   /* pick launch shapes by timing (cached per size) */
 } lamino_recon_params;
 void lamino_recon_params_default(lamino_recon_params *p);
 /* method 1, 2 or 3.  projs[i]: [proj_dims[3i]][proj_dims[3i+1]][proj_dims[3i+2]];

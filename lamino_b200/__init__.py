@@ -211,14 +211,13 @@ class NufftPlan:
         self._h = h
 
     def set_bins(self, b1: int, b2: int, b3: int):
-        """Fine-grid bin size of the shared-memory spreading / interpolation."""
+        """Fine-grid bin size, a hint: results and times do not depend on it."""
         _check(lib().lamino_plan_set_bins(self._h, int(b1), int(b2), int(b3)))
         return self
 
     def autotune(self, grids, objective: str = "normal"):
-        """Time candidate bin layouts on `grids` and keep the fastest for
-        'adjoint' (one setup pass incl. the sort) or 'normal' (repeated sysmat);
-        returns (bins, best_ms)."""
+        """Time the plan's operator on `grids`: 'adjoint' (one setup pass) or
+        'normal' (sysmat); returns (bins, best_ms)."""
         arr = (ctypes.c_void_p * len(grids))(*[g._h.value for g in grids])
         b = (ctypes.c_int * 3)()
         ms = ctypes.c_double()
@@ -535,7 +534,7 @@ class ReconParams:
     form: op_kind 'toeplitz' (FP32 spectra), 'toeplitz_fp16', 'nufft' or 'mixed'
     (FP16 correction solves in `refinements` FP32-residual cycles), and
     use_graphs (replay each solver iteration's operator work as a CUDA graph) and
-    autotune (launch shapes / bin layouts picked by timing, cached per size)."""
+    autotune (launch shapes picked by timing, cached per size)."""
 
     def __init__(self, **kw):
         c = _ReconParamsC()
