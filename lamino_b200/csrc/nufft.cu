@@ -380,6 +380,7 @@ struct LatView {
     double cg, sg, h;
     int nc, nT, T0;
     int first, ncols;
+    double p1, p3, kX, kT;  // position per z and x cell, columns and T lines per position
 };
 // footprint of node (line t, column k) in the (z, x) plane
 template <int W>
@@ -609,23 +610,22 @@ __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int 
         __syncthreads();
         n = 0;
     };
-    const double dX = 2 * M_PI / L.ncols;
     // copies of the cells, one period apart, that the lattice reaches: the
     // footprints lie in [-reach, reach] along each axis
     const int m1 = (reach1 + c1 + kCell) / F.nf1, m3 = (reach3 + c3 + kCell) / F.nf3;
     for (int b1 = c1 - m1 * F.nf1; b1 <= reach1; b1 += F.nf1)
         for (int b3 = c3 - m3 * F.nf3; b3 <= reach3; b3 += F.nf3) {
             // positions whose footprint starts in [b - W + 1, b + kCell - 1]
-            const double zlo = (b1 - W + 0.5 * W) / F.s1, zhi = (b1 + kCell - 1 + 0.5 * W) / F.s1;
-            const double xlo = (b3 - W + 0.5 * W) / F.s3, xhi = (b3 + kCell - 1 + 0.5 * W) / F.s3;
+            const double zlo = (b1 - W + 0.5 * W) * L.p1, zhi = (b1 + kCell - 1 + 0.5 * W) * L.p1;
+            const double xlo = (b3 - W + 0.5 * W) * L.p3, xhi = (b3 + kCell - 1 + 0.5 * W) * L.p3;
             const double xm = 0.5 * (xlo + xhi), zm = 0.5 * (zlo + zhi), xr = 0.5 * (xhi - xlo), zr = 0.5 * (zhi - zlo);
             const double Xm = xm * L.cg - zm * L.sg, Xr = xr * fabs(L.cg) + zr * fabs(L.sg);
             const double Tm = xm * L.sg + zm * L.cg, Tr = xr * fabs(L.sg) + zr * fabs(L.cg);
             // one column / line of margin for the rounding of the positions
-            const int ka = max(0, (int)floor((Xm - Xr + M_PI) / dX - 0.5) - 1 - L.first);
-            const int kb = min(L.nc - 1, (int)ceil((Xm + Xr + M_PI) / dX - 0.5) + 1 - L.first);
-            const int ta = max(0, (int)floor((Tm - Tr) / L.h) - L.T0 - 1);
-            const int tb = min(L.nT - 1, (int)ceil((Tm + Tr) / L.h) - L.T0 + 1);
+            const int ka = max(0, (int)floor((Xm - Xr + M_PI) * L.kX - 0.5) - 1 - L.first);
+            const int kb = min(L.nc - 1, (int)ceil((Xm + Xr + M_PI) * L.kX - 0.5) + 1 - L.first);
+            const int ta = max(0, (int)floor((Tm - Tr) * L.kT) - L.T0 - 1);
+            const int tb = min(L.nT - 1, (int)ceil((Tm + Tr) * L.kT) - L.T0 + 1);
             if (ka > kb || ta > tb) continue;
             const int nk = kb - ka + 1, cnt = nk * (tb - ta + 1);
             for (int base = 0; base < cnt; base += blockDim.x) {
@@ -1230,9 +1230,9 @@ static Fine fine_of(const NufftPlan &pl) {
     return F;
 }
 static unsigned volume_tiles(const Dims3 &v) { return (unsigned)(v.n1 * ((v.n2 + 31) / 32) * ((v.n3 + 31) / 32)); }
-static LatView lat_view(const Lattice &l, const Geom &g, int64_t first) {
+static LatView lat_view(const Lattice &l, const Geom &g, const Fine &F, int64_t first) {
     return LatView{l.X + first, l.cg, l.sg, l.h, (int)std::min<int64_t>(l.ncc, g.ncols - first), l.nT, l.T0, (int)first,
-                   (int)g.ncols};
+                   (int)g.ncols, 1.0 / F.s1, 1.0 / F.s3, g.ncols * (0.5 / M_PI), 1.0 / l.h};
 }
 static void check_points(const Geom &g) {
     if (g.npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "too many points in one geometry");
@@ -1578,7 +1578,7 @@ void NufftPlan::nodes_to_rows(const Lattice &l, const Geom &g, float2 *rows, cud
         auto ng = K == 16 ? k_nodes_gather<W, 16> : k_nodes_gather<W, 8>;
         raise_smem_limit((const void *)ng, smem);
         for (int64_t k0 = 0; k0 < g.ncols; k0 += l.ncc) {
-            const LatView L = lat_view(l, g, k0);
+            const LatView L = lat_view(l, g, F, k0);
             ng<<<b1, 256, smem, s>>>(L, F, grid.p, work.p, pitch, ktiles, ychunk, ydiv, nchunk, boxcap);
             LAMINO_LAUNCH("k_nodes_gather");
             k_rows_gather<W><<<(unsigned)groups * ((L.nc + 63) / 64), 256, 0, s>>>(
@@ -1614,7 +1614,7 @@ void NufftPlan::rows_to_nodes(const Lattice &l, const Geom &g, const float2 *row
         auto rs = from == ROWS_SYSMAT ? k_rows_spread<W, ROWS_SYSMAT>
                   : from == ROWS_HALF ? k_rows_spread<W, ROWS_HALF> : k_rows_spread<W, ROWS_PLAIN>;
         for (int64_t k0 = 0; k0 < g.ncols; k0 += l.ncc) {
-            const LatView L = lat_view(l, g, k0);
+            const LatView L = lat_view(l, g, F, k0);
             k_tiles_zero<<<(unsigned)std::min(l.max_items, 148 * 8), 256, 0, s>>>(l.nitem, l.items, l.nT, l.ntile, (int)nf2,
                                                                                   L.nc, work.p);
             LAMINO_LAUNCH("k_tiles_zero");
