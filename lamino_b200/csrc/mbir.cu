@@ -96,17 +96,23 @@ int64_t mbir_footprint(int method, const std::vector<std::array<int64_t, 3>> &pr
     const Dims3 od = padded_dims(method, recon, prm);
     const float pf = proj_pad_factor(method, prm);
     const int64_t V = od.size();
-    int64_t raw = 0, maxpts = 0;
+    int64_t raw = 0, maxpts = 0, maxcols = 0;
     for (auto &d : proj_dims) {
         raw += d[0] * d[1] * d[2] * 4;
         maxpts = std::max<int64_t>(maxpts, d[0] * pad2d_len(d[1], pf) * pad2d_len(d[2], pf));
+        maxcols = std::max<int64_t>(maxcols, pad2d_len(d[2], pf));
     }
     const int w = es_width(prm.eps);
-    const int64_t nf = next_smooth_even(std::max<int64_t>(2 * od.n1, 2 * w)) *
-                       next_smooth_even(std::max<int64_t>(2 * od.n2, 2 * w)) *
+    const int64_t nf2 = next_smooth_even(std::max<int64_t>(2 * od.n2, 2 * w));
+    const int64_t nf = next_smooth_even(std::max<int64_t>(2 * od.n1, 2 * w)) * nf2 *
                        next_smooth_even(std::max<int64_t>(2 * od.n3, 2 * w));
+    // the NUFFT's grids: seven fine grids cover one, its FFT work and the node grid,
+    // but for detectors far wider than the volume (T lines of the steepest tilt)
+    const int64_t lines = 2 * (int64_t)std::ceil(std::hypot((double)od.n1, (double)od.n3)) + 3 * w + 6;
+    const int64_t nodes = NufftPlan::node_bytes(lines, nf2, maxcols);
+    const int64_t grids = std::max<int64_t>((6 + 1) * nf * 8, 3 * nf * 8 + nodes);
     // setup: raw + padded projections, projection spectra + 2-D FFT work, fine grids + 3-D FFT work
-    const int64_t setup = raw + maxpts * 4 + 2 * maxpts * 8 + (6 + 1) * nf * 8 + 3 * V * 4;
+    const int64_t setup = raw + maxpts * 4 + 2 * maxpts * 8 + grids + 3 * V * 4;
     const int64_t L1 = next_smooth_even(2 * od.n1), L2 = next_smooth_even(2 * od.n2), L3 = next_smooth_even(2 * od.n3);
     const int64_t S = L1 * L2 * (L3 / 2 + 1), L = L1 * L2 * L3;
     const int64_t n1p = (od.n1 + 7) / 8 * 8;
@@ -115,7 +121,7 @@ int64_t mbir_footprint(int method, const std::vector<std::array<int64_t, 3>> &pr
     int64_t op = 6 * S * kb + inter;
     const int64_t build = 6 * L * 4 + 2 * S * 8;  // transient kernel grids + R2C output and work
     if (method == 3) op += (int64_t)proj_dims.size() * (6 * S * 4 + inter);  // per-gamma operators for the loss
-    if (prm.op_kind == OP_NUFFT) op = (6 + 1) * nf * 8 + 2 * maxpts * 8;
+    if (prm.op_kind == OP_NUFFT) op = grids + 2 * maxpts * 8;
     const int64_t state = (method == 2 ? 40 : 12) * V * 4 + 3 * V * 4;
     const int64_t solve = op + state + (prm.op_kind == OP_NUFFT ? 0 : build);
     const int64_t peak = std::max(setup, solve + 3 * V * 4 + raw);

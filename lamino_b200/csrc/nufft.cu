@@ -1475,12 +1475,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->nstart = l->nT - w + 1;
     const int64_t np = g.nproj, nrow = np * g.nrows, cells = (int64_t)l->nstart * nf2;
     if (cells > (int64_t)INT32_MAX - 1) throw Error(ERR_ARG, "node grid too large");
-    // Columns at a time: a wide detector over a thin volume has far more nodes than
-    // fine-grid cells (2400 T lines x 4096 y x 2048 columns for 16 x 2048 x 2048 at 35
-    // degrees: 161 GB), and the columns don't meet before the fine grid.  16 GiB hold
-    // the 955 x 1458 x 1233 nodes of the largest usual case at once.
-    constexpr int64_t kNodeBytes = 16LL << 30;
-    l->ncc = (int)std::min(g.ncols, std::max<int64_t>(64, kNodeBytes / (l->nT * nf2 * (int64_t)sizeof(float2)) / 64 * 64));
+    l->ncc = (int)node_columns(l->nT, nf2, g.ncols);
     // Segments of k_rows_spread: 256 rows, fewer where that would leave less than
     // about 16 CTAs per SM (a row meets 6 to 9 tiles).
     l->ntile = (l->nT + kCell - 1) / kCell;

@@ -115,7 +115,19 @@ struct NufftPlan {
     enum RowSource { ROWS_PLAIN, ROWS_SYSMAT, ROWS_HALF };  // see k_rows_spread
     void rows_to_nodes(const Lattice &lat, const Geom &g, const float2 *rows, RowSource from, cudaStream_t s);
     // whole 128-byte lines, so that a run of columns never straddles one
-    int64_t node_pitch(int64_t ncols) const { return (ncols + 15) / 16 * 16; }
+    static int64_t node_pitch(int64_t ncols) { return (ncols + 15) / 16 * 16; }
+    // columns of the node grid at a time (Lattice::ncc), and the bytes they take.  A wide
+    // detector over a thin volume has far more nodes than fine-grid cells (2400 T
+    // lines x 4096 y x 2048 columns for 16 x 2048 x 2048 at 35 degrees: 161 GB), and the
+    // columns don't meet before the fine grid.  The largest usual case (721 x 71 x 721, 1233
+    // columns) takes 2.9 GB, in one piece.
+    static int64_t node_columns(int64_t lines, int64_t nf2, int64_t ncols) {
+        constexpr int64_t kBytes = 4LL << 30;
+        return std::min(ncols, std::max<int64_t>(64, kBytes / (lines * nf2 * (int64_t)sizeof(float2)) / 64 * 64));
+    }
+    static int64_t node_bytes(int64_t lines, int64_t nf2, int64_t ncols) {
+        return lines * nf2 * node_pitch(node_columns(lines, nf2, ncols)) * (int64_t)sizeof(float2);
+    }
 };
 
 }  // namespace lamino

@@ -55,8 +55,8 @@ def test_lattice_transforms_vs_oracle(L, O, dims, nproj, nrows, ncols, gamma, ep
 
 
 def test_columns_in_several_chunks(L, O):
-    """A detector so wide that the node grid passes 16 GiB is taken in chunks of
-    columns (here 25 T lines x 800 y x 8 bytes a column, 107328 columns at a time);
+    """A detector so wide that the node grid passes 4 GiB is taken in chunks of
+    columns (here 25 T lines x 800 y x 8 bytes a column, 26816 columns at a time);
     a thin volume leaves sums that the oracle takes term by term.  Type 1 adds up to
     750 thousand nodes into a cell one after the other, whose rounding grows with
     the root of their number: 2^-24 sqrt(750e3) = 5e-5 beside the other 2.2e-5."""
