@@ -687,15 +687,20 @@ __global__ void __launch_bounds__(256, 3) k_nodes_spread(LatView L, Fine F, int 
 // ---------------------------------------------------------------------------
 
 // Nodes -> rows.  A CTA takes 32 rows, consecutive in cell order, and 64
-// columns; a warp one row at a time, two columns per lane, w^2 16-byte loads
+// columns; a warp two rows at a time, two columns per lane, 16-byte loads
 // of contiguous columns.  Rows of neighbouring cells share most of their taps,
-// which stay in L1.
+// which stay in L1, whose bandwidth is the bound.  There are 0.7 to 1.7 rows per
+// cell, so the next row mostly starts in the same T line or the next one: w + 1
+// lines then hold the taps of both, with the weights padded by zeros, and each value
+// is read once for the two (the weights in registers, at three CTAs per SM).
+// Measured (before: one row at a time): 2 x 91 x 309^2 270 -> 212 us, 181 x 362^2
+// 398 -> 340 us, 90 x 200 x 181 58.8 -> 50.9 us.
 constexpr int kRowGroup = 32;
 template <int W>
-__global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nrow,
+__global__ void __launch_bounds__(256, 3) k_rows_gather(const int4 *__restrict__ pt, const float2 *__restrict__ pd, int nrow,
                                                      const float2 *__restrict__ G, int nf2, int pitch, int nc, int ncols,
                                                      int groups, float beta, float2 *__restrict__ out) {
-    __shared__ float wT[kRowGroup][W], wy[kRowGroup][W];
+    __shared__ float wT[kRowGroup][W + 2], wy[kRowGroup][W];  // wT between two zeros
     __shared__ int4 info[kRowGroup];
     const int kb = blockIdx.x / groups, base = (blockIdx.x - kb * groups) * kRowGroup, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x < 2 * kRowGroup) {
@@ -705,7 +710,8 @@ __global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt
             if (threadIdx.x < kRowGroup) {
                 info[r] = pt[q];
 #pragma unroll
-                for (int t = 0; t < W; ++t) wT[r][t] = es_weight<W>(d.x, t, beta);
+                for (int t = 0; t < W; ++t) wT[r][t + 1] = es_weight<W>(d.x, t, beta);
+                wT[r][0] = wT[r][W + 1] = 0.f;
             } else {
 #pragma unroll
                 for (int t = 0; t < W; ++t) wy[r][t] = es_weight<W>(d.y, t, beta);
@@ -716,29 +722,68 @@ __global__ void __launch_bounds__(256) k_rows_gather(const int4 *__restrict__ pt
     const int k = kb * 64 + 2 * lane;
     if (k >= nc) return;
     const int64_t line = (int64_t)nf2 * pitch;
-    for (int r = warp; r < kRowGroup && base + r < nrow; r += 8) {
-        const int4 I = info[r];
-        const float2 *p = G + I.y * line + k;
-        float2 a0 = make_float2(0.f, 0.f), a1 = a0;
-#pragma unroll
-        for (int t2 = 0; t2 < W; ++t2) {
-            int yy = I.z + t2; if (yy >= nf2) yy -= nf2;
-            const float2 *q = p + (int64_t)yy * pitch;
-            float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll
-            for (int t1 = 0; t1 < W; ++t1) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(q + t1 * line));
-                const float u = wT[r][t1];
-                s0 = __ffma2_rn(make_float2(u, u), make_float2(v.x, v.y), s0);
-                s1 = __ffma2_rn(make_float2(u, u), make_float2(v.z, v.w), s1);
-            }
-            const float u = wy[r][t2];
-            a0 = __ffma2_rn(make_float2(u, u), s0, a0);
-            a1 = __ffma2_rn(make_float2(u, u), s1, a1);
-        }
-        float2 *o = out + (int64_t)I.x * ncols + k;
+    auto store = [&](int id, float2 a0, float2 a1) {
+        float2 *o = out + (int64_t)id * ncols + k;
         o[0] = a0;
         if (k + 1 < nc) o[1] = a1;
+    };
+    auto tap = [](float u, float4 v, float2 &s0, float2 &s1) {
+        s0 = __ffma2_rn(make_float2(u, u), make_float2(v.x, v.y), s0);
+        s1 = __ffma2_rn(make_float2(u, u), make_float2(v.z, v.w), s1);
+    };
+    for (int r = 2 * warp; r < kRowGroup && base + r < nrow; r += 16) {
+        const int4 I = info[r], J = info[r + 1];
+        const bool two = base + r + 1 < nrow;
+        const int d = J.y - I.y;
+        if (two && J.z == I.z && (unsigned)d <= 1u) {  // W + 1 lines hold the taps of both
+            const float2 *p = G + I.y * line + k;
+            float wa[W + 1], wb[W + 1];
+#pragma unroll
+            for (int t = 0; t <= W; ++t) {
+                wa[t] = wT[r][t + 1];
+                wb[t] = wT[r + 1][t + 1 - d];
+            }
+            float2 a0 = make_float2(0.f, 0.f), a1 = a0, b0 = a0, b1 = a0;
+#pragma unroll
+            for (int t2 = 0; t2 < W; ++t2) {
+                int yy = I.z + t2; if (yy >= nf2) yy -= nf2;
+                const float2 *q = p + (int64_t)yy * pitch;
+                float2 s0 = make_float2(0.f, 0.f), s1 = s0, u0 = s0, u1 = s0;
+#pragma unroll
+                for (int t1 = 0; t1 <= W; ++t1) {
+                    // (with d = 0 the line after the last one may not exist; its weights are zero)
+                    const float4 v = __ldg(reinterpret_cast<const float4 *>(q + (t1 < W ? t1 : W - 1 + d) * line));
+                    tap(wa[t1], v, s0, s1);
+                    tap(wb[t1], v, u0, u1);
+                }
+                const float fa = wy[r][t2], fb = wy[r + 1][t2];
+                a0 = __ffma2_rn(make_float2(fa, fa), s0, a0);
+                a1 = __ffma2_rn(make_float2(fa, fa), s1, a1);
+                b0 = __ffma2_rn(make_float2(fb, fb), u0, b0);
+                b1 = __ffma2_rn(make_float2(fb, fb), u1, b1);
+            }
+            store(I.x, a0, a1);
+            store(J.x, b0, b1);
+            continue;
+        }
+        for (int e = 0; e < 1 + two; ++e) {
+            const int4 R = e ? J : I;
+            const float2 *p = G + R.y * line + k;
+            float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+#pragma unroll
+            for (int t2 = 0; t2 < W; ++t2) {
+                int yy = R.z + t2; if (yy >= nf2) yy -= nf2;
+                const float2 *q = p + (int64_t)yy * pitch;
+                float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll
+                for (int t1 = 0; t1 < W; ++t1)
+                    tap(wT[r + e][t1 + 1], __ldg(reinterpret_cast<const float4 *>(q + t1 * line)), s0, s1);
+                const float u = wy[r + e][t2];
+                a0 = __ffma2_rn(make_float2(u, u), s0, a0);
+                a1 = __ffma2_rn(make_float2(u, u), s1, a1);
+            }
+            store(R.x, a0, a1);
+        }
     }
 }
 
