@@ -1432,7 +1432,7 @@ void NufftPlan::set_bins(int c1, int c2, int c3) {
     b1 = c1; b2 = c2; b3 = c3;
 }
 
-// exclusive scan of the bin counts (one CTA of 1024 threads, 4096 bins per pass)
+// exclusive scan of the cell counts (one CTA of 1024 threads, 4096 cells per pass)
 __global__ void __launch_bounds__(1024) k_scan_offsets(const uint32_t *__restrict__ cnt, int n,
                                                        uint32_t *__restrict__ start, uint32_t *__restrict__ cursor) {
     __shared__ uint32_t wsum[32];

@@ -203,63 +203,6 @@ __global__ void k_to_half(const float *__restrict__ K, int64_t n, int L1, const 
 // independent global loads kept in flight per thread in the load phases
 constexpr int LD_BATCH = 8;
 
-// Rows of M3 = 729 (schedule 9, 9, 9): the first radix-9 stage (one block, 81
-// offsets) runs in registers on the way in (k_r2c_rows) and its inverse on the
-// way out (k_c2r_rows).  Item (r, n) holds the packed values n + 81 j of row r.
-constexpr int R729_OFS = 81;
-
-__device__ __forceinline__ void rows729_load(const float *xb, int nr, int n3,
-                                             const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps,
-                                             int tid, int nth) {
-    for (int t = tid; t < nr * R729_OFS; t += nth) {
-        const int r = t / R729_OFS, n = t - r * R729_OFS;
-        const float *xr = xb + (int64_t)r * n3;
-        float2 x[9];
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const int i = 2 * (n + R729_OFS * j);
-            x[j].x = i < n3 ? xr[i] : 0.f;
-            x[j].y = i + 1 < n3 ? xr[i + 1] : 0.f;
-        }
-        dft_small<9, false>(x);
-        if (n != 0) {
-            float2 w[9];
-            twiddle_powers<9>(tw3, n, w);
-#pragma unroll
-            for (int k = 1; k < 9; ++k) x[k] = c_mul(x[k], w[k]);
-        }
-        float2 *sp = sm + r * ps + n;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) sp[R729_OFS * k] = x[k];
-    }
-}
-
-__device__ __forceinline__ void rows729_store(const float2 *__restrict__ sm, int nr, int ps, int n3,
-                                              const float2 *__restrict__ tw3, float *__restrict__ yb, int tid,
-                                              int nth) {
-    for (int t = tid; t < nr * R729_OFS; t += nth) {
-        const int r = t / R729_OFS, n = t - r * R729_OFS;
-        const float2 *sp = sm + r * ps + n;
-        float2 a[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) a[k] = sp[R729_OFS * k];
-        if (n != 0) {
-            float2 w[9];
-            twiddle_powers<9>(tw3, n, w);
-#pragma unroll
-            for (int k = 1; k < 9; ++k) a[k] = c_mulc(a[k], w[k]);
-        }
-        dft_small<9, true>(a);
-        float *yr = yb + (int64_t)r * n3;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const int i = 2 * (n + R729_OFS * j);
-            if (i < n3) yr[i] = a[j].x;
-            if (i + 1 < n3) yr[i + 1] = a[j].y;
-        }
-    }
-}
-
 // ---- register DFTs of composite lengths (two-stage row and pencil transforms) ----
 // cos / sin of 2 pi m / R for the composite register DFTs (R = 15, 18, 25)
 __host__ __device__ constexpr float wr_c(int R, int m) {
@@ -585,7 +528,7 @@ __host__ __device__ constexpr int rows_threads(int M3, int R) {
 
 // The first stage of a runtime-length row transform (radix R0 over the whole
 // packed row of M3, m0 = M3 / R0 offsets) in registers on the way in and its
-// inverse on the way out, as rows729_load / rows729_store for other lengths.
+// inverse on the way out.
 template <int R0>
 __device__ __forceinline__ void rowslead_load(const float *xb, int nr, int n3, int M3,
                                               const float2 *__restrict__ tw3, float2 *__restrict__ sm, int ps,
@@ -1499,8 +1442,8 @@ __device__ __forceinline__ void pencil_inverse(float2 *pv, int64_t cs, int n1, c
 
 // B: one (p2, k3) pencil of the 3 components along n1: DIF (zero-padded), 3x3
 // symmetric multiply with the spectra (same position order), undo, first n1 kept.
-// In place on xa.  N1: compile-time L1 or 0.  At L1 = 1458, five CTAs of 256
-// threads per SM (48 registers, 35 KB of shared memory each); four otherwise.
+// In place on xa.  N1: compile-time L1 or 0 (threads and CTAs per SM: pencil_threads,
+// pencil_ctas).
 template <bool HALF, int N1>
 __global__ void __launch_bounds__(pencil_threads(N1), pencil_ctas(N1)) k_pencil(float2 *__restrict__ xa, int n1, int n1p, int L2, int L3h, FftLen F1,
                                                 const float2 *__restrict__ tw1, const float *__restrict__ K,
