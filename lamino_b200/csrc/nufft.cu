@@ -394,9 +394,10 @@ __device__ __forceinline__ void node_pos(const LatView &L, const Fine &F, int t,
 // Fine grid -> nodes.  A CTA owns 128 nodes (16 columns x 8 T lines, or 8 x 16).
 // Per chunk of up to 16 y it stages the (z, x) box of cells that the nodes'
 // footprints cover in shared memory; a thread then takes two nodes, one T line
-// apart, and two y: the lattice keeps T lines at most one cell apart, so both
+// apart, and two y: the lattice keeps T lines at most one cell apart (see lattice()), so both
 // footprints lie in (W + 1)^2 cells, each read once (16 bytes) and weighted for
-// both nodes with the weights padded by zeros.  Results go through shared memory
+// both nodes with the weights padded by zeros.  A tile with a pair that starts
+// further apart, which rounding alone could bring about, goes tap by tap.  Results go through shared memory
 // to the node grid [T][y][X], X fastest.  Bound by shared-memory wavefronts:
 // 64 16-byte reads per four values where one node and one y at a time takes 196
 // of 8 bytes.  A box that does not fit (a detector far coarser than the fine
@@ -442,9 +443,14 @@ __global__ void __launch_bounds__(256, 2) k_nodes_gather(LatView L, Fine F, cons
         for (int r = 0; r < W; ++r) wt[r + 1][n] = es_weight<W>(z ? d1 : d3, r, F.beta);
     }
     __syncthreads();
+    bool far = false;
+    if (tid < kPairs) {
+        const int a = tid / kNodeK * 2 * kNodeK + tid % kNodeK, b = a + kNodeK;
+        far = abs(n1[a] - n1[b]) > 1 || abs(n3[a] - n3[b]) > 1;
+    }
     const int B1 = hi1 - lo1 + W + 1, B3 = hi3 - lo3 + W + 1;
     const int base1 = wrap(lo1, F.nf1), base3 = wrap(lo3, F.nf3);
-    const bool staged = (int64_t)B1 * B3 <= boxcap;
+    const bool staged = !__syncthreads_or(far) && (int64_t)B1 * B3 <= boxcap;
     const int half = ychunk / 2;
     for (int c = blockIdx.y; c < nchunk; c += gridDim.y) {
         const int y0 = c * ychunk, ny = min(ychunk, F.nf2 - y0);
@@ -1510,8 +1516,12 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     // twice the volume's extent along t, in cells over the period 2 pi
     const double band = vol.n3 * std::fabs(l->sg) + vol.n1 * std::fabs(l->cg);
     int nTf = band > w ? 2 * (int)std::ceil(band - 1e-9) : 2 * w;  // (also for a NaN tilt)
-    // and no T line more than one cell of the fine grid from the next (k_nodes_gather)
-    const double near = std::max(nf1 * std::fabs(l->cg), nf3 * std::fabs(l->sg));
+    // and no T line more than one cell of the fine grid from the next (k_nodes_gather).
+    // Lines exactly one cell apart (no tilt, or a quarter turn) lie at the cells: the
+    // footprints of odd widths then start half a cell from an integer, those of even widths
+    // at an integer up to rounding, which puts some lines' first taps two cells
+    // apart.  Even widths take their lines closer than one cell.
+    const double near = std::max(nf1 * std::fabs(l->cg), nf3 * std::fabs(l->sg)) + (w % 2 ? 0 : 1);
     if (near > nTf) nTf = 2 * (int)std::ceil(0.5 * near);
     l->h = 2 * M_PI / nTf;
     // |T| <= pi up to float rounding: footprints start in [-nTf/2 - w/2, nTf/2 - w/2 + 1)

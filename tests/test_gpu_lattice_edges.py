@@ -1,0 +1,41 @@
+"""The lattice transforms where their assumptions are tight: lines exactly one
+cell apart, fine grids that end in part of a tile, angles that are not numbers,
+memory that runs out between calls, more datasets than a plan's usual number."""
+import numpy as np
+import pytest
+
+from conftest import rel
+
+pytestmark = pytest.mark.gpu
+
+
+def _grids(L, O, rng, nproj, nrows, ncols, gamma):
+    th = rng.uniform(0, 2 * np.pi, nproj).astype(np.float32)
+    return L.PolarGrid(th, nrows, ncols, np.float32(gamma)), O.PolarGrid(th, nrows, ncols, np.float32(gamma))
+
+
+def _check_all(L, O, rng, dims, pg, opg, eps):
+    """Every lattice operator within 1e-5 (float positions and sums) plus 10 eps (the
+    kernel's error in the four interpolated axes) of the FP64 oracle."""
+    tol = 1e-5 + 10 * eps
+    plan, plan_o = L.NufftPlan(dims, eps), O.NufftPlan(dims, eps=1e-12)
+    f = (rng.standard_normal(dims) + 1j * rng.standard_normal(dims)).astype(np.complex64)
+    c = (rng.standard_normal(pg.dims()) + 1j * rng.standard_normal(pg.dims())).astype(np.complex64)
+    assert rel(L.nufft3d2(f, pg, plan=plan), O.nufft3d2(f.astype(np.complex128), opg, plan_o)) < tol
+    assert rel(L.nufft3d1(c, pg, dims, plan=plan), O.nufft3d1(c.astype(np.complex128), opg, plan_o)) < tol
+    m = rng.standard_normal((3,) + dims).astype(np.float32)
+    p = rng.standard_normal(pg.dims()).astype(np.float32)
+    assert rel(L.forward(m, pg, plan=plan), O.forward(m, opg, opg.gamma, plan_o)) < tol
+    assert rel(L.adjoint(p, pg, dims, plan=plan), O.adjoint(p, opg, dims, opg.gamma, plan_o)) < tol
+    assert rel(L.sysmat(m, pg, plan=plan), O.sysmat(m, opg, opg.gamma, plan_o)) < tol
+
+
+@pytest.mark.parametrize("eps", [1e-3, 1e-5, 1e-7])
+@pytest.mark.parametrize("gamma", [0.0, np.pi / 2, np.pi])
+@pytest.mark.parametrize("dims", [(90, 6, 64), (64, 5, 90)])
+def test_lines_one_cell_apart_even_widths(L, O, dims, gamma, eps):
+    """No tilt, a quarter and half a turn: the T lines would lie on the cells of the
+    fine grid, where the even kernel widths' footprints start at integers."""
+    rng = np.random.default_rng(3)
+    pg, opg = _grids(L, O, rng, 6, 24, 33, gamma)
+    _check_all(L, O, rng, dims, pg, opg, eps)
