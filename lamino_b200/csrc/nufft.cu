@@ -793,10 +793,12 @@ __global__ void __launch_bounds__(256, 3) k_rows_gather(const int4 *__restrict__
     }
 }
 
-// the run of rows (first, count) that start in y cell c2 - (W - 1) + r and whose
-// footprint meets T cells [c1, c1 + kCell)
+// the run of rows (first, count) that start in y cell c2 - (W - 1) + r, if the
+// tile's y cells (the last tile has fewer than kCell where nf2 is no multiple of it) lie
+// in the footprint, and whose footprint meets T cells [c1, c1 + kCell)
 template <int W>
 __device__ __forceinline__ int2 tile_run(const uint32_t *__restrict__ start, int nstart, int nf2, int c1, int c2, int r) {
+    if (r - (W - 1) >= nf2 - c2) return make_int2(0, 0);
     const int lo = max(0, c1 - (W - 1)), hi = min(nstart - 1, c1 + kCell - 1);
     const uint32_t *o = start + (int64_t)wrap(c2 - (W - 1) + r, nf2) * nstart;
     return make_int2((int)o[lo], (int)(o[hi + 1] - o[lo]));
@@ -1271,6 +1273,15 @@ __global__ void __launch_bounds__(256) k_sysmat_points(GeomView g, const float2 
 
 constexpr int64_t kHalfPrime = 13;  // see halved()
 
+// tiles of kCell cells along y that a footprint of w cells meets, at most: one
+// that wraps past the end of the fine grid may meet the short last tile besides
+static int64_t y_tiles_met(int w, int nf2) {
+    int most = (w + kCell - 2) / kCell + 1;
+    for (int s = nf2 - w + 1; s < nf2; ++s)  // first cell; last cell s + w - 1 - nf2 (nf2 >= 2 w)
+        most = std::max(most, (nf2 - 1) / kCell - s / kCell + 1 + (s + w - 1 - nf2) / kCell + 1);
+    return most;
+}
+
 static Fine fine_of(const NufftPlan &pl) {
     Fine F;
     F.nf1 = (int)pl.nf1; F.nf2 = (int)pl.nf2; F.nf3 = (int)pl.nf3;
@@ -1536,8 +1547,8 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->ntile = (l->nT + kCell - 1) / kCell;
     const int64_t ntiles = (int64_t)l->ntile * ((nf2 + kCell - 1) / kCell);
     l->seg = (int)std::min<int64_t>(256, std::max<int64_t>(32, nrow * 6 * ((g.ncols + 255) / 256) / (148 * 16) / 32 * 32));
-    const int64_t meet = (w + kCell - 2) / kCell + 1;  // tiles a footprint meets along one axis, at most
-    const int64_t max_items = ntiles + nrow * meet * meet / l->seg + 1;
+    const int64_t meet = (w + kCell - 2) / kCell + 1;  // tiles a footprint meets along T, at most
+    const int64_t max_items = ntiles + nrow * meet * y_tiles_met(w, (int)nf2) / l->seg + 1;
     l->max_items = (int)max_items;
     // one allocation for all tables
     size_t bytes = 0;

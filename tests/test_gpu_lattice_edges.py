@@ -39,3 +39,15 @@ def test_lines_one_cell_apart_even_widths(L, O, dims, gamma, eps):
     rng = np.random.default_rng(3)
     pg, opg = _grids(L, O, rng, 6, 24, 33, gamma)
     _check_all(L, O, rng, dims, pg, opg, eps)
+
+
+@pytest.mark.parametrize("eps", [1e-3, 1e-4, 1e-7])
+@pytest.mark.parametrize("dims,nproj,nrows,spread", [((9, 9, 9), 100, 120, 2 * np.pi), ((32, 9, 32), 200, 154, 2 * np.pi),
+                                                     ((30, 15, 30), 240, 154, 0.2), ((9, 25, 9), 300, 120, 0.02)])
+def test_short_last_tile(L, O, dims, nproj, nrows, spread, eps):
+    """Fine grids along y of 18, 30 and 50 cells end in half a tile; many rows, all of
+    them near y = 0 with a small spread of angles, meet it and both its neighbours."""
+    rng = np.random.default_rng(8)
+    th = rng.uniform(0, spread, nproj).astype(np.float32)
+    g = np.float32(0.5)
+    _check_all(L, O, rng, dims, L.PolarGrid(th, nrows, 7, g), O.PolarGrid(th, nrows, 7, g), eps)
