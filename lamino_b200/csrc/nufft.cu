@@ -322,13 +322,15 @@ __device__ __forceinline__ int64_t half_row(int p, int j, int np, int nr) {
     const int jh = (nr + 1) / 2;
     return j < jh ? (int64_t)p * jh + j : (int64_t)np * jh + (int64_t)p * (nr - jh) + (j - jh);
 }
-// the (T, y) position of detector row `id` = p nrows + j and its footprint
+// the (T, y) position of detector row `id` = p nrows + j and its footprint; a row
+// of an angle that is not a number gets some cell of the lattice and a footprint
+// whose weights are all zero
 struct RowPos {
     int p, j, lT, ly;
     float dT, dy;
 };
 template <int W>
-__device__ __forceinline__ RowPos row_pos(const GeomView &g, bool raw, double invh, int T0,
+__device__ __forceinline__ RowPos row_pos(const GeomView &g, bool raw, double invh, int T0, int nstart,
                                           const Fine &F, int id) {
     RowPos r;
     r.p = id / g.nrows;
@@ -343,7 +345,7 @@ __device__ __forceinline__ RowPos row_pos(const GeomView &g, bool raw, double in
         T = qy * (double)__ldg(g.ct + r.p);
         y = -qy * (double)__ldg(g.st + r.p);
     }
-    r.lT = es_first<W>(T, invh, r.dT) - T0;
+    r.lT = max(0, min(es_first<W>(T, invh, r.dT) - T0, nstart - 1));
     r.ly = wrap(es_first<W>(y, F.s2, r.dy), F.nf2);
     return r;
 }
@@ -352,7 +354,7 @@ __global__ void __launch_bounds__(256) k_rows_count(GeomView g, bool raw, double
                                                     int T0, int nstart, Fine F, uint32_t *__restrict__ cnt) {
     const int n = g.nproj * g.nrows;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
-        const RowPos r = row_pos<W>(g, raw, invh, T0, F, id);
+        const RowPos r = row_pos<W>(g, raw, invh, T0, nstart, F, id);
         atomicAdd(cnt + (int64_t)r.ly * nstart + r.lT, 1u);
     }
 }
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(256) k_rows_place(GeomView g, bool raw, double
                                                     int4 *__restrict__ pt, float2 *__restrict__ pd) {
     const int n = g.nproj * g.nrows;
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
-        const RowPos r = row_pos<W>(g, raw, invh, T0, F, id);
+        const RowPos r = row_pos<W>(g, raw, invh, T0, nstart, F, id);
         const uint32_t at = atomicAdd(cursor + (int64_t)r.ly * nstart + r.lT, 1u);
         pt[at] = make_int4(half ? (int)half_row(r.p, r.j, g.nproj, g.nrows) : id, r.lT, r.ly, id);
         pd[at] = make_float2(r.dT, r.dy);

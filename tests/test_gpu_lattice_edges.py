@@ -51,3 +51,25 @@ def test_short_last_tile(L, O, dims, nproj, nrows, spread, eps):
     th = rng.uniform(0, spread, nproj).astype(np.float32)
     g = np.float32(0.5)
     _check_all(L, O, rng, dims, L.PolarGrid(th, nrows, 7, g), O.PolarGrid(th, nrows, 7, g), eps)
+
+
+@pytest.mark.parametrize("nrows,ncols", [(16, 20), (17, 19)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_angles_that_are_not_numbers(L, bad, nrows, ncols):
+    """Such an angle has no positions: its rows are not numbers, the others are those
+    of the geometry without it, and sums over all rows are not numbers."""
+    rng = np.random.default_rng(6)
+    dims, g = (10, 6, 12), np.float32(0.5)
+    th = rng.uniform(0, 2 * np.pi, 4).astype(np.float32)
+    pg = L.PolarGrid(np.concatenate([th[:1], [np.float32(bad)], th[1:]]), nrows, ncols, g)
+    clean = L.PolarGrid(th, nrows, ncols, g)
+    others = [0, 2, 3, 4]
+    plan = L.NufftPlan(dims)
+    m = rng.standard_normal((3,) + dims).astype(np.float32)
+    got = L.forward(m, pg, plan=plan)
+    assert np.isnan(got[1]).all()
+    assert rel(got[others], L.forward(m, clean, plan=plan)) < 1e-6
+    f = (rng.standard_normal(dims) + 1j * rng.standard_normal(dims)).astype(np.complex64)
+    assert rel(L.nufft3d2(f, pg, plan=plan)[others], L.nufft3d2(f, clean, plan=plan)) < 1e-6
+    assert np.isnan(L.adjoint(rng.standard_normal(pg.dims()).astype(np.float32), pg, dims, plan=plan)).all()
+    assert np.isnan(L.sysmat(m, pg, plan=plan)).all()
