@@ -1507,9 +1507,24 @@ const Lattice *NufftPlan::find_lattice(const Geom &g, bool raw) const {
     return nullptr;
 }
 
+void NufftPlan::need_work(int64_t n) {
+    if ((int64_t)work.n >= n) return;
+    const size_t had = std::max<size_t>(work.n, (size_t)(nf() + nf() / 4));
+    try {
+        work.alloc((size_t)n);
+    } catch (...) {  // the other geometries still work with what there was
+        try {
+            work.alloc(had);
+        } catch (const Error &) {
+        }
+        throw;
+    }
+}
+
 const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     for (auto &l : lats)
         if (l->uid == g.uid && l->raw == raw) {
+            need_work(node_values(*l));
             l->last_use = ++use_clock;
             return *l;
         }
@@ -1577,8 +1592,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
     l->nitem = reinterpret_cast<int *>(m0 + oni);
     l->items = reinterpret_cast<int2 *>(m0 + oit);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(m0 + ocnt);  // counts, then placement cursors
-    const int64_t need = (int64_t)l->nT * nf2 * node_pitch(l->ncc);
-    if ((int64_t)work.n < need) work.alloc(need);
+    need_work(node_values(*l));
     LAMINO_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(reinterpret_cast<char *>(l->items) - reinterpret_cast<char *>(cnt)), s));
     const Fine F = fine_of(*this);
     const GeomView gv = g.view();
@@ -1803,7 +1817,9 @@ void NufftPlan::normal_ptrs(const Geom *const *gs, int ng, const float *x3, floa
         if (!gs[i] || gs[i]->npts() > (int64_t)UINT32_MAX / 2) throw Error(ERR_ARG, "bad geometry");
     for (int i = 0; i < ng; ++i) {
         const Lattice *l = find_lattice(*gs[i], false);
-        if (l && (int64_t)pbuf.n < gs[i]->npts()) l = nullptr;  // no row buffer from an earlier call
+        if (l && ((int64_t)pbuf.n < gs[i]->npts() || (int64_t)work.n < node_values(*l)))
+            l = nullptr;  // no row buffer or node grid from an earlier call
+        if ((int64_t)work.n < nf()) throw Error(ERR_OOM, "the plan lost its scratch to a failed allocation");
         normal_one(*gs[i], l, x3, y3, i > 0, s);
     }
 }

@@ -77,6 +77,10 @@ struct NufftPlan {
 
     NufftPlan(Dims3 d, double eps);
     int64_t nf() const { return nf1 * nf2 * nf3; }
+    // values of a lattice's node grid, and at least n values in `work`: if there is no
+    // memory for them, `work` keeps its size and the error goes on to the caller
+    int64_t node_values(const Lattice &l) const { return (int64_t)l.nT * nf2 * node_pitch(l.ncc); }
+    void need_work(int64_t n);
     void ensure_proj(const Geom &g);
     // projection space <-> rows (see Lattice::half): proj is read / written
     void rows_to_proj(const Lattice &lat, const Geom &g, float *proj, cudaStream_t s);

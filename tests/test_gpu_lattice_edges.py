@@ -73,3 +73,40 @@ def test_angles_that_are_not_numbers(L, bad, nrows, ncols):
     assert rel(L.nufft3d2(f, pg, plan=plan)[others], L.nufft3d2(f, clean, plan=plan)) < 1e-6
     assert np.isnan(L.adjoint(rng.standard_normal(pg.dims()).astype(np.float32), pg, dims, plan=plan)).all()
     assert np.isnan(L.sysmat(m, pg, plan=plan)).all()
+
+
+SCRATCH = """
+import numpy as np, torch
+import lamino_b200 as L
+rng = np.random.default_rng(2)
+dims = (16, 64, 16)
+grid = lambda n: L.PolarGrid(np.array([0.3], np.float32), 4, n, np.float32(0.6))
+small, wide = grid(24), grid(50_000)   # node grids of 2 MB and 3 GB
+m = torch.from_numpy(rng.standard_normal((3,) + dims).astype(np.float32)).cuda()
+plan = L.NufftPlan(dims)
+want = L.forward(m, small, plan=plan).clone()
+free, _ = torch.cuda.mem_get_info()
+filler = torch.empty(free - (1 << 30), dtype=torch.uint8, device="cuda")
+try:
+    L.forward(m, wide, plan=plan)
+    raise SystemExit("the wide detector fitted")
+except L.LaminoError as e:
+    assert e.code == 2, e
+assert torch.equal(L.forward(m, small, plan=plan), want)
+del filler
+torch.cuda.empty_cache()
+assert torch.isfinite(L.forward(m, wide, plan=plan)).all()
+assert torch.equal(L.forward(m, small, plan=plan), want)
+print("kept")
+"""
+
+
+def test_scratch_survives_a_failed_allocation():
+    """A node grid that finds no memory is an error of that call alone: the geometries
+    the plan already knows go on with the scratch that it had.  In a process of its
+    own, whose memory nothing else holds."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    r = subprocess.run([sys.executable, "-c", SCRATCH], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "kept", r.stdout + r.stderr
