@@ -1208,14 +1208,16 @@ __global__ void __launch_bounds__(256) k_half_post(const float2 *__restrict__ z,
 // ---------------------------------------------------------------------------
 // direct sysmat per point, for calls that may not allocate a lattice: w^3 taps
 // per point from the fine grid of W and atomics into the fine grid of U, at q
-// and at -q (float positions, so -q is not a lattice point)
+// and at -q.  The points are the lattice's (the antisymmetric part of the float
+// frequencies, products and sums in double), so that the result does not depend on
+// whether an earlier call has built one.
 // ---------------------------------------------------------------------------
 
 template <int W>
 struct Taps {
     float w1[W], w2[W], w3[W];
     int l1, l2, l3;
-    __device__ __forceinline__ Taps(const Fine &F, float x, float y, float z) {
+    __device__ __forceinline__ Taps(const Fine &F, double x, double y, double z) {
         float d1, d2, d3;
         l3 = wrap(es_first<W>(x, F.s3, d3), F.nf3);
         l2 = wrap(es_first<W>(y, F.s2, d2), F.nf2);
@@ -1252,8 +1254,8 @@ __global__ void __launch_bounds__(256) k_sysmat_points(GeomView g, const float2 
         const int p = (int)(pid / plane);
         const uint32_t r = pid - (uint32_t)p * plane;
         const int j = (int)(r / (uint32_t)g.ncols), k = (int)(r - (uint32_t)j * g.ncols);
-        float x, y, z;
-        point_xyz(g, p, j, k, x, y, z);
+        const double X = odd_part(g.qX, k, g.ncols), Y = odd_part(g.qY, j, g.nrows), T = Y * (double)__ldg(g.ct + p);
+        const double x = X * g.cg + T * g.sg, y = -Y * (double)__ldg(g.st + p), z = T * g.cg - X * g.sg;
         const float ax = 0.5f * __ldg(g.st + p), ay = -0.5f * __ldg(g.ct + p);
         const Taps<W> tq(F, x, y, z), tm(F, -x, -y, -z);
         float2 f = make_float2(0.f, 0.f), h = f;
