@@ -1531,7 +1531,7 @@ const Lattice &NufftPlan::lattice(const Geom &g, bool raw, cudaStream_t s) {
             return *l;
         }
     check_points(g);
-    if ((int)lats.size() >= kMaxLattices) {
+    if (lats.size() >= keep_lattices) {
         size_t lru = 0;
         for (size_t i = 1; i < lats.size(); ++i)
             if (lats[i]->last_use < lats[lru]->last_use) lru = i;
@@ -1809,6 +1809,7 @@ void NufftPlan::normal(const std::vector<const Geom *> &gs, const float *x3, flo
         check_points(*g);
         if ((int64_t)pbuf.n < g->npts()) pbuf.alloc(g->npts());
     }
+    keep_lattices = std::max(keep_lattices, gs.size());
     for (const Geom *g : gs) lattice(*g, false, s);
     for (size_t i = 0; i < gs.size(); ++i) normal_one(*gs[i], &lattice(*gs[i], false, s), x3, y3, i > 0, s);
 }

@@ -72,7 +72,10 @@ struct NufftPlan {
     // lattices of the geometries used with this plan (bounded LRU)
     std::vector<std::unique_ptr<Lattice>> lats;
     uint64_t use_clock = 0;
-    static constexpr int kMaxLattices = 16;
+    // how many: 16, or the geometries of the largest sum so far.  A sum with more than are
+    // kept would build them anew in every call, also in one that is being captured,
+    // where their memory would become the graph's.
+    size_t keep_lattices = 16;
     int b1 = 4, b2 = 8, b3 = 16;   // bin layout of lamino_plan_set_bins (a hint, see set_bins)
 
     NufftPlan(Dims3 d, double eps);

@@ -110,3 +110,26 @@ def test_scratch_survives_a_failed_allocation():
     from conftest import ROOT
     r = subprocess.run([sys.executable, "-c", SCRATCH], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "kept", r.stdout + r.stderr
+
+
+def test_more_datasets_than_a_plan_usually_keeps(L, O):
+    """A solver over 18 tilts in the NUFFT form captures its operator after one call;
+    by then every lattice is there.  Same result as without graphs, in float sums
+    of another order at most."""
+    rng = np.random.default_rng(12)
+    recon = (8, 4, 8)
+    data = [(rng.random((3, 8, 9), dtype=np.float32), rng.uniform(0, 2 * np.pi, 3).astype(np.float32), np.float32(0.15 * i))
+            for i in range(18)]
+    par = dict(maxIters=4, op_kind="nufft", tol=0.0, xtol=0.0)
+    got = L.MBIR1(data, recon, L.ReconParams(**par))
+    assert rel(got, L.MBIR1(data, recon, L.ReconParams(use_graphs=0, **par))) < 1e-5
+    got = L.MBIR3(data, recon, L.ReconParams(**par))
+    assert rel(got, L.MBIR3(data, recon, L.ReconParams(use_graphs=0, **par))) < 1e-5
+    # and the operator over them, twice in a row
+    pgs = [L.PolarGrid(th, 20, 21, g) for _, th, g in data]
+    opgs = [O.PolarGrid(th, 20, 21, g) for _, th, g in data]
+    x = rng.standard_normal((3, 11, 6, 11)).astype(np.float32)
+    plan, plan_o = L.NufftPlan(x.shape[1:]), O.NufftPlan(x.shape[1:], eps=1e-12)
+    want = O.normal(x, opgs, [p.gamma for p in opgs], plan_o)
+    for _ in range(2):
+        assert rel(L.sysmat(x, pgs, plan=plan), want) < 2.2e-5
