@@ -186,11 +186,6 @@ void MbirJob::prepare() {
     const bool mixed = prm.op_kind == OP_TOEPLITZ_MIXED;
     if (prm.op_kind == OP_NUFFT) {
         NufftPlan *pl = plan_.get();
-        if (prm.autotune) {
-            const double tt = now_s();
-            pl->autotune_bins(gptr_, 1, s);
-            t_tune_ += now_s() - tt;
-        }
         A_raw_ = [pl, this](const float *x, float *y, cudaStream_t st) { pl->normal(gptr_, x, y, st); };
         if (method == 3)
             for (const Geom *g : gptr_)
