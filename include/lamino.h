@@ -70,7 +70,8 @@ int lamino_plan_destroy(lamino_plan_t p);
  * cuFINUFFT). */
 int lamino_plan_set_bins(lamino_plan_t p, int b1, int b2, int b3);
 /* Times the plan's operator on the given geometries for objective 0 (adjoint of
- * geoms[0], a setup pass) or 1 (sum over geoms of sysmat, a solver's operator).
+ * geoms[0], a setup pass with its tables) or 1 (sum over geoms of sysmat, a solver's
+ * operator, its tables built before).
  * Cached per fine grid, kernel width, objective and point count for the process.
  * bins[3] (may be NULL) receives the plan's bin layout, *best_ms (may be
  * NULL) the time (0 when taken from the cache). */

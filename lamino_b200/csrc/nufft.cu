@@ -1740,6 +1740,7 @@ double NufftPlan::autotune_bins(const std::vector<const Geom *> &gs, int objecti
         k_fill<<<grid_for(gs[0]->npts(), 256), 256, 0, s>>>(proj.p, gs[0]->npts(), 1.0f);
         LAMINO_LAUNCH("k_fill");
     }
+    if (objective == 1) normal(gs, x.p, y.p, s);  // builds the lattices
     cudaEvent_t e0, e1;
     LAMINO_CUDA(cudaEventCreate(&e0));
     LAMINO_CUDA(cudaEventCreate(&e1));

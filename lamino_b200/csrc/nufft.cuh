@@ -94,9 +94,10 @@ struct NufftPlan {
     // the geometry's lattice (built on first use, then cached) with the node grid allocated
     const Lattice &lattice(const Geom &g, bool raw, cudaStream_t s);
     const Lattice *find_lattice(const Geom &g, bool raw) const;
-    // one pass of the adjoint (objective 0) or of the sum over the geometries of
-    // sysmat (objective 1) timed; cached per (fine grid, width, objective, points)
-    // for the process.  Returns its time in ms (0 when taken from the cache).
+    // one pass of the adjoint (objective 0, with the building of its lattice: a setup
+    // pass) or of the sum over the geometries of sysmat (objective 1, without) timed;
+    // cached per (fine grid, width, objective, points) for the process.  Returns its
+    // time in ms (0 when taken from the cache).
     double autotune_bins(const std::vector<const Geom *> &gs, int objective, cudaStream_t s);
 
     // --- operators (device pointers; volumes are 3 contiguous components) ---
