@@ -96,22 +96,25 @@ int64_t mbir_footprint(int method, const std::vector<std::array<int64_t, 3>> &pr
     const Dims3 od = padded_dims(method, recon, prm);
     const float pf = proj_pad_factor(method, prm);
     const int64_t V = od.size();
-    int64_t raw = 0, maxpts = 0, maxcols = 0;
+    int64_t raw = 0, maxpts = 0, maxcols = 0, rows = 0;
     for (auto &d : proj_dims) {
         raw += d[0] * d[1] * d[2] * 4;
         maxpts = std::max<int64_t>(maxpts, d[0] * pad2d_len(d[1], pf) * pad2d_len(d[2], pf));
         maxcols = std::max<int64_t>(maxcols, pad2d_len(d[2], pf));
+        rows += d[0] * pad2d_len(d[1], pf);
     }
     const int w = es_width(prm.eps);
     const int64_t nf2 = next_smooth_even(std::max<int64_t>(2 * od.n2, 2 * w));
     const int64_t nf = next_smooth_even(std::max<int64_t>(2 * od.n1, 2 * w)) * nf2 *
                        next_smooth_even(std::max<int64_t>(2 * od.n3, 2 * w));
-    // the NUFFT's grids: seven fine grids cover one, its FFT work and the node grid,
-    // but for detectors far wider than the volume (T lines of the steepest tilt)
+    // the NUFFT: its fine grid, cuFFT's work (measured: up to 1.25 fine grids; counted as
+    // two) and the node grid (T lines of the steepest tilt); tables of every dataset's
+    // lattice (24 bytes and some work items a row, two counts a cell, a factor a mode)
     const int64_t lines = 2 * (int64_t)std::ceil(std::hypot((double)od.n1, (double)od.n3)) + 3 * w + 6;
-    const int64_t nodes = NufftPlan::node_bytes(lines, nf2, maxcols);
-    const int64_t grids = std::max<int64_t>((6 + 1) * nf * 8, 3 * nf * 8 + nodes);
-    // setup: raw + padded projections, projection spectra + 2-D FFT work, fine grids + 3-D FFT work
+    const int64_t nodes = NufftPlan::node_bytes(lines, nf2, maxcols), nds = (int64_t)proj_dims.size();
+    const int64_t tables = 40 * rows + nds * (lines * nf2 * 10 + od.n1 * od.n3 * 4);
+    const int64_t grids = 3 * nf * 8 + std::max<int64_t>(nf * 10, nodes) + tables;
+    // setup: raw + padded projections, projection spectra + 2-D FFT work, the NUFFT
     const int64_t setup = raw + maxpts * 4 + 2 * maxpts * 8 + grids + 3 * V * 4;
     const int64_t L1 = next_smooth_even(2 * od.n1), L2 = next_smooth_even(2 * od.n2), L3 = next_smooth_even(2 * od.n3);
     const int64_t S = L1 * L2 * (L3 / 2 + 1), L = L1 * L2 * L3;
@@ -119,8 +122,15 @@ int64_t mbir_footprint(int method, const std::vector<std::array<int64_t, 3>> &pr
     const int64_t kb = prm.op_kind == OP_TOEPLITZ_FP32 ? 4 : (prm.op_kind == OP_TOEPLITZ_FP16 ? 2 : 6);
     const int64_t inter = 3 * od.n1 * od.n2 * (L3 / 2 + 1) * 8 + 3 * L2 * (L3 / 2 + 1) * n1p * 8;
     int64_t op = 6 * S * kb + inter;
-    const int64_t build = 6 * L * 4 + 2 * S * 8;  // transient kernel grids + R2C output and work
-    if (method == 3) op += (int64_t)proj_dims.size() * (6 * S * 4 + inter);  // per-gamma operators for the loss
+    int64_t build = 6 * L * 4 + 2 * S * 8;  // transient kernel grids + R2C output and work
+    if (method == 3) {
+        // three spectra and the forms' partial sums per dataset, the sum's six only for
+        // more than two datasets or other precisions; one dataset's kernels at a time; the
+        // last padded projections stay until the solver's state stands
+        const int64_t sum = nds > 2 || prm.op_kind != OP_TOEPLITZ_FP32 ? 6 * S * kb : 0;
+        op = nds * 3 * S * 4 + L2 * (L3 / 2 + 1) * 3 * 8 * std::min<int64_t>(nds, 4) + sum + inter + maxpts * 4;
+        build = 3 * L * 4 + 2 * S * 8;
+    }
     if (prm.op_kind == OP_NUFFT) op = grids + 2 * maxpts * 8;
     const int64_t state = (method == 2 ? 40 : 12) * V * 4 + 3 * V * 4;
     const int64_t solve = op + state + (prm.op_kind == OP_NUFFT ? 0 : build);
