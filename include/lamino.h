@@ -230,6 +230,11 @@ typedef struct {
     int autotune;   /* pick launch shapes by timing (cached per size) */
 } lamino_recon_params;
 void lamino_recon_params_default(lamino_recon_params *p);
+/* lamino_mbir and lamino_ramp_precond take their buffers from a memory pool of
+ * this library's own and leave up to 4 GiB of it on the current device for the
+ * next call; an allocation of this library that fails takes it back.  lamino_trim
+ * gives what no call is using back to the device, for other allocators. */
+int lamino_trim(void);
 /* method 1, 2 or 3.  projs[i]: [proj_dims[3i]][proj_dims[3i+1]][proj_dims[3i+2]];
  * angles[i]: proj_dims[3i] radians (host); out3: [3][r1][r2][r3]. */
 int lamino_mbir(int method, int ndatasets, const float *const *projs, const int64_t *proj_dims,

@@ -20,7 +20,7 @@ __all__ = [
     "LaminoError", "lib", "PolarGrid", "NufftPlan", "ToeplitzNormal", "beam_dir_vector",
     "forward", "adjoint", "sysmat", "gradient", "residual", "nufft3d1", "nufft3d2",
     "MBIR1", "MBIR2", "MBIR3", "ReconParams", "opt", "padded_volume_dims", "mbir_footprint",
-    "mbir_phases", "mbir3_batch",
+    "mbir_phases", "mbir3_batch", "trim",
     "ReconServer",
 ]
 
@@ -94,6 +94,7 @@ def lib():
         "lamino_server_create": ([i64, i32, i32, f64, P(vp)], i32),
         "lamino_server_submit": ([vp, i32, i32, P(vp), P(i64), P(vp), P(f32), i64, i64, i64, vp, P(i64)], i32),
         "lamino_server_wait": ([vp, i64, f64, vp, P(f64), P(f64), P(f64), P(f64)], i32),
+        "lamino_trim": ([], i32),
         "lamino_mbir_phases": ([P(f64), P(f64), P(f64), P(i64), P(f64)], i32),
         "lamino_server_stats": ([vp, P(i64)], i32),
         "lamino_server_destroy": ([vp], i32),
@@ -589,6 +590,12 @@ def _mbir(method, datasets, recon_dims, params):
     _check(lib().lamino_mbir(method, n, projs, dims, angs, gam, *[int(d) for d in recon_dims],
                              ctypes.byref(pc), _ptr(out), _stream(ref)))
     return out
+
+
+def trim() -> None:
+    """Give the device memory that MBIR1 / 2 / 3 and opt.ramp_precond keep for their
+    next call (up to 4 GiB) back to the device, for other allocators."""
+    _check(lib().lamino_trim())
 
 
 def mbir_phases() -> dict:

@@ -721,6 +721,12 @@ int lamino_mbir(int method, int nds, const float *const *projs, const int64_t *p
     API_END
 }
 
+int lamino_trim(void) {
+    API_BEGIN
+    trim_call_pool();
+    API_END
+}
+
 int lamino_mbir_phases(double *setup_s, double *build_s, double *solve_s, int64_t *applies, double *parts) {
     API_BEGIN
     const MbirPhases &p = last_mbir_phases();
