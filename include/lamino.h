@@ -227,7 +227,7 @@ typedef struct {
     double eps;
     int refinements;
     int use_graphs; /* replay each solver iteration's operator work as a CUDA graph (non-default streams) */
-    int autotune;   /* pick launch shapes by timing (cached per size) */
+    int autotune;   /* pick the Toeplitz form's launch shapes by timing (cached per size) */
 } lamino_recon_params;
 void lamino_recon_params_default(lamino_recon_params *p);
 /* lamino_mbir and lamino_ramp_precond take their buffers from a memory pool of

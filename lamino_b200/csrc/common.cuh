@@ -55,7 +55,9 @@ inline unsigned grid_for(int64_t n, int block, int64_t cap = 148LL * 64) {
 // every CTA of the one before has called allow_next(); the kernel reads and writes
 // nothing of earlier kernels before wait_previous(), which returns when they have
 // completed and their writes are visible.  A kernel of either kind may come before
-// or after.  Data of the kernel before is read by plain loads (no __restrict__ const,
+// or after.  wait_previous() waits for the one kernel before; that it stands for all earlier
+// ones as well takes a wait in at least one CTA of every kernel launched this way (others
+// may return without one, as the empty work items of k_rows_spread do).  Data of the kernel before is read by plain loads (no __restrict__ const,
 // no __ldg): the read-only path assumes that nothing writes it while the kernel
 // runs, and here the kernel runs before the writes are done.  What is gained is the launch latency between short kernels.
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

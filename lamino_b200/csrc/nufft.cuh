@@ -69,7 +69,7 @@ struct NufftPlan {
     FftPlan fft2;                  // 2-D; or, halved (Lattice::half), along the detector rows ...
     FftPlan fft2n;                 // ... and along the columns, two real ones at a time
     int64_t f2_np = -1, f2_nr = -1, f2_nc = -1;
-    // lattices of the geometries used with this plan (bounded LRU)
+    // lattices of the geometries used with this plan (least recently used goes first)
     std::vector<std::unique_ptr<Lattice>> lats;
     uint64_t use_clock = 0;
     // how many: 16, or the geometries of the largest sum so far.  A sum with more than are

@@ -1263,7 +1263,7 @@ __device__ __forceinline__ void p1458_inverse(const PencilRows &rows, const floa
 // Its threads take the items of a stage in a row (unit (h, c) major: 6 B in the
 // stage over A values, 6 A in the other), so that all lanes but the last few work;
 // a warp per (c, h) left 14 to 17 of 32 idle at 540.  Pencil at the padded sizes of
-// the batched mix, before -> after: 540 186 -> 129 us (270 x 32 x 270), 750 433 ->
+// the batched mix, before -> after: 540 186 -> 131 us (270 x 32 x 270), 750 433 ->
 // 338 us (362 x 44 x 362); 360 and 180, then shared-memory schedules, 68 -> 47 us
 // (180 x 22 x 180) and 14 -> 12 us (90 x 10 x 90).
 template <int A, int B>
@@ -1593,10 +1593,10 @@ __global__ void __launch_bounds__(pencil_threads(N1)) k_pencil_quad(const float2
 // as k_pencil_quad) to part[pencil][g][i]; the reconstruction step with two
 // datasets gets the product and the loss of one volume from one pass that reads
 // as many spectra as the product alone did.
-// Measured at 270 x 32 x 270 (embedding 540 x 64 x 540) with two datasets: 193 us
-// on average over products, forms and both at once, where k_pencil takes 183 us
-// and k_pencil_quad, which reads 12 spectra and adds every pencil's sums to the
-// same six doubles by atomics, 296 us.
+// Measured at 270 x 32 x 270 (embedding 540 x 64 x 540) with two datasets: both at
+// once 168 us, the forms alone 113, where k_pencil takes 131 us and k_pencil_quad,
+// which reads 12 spectra and adds every pencil's sums to the same six doubles by
+// atomics, 162.
 constexpr int kMaxTilts = 4;
 struct Tilts {
     const float *K[kMaxTilts];
